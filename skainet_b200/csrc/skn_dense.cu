@@ -885,7 +885,8 @@ skn_dense_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
     __shared__ uint64_t full_bar[DTC_MAX_STAGES], empty_bar[DTC_MAX_STAGES], acc_full[2], acc_empty[2];
     __shared__ uint32_t tmem_slot, last_flag;
     __shared__ int start[GROUPS ? SKN_MAX_EXPERTS + 1 : 1], off[GROUPS ? SKN_MAX_EXPERTS + 1 : 1];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    // (through a shuffle: the compiler then knows that a warp's threads take one role together)
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
     const int stage_bytes = DTC_A_BYTES + NT * DTC_BK * 2;
     const int acc_cols = NT < 32 ? 32 : NT;
     uint32_t tmem_cols = 32;
@@ -979,37 +980,39 @@ skn_dense_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
                 }
         }
     } else if (warp == DTC_MMA) {
-        if (lane == 0) {
-            uint32_t idesc = tc_idesc(DTC_BM, NT);
-            bool ok = true;
-            int it = 0, tile = 0;
-            for (int u = blockIdx.x; u < units && ok; u += gridDim.x, ++tile) {
-                const int sp = GROUPS ? 0 : (u / mt) % splits;
-                const int kb = (int)((int64_t)ksteps * sp / splits), ke = (int)((int64_t)ksteps * (sp + 1) / splits);
-                const int b = tile & 1;
-                if (GROUPS) idesc = tc_idesc(DTC_BM, max(16, (tile_of(u).cols + 15) / 16 * 16));
-                if (!skn_mbar_wait(&acc_empty[b], ((uint32_t)(tile >> 1) & 1u) ^ 1u)) {
-                    atomicExch(status, SKN_ERR_TIMEOUT);
+        // the whole warp follows the barriers, one elected lane issues
+        uint32_t idesc = tc_idesc(DTC_BM, NT);
+        bool ok = true;
+        int s = 0, tile = 0;
+        uint32_t ph = 0;
+        for (int u = blockIdx.x; u < units && ok; u += gridDim.x, ++tile) {
+            const int sp = GROUPS ? 0 : (u / mt) % splits;
+            const int kb = (int)((int64_t)ksteps * sp / splits), ke = (int)((int64_t)ksteps * (sp + 1) / splits);
+            const int b = tile & 1;
+            if (GROUPS) idesc = tc_idesc(DTC_BM, max(16, (tile_of(u).cols + 15) / 16 * 16));
+            if (!skn_mbar_wait(&acc_empty[b], ((uint32_t)(tile >> 1) & 1u) ^ 1u)) {
+                if (lane == 0) atomicExch(status, SKN_ERR_TIMEOUT);
+                break;
+            }
+            tc_fence_after();
+            const uint32_t d = tmem + (uint32_t)(b * acc_cols);
+            for (int k = kb; k < ke; ++k) {
+                if (!skn_mbar_wait(&full_bar[s], ph)) {
+                    if (lane == 0) atomicExch(status, SKN_ERR_TIMEOUT);
+                    ok = false;
                     break;
                 }
                 tc_fence_after();
-                const uint32_t d = tmem + (uint32_t)(b * acc_cols);
-                for (int k = kb; k < ke; ++k, ++it) {
-                    const int s = it % stages;
-                    if (!skn_mbar_wait(&full_bar[s], (uint32_t)(it / stages) & 1u)) {
-                        atomicExch(status, SKN_ERR_TIMEOUT);
-                        ok = false;
-                        break;
-                    }
-                    tc_fence_after();
-                    const uint32_t base = skn_smem_u32(smem + (size_t)s * stage_bytes);
-                    const uint64_t ad = tc_smem_desc(base), bd = tc_smem_desc(base + DTC_A_BYTES);
+                const uint32_t base = skn_smem_u32(smem + (size_t)s * stage_bytes);
+                const uint64_t ad = tc_smem_desc(base), bd = tc_smem_desc(base + DTC_A_BYTES);
+                if (tc_elect()) {
 #pragma unroll
                     for (int j = 0; j < DTC_BK / 16; ++j) tc_mma_bf16(d, ad + 2 * j, bd + 2 * j, idesc, (k > kb || j > 0) ? 1u : 0u);
                     tc_commit(&empty_bar[s]);
                 }
-                tc_commit(&acc_full[b]);
+                if (++s == stages) { s = 0; ph ^= 1u; }
             }
+            if (ok && tc_elect()) tc_commit(&acc_full[b]);
         }
     } else {
         // epilogue: TMEM lane = weight row, column = token; a warp's store covers 32 consecutive outputs of one token

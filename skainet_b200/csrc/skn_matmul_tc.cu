@@ -97,13 +97,6 @@ __device__ __forceinline__ bool tc_wait_warp(uint64_t *bar, uint32_t parity, int
     if (lane == 0) ok = skn_mbar_wait(bar, parity);
     return __shfl_sync(0xffffffffu, (int)ok, 0) != 0;
 }
-// One lane of a converged warp, chosen by the instruction made for it: under a plain `lane == 0` the operands of every
-// tcgen05 instruction take a detour through vector registers (445 clocks instead of 100 for the MMAs of a stage).
-__device__ __forceinline__ bool tc_elect() {
-    uint32_t p;
-    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
-    return p != 0;
-}
 __device__ __forceinline__ uint4 tc_lds128(uint32_t addr) {
     uint4 v;
     asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr));

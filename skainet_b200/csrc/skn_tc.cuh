@@ -6,6 +6,15 @@
 #include <cuda.h>
 #include <cuda_bf16.h>
 
+// One lane of a converged warp, chosen by the instruction made for it: under a plain `lane == 0` the operands of every
+// tcgen05 instruction take a detour through vector registers (measured for the four MMAs of a 64-column stage: 445 clocks
+// instead of 100, more than the 256 to 512 that the tensor cores need for them).
+__device__ __forceinline__ bool tc_elect() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+    return p != 0;
+}
+
 // ---- tcgen05 wrappers ---------------------------------------------------------------------
 __device__ __forceinline__ void tc_alloc(uint32_t *slot_smem, uint32_t ncols) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(skn_smem_u32(slot_smem)),
