@@ -286,8 +286,8 @@ int32_t skn_llama_forward_dev(skn_llama *m, const int32_t *tokens_dev, int32_t T
         for (auto &l : m->layers) {
             const skn_tensor *qkv[3] = {l.wq, l.wk, l.wv}, *gu[2] = {l.wg, l.wu};
             fold = fold && l.wk->type == l.wq->type && l.wv->type == l.wq->type && l.wq->pitch == l.wk->pitch &&
-                   l.wq->pitch == l.wv->pitch && skn_rows_max_acts(ctx, 3, qkv) >= 4 && l.wu->type == l.wg->type &&
-                   l.wu->pitch == l.wg->pitch && skn_rows_max_acts(ctx, 2, gu) >= 4;
+                   l.wq->pitch == l.wv->pitch && ((M >= SKN_BATCH_MIN && skn_batch_covers(3, qkv)) || skn_rows_max_acts(ctx, 3, qkv) >= 4) && l.wu->type == l.wg->type &&
+                   l.wu->pitch == l.wg->pitch && ((M >= SKN_BATCH_MIN && skn_batch_covers(2, gu)) || skn_rows_max_acts(ctx, 2, gu) >= 4);
         }
     }
     auto fused = [&](int n, const skn_tensor *const *ws, const float *x, float *const *ys, const float *const *add,

@@ -72,35 +72,10 @@ __device__ __forceinline__ void tc2_tma_load_2d(void *dst_smem, const CUtensorMa
         ::"r"(skn_smem_u32(dst_smem)), "l"(reinterpret_cast<uint64_t>(tmap)), "r"(x), "r"(y), "r"(bar_cluster)
         : "memory");
 }
-__device__ __forceinline__ uint32_t tc_cluster_rank() {
-    uint32_t r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-}
-__device__ __forceinline__ uint32_t tc_mapa(uint32_t addr, uint32_t rank) {
-    uint32_t r;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
-    return r;
-}
 // What the arrival announces is read by the tensor cores only and was handed to their proxy by a fence before, so the
 // default scope does: `.release.cluster` waits for all of the warp's stores to be acknowledged.
 __device__ __forceinline__ void tc_arrive_remote(uint32_t cluster_addr) {
     asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
-}
-__device__ __forceinline__ void tc_cluster_sync() {
-    asm volatile("barrier.cluster.arrive.release;" ::: "memory");
-    asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
-}
-// one lane of a warp polls for all of it
-__device__ __forceinline__ bool tc_wait_warp(uint64_t *bar, uint32_t parity, int lane) {
-    bool ok = true;
-    if (lane == 0) ok = skn_mbar_wait(bar, parity);
-    return __shfl_sync(0xffffffffu, (int)ok, 0) != 0;
-}
-__device__ __forceinline__ uint4 tc_lds128(uint32_t addr) {
-    uint4 v;
-    asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr));
-    return v;
 }
 
 // ---- raw blocks -> bf16 ----------------------------------------------------------------------------------------
@@ -132,29 +107,6 @@ __device__ __forceinline__ void tc_quad(uint32_t w, __half2 base, uint64_t scale
         out[i] = tc_pack_bf16(lo, hi);
     }
 }
-// words of a byte run that starts `sel` words and sh bits (0 or 16) into an aligned window (sel: the same for the warp)
-template <int SEL, int N, int W>
-__device__ __forceinline__ void tc_cut(const uint32_t (&win)[W], uint32_t sh, uint32_t (&out)[N]) {
-#pragma unroll
-    for (int i = 0; i < N; ++i) out[i] = __funnelshift_rc(win[i + SEL], (i + SEL + 1 < W) ? win[i + SEL + 1 < W ? i + SEL + 1 : 0] : 0u, sh);
-}
-template <int N, int W>
-__device__ __forceinline__ void tc_shift(const uint32_t (&win)[W], int sel, uint32_t sh, uint32_t (&out)[N]) {
-    switch (sel) {
-    case 0: tc_cut<0>(win, sh, out); break;
-    case 1: tc_cut<1>(win, sh, out); break;
-    case 2: tc_cut<2>(win, sh, out); break;
-    default: tc_cut<3>(win, sh, out); break;
-    }
-}
-template <int N> __device__ __forceinline__ void tc_window(uint32_t addr, uint32_t (&w)[N]) {
-#pragma unroll
-    for (int i = 0; i < N / 4; ++i) {
-        const uint4 v = tc_lds128(addr + 16 * i);
-        w[4 * i] = v.x; w[4 * i + 1] = v.y; w[4 * i + 2] = v.z; w[4 * i + 3] = v.w;
-    }
-}
-
 constexpr uint64_t TC_NEG_ZERO2 = 0x8000000080000000ull;   // (-0, -0): v * s + (-0) is the rounded product
 
 // Stage u (weights 64 u .. 64 u + 63 of the super-block) of the row at `row`: what both halves share, then half g as
@@ -602,20 +554,6 @@ static tc_plan tc_make_plan(int type, int M, int64_t tiles, int K, const int *pa
     return best;
 }
 
-// boxes of `rows` rows x one super-block column of the raw blocks, in 4-byte units
-static cudaError_t tc_weight_map(const skn_tensor *w, int rows, CUtensorMap *out) {
-    skn_encode_tiled_fn encode = nullptr;
-    const cudaError_t e = skn_tmap_encoder(&encode);
-    if (e != cudaSuccess) return e;
-    const cuuint64_t gdim[2] = {(cuuint64_t)((w->row_bytes + 3) / 4), (cuuint64_t)w->n_rows};
-    const cuuint64_t gstride[1] = {(cuuint64_t)w->pitch};
-    const cuuint32_t box[2] = {(cuuint32_t)(tc_row_bytes(w->type) / 4), (cuuint32_t)rows};
-    const cuuint32_t estr[2] = {1, 1};
-    const CUresult r = encode(out, CU_TENSOR_MAP_DATA_TYPE_UINT32, 2, w->d_blocks, gdim, gstride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                              CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
-}
-
 static cudaLaunchConfig_t tc_config(dim3 grid, int split, size_t smem, cudaStream_t stream, cudaLaunchAttribute *attr) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
@@ -661,8 +599,8 @@ static cudaError_t launch_tc(const __nv_bfloat16 *A, int M, int K, const skn_ten
     const tc_plan pl = tc_make_plan(TYPE, M, tiles, K, pairs);
     CUtensorMap tx, tw, tw2;
     if ((e = skn_tmap_bf16(A, M, K, (int64_t)K * 2, pl.nn / 2, &tx)) != cudaSuccess) return e;
-    if ((e = tc_weight_map(w, DUAL ? 16 : TC_ROWS, &tw)) != cudaSuccess) return e;
-    if ((e = tc_weight_map(DUAL ? w2 : w, DUAL ? 16 : TC_ROWS, &tw2)) != cudaSuccess) return e;
+    if ((e = skn_tmap_blocks(w, TcFmt<TYPE>::ROW, DUAL ? 16 : TC_ROWS, &tw)) != cudaSuccess) return e;
+    if ((e = skn_tmap_blocks(DUAL ? w2 : w, TcFmt<TYPE>::ROW, DUAL ? 16 : TC_ROWS, &tw2)) != cudaSuccess) return e;
     const cudaLaunchConfig_t cfg = tc_config(dim3((unsigned)(tiles * 2 * pl.split), (unsigned)pl.blocks), pl.split, pl.smem, stream, attr);
     return cudaLaunchKernelEx(&cfg, kern, tx, tw, tw2, M, K, (int)w->n_rows, pl, out, status);
 }

@@ -966,6 +966,30 @@ cudaError_t skn_launch_matvec_acts(skn_ctx *ctx, int n, const skn_tensor *const 
     }
     if ((w[0]->pitch % 16) != 0) return cudaErrorNotSupported;
     const int64_t K = w[0]->n_cols;
+    // nine rows or more: tcgen05, up to 32 rows per pass over the weights; it has no rotary epilogue and no exchange.  Its time
+    // hardly depends on the rows, that of the many-row kernel below grows with them: Q4_K 14336 x 4096 29 us at 3 to 16 rows
+    // against 18 / 34 / 69 at 4 / 8 / 16; 4096 x 4096 13.5 against 10.5 / 12.2 / 22; Q8_0 14336 x 4096 42 (M = 4), 50 (M = 16) against 20, 73.
+    if (M >= SKN_BATCH_MIN && !xc && !rope && skn_batch_covers(n, w)) {
+        const int rows = skn_batch_rows(w[0]->type), launches = (M + rows - 1) / rows;
+        for (int i = 0, m0 = 0; i < launches; ++i) {
+            const int na = (M - m0 + (launches - i) - 1) / (launches - i);       // even shares
+            float *ys[3] = {nullptr, nullptr, nullptr};
+            const float *as[3] = {nullptr, nullptr, nullptr};
+            for (int t = 0; t < n; ++t) {
+                ys[t] = y[t] + (int64_t)m0 * w[swiglu ? 0 : t]->n_rows;
+                if (add && add[t]) as[t] = add[t] + (add_per_act ? (int64_t)m0 * w[t]->n_rows : 0);
+            }
+            cudaError_t err = cudaSuccess;
+            if (!skn_batch_try_group(ctx, n, w, x + (int64_t)m0 * K, na, ys, add ? as : nullptr, add_per_act, norm_gain, norm_eps,
+                                     silu_u ? silu_u + (int64_t)m0 * K : nullptr, swiglu, stream, err)) {
+                if (i == 0) break;                                        // not covered after all: the routes below
+                return cudaErrorUnknown;
+            }
+            if (err != cudaSuccess) return err;
+            m0 += na;
+            if (m0 == M) return cudaSuccess;
+        }
+    }
     // three rows or more: the many-row kernel (x prepared once per launch by its own kernel, up to sixteen rows
     // per pass over the weights); it has no rotary epilogue and no exchange
     if (M >= 3 && !xc && !rope) {

@@ -1,0 +1,702 @@
+// K2 for batches of some activation rows (up to 32 in one launch): Y[M, N] = X[M, K] . W_q[N, K]^T in the accuracy of the
+// single-row kernels, on the 5th-generation tensor cores.
+//
+// The arithmetic is the one of skn_matvec_mma.cu -- 30-bit fixed-point activations per super-block, integer products,
+// exact sums per scale block, outliers apart in fp32 -- in numbers that tcgen05 takes: a weight's integer (Q4_K: quant
+// times 6-bit sub-block scale, at most 945; Q4_0, Q8_0: the signed quant) is an exact fp16 number, an activation is
+// three exact fp16 digits (X = d0 2^22 + d1 2^11 + d2, |d0| <= 256, |d1|, |d2| <= 1024), and an fp32 accumulator holds
+// sums of such products exactly below 2^24, which those of the leading digit stay under but for contrived blocks (and
+// then lose one part in 2^23).  The scale d of a block multiplies the accumulator when it is drained: once per 256
+// columns for Q4_K, once per 32 for Q4_0 and Q8_0.
+//
+// What bounded the mma.sync form of this (skn_matvec_rows.cu) was the chain load, MMA, integer multiply-add per 16 rows x
+// 32 columns of eight warps; here a thread that unpacks 64 weights needs about two instructions per weight, one thread
+// issues the MMAs for 128 rows, and a drained number stands for 256 (32) products.
+//
+// A CTA owns 128 weight rows (DUAL: 16 gate rows, 16 up rows, ...) x a part of K; the c CTAs of a cluster share K and add their
+// sums through distributed shared memory in rank order.
+//   warps 4 i, i < 4  warp 0 issues MMAs, warp 4 the TMA of the digit planes, warp 8 that of the raw blocks and block records
+//   other warps < 16  unpack: raw super-block columns -> fp16 operand tiles, in three groups of four
+//   warps 16-23       drain: lane = weight row; scales, offsets (fp32 sums of x), outliers, sums over K in registers; output
+//
+// Measured (B200, graph of distinct weights, us per call with the preparation of x, before -> now):
+//   Q4_K 14336 x 4096: 8 rows 34 -> 31, 16 rows 69 -> 29, 32 rows 137 -> 37; 28672 x 4096: 16 rows 110 -> 57; 4096 x 4096: 22 -> 13.4
+//   Q4_0 4096 x 14336: 16 rows 75 -> 41, 60 rows 299 -> 116; Q8_0 14336 x 4096: 16 rows 73 -> 50
+// Bound now: 600 clocks per 64 columns of 128 rows in the hand-overs between unpacking, issuing and draining warps (the products and the
+// arithmetic of each take less than half of that), and about 10 us a call of preparation, start and exchange.
+#include "skn_mma_common.cuh"
+#include "skn_tc.cuh"
+
+#include <atomic>
+
+constexpr int MB_ROWS = 128, MB_BK = 128;          // a stage: two 128-byte wide operand tiles of 64 columns (one tile per
+                                                  // stage left the issuing thread with 680 clocks of waits and commits per 64 columns)
+constexpr int MB_A_TILE = MB_ROWS * 128, MB_A_BYTES = 2 * MB_A_TILE;
+constexpr int MB_THREADS = 24 * 32;
+constexpr int MB_DQ_WARPS = 12, MB_DQ_GROUPS = 3, MB_DRAIN = 16, MB_DRAIN_WARPS = 8;
+constexpr int MB_MMA = 0, MB_TMA_X = 4, MB_TMA_W = 8;
+constexpr int MB_CHUNK = 8, MB_COLS = 32;         // activation rows of a chunk; its columns (three digits of eight rows, eight unused)
+constexpr int MB_MAX_A = 4, MB_MAX_B = 6, MB_MAX_RAW = 4, MB_MAX_D = 8, MB_MAX_SPLIT = 8;
+constexpr int MB_SMEM_MAX = 224 * 1024;
+
+// record of one (super-block, activation row), the layout of mm_digitize's outputs
+struct __align__(16) mb_meta {
+    float scale;                                  // 2^(e-29) (NaN: the block is not finite)
+    uint32_t ocnt, oidx, pad;                     // outliers: count, positions (one byte each)
+    float oval[MM_MAX_OUT];                       // ... and values
+    float xsum[8];                                // sums of 32 activations, outliers excluded
+};
+constexpr int MB_META = (int)sizeof(mb_meta);
+static_assert(MB_META == 64, "block record layout");
+
+// ---- activations -> digit planes and block records ------------------------------------------------------------------
+// One CTA per activation row; f(x) = x, x / rms(x) * gain, or silu(x) * u.  Row a's digit p goes to row
+// (a / 8) * 32 + p * 8 + a % 8 of `planes` ([32 * chunks][K] fp16); records to meta[super-block][8 * chunks].
+__global__ void __launch_bounds__(1024)
+skn_xsplit_kernel(const float *__restrict__ x, int K, const float *__restrict__ gain, float eps, const float *__restrict__ silu_u,
+                  __half *__restrict__ planes, mb_meta *__restrict__ meta, int rows_pad) {
+    skn_pdl_launch_dependents();                  // the product's CTAs may come in and unpack their first weights
+    skn_pdl_wait();                               // x is the previous kernel's output; the planes may still be read by it
+    const int a = blockIdx.x, nb = K / 256;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    const float4 *xr = reinterpret_cast<const float4 *>(x + (size_t)a * K);
+    const float4 *ur = silu_u ? reinterpret_cast<const float4 *>(silu_u + (size_t)a * K) : nullptr;
+    __shared__ float s_ss[32];
+    float rs = 1.f;
+    if (gain) {
+        float ss = 0.f;
+        for (int i = threadIdx.x; i < K / 4; i += blockDim.x) {
+            const float4 v = __ldg(xr + i);
+            ss += (v.x * v.x + v.y * v.y) + (v.z * v.z + v.w * v.w);
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+        if (lane == 0) s_ss[warp] = ss;
+        __syncthreads();
+        float tot = 0.f;
+        for (int w = 0; w < nw; ++w) tot += s_ss[w];
+        rs = rsqrtf(tot / (float)K + eps);
+    }
+    auto load = [&](int f) {
+        float4 v = __ldg(xr + f);
+        if (ur) {
+            const float4 u = __ldg(ur + f);
+            v.x = v.x / (1.f + expf(-v.x)) * u.x; v.y = v.y / (1.f + expf(-v.y)) * u.y;
+            v.z = v.z / (1.f + expf(-v.z)) * u.z; v.w = v.w / (1.f + expf(-v.w)) * u.w;
+        }
+        if (gain) {
+            const float4 g = __ldg(reinterpret_cast<const float4 *>(gain) + f);
+            v.x = v.x * rs * g.x; v.y = v.y * rs * g.y; v.z = v.z * rs * g.z; v.w = v.w * rs * g.w;
+        }
+        return v;
+    };
+    __half *row = planes + ((size_t)(a / MB_CHUNK) * MB_COLS + a % MB_CHUNK) * K;
+    for (int sb = warp; sb < nb; sb += nw) {
+        const float4 v0 = load(sb * 64 + lane), v1 = load(sb * 64 + 32 + lane);
+        mb_meta *m = meta + (size_t)sb * rows_pad + a;
+        int X[8];
+        mm_fixed_point<false>(v0, v1, 0, lane, X, &m->scale, m->xsum, m->oval, &m->oidx, reinterpret_cast<uint8_t *>(&m->ocnt), nullptr);
+        __half dig[3][8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const int d2 = ((X[i] + 1024) & 2047) - 1024, h = (X[i] - d2) >> 11;
+            const int d1 = ((h + 1024) & 2047) - 1024;
+            dig[0][i] = __int2half_rn((h - d1) >> 11);
+            dig[1][i] = __int2half_rn(d1);
+            dig[2][i] = __int2half_rn(d2);
+        }
+#pragma unroll
+        for (int p = 0; p < 3; ++p) {
+            uint2 *to = reinterpret_cast<uint2 *>(row + (size_t)p * MB_CHUNK * K + sb * 256) + lane;
+            to[0] = *reinterpret_cast<const uint2 *>(&dig[p][0]);
+            to[32] = *reinterpret_cast<const uint2 *>(&dig[p][4]);
+        }
+    }
+}
+
+// ---- raw blocks -> fp16 integers --------------------------------------------------------------------------------------
+template <int TYPE> struct MbFmt;
+template <> struct MbFmt<SKN_TYPE_Q4_K> { static constexpr int ROW = 144, MM = MM_FMT_Q4K, BLOCKS = 1; };
+template <> struct MbFmt<SKN_TYPE_Q4_0> { static constexpr int ROW = 144, MM = MM_FMT_Q40, BLOCKS = 8; };
+template <> struct MbFmt<SKN_TYPE_Q8_0> { static constexpr int ROW = 272, MM = MM_FMT_Q80, BLOCKS = 8; };
+
+// four bytes b of w -> fp16 (b + 1024) * mul + add: 1024 + b is the byte under the high byte 0x64; all values here are exact
+__device__ __forceinline__ void mb_quad(uint32_t w, __half2 mul, __half2 add, uint32_t *out) {
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        const uint32_t h = __byte_perm(w, 0x64646464u, i ? 0x4342 : 0x4140);
+        const __half2 v = __hfma2(*reinterpret_cast<const __half2 *>(&h), mul, add);
+        out[i] = *reinterpret_cast<const uint32_t *>(&v);
+    }
+}
+// half g of stage u of the row at `row` (see the formats' notes in skn_matmul_tc.cu: same cut, same chunks)
+template <int TYPE>
+__device__ __forceinline__ void mb_half(uint32_t row, int u, int g, uint32_t sc2, uint32_t (&out)[16]) {
+    if constexpr (TYPE == SKN_TYPE_Q4_K) {
+        const uint4 q = tc_lds128(row + 16 + 32 * u + 16 * g);
+        const uint32_t qw[4] = {q.x, q.y, q.z, q.w};
+        const __half2 s0 = __half2half2(__uint2half_rn(sc2 & 0xFFu)), s1 = __half2half2(__uint2half_rn(sc2 >> 8));
+        const __half2 a0 = __hmul2(s0, __float2half2_rn(-1024.f)), a1 = __hmul2(s1, __float2half2_rn(-1024.f));
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            mb_quad(qw[i] & 0x0F0F0F0Fu, s0, a0, out + 2 * i);
+            mb_quad((qw[i] >> 4) & 0x0F0F0F0Fu, s1, a1, out + 8 + 2 * i);
+        }
+    } else if constexpr (TYPE == SKN_TYPE_Q4_0) {
+        uint32_t win[8], w[5];
+        tc_window(row + 32 * u + 16 * g, win);
+        tc_shift(win, u, 16u * g, w);
+        const __half2 one = __float2half2_rn(1.f), add = __float2half2_rn(-1032.f);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const uint32_t q = __funnelshift_r(w[i], w[i + 1], 16);
+            mb_quad(q & 0x0F0F0F0Fu, one, add, out + 2 * i);
+            mb_quad((q >> 4) & 0x0F0F0F0Fu, one, add, out + 8 + 2 * i);
+        }
+    } else {
+        uint32_t win[12], w[9];
+        tc_window(row + 64 * u + 32 * g, win);
+        tc_shift(win, u, 16u * g, w);
+        const __half2 one = __float2half2_rn(1.f), add = __float2half2_rn(-1152.f);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) mb_quad(__funnelshift_r(w[i], w[i + 1], 16) ^ 0x80808080u, one, add, out + 2 * i);
+    }
+}
+// 6-bit scales (word 1) and minima (word 2) of a Q4_K header as bytes: sub-blocks 0-3, 4-7
+__device__ __forceinline__ void mb_q4k_scales(const uint4 &h, uint32_t (&sc)[2], uint32_t (&mn)[2]) {
+    sc[0] = h.y & 0x3F3F3F3Fu;
+    sc[1] = (h.w & 0x0F0F0F0Fu) | ((h.y >> 2) & 0x30303030u);
+    mn[0] = h.z & 0x3F3F3F3Fu;
+    mn[1] = ((h.w >> 4) & 0x0F0F0F0Fu) | ((h.z >> 2) & 0x30303030u);
+}
+__device__ __forceinline__ float mb_byte(uint32_t w, int i) {       // byte i as a float: 2^23 + byte, exactly, less 2^23
+    return __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7440 + i)) - 8388608.f;
+}
+
+struct mb_args {
+    int count, n_act;
+    int tcum[4];                                  // tiles before tensor t
+    int64_t n_rows[3];
+    float *y[3];
+    const float *add[3];
+    int64_t addstride[3];
+};
+struct mb_plan {
+    int split, a, b, raw, d;                      // CTAs that share K; ring depths (weight tiles, digit tiles, raw columns, accumulators)
+    size_t smem;
+};
+
+template <int TYPE, int NCH, bool DUAL>
+__global__ void __launch_bounds__(MB_THREADS, 1)
+skn_matvec_batch_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_w0, const __grid_constant__ CUtensorMap tm_w1,
+                        const __grid_constant__ CUtensorMap tm_w2, const mb_args ar, int K, const mb_plan pl, const mb_meta *__restrict__ meta,
+                        int32_t *__restrict__ status) {
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    constexpr int ROW = MbFmt<TYPE>::ROW, RAW_BYTES = MB_ROWS * ROW, BLOCKS = MbFmt<TYPE>::BLOCKS;
+    constexpr int NCOL = NCH * MB_COLS, SET_COLS = BLOCKS == 1 ? NCOL : 2 * NCOL, B_TILE = NCOL * 128, B_BYTES = 2 * B_TILE, META_BYTES = NCH * MB_CHUNK * MB_META;
+    __shared__ uint64_t a_full[MB_MAX_A], a_empty[MB_MAX_A], b_full[MB_MAX_B], b_empty[MB_MAX_B], raw_full[MB_MAX_RAW], meta_full[MB_MAX_RAW],
+        raw_empty[MB_MAX_RAW], d_full[MB_MAX_D], d_empty[MB_MAX_D];
+    __shared__ uint32_t tmem_slot;
+
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+    const int c = pl.split, kr = c > 1 ? (int)tc_cluster_rank() : 0, tile = (int)blockIdx.x / c;
+    const int na = pl.a, nb = pl.b, nraw = pl.raw, nd = pl.d;
+    uint8_t *b_ring = smem + (size_t)na * MB_A_BYTES, *raw_ring = b_ring + (size_t)nb * B_BYTES, *meta_ring = raw_ring + (size_t)nraw * RAW_BYTES;
+    float *slots = reinterpret_cast<float *>(smem);                // over the rings, once all CTAs of the cluster are done with them
+    const int nsb = K / 256, sb0 = kr * nsb / c, sb1 = (kr + 1) * nsb / c, steps = 2 * (sb1 - sb0);
+    // the tile's tensor and first row
+    int t = 0;
+    if (!DUAL) t = (tile >= ar.tcum[1] ? 1 : 0) + (ar.count > 2 && tile >= ar.tcum[2] ? 1 : 0);
+    const int n0 = DUAL ? tile * (MB_ROWS / 2) : (tile - ar.tcum[t]) * MB_ROWS;
+    constexpr uint32_t TMEM_COLS = 512;
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < na; ++s) {
+            skn_mbar_init(&a_full[s], 4);
+            skn_mbar_init(&a_empty[s], 1);
+        }
+        for (int s = 0; s < nb; ++s) {
+            skn_mbar_init(&b_full[s], 1);
+            skn_mbar_init(&b_empty[s], 1);
+        }
+        for (int s = 0; s < nd; ++s) {
+            skn_mbar_init(&d_full[s], 1);
+            skn_mbar_init(&d_empty[s], MB_DRAIN_WARPS);
+        }
+        skn_fence_mbar_init();
+    }
+    auto load_raw = [&](int sb, int rs) {
+        uint8_t *dst = raw_ring + (size_t)rs * RAW_BYTES;
+        skn_mbar_expect_tx(&raw_full[rs], RAW_BYTES);
+        const int x = sb * (ROW / 4);
+        if (DUAL) {
+            for (int i = 0; i < 4; ++i) {
+                tc_tma_load_2d(dst + 32 * i * ROW, &tm_w0, x, n0 + 16 * i, &raw_full[rs]);
+                tc_tma_load_2d(dst + (32 * i + 16) * ROW, &tm_w1, x, n0 + 16 * i, &raw_full[rs]);
+            }
+        } else {
+            tc_tma_load_2d(dst, t == 0 ? &tm_w0 : (t == 1 ? &tm_w1 : &tm_w2), x, n0, &raw_full[rs]);
+        }
+    };
+    auto load_meta = [&](int sb, int rs) {
+        skn_mbar_expect_tx(&meta_full[rs], META_BYTES);
+        skn_bulk_g2s(meta_ring + (size_t)rs * META_BYTES, meta + (size_t)sb * (NCH * MB_CHUNK), META_BYTES, &meta_full[rs]);
+    };
+    const int early = min(nraw, sb1 - sb0);
+    if (warp == MB_TMA_W && lane == 0) {
+        for (int s = 0; s < nraw; ++s) {
+            skn_mbar_init(&raw_full[s], 1);
+            skn_mbar_init(&meta_full[s], 1);
+            skn_mbar_init(&raw_empty[s], MB_DQ_WARPS + MB_DRAIN_WARPS);
+        }
+        skn_fence_mbar_init();
+        skn_fence_proxy_async();
+        for (int i = 0; i < early; ++i) load_raw(sb0 + i, i);      // the weights depend on no launch before this one
+    }
+    if (warp == MB_MMA) tc_alloc(&tmem_slot, TMEM_COLS);
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem_base = tmem_slot;
+
+    bool failed = false;
+    auto give_up = [&]() {
+        failed = true;
+        atomicExch(status, SKN_ERR_TIMEOUT);
+    };
+    if (warp < MB_DRAIN && (warp & 3)) {
+        // ---------------- unpack: group `turn` takes the stages 3 i + turn ----------------
+        const int dq = (warp >> 2) * 3 + (warp & 3) - 1, turn = dq >> 2, r = (dq & 3) * 32 + lane;
+        const uint32_t raw0 = skn_smem_u32(raw_ring) + (uint32_t)(r * ROW);
+        int s = turn % na, rs = 0, it = turn;
+        uint32_t ph = (uint32_t)(turn / na), rph = 0;
+#pragma unroll 1
+        for (int sb = 0; sb < steps / 2; ++sb) {           // (every group sees every super-block, with a stage of its own in it or not)
+            if (!failed && !tc_wait_warp(&raw_full[rs], rph, lane)) give_up();
+            if (it >> 1 == sb) {
+                const uint32_t row = raw0 + (uint32_t)(rs * RAW_BYTES);
+                uint32_t sc[2] = {0, 0}, mn[2];
+                if (TYPE == SKN_TYPE_Q4_K) mb_q4k_scales(tc_lds128(row), sc, mn);
+                const uint32_t sc4 = sc[it & 1];           // scales of the stage's four sub-blocks
+#pragma unroll 1
+                for (int v = 0; v < 2; ++v) {              // the stage's tiles of 64 columns
+                    uint8_t *tile_a = smem + (size_t)s * MB_A_BYTES + v * MB_A_TILE;
+#pragma unroll
+                    for (int g = 0; g < 2; ++g) {
+                        uint32_t p[16];
+                        mb_half<TYPE>(row, 2 * (it & 1) + v, g, (sc4 >> (16 * v)) & 0xFFFFu, p);
+                        if (v == 0 && g == 0 && !failed && !tc_wait_warp(&a_empty[s], ph ^ 1u, lane)) give_up();
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) {
+                            const int chunk = TYPE == SKN_TYPE_Q4_K ? 4 * (i >> 1) + 2 * g + (i & 1) : 4 * g + i;
+                            tc_store_chunk(tile_a, r, chunk, make_uint4(p[4 * i], p[4 * i + 1], p[4 * i + 2], p[4 * i + 3]));
+                        }
+                    }
+                }
+                skn_fence_proxy_async();
+                __syncwarp();
+                if (lane == 0) skn_mbar_arrive(&a_full[s]);
+                for (s += MB_DQ_GROUPS; s >= na; s -= na) ph ^= 1u;
+                it += MB_DQ_GROUPS;
+            }
+            __syncwarp();
+            if (lane == 0) skn_mbar_arrive(&raw_empty[rs]);
+            if (++rs == nraw) { rs = 0; rph ^= 1u; }
+        }
+    } else if (warp == MB_TMA_W) {
+        // ---------------- raw blocks, and the block records of the activations (previous launch's output) ----------------
+        if (lane == 0) {
+            skn_pdl_wait();
+            for (int i = 0; i < early; ++i) load_meta(sb0 + i, i);
+            int rs = 0;
+            uint32_t rph = 0;
+            for (int sb = sb0 + early; sb < sb1; ++sb) {
+                if (!failed && !skn_mbar_wait(&raw_empty[rs], rph)) give_up();
+                skn_fence_proxy_async();
+                load_raw(sb, rs);
+                load_meta(sb, rs);
+                if (++rs == nraw) { rs = 0; rph ^= 1u; }
+            }
+        }
+    } else if (warp == MB_TMA_X) {
+        if (lane == 0) {
+            skn_pdl_wait();
+            int s = 0;
+            uint32_t ph = 0;
+            for (int it = 0; it < steps; ++it) {
+                if (!failed && !skn_mbar_wait(&b_empty[s], ph ^ 1u)) give_up();
+                skn_mbar_expect_tx(&b_full[s], B_BYTES);
+                for (int v = 0; v < 2; ++v)
+                    tc_tma_load_2d(b_ring + (size_t)s * B_BYTES + v * B_TILE, &tm_x, (sb0 * 2 + it) * MB_BK + 64 * v, 0, &b_full[s]);
+                if (++s == nb) { s = 0; ph ^= 1u; }
+            }
+        }
+    } else if (warp == MB_MMA) {
+        // ---------------- MMAs: 128 rows x NCOL columns, fp16 operands, one accumulator per scale block ----------------
+        constexpr uint32_t idesc = (1u << 4) | ((uint32_t)(NCOL >> 3) << 17) | ((uint32_t)(MB_ROWS >> 4) << 24);
+        const uint64_t a0 = tc_smem_desc(skn_smem_u32(smem)), b0 = tc_smem_desc(skn_smem_u32(b_ring));
+        int s = 0, tb = 0, d = 0;
+        uint32_t ph = 0, pb = 0, pd = 0;
+        for (int it = 0; it < steps; ++it) {
+            if (!failed && !skn_mbar_wait(&b_full[tb], pb)) failed = true;
+            if (!failed && !skn_mbar_wait(&a_full[s], ph)) failed = true;
+            const uint64_t ad = a0 + (uint64_t)(s * (MB_A_BYTES >> 4)), bd = b0 + (uint64_t)(tb * (B_BYTES >> 4));
+            // K step k (16 columns): 32 bytes inside a tile's swizzle atom = +2 in the address field
+            if constexpr (BLOCKS == 1) {
+                if ((it & 1) == 0 && !failed && !skn_mbar_wait(&d_empty[d], pd ^ 1u)) failed = true;
+                tc_fence_after();
+                if (tc_elect()) {
+#pragma unroll
+                    for (int k = 0; k < 8; ++k)
+                        tc_mma_bf16(tmem_base + d * SET_COLS, ad + (k >> 2) * (MB_A_TILE >> 4) + 2 * (k & 3), bd + (k >> 2) * (B_TILE >> 4) + 2 * (k & 3), idesc,
+                                    ((it & 1) || k) ? 1u : 0u);
+                    if (it & 1) tc_commit(&d_full[d]);
+                }
+                if ((it & 1) && ++d == nd) { d = 0; pd ^= 1u; }
+            } else {
+                // two blocks of 32 columns per tile, an accumulator each
+#pragma unroll
+                for (int v = 0; v < 2; ++v) {
+                    if (!failed && !skn_mbar_wait(&d_empty[d], pd ^ 1u)) failed = true;
+                    tc_fence_after();
+                    if (tc_elect()) {
+#pragma unroll
+                        for (int k = 0; k < 4; ++k)
+                            tc_mma_bf16(tmem_base + d * SET_COLS + (k >> 1) * NCOL, ad + v * (MB_A_TILE >> 4) + 2 * k, bd + v * (B_TILE >> 4) + 2 * k, idesc, (uint32_t)(k & 1));
+                        tc_commit(&d_full[d]);
+                    }
+                    if (++d == nd) { d = 0; pd ^= 1u; }
+                }
+            }
+            if (tc_elect()) {
+                tc_commit(&a_empty[s]);
+                tc_commit(&b_empty[tb]);
+            }
+            if (++s == na) { s = 0; ph ^= 1u; }
+            if (++tb == nb) { tb = 0; pb ^= 1u; }
+        }
+        if (failed && lane == 0) atomicExch(status, SKN_ERR_TIMEOUT);
+    } else if (warp >= MB_DRAIN) {
+        // ---------------- drain: lane = weight row ----------------
+        const int wq = warp & 3, r = wq * 32 + lane, odd = (warp - MB_DRAIN) >> 2;     // the two warps of a row quarter take the chunks in turn
+        constexpr int MINE = (NCH + 1) / 2;
+        const uint32_t raw0 = skn_smem_u32(raw_ring) + (uint32_t)(r * ROW), meta0 = skn_smem_u32(meta_ring);
+        float y[MINE * MB_CHUNK];
+#pragma unroll
+        for (int a = 0; a < MINE * MB_CHUNK; ++a) y[a] = 0.f;
+        int rs = 0, d = 0;
+        uint32_t rph = 0, pd = 0;
+#pragma unroll 1
+        for (int sb = sb0; sb < sb1; ++sb) {
+            if (!failed && !tc_wait_warp(&raw_full[rs], rph, lane)) give_up();
+            if (!failed && !tc_wait_warp(&meta_full[rs], rph, lane)) give_up();
+            const uint32_t row = raw0 + (uint32_t)(rs * RAW_BYTES), mt = meta0 + (uint32_t)(rs * META_BYTES);
+            if constexpr (BLOCKS == 1) {
+                const uint4 hdr = tc_lds128(row);
+                const float2 dd = __half22float2(*reinterpret_cast<const __half2 *>(&hdr.x));
+                uint32_t sc[2], mn[2];
+                mb_q4k_scales(hdr, sc, mn);
+                float mf[8];
+#pragma unroll
+                for (int j = 0; j < 8; ++j) mf[j] = mb_byte(mn[j >> 2], j & 3);
+                if (!failed && !tc_wait_warp(&d_full[d], pd, lane)) give_up();
+                tc_fence_after();
+#pragma unroll
+                for (int i = 0; i < MINE; ++i) {
+                    const int ch = 2 * i + odd;
+                    if (ch >= NCH) break;
+                    uint32_t D[32];
+                    tc_ld32(tmem_base + (uint32_t)(d * NCOL + ch * MB_COLS) + ((uint32_t)(wq * 32) << 16), D);
+#pragma unroll
+                    for (int a = 0; a < MB_CHUNK; ++a) {
+                        const uint32_t m = mt + (uint32_t)((ch * MB_CHUNK + a) * MB_META);
+                        const float sx = mm_lds32f(m);
+                        const uint4 s0 = tc_lds128(m + 32), s1 = tc_lds128(m + 48);
+                        const float v = fmaf(__uint_as_float(D[a]), 4194304.f, fmaf(__uint_as_float(D[8 + a]), 2048.f, __uint_as_float(D[16 + a])));
+                        float off = mf[0] * __uint_as_float(s0.x);
+                        off = fmaf(mf[1], __uint_as_float(s0.y), off); off = fmaf(mf[2], __uint_as_float(s0.z), off);
+                        off = fmaf(mf[3], __uint_as_float(s0.w), off); off = fmaf(mf[4], __uint_as_float(s1.x), off);
+                        off = fmaf(mf[5], __uint_as_float(s1.y), off); off = fmaf(mf[6], __uint_as_float(s1.z), off);
+                        off = fmaf(mf[7], __uint_as_float(s1.w), off);
+                        y[i * MB_CHUNK + a] += fmaf(v, dd.x * sx, -dd.y * off);
+                    }
+                }
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) skn_mbar_arrive(&d_empty[d]);
+                if (++d == nd) { d = 0; pd ^= 1u; }
+            } else {
+                float z[MINE * MB_CHUNK];                           // sums over the super-block: short chains of roundings
+#pragma unroll
+                for (int a = 0; a < MINE * MB_CHUNK; ++a) z[a] = 0.f;
+#pragma unroll 1
+                for (int u = 0; u < 4; ++u) {
+                    if (!failed && !tc_wait_warp(&d_full[d], pd, lane)) give_up();
+                    tc_fence_after();
+#pragma unroll
+                    for (int j = 0; j < 2; ++j) {
+                        const float dj = mm_lds_half(row + (uint32_t)((2 * u + j) * (TYPE == SKN_TYPE_Q4_0 ? 18 : 34)));
+#pragma unroll
+                        for (int i = 0; i < MINE; ++i) {
+                            const int ch = 2 * i + odd;
+                            if (ch >= NCH) break;
+                            uint32_t D[32];
+                            tc_ld32(tmem_base + (uint32_t)(d * SET_COLS + j * NCOL + ch * MB_COLS) + ((uint32_t)(wq * 32) << 16), D);
+#pragma unroll
+                            for (int a = 0; a < MB_CHUNK; ++a) {
+                                const float v = fmaf(__uint_as_float(D[a]), 4194304.f, fmaf(__uint_as_float(D[8 + a]), 2048.f, __uint_as_float(D[16 + a])));
+                                z[i * MB_CHUNK + a] = fmaf(v, dj, z[i * MB_CHUNK + a]);
+                            }
+                        }
+                    }
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) skn_mbar_arrive(&d_empty[d]);
+                    if (++d == nd) { d = 0; pd ^= 1u; }
+                }
+#pragma unroll
+                for (int a = 0; a < MINE * MB_CHUNK; ++a)
+                    if (2 * (a / MB_CHUNK) + odd < NCH) y[a] = fmaf(z[a], mm_lds32f(mt + (uint32_t)((MB_CHUNK * (2 * (a / MB_CHUNK) + odd) + a % MB_CHUNK) * MB_META)), y[a]);
+            }
+            // outliers (rare): their products with the whole dequantised weight
+            uint32_t any = 0;
+            for (int a = lane; a < ar.n_act; a += 32) any |= mm_lds32(mt + (uint32_t)(a * MB_META) + 4) & 0xFFu;
+            if (__any_sync(0xffffffffu, any != 0)) {
+#pragma unroll
+                for (int a = 0; a < MINE * MB_CHUNK; ++a) {
+                    const int act = MB_CHUNK * (2 * (a / MB_CHUNK) + odd) + a % MB_CHUNK;
+                    const uint32_t m = mt + (uint32_t)(act * MB_META);
+                    const int n = act < ar.n_act ? (int)(mm_lds32(m + 4) & 0xFFu) : 0;
+                    float add = 0.f;
+#pragma unroll 1
+                    for (int i = 0; i < n; ++i)
+                        add = fmaf(mm_weight_at<MbFmt<TYPE>::MM>(row, (int)mm_lds8(m + 8 + (uint32_t)i)), mm_lds32f(m + 16 + 4 * (uint32_t)i), add);
+                    y[a] += add;
+                }
+            }
+            __syncwarp();
+            if (lane == 0) skn_mbar_arrive(&raw_empty[rs]);
+            if (++rs == nraw) { rs = 0; rph ^= 1u; }
+        }
+        skn_pdl_launch_dependents();
+        skn_pdl_wait();                                            // y and add belong to earlier launches
+        // partial sums to the CTA that adds up a chunk: [owned chunk][source][row of x][weight row]
+        if (c > 1) {
+            tc_cluster_sync();
+#pragma unroll
+            for (int i = 0; i < MINE; ++i) {
+                const int ch = 2 * i + odd, owner = ch % c;
+                if (ch >= NCH || owner == kr) continue;
+                const uint32_t to = tc_mapa(skn_smem_u32(slots) + (uint32_t)(((ch / c) * (c - 1) + (kr < owner ? kr : kr - 1)) * (MB_CHUNK * MB_ROWS) + r) * 4u,
+                                            (uint32_t)owner);
+#pragma unroll
+                for (int a = 0; a < MB_CHUNK; ++a)
+                    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(to + (uint32_t)(a * MB_ROWS * 4)), "f"(y[i * MB_CHUNK + a]) : "memory");
+            }
+            tc_cluster_sync();
+        }
+        float *yo = ar.y[t];
+        const float *ao = ar.add[t];
+        const int64_t N = ar.n_rows[t];
+#pragma unroll
+        for (int i = 0; i < MINE; ++i) {
+            const int ch = 2 * i + odd;
+            if (ch >= NCH || ch % c != kr) continue;
+            float v[MB_CHUNK];
+#pragma unroll
+            for (int a = 0; a < MB_CHUNK; ++a) v[a] = y[i * MB_CHUNK + a];
+            if (c > 1) {
+#pragma unroll 1
+                for (int j = 0; j < c; ++j) {                      // in the order of K, whoever adds
+                    const float *from = slots + ((ch / c) * (c - 1) + (j < kr ? j : j - 1)) * (MB_CHUNK * MB_ROWS) + r;
+#pragma unroll
+                    for (int a = 0; a < MB_CHUNK; ++a) {
+                        const float p = j == kr ? y[i * MB_CHUNK + a] : from[a * MB_ROWS];
+                        v[a] = j == 0 ? p : v[a] + p;
+                    }
+                }
+            }
+            if (DUAL) {
+                // lane l holds gate (l < 16) or up of column l & 15: the halves trade rows of x, each forms every other product
+                const bool low = lane < 16;
+                const int f = n0 + 16 * wq + (lane & 15);
+#pragma unroll
+                for (int a = 0; a < MB_CHUNK; a += 2) {
+                    const float got = __shfl_xor_sync(0xffffffffu, low ? v[a + 1] : v[a], 16);
+                    const float gate = low ? v[a] : got, up = low ? got : v[a + 1];
+                    const int m = ch * MB_CHUNK + a + (low ? 0 : 1);
+                    if (m < ar.n_act && f < N) yo[(int64_t)m * N + f] = gate / (1.f + expf(-gate)) * up;
+                }
+            } else if (n0 + r < N) {
+#pragma unroll
+                for (int a = 0; a < MB_CHUNK; ++a) {
+                    const int m = ch * MB_CHUNK + a;
+                    if (m < ar.n_act) yo[(int64_t)m * N + n0 + r] = v[a] + (ao ? ao[(int64_t)m * ar.addstride[t] + n0 + r] : 0.f);
+                }
+            }
+        }
+    }
+    __syncwarp();
+    if (c > 1 && warp < MB_DRAIN) {                                // the other warps' part of the two cluster barriers
+        tc_cluster_sync();
+        tc_cluster_sync();
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == MB_MMA) {
+        tc_fence_after();
+        tc_dealloc(tmem_base, TMEM_COLS);
+    }
+}
+
+// ---- launch --------------------------------------------------------------------------------------------------------
+static int mb_row_bytes(int type) { return type == SKN_TYPE_Q8_0 ? MbFmt<SKN_TYPE_Q8_0>::ROW : MbFmt<SKN_TYPE_Q4_K>::ROW; }
+
+// K over as many CTAs of a cluster as make the launch shortest, in SM clocks: a start and end of 9000, MB_STAGE_CLOCKS per 64 columns
+// of 128 rows.  `fit[s]` = CTAs in flight in clusters of s.
+constexpr int MB_STAGE_CLOCKS = 500;
+static mb_plan mb_make_plan(int type, int nch, int64_t tiles, int K, const int *fit) {
+    mb_plan pl = {};
+    const int raw_bytes = MB_ROWS * mb_row_bytes(type) + nch * MB_CHUNK * MB_META, b_bytes = nch * MB_COLS * MB_BK * 2, nsb = K / 256;
+    int64_t best = 0;
+    for (int c = 1; c <= MB_MAX_SPLIT && c <= nsb; ++c) {
+        if (fit[c] < 1 && c > 1) continue;
+        const int64_t f = fit[c] > 0 ? fit[c] : 1, waves = (tiles * c + f - 1) / f;
+        const int64_t cost = waves * (9000 + (c > 1 ? 2000 : 0) + (int64_t)((nsb + c - 1) / c) * 4 * MB_STAGE_CLOCKS);
+        if (best == 0 || cost < best) { best = cost; pl.split = c; }
+    }
+    pl.d = 512 / (nch * MB_COLS * (type == SKN_TYPE_Q4_K ? 1 : 2));
+    if (pl.d > MB_MAX_D) pl.d = MB_MAX_D;
+    // a weight tile per unpacking group at least (a group tells its tile's turn by the parity of a phase)
+    pl.a = MB_DQ_GROUPS;
+    pl.b = pl.raw = 2;
+    auto fits = [&](int a, int b, int raw) { return a * MB_A_BYTES + b * b_bytes + raw * raw_bytes <= MB_SMEM_MAX - 1024; };
+    for (bool grown = true; grown;) {
+        grown = false;
+        if (pl.raw < MB_MAX_RAW && fits(pl.a, pl.b, pl.raw + 1)) { ++pl.raw; grown = true; }
+        if (pl.b < MB_MAX_B && fits(pl.a, pl.b + 1, pl.raw)) { ++pl.b; grown = true; }
+        if (pl.a < MB_MAX_A && fits(pl.a + 1, pl.b, pl.raw)) { ++pl.a; grown = true; }
+    }
+    pl.smem = (size_t)pl.a * MB_A_BYTES + (size_t)pl.b * b_bytes + (size_t)pl.raw * raw_bytes + 1024;      // (the partial sums, 28 KB at most, meet in it)
+    return pl;
+}
+
+static cudaLaunchConfig_t mb_config(dim3 grid, dim3 block, int cluster, size_t smem, cudaStream_t stream, cudaLaunchAttribute *attr) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = cluster;
+    attr[1].val.clusterDim.y = 1;
+    attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = cluster > 1 ? 2 : 1;
+    return cfg;
+}
+
+template <int TYPE, int NCH, bool DUAL>
+static cudaError_t mb_launch(skn_ctx *ctx, int n, const skn_tensor *const *w, const float *x, int M, const mb_args &ar, int64_t tiles, const float *gain,
+                             float eps, const float *silu_u, cudaStream_t stream, bool &covered) {
+    auto kern = skn_matvec_batch_kernel<TYPE, NCH, DUAL>;
+    // per device: CTAs in flight in clusters of 1 .. 8 (0: not asked yet)
+    static std::atomic<int> fits[64][MB_MAX_SPLIT + 1];
+    std::atomic<int> *fit = fits[ctx->device & 63];
+    cudaLaunchAttribute attr[2];
+    cudaError_t e;
+    if (fit[MB_MAX_SPLIT].load(std::memory_order_acquire) == 0) {
+        e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, MB_SMEM_MAX);
+        if (e != cudaSuccess) return e;
+        for (int s = 1; s <= MB_MAX_SPLIT; ++s) {
+            const cudaLaunchConfig_t cfg = mb_config(dim3(s), dim3(MB_THREADS), s, MB_SMEM_MAX, stream, attr);
+            int k = ctx->sm_count;
+            if (s > 1 && (e = cudaOccupancyMaxActiveClusters(&k, kern, &cfg)) != cudaSuccess) return e;
+            fit[s].store(k > 0 ? k * s : -1, std::memory_order_release);
+        }
+    }
+    int f[MB_MAX_SPLIT + 1] = {0};
+    for (int s = 1; s <= MB_MAX_SPLIT; ++s) f[s] = fit[s].load(std::memory_order_acquire);
+    const int K = (int)w[0]->n_cols, rows_pad = NCH * MB_CHUNK;
+    const mb_plan pl = mb_make_plan(TYPE, NCH, tiles, K, f);
+    const size_t planes = (size_t)NCH * MB_COLS * K * 2;           // a multiple of 1024
+    if (skn_stage_reserve(ctx, &ctx->d_xq, &ctx->d_xq_bytes, planes + (size_t)(K / 256) * rows_pad * MB_META) != SKN_OK) return cudaErrorMemoryAllocation;
+    __half *xp = (__half *)ctx->d_xq;
+    mb_meta *meta = reinterpret_cast<mb_meta *>((uint8_t *)ctx->d_xq + planes);
+    CUtensorMap tx, tw[3];
+    if ((e = skn_tmap_bf16(xp, NCH * MB_COLS, K, (int64_t)K * 2, NCH * MB_COLS, &tx)) != cudaSuccess) return e;   // 16-bit elements, whatever they are
+    for (int t = 0; t < 3; ++t)
+        if ((e = skn_tmap_blocks(w[t < n ? t : 0], MbFmt<TYPE>::ROW, DUAL ? 16 : MB_ROWS, &tw[t])) != cudaSuccess) return e;
+    covered = true;
+    const int warps = K / 256 < 32 ? K / 256 : 32;
+    const cudaLaunchConfig_t prep = mb_config(dim3((unsigned)M), dim3((unsigned)warps * 32), 1, 0, stream, attr);
+    if ((e = cudaLaunchKernelEx(&prep, skn_xsplit_kernel, x, K, gain, eps, silu_u, xp, meta, rows_pad)) != cudaSuccess) return e;
+    const cudaLaunchConfig_t cfg = mb_config(dim3((unsigned)(tiles * pl.split)), dim3(MB_THREADS), pl.split, pl.smem, stream, attr);
+    return cudaLaunchKernelEx(&cfg, kern, tx, tw[0], tw[1], tw[2], ar, K, pl, (const mb_meta *)meta, ctx->d_status);
+}
+
+// most rows of a launch: what the shared memory holds beside two raw columns (Q8_0: 35 KB each) and three weight stages
+int skn_batch_rows(int32_t type) { return type == SKN_TYPE_Q8_0 ? 24 : 32; }
+
+// whether skn_batch_try_group takes these tensors
+bool skn_batch_covers(int n, const skn_tensor *const *w) {
+    const skn_tensor *w0 = w[0];
+    if (w0->type != SKN_TYPE_Q4_K && w0->type != SKN_TYPE_Q4_0 && w0->type != SKN_TYPE_Q8_0) return false;
+    if (n < 1 || n > 3 || w0->n_cols % 256 || w0->n_cols < 256 || w0->n_cols > (1 << 18) || w0->pitch % 16) return false;
+    for (int t = 0; t < n; ++t)
+        if (w[t]->type != w0->type || w[t]->n_cols != w0->n_cols || w[t]->pitch != w0->pitch || w[t]->n_rows < 1 || w[t]->n_rows > (1 << 28)) return false;
+    return true;
+}
+
+template <int TYPE, bool DUAL, class... A>
+static cudaError_t mb_by_rows(int M, A &&...a) {
+    switch ((M + MB_CHUNK - 1) / MB_CHUNK) {
+    case 1: return mb_launch<TYPE, 1, DUAL>(a...);
+    case 2: return mb_launch<TYPE, 2, DUAL>(a...);
+    case 3: return mb_launch<TYPE, 3, DUAL>(a...);
+    default: return mb_launch<TYPE, 4, DUAL>(a...);
+    }
+}
+template <bool DUAL, class... A>
+static cudaError_t mb_by_type(int type, int M, A &&...a) {
+    switch (type) {
+    case SKN_TYPE_Q4_K: return mb_by_rows<SKN_TYPE_Q4_K, DUAL>(M, a...);
+    case SKN_TYPE_Q4_0: return mb_by_rows<SKN_TYPE_Q4_0, DUAL>(M, a...);
+    default: return mb_by_rows<SKN_TYPE_Q8_0, DUAL>(M, a...);
+    }
+}
+
+// Y[t][m] = W[t] . f(x[m]) (+ add[t]) for n <= 3 tensors of one type, K and pitch and 1 <= M <= skn_batch_rows() activation rows;
+// arguments as of skn_rows_try_group.  Returns false when the tensors are not covered (nothing launched).
+bool skn_batch_try_group(skn_ctx *ctx, int n, const skn_tensor *const *w, const float *x, int M, float *const *y, const float *const *add,
+                         bool add_per_act, const float *norm_gain, float norm_eps, const float *silu_u, bool swiglu, cudaStream_t stream,
+                         cudaError_t &err) {
+    err = cudaSuccess;
+    if (M < 1 || M > skn_batch_rows(w[0]->type) || !skn_batch_covers(n, w)) return false;
+    if (swiglu && (n != 2 || w[0]->n_rows != w[1]->n_rows)) return false;
+    mb_args ar = {};
+    ar.count = n;
+    ar.n_act = M;
+    int64_t tiles = 0;
+    for (int t = 0; t < n; ++t) {
+        ar.tcum[t] = (int)tiles;
+        if (!swiglu) tiles += (w[t]->n_rows + MB_ROWS - 1) / MB_ROWS;
+        ar.n_rows[t] = w[t]->n_rows;
+        ar.y[t] = y[t];
+        ar.add[t] = add ? add[t] : nullptr;
+        ar.addstride[t] = add_per_act ? w[t]->n_rows : 0;
+    }
+    for (int t = n; t < 4; ++t) ar.tcum[t] = (int)tiles + 1;
+    if (swiglu) tiles = (w[0]->n_rows + MB_ROWS / 2 - 1) / (MB_ROWS / 2);
+    bool covered = false;
+    err = swiglu ? mb_by_type<true>(w[0]->type, M, ctx, n, w, x, M, ar, tiles, norm_gain, norm_eps, silu_u, stream, covered)
+                 : mb_by_type<false>(w[0]->type, M, ctx, n, w, x, M, ar, tiles, norm_gain, norm_eps, silu_u, stream, covered);
+    if (!covered && (err == cudaErrorInvalidValue || err == cudaErrorNotSupported)) {
+        err = cudaSuccess;
+        return false;
+    }
+    return true;
+}

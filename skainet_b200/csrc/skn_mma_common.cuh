@@ -212,16 +212,15 @@ static __device__ __noinline__ mm_outlier_result mm_take_outliers(float i0, floa
 }
 
 // One super-block (256 activations, two float4 per lane: elements 4*lane.. and 128 + 4*lane..)
-// -> four digit planes (byte k of a plane = that digit of activation k), the scale 2^(e-29)
+// -> 30-bit fixed-point integers (mm_fixed_point) or their four digit planes (byte k of a plane = that digit of activation k), the scale 2^(e-29)
 // (NaN when the block holds a NaN or an infinity), the eight 32-element sums (outliers excluded: their whole
 // product, offset terms included, is formed in fp32) and the block's outlier record:
 // ocnt[sbi] = how many (0..4), oval[4 * sbi + i] their values, oidx[sbi] their positions (one byte each).
 // XS16: sixteen 16-element sums instead of the eight 32-element ones.  any_out (may be NULL): set to 1 when the
 // block has outliers.
 template <bool XS16>
-static __device__ __forceinline__ void mm_digitize(const float4 v0, const float4 v1, int sbi, int lane, uint8_t *dig, int PL,
-                                                   float *sgrp, float *xsum, float *oval, uint32_t *oidx, uint8_t *ocnt,
-                                                   int *any_out = nullptr) {
+static __device__ __forceinline__ void mm_fixed_point(const float4 v0, const float4 v1, int sbi, int lane, int (&X)[8], float *sgrp, float *xsum,
+                                                      float *oval, uint32_t *oidx, uint8_t *ocnt, int *any_out) {
     float in[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
     const float mx = fmaxf(fmaxf(fmaxf(fabsf(v0.x), fabsf(v0.y)), fmaxf(fabsf(v0.z), fabsf(v0.w))),
                            fmaxf(fmaxf(fabsf(v1.x), fabsf(v1.y)), fmaxf(fabsf(v1.z), fabsf(v1.w))));
@@ -244,14 +243,25 @@ static __device__ __forceinline__ void mm_digitize(const float4 v0, const float4
         tot = r.tot; n_out = r.n_out; ES = r.ES;
     }
     const float mul = __int_as_float((283 - ES) << 23);           // 2^(29-e)
-    uint32_t D[8];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) D[i] = ((uint32_t)__float2int_rn(in[i] * mul) + 0x80808080u) ^ 0x80808080u;
-    mm_store_planes(D, dig, PL, sbi * 64 + lane);
+    for (int i = 0; i < 8; ++i) X[i] = __float2int_rn(in[i] * mul);
     if (lane == 0) {
         ocnt[sbi] = (uint8_t)n_out;
         sgrp[sbi] = (fabsf(tot) <= 3.4028234e38f && mxb < 0x7F800000u) ? __int_as_float((ES - 29) << 23) : __int_as_float(0x7FC00000);
     }
+}
+
+// ... and their four signed bytes as planes
+template <bool XS16>
+static __device__ __forceinline__ void mm_digitize(const float4 v0, const float4 v1, int sbi, int lane, uint8_t *dig, int PL,
+                                                   float *sgrp, float *xsum, float *oval, uint32_t *oidx, uint8_t *ocnt,
+                                                   int *any_out = nullptr) {
+    int X[8];
+    mm_fixed_point<XS16>(v0, v1, sbi, lane, X, sgrp, xsum, oval, oidx, ocnt, any_out);
+    uint32_t D[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) D[i] = ((uint32_t)X[i] + 0x80808080u) ^ 0x80808080u;
+    mm_store_planes(D, dig, PL, sbi * 64 + lane);
 }
 
 // The weight at column k (0..255) of the super-block at shared address `blk`, dequantised as the format defines

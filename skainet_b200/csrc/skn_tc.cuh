@@ -1,6 +1,7 @@
 // tcgen05 / TMEM / tiled-TMA wrappers shared by the tensor-core kernels (K-major bf16 operand tiles of 64 columns
 // with 128-byte swizzle, fp32 accumulators).
 #pragma once
+#include "skn_internal.cuh"
 #include "skn_ptx.cuh"
 
 #include <cuda.h>
@@ -55,6 +56,57 @@ __device__ __forceinline__ void tc_ld32(uint32_t taddr, uint32_t (&r)[32]) {
         : "memory");
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
+
+// ---- clusters, warp-wide waits, shared-memory windows ------------------------------------------------------------
+__device__ __forceinline__ uint32_t tc_cluster_rank() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ uint32_t tc_mapa(uint32_t addr, uint32_t rank) {
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void tc_cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+}
+// one lane of a warp polls for all of it
+__device__ __forceinline__ bool tc_wait_warp(uint64_t *bar, uint32_t parity, int lane) {
+    bool ok = true;
+    if (lane == 0) ok = skn_mbar_wait(bar, parity);
+    return __shfl_sync(0xffffffffu, (int)ok, 0) != 0;
+}
+__device__ __forceinline__ uint4 tc_lds128(uint32_t addr) {
+    uint4 v;
+    asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr));
+    return v;
+}
+
+// words of a byte run that starts `sel` words and sh bits (0 or 16) into an aligned window (sel: the same for the warp)
+template <int SEL, int N, int W>
+__device__ __forceinline__ void tc_cut(const uint32_t (&win)[W], uint32_t sh, uint32_t (&out)[N]) {
+#pragma unroll
+    for (int i = 0; i < N; ++i) out[i] = __funnelshift_rc(win[i + SEL], (i + SEL + 1 < W) ? win[i + SEL + 1 < W ? i + SEL + 1 : 0] : 0u, sh);
+}
+template <int N, int W>
+__device__ __forceinline__ void tc_shift(const uint32_t (&win)[W], int sel, uint32_t sh, uint32_t (&out)[N]) {
+    switch (sel) {
+    case 0: tc_cut<0>(win, sh, out); break;
+    case 1: tc_cut<1>(win, sh, out); break;
+    case 2: tc_cut<2>(win, sh, out); break;
+    default: tc_cut<3>(win, sh, out); break;
+    }
+}
+template <int N> __device__ __forceinline__ void tc_window(uint32_t addr, uint32_t (&w)[N]) {
+#pragma unroll
+    for (int i = 0; i < N / 4; ++i) {
+        const uint4 v = tc_lds128(addr + 16 * i);
+        w[4 * i] = v.x; w[4 * i + 1] = v.y; w[4 * i + 2] = v.z; w[4 * i + 3] = v.w;
+    }
+}
+
 
 // 2-D tiled TMA load (no multicast) of a box at element coordinates (x = column, y = row); the
 // tensor map's 128-byte swizzle lays the box out exactly as tc_store_chunk does
@@ -123,5 +175,19 @@ static inline cudaError_t skn_tmap_bf16(const void *base, int64_t rows, int64_t 
     const CUresult r = encode(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void *>(base), gdim, gstride, box, estr,
                               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
+}
+
+// Tensor map of a tensor's raw blocks: boxes of `rows` rows x box_bytes bytes, coordinates in 4-byte units
+static inline cudaError_t skn_tmap_blocks(const skn_tensor *w, int box_bytes, int rows, CUtensorMap *out) {
+    skn_encode_tiled_fn encode = nullptr;
+    const cudaError_t e = skn_tmap_encoder(&encode);
+    if (e != cudaSuccess) return e;
+    const cuuint64_t gdim[2] = {(cuuint64_t)((w->row_bytes + 3) / 4), (cuuint64_t)w->n_rows};
+    const cuuint64_t gstride[1] = {(cuuint64_t)w->pitch};
+    const cuuint32_t box[2] = {(cuuint32_t)(box_bytes / 4), (cuuint32_t)rows};
+    const cuuint32_t estr[2] = {1, 1};
+    const CUresult r = encode(out, CU_TENSOR_MAP_DATA_TYPE_UINT32, 2, w->d_blocks, gdim, gstride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                              CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
 }

@@ -1,0 +1,91 @@
+"""Batches of 9 to 63 activation rows (tcgen05 with exact fp16 integers) against the fp64 oracle, at the edges of chunks, tiles,
+launches and parts of K; the tolerance of the single-row kernels."""
+import numpy as np
+import pytest
+
+import skainet_b200 as skn
+from conftest import FP32_TOL, assert_close_dot
+from oracle import oracle
+from skainet_b200 import synth
+from skainet_b200.llama import LlamaConfig, LlamaDecoder
+
+pytestmark = pytest.mark.gpu
+TYPES = [synth.Q4_0, synth.Q8_0, synth.Q4_K]
+
+
+def check(ctx, qt, w, x, N, K, bias=None):
+    t = skn.QuantTensor(ctx, (N, K), qt, w)
+    y = t.matmul_t(x, bias)
+    t.close()
+    ref, absdot = oracle.matmul(qt, w, N, K, x)
+    if bias is not None:
+        ref, absdot = ref + bias.astype(np.float64), absdot + np.abs(bias.astype(np.float64))
+    assert_close_dot(y, ref, absdot, FP32_TOL, f"type {qt} {N}x{K} M={x.shape[0]}")
+
+
+@pytest.mark.parametrize("qt", TYPES)
+@pytest.mark.parametrize("M,N,K", [(9, 1, 256), (16, 127, 512), (17, 130, 768), (24, 128, 2304), (25, 300, 1024), (32, 16, 4096), (33, 257, 256), (63, 40, 1792)])
+def test_batch_edges(ctx, qt, M, N, K):
+    g = synth.rng(M + N + K)
+    check(ctx, qt, synth.make_weight(g, qt, N, K), synth.make_activations(g, M, K), N, K, g.standard_normal(N).astype(np.float32) if M % 2 else None)
+
+
+@pytest.mark.parametrize("qt", TYPES)
+def test_batch_outliers_zeros_and_scales(ctx, qt):
+    """Rows of zeros, of one element, of outliers up to 1e6 in the block, of very different sizes; the towering elements meet zero weights."""
+    g = synth.rng(5)
+    M, N, K = 12, 48, 1024
+    w = synth.make_weight(g, qt, N, K)
+    x = synth.make_activations(g, M, K)
+    x[0] = 0
+    x[1] = 0
+    x[1, 700] = 3.5
+    for m, size in ((2, 1e3), (3, 1e4), (4, 1e6)):
+        x[m, 5::256] *= size
+        x[m, 130::256] *= -size
+    x[5] *= 1e-20
+    x[6] *= 1e20
+    check(ctx, qt, w, x, N, K)
+
+
+@pytest.mark.parametrize("qt", TYPES)
+def test_batch_rows_that_are_not_finite_stay_apart(ctx, qt):
+    g = synth.rng(6)
+    M, N, K = 10, 33, 512
+    w, x = synth.make_weight(g, qt, N, K), synth.make_activations(g, M, K)
+    t = skn.QuantTensor(ctx, (N, K), qt, w)
+    clean = t.matmul_t(x)
+    x[3, 17], x[7, 300] = np.inf, np.nan
+    y = t.matmul_t(x)
+    t.close()
+    assert not np.isfinite(y[3]).any() and not np.isfinite(y[7]).any()
+    keep = [m for m in range(M) if m not in (3, 7)]
+    assert np.array_equal(y[keep], clean[keep])
+
+
+@pytest.mark.parametrize("batch", [9, 20, 40])
+def test_decoder_batch_agrees_with_single_sequences(ctx, batch):
+    """Q/K/V grouped, gate / up / SwiGLU interleaved, residuals and folded norms: a batch of sequences against the same
+    sequences one by one (single-row kernels), both in fp32 sums: 1e-5 a product, a few dozen in a row."""
+    g = synth.rng(batch)
+    cfg = LlamaConfig(n_layers=2, d_model=512, n_heads=4, n_kv_heads=2, head_dim=128, ffn_dim=768, vocab=320)
+    shapes = dict(wq=(512, 512), wk=(256, 512), wv=(256, 512), wo=(512, 512), w_gate=(768, 512), w_up=(768, 512), w_down=(512, 768))
+    layers = [{n: synth.make_weight(g, synth.Q4_K, *s) for n, s in shapes.items()} for _ in range(2)]
+    embed, head = (synth.make_weight(g, synth.Q6_K, 320, 512) for _ in range(2))
+    gain = np.ones(512, dtype=np.float32)
+    tokens = g.integers(0, 320, size=(batch, 3)).astype(np.int32)
+
+    def logits(rows):
+        m = LlamaDecoder(ctx, cfg, batch=len(rows), max_tokens=1, max_ctx=8)
+        for i, l in enumerate(layers):
+            m.set_layer(i, l, gain, gain)
+        m.set_head(embed, gain, head)
+        out = np.stack([m.forward(np.ascontiguousarray(rows[:, i:i + 1]), want_logits=True)[1] for i in range(rows.shape[1])])
+        m.close()
+        return out.astype(np.float64)
+
+    many = logits(tokens)
+    assert np.isfinite(many).all()
+    for b in (0, 8, batch - 1):
+        one = logits(tokens[b:b + 1])[:, 0]
+        assert np.linalg.norm(many[:, b] - one) <= 1e-3 * np.linalg.norm(one)
