@@ -22,6 +22,7 @@
 // Measured (B200, graph of distinct weights, us per call with the preparation of x, before -> now):
 //   Q4_K 14336 x 4096: 8 rows 34 -> 31, 16 rows 69 -> 29, 32 rows 137 -> 37; 28672 x 4096: 16 rows 110 -> 57; 4096 x 4096: 22 -> 13.4
 //   Q4_0 4096 x 14336: 16 rows 75 -> 41, 60 rows 299 -> 116; Q8_0 14336 x 4096: 16 rows 73 -> 50
+//   Q6_K 32000 x 4096: 16 rows 236 -> 123; 4096 x 14336: 191 -> 57 (they ran four rows a launch)
 // Bound now: 600 clocks per 64 columns of 128 rows in the hand-overs between unpacking, issuing and draining warps (the products and the
 // arithmetic of each take less than half of that), and about 10 us a call of preparation, start and exchange.
 #include "skn_mma_common.cuh"
@@ -29,7 +30,7 @@
 
 #include <atomic>
 
-constexpr int MB_ROWS = 128, MB_BK = 128;          // a stage: two 128-byte wide operand tiles of 64 columns (one tile per
+constexpr int MB_ROWS = 128;                       // a stage: two 128-byte wide operand tiles of 64 columns (one tile per
                                                   // stage left the issuing thread with 680 clocks of waits and commits per 64 columns)
 constexpr int MB_A_TILE = MB_ROWS * 128, MB_A_BYTES = 2 * MB_A_TILE;
 constexpr int MB_THREADS = 24 * 32;
@@ -116,9 +117,12 @@ skn_xsplit_kernel(const float *__restrict__ x, int K, const float *__restrict__ 
 
 // ---- raw blocks -> fp16 integers --------------------------------------------------------------------------------------
 template <int TYPE> struct MbFmt;
-template <> struct MbFmt<SKN_TYPE_Q4_K> { static constexpr int ROW = 144, MM = MM_FMT_Q4K, BLOCKS = 1; };
-template <> struct MbFmt<SKN_TYPE_Q4_0> { static constexpr int ROW = 144, MM = MM_FMT_Q40, BLOCKS = 8; };
-template <> struct MbFmt<SKN_TYPE_Q8_0> { static constexpr int ROW = 272, MM = MM_FMT_Q80, BLOCKS = 8; };
+template <> struct MbFmt<SKN_TYPE_Q4_K> { static constexpr int ROW = 144, MM = MM_FMT_Q4K, BLOCKS = 1, STAGES = 2; };
+template <> struct MbFmt<SKN_TYPE_Q4_0> { static constexpr int ROW = 144, MM = MM_FMT_Q40, BLOCKS = 8, STAGES = 2; };
+template <> struct MbFmt<SKN_TYPE_Q8_0> { static constexpr int ROW = 272, MM = MM_FMT_Q80, BLOCKS = 8, STAGES = 2; };
+// Q6_K: quant times 8-bit scale needs 12 bits.  The scale is taken as 2 h + b, b = 0 or 1: a stage is 64 columns in two weight
+// tiles, (q - 32) h and (q - 32) b, against one tile of digits, into two accumulators
+template <> struct MbFmt<SKN_TYPE_Q6_K> { static constexpr int ROW = 240, MM = MM_FMT_Q6K, BLOCKS = 1, STAGES = 4; };
 
 // four bytes b of w -> fp16 (b + 1024) * mul + add: 1024 + b is the byte under the high byte 0x64; all values here are exact
 __device__ __forceinline__ void mb_quad(uint32_t w, __half2 mul, __half2 add, uint32_t *out) {
@@ -131,7 +135,7 @@ __device__ __forceinline__ void mb_quad(uint32_t w, __half2 mul, __half2 add, ui
 }
 // half g of stage u of the row at `row` (see the formats' notes in skn_matmul_tc.cu: same cut, same chunks)
 template <int TYPE>
-__device__ __forceinline__ void mb_half(uint32_t row, int u, int g, uint32_t sc2, uint32_t (&out)[16]) {
+__device__ __forceinline__ void mb_half(uint32_t row, int u, int g, uint32_t sc2, uint32_t (&out)[16], int lead = 0, int v = 0) {
     if constexpr (TYPE == SKN_TYPE_Q4_K) {
         const uint4 q = tc_lds128(row + 16 + 32 * u + 16 * g);
         const uint32_t qw[4] = {q.x, q.y, q.z, q.w};
@@ -152,6 +156,26 @@ __device__ __forceinline__ void mb_half(uint32_t row, int u, int g, uint32_t sc2
             const uint32_t q = __funnelshift_r(w[i], w[i + 1], 16);
             mb_quad(q & 0x0F0F0F0Fu, one, add, out + 2 * i);
             mb_quad((q >> 4) & 0x0F0F0F0Fu, one, add, out + 8 + 2 * i);
+        }
+    } else if constexpr (TYPE == SKN_TYPE_Q6_K) {
+        const uint32_t sh = (uint32_t)(lead & 2) * 8u;
+        uint32_t wl[12], wh[12], ql[8], qh[8], s8;
+        tc_window(row + 64 * (u >> 1) + 32 * g, wl);
+        tc_window(row + 128 + 32 * (u >> 1), wh);
+        tc_shift(wl, lead >> 2, sh, ql);
+        tc_shift(wh, lead >> 2, sh, qh);
+        asm volatile("ld.shared.u16 %0, [%1];" : "=r"(s8) : "r"(row + (uint32_t)lead + 192 + 8 * (u >> 1) + 4 * (u & 1) + 2 * g));   // two int8 scales
+        const int i0 = (int)(int8_t)(s8 & 0xFFu), i1 = (int)(int8_t)(s8 >> 8);
+        const __half2 s0 = __half2half2(__int2half_rn(v ? i0 & 1 : i0 >> 1)), s1 = __half2half2(__int2half_rn(v ? i1 & 1 : i1 >> 1));
+        const int lsh = 4 * (u & 1), hsh = 4 * (u & 1) + 2 * g;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            mb_quad(((ql[i] >> lsh) & 0x0F0F0F0Fu) | (((qh[i] >> hsh) & 0x03030303u) << 4), __float2half2_rn(1.f), __float2half2_rn(-1056.f), out + 2 * i);
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const __half2 w = __hmul2(*reinterpret_cast<const __half2 *>(&out[2 * i + e]), i < 4 ? s0 : s1);
+                out[2 * i + e] = *reinterpret_cast<const uint32_t *>(&w);
+            }
         }
     } else {
         uint32_t win[12], w[9];
@@ -194,7 +218,7 @@ skn_matvec_batch_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_c
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     constexpr int ROW = MbFmt<TYPE>::ROW, RAW_BYTES = MB_ROWS * ROW, BLOCKS = MbFmt<TYPE>::BLOCKS;
-    constexpr int NCOL = NCH * MB_COLS, SET_COLS = BLOCKS == 1 ? NCOL : 2 * NCOL, B_TILE = NCOL * 128, B_BYTES = 2 * B_TILE, META_BYTES = NCH * MB_CHUNK * MB_META;
+    constexpr int NCOL = NCH * MB_COLS, SET_COLS = TYPE == SKN_TYPE_Q4_K ? NCOL : 2 * NCOL, B_TILE = NCOL * 128, STAGES = MbFmt<TYPE>::STAGES, B_TILES = 4 / STAGES, B_BYTES = B_TILES * B_TILE, META_BYTES = NCH * MB_CHUNK * MB_META;
     __shared__ uint64_t a_full[MB_MAX_A], a_empty[MB_MAX_A], b_full[MB_MAX_B], b_empty[MB_MAX_B], raw_full[MB_MAX_RAW], meta_full[MB_MAX_RAW],
         raw_empty[MB_MAX_RAW], d_full[MB_MAX_D], d_empty[MB_MAX_D];
     __shared__ uint32_t tmem_slot;
@@ -204,7 +228,7 @@ skn_matvec_batch_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_c
     const int na = pl.a, nb = pl.b, nraw = pl.raw, nd = pl.d;
     uint8_t *b_ring = smem + (size_t)na * MB_A_BYTES, *raw_ring = b_ring + (size_t)nb * B_BYTES, *meta_ring = raw_ring + (size_t)nraw * RAW_BYTES;
     float *slots = reinterpret_cast<float *>(smem);                // over the rings, once all CTAs of the cluster are done with them
-    const int nsb = K / 256, sb0 = kr * nsb / c, sb1 = (kr + 1) * nsb / c, steps = 2 * (sb1 - sb0);
+    const int nsb = K / 256, sb0 = kr * nsb / c, sb1 = (kr + 1) * nsb / c, steps = STAGES * (sb1 - sb0);
     // the tile's tensor and first row
     int t = 0;
     if (!DUAL) t = (tile >= ar.tcum[1] ? 1 : 0) + (ar.count > 2 && tile >= ar.tcum[2] ? 1 : 0);
@@ -229,7 +253,7 @@ skn_matvec_batch_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_c
     auto load_raw = [&](int sb, int rs) {
         uint8_t *dst = raw_ring + (size_t)rs * RAW_BYTES;
         skn_mbar_expect_tx(&raw_full[rs], RAW_BYTES);
-        const int x = sb * (ROW / 4);
+        const int x = TYPE == SKN_TYPE_Q6_K ? ((sb * 210) >> 4) * 4 : sb * (ROW / 4);
         if (DUAL) {
             for (int i = 0; i < 4; ++i) {
                 tc_tma_load_2d(dst + 32 * i * ROW, &tm_w0, x, n0 + 16 * i, &raw_full[rs]);
@@ -272,20 +296,22 @@ skn_matvec_batch_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_c
         int s = turn % na, rs = 0, it = turn;
         uint32_t ph = (uint32_t)(turn / na), rph = 0;
 #pragma unroll 1
-        for (int sb = 0; sb < steps / 2; ++sb) {           // (every group sees every super-block, with a stage of its own in it or not)
+        for (int sb = 0; sb < steps / STAGES; ++sb) {           // (every group sees every super-block, with a stage of its own in it or not)
             if (!failed && !tc_wait_warp(&raw_full[rs], rph, lane)) give_up();
-            if (it >> 1 == sb) {
-                const uint32_t row = raw0 + (uint32_t)(rs * RAW_BYTES);
+            const uint32_t row = raw0 + (uint32_t)(rs * RAW_BYTES);
+            const int lead = TYPE == SKN_TYPE_Q6_K ? ((sb0 + sb) * 210) & 15 : 0;
+#pragma unroll 1
+            for (; it / STAGES == sb; it += MB_DQ_GROUPS) {
                 uint32_t sc[2] = {0, 0}, mn[2];
                 if (TYPE == SKN_TYPE_Q4_K) mb_q4k_scales(tc_lds128(row), sc, mn);
                 const uint32_t sc4 = sc[it & 1];           // scales of the stage's four sub-blocks
 #pragma unroll 1
-                for (int v = 0; v < 2; ++v) {              // the stage's tiles of 64 columns
+                for (int v = 0; v < 2; ++v) {              // the stage's two tiles
                     uint8_t *tile_a = smem + (size_t)s * MB_A_BYTES + v * MB_A_TILE;
 #pragma unroll
                     for (int g = 0; g < 2; ++g) {
                         uint32_t p[16];
-                        mb_half<TYPE>(row, 2 * (it & 1) + v, g, (sc4 >> (16 * v)) & 0xFFFFu, p);
+                        mb_half<TYPE>(row, STAGES == 4 ? it & 3 : 2 * (it & 1) + v, g, (sc4 >> (16 * v)) & 0xFFFFu, p, lead, v);
                         if (v == 0 && g == 0 && !failed && !tc_wait_warp(&a_empty[s], ph ^ 1u, lane)) give_up();
 #pragma unroll
                         for (int i = 0; i < 4; ++i) {
@@ -298,7 +324,6 @@ skn_matvec_batch_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_c
                 __syncwarp();
                 if (lane == 0) skn_mbar_arrive(&a_full[s]);
                 for (s += MB_DQ_GROUPS; s >= na; s -= na) ph ^= 1u;
-                it += MB_DQ_GROUPS;
             }
             __syncwarp();
             if (lane == 0) skn_mbar_arrive(&raw_empty[rs]);
@@ -327,8 +352,8 @@ skn_matvec_batch_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_c
             for (int it = 0; it < steps; ++it) {
                 if (!failed && !skn_mbar_wait(&b_empty[s], ph ^ 1u)) give_up();
                 skn_mbar_expect_tx(&b_full[s], B_BYTES);
-                for (int v = 0; v < 2; ++v)
-                    tc_tma_load_2d(b_ring + (size_t)s * B_BYTES + v * B_TILE, &tm_x, (sb0 * 2 + it) * MB_BK + 64 * v, 0, &b_full[s]);
+                for (int v = 0; v < B_TILES; ++v)
+                    tc_tma_load_2d(b_ring + (size_t)s * B_BYTES + v * B_TILE, &tm_x, (sb0 * STAGES + it) * (64 * B_TILES) + 64 * v, 0, &b_full[s]);
                 if (++s == nb) { s = 0; ph ^= 1u; }
             }
         }
@@ -343,7 +368,18 @@ skn_matvec_batch_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_c
             if (!failed && !skn_mbar_wait(&a_full[s], ph)) failed = true;
             const uint64_t ad = a0 + (uint64_t)(s * (MB_A_BYTES >> 4)), bd = b0 + (uint64_t)(tb * (B_BYTES >> 4));
             // K step k (16 columns): 32 bytes inside a tile's swizzle atom = +2 in the address field
-            if constexpr (BLOCKS == 1) {
+            if constexpr (TYPE == SKN_TYPE_Q6_K) {
+                if ((it & 3) == 0 && !failed && !skn_mbar_wait(&d_empty[d], pd ^ 1u)) failed = true;
+                tc_fence_after();
+                if (tc_elect()) {
+#pragma unroll
+                    for (int k = 0; k < 8; ++k)
+                        tc_mma_bf16(tmem_base + d * SET_COLS + (k >> 2) * NCOL, ad + (k >> 2) * (MB_A_TILE >> 4) + 2 * (k & 3), bd + 2 * (k & 3), idesc,
+                                    ((it & 3) || (k & 3)) ? 1u : 0u);
+                    if ((it & 3) == 3) tc_commit(&d_full[d]);
+                }
+                if ((it & 3) == 3 && ++d == nd) { d = 0; pd ^= 1u; }
+            } else if constexpr (BLOCKS == 1) {
                 if ((it & 1) == 0 && !failed && !skn_mbar_wait(&d_empty[d], pd ^ 1u)) failed = true;
                 tc_fence_after();
                 if (tc_elect()) {
@@ -392,7 +428,34 @@ skn_matvec_batch_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_c
             if (!failed && !tc_wait_warp(&raw_full[rs], rph, lane)) give_up();
             if (!failed && !tc_wait_warp(&meta_full[rs], rph, lane)) give_up();
             const uint32_t row = raw0 + (uint32_t)(rs * RAW_BYTES), mt = meta0 + (uint32_t)(rs * META_BYTES);
-            if constexpr (BLOCKS == 1) {
+            const uint32_t blk = TYPE == SKN_TYPE_Q6_K ? row + (uint32_t)((sb * 210) & 15) : row;
+            if constexpr (TYPE == SKN_TYPE_Q6_K) {
+                const float db = mm_lds_half(blk + 208);
+                if (!failed && !tc_wait_warp(&d_full[d], pd, lane)) give_up();
+                tc_fence_after();
+#pragma unroll
+                for (int i = 0; i < MINE; ++i) {
+                    const int ch = 2 * i + odd;
+                    if (ch >= NCH) break;
+                    const uint32_t at = tmem_base + (uint32_t)(d * SET_COLS + ch * MB_COLS) + ((uint32_t)(wq * 32) << 16);
+                    float hi[MB_CHUNK];
+#pragma unroll
+                    for (int v = 0; v < 2; ++v) {
+                        uint32_t D[32];
+                        tc_ld32(at + (uint32_t)(v * NCOL), D);
+#pragma unroll
+                        for (int a = 0; a < MB_CHUNK; ++a) {
+                            const float t = fmaf(__uint_as_float(D[a]), 4194304.f, fmaf(__uint_as_float(D[8 + a]), 2048.f, __uint_as_float(D[16 + a])));
+                            if (v == 0) hi[a] = t;
+                            else y[i * MB_CHUNK + a] = fmaf(fmaf(hi[a], 2.f, t), db * mm_lds32f(mt + (uint32_t)((ch * MB_CHUNK + a) * MB_META)), y[i * MB_CHUNK + a]);
+                        }
+                    }
+                }
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) skn_mbar_arrive(&d_empty[d]);
+                if (++d == nd) { d = 0; pd ^= 1u; }
+            } else if constexpr (BLOCKS == 1) {
                 const uint4 hdr = tc_lds128(row);
                 const float2 dd = __half22float2(*reinterpret_cast<const __half2 *>(&hdr.x));
                 uint32_t sc[2], mn[2];
@@ -471,7 +534,7 @@ skn_matvec_batch_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_c
                     float add = 0.f;
 #pragma unroll 1
                     for (int i = 0; i < n; ++i)
-                        add = fmaf(mm_weight_at<MbFmt<TYPE>::MM>(row, (int)mm_lds8(m + 8 + (uint32_t)i)), mm_lds32f(m + 16 + 4 * (uint32_t)i), add);
+                        add = fmaf(mm_weight_at<MbFmt<TYPE>::MM>(blk, (int)mm_lds8(m + 8 + (uint32_t)i)), mm_lds32f(m + 16 + 4 * (uint32_t)i), add);
                     y[a] += add;
                 }
             }
@@ -551,19 +614,21 @@ skn_matvec_batch_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_c
 }
 
 // ---- launch --------------------------------------------------------------------------------------------------------
-static int mb_row_bytes(int type) { return type == SKN_TYPE_Q8_0 ? MbFmt<SKN_TYPE_Q8_0>::ROW : MbFmt<SKN_TYPE_Q4_K>::ROW; }
+static int mb_row_bytes(int type) {
+    return type == SKN_TYPE_Q8_0 ? MbFmt<SKN_TYPE_Q8_0>::ROW : (type == SKN_TYPE_Q6_K ? MbFmt<SKN_TYPE_Q6_K>::ROW : MbFmt<SKN_TYPE_Q4_K>::ROW);
+}
 
 // K over as many CTAs of a cluster as make the launch shortest, in SM clocks: a start and end of 9000, MB_STAGE_CLOCKS per 64 columns
 // of 128 rows.  `fit[s]` = CTAs in flight in clusters of s.
 constexpr int MB_STAGE_CLOCKS = 500;
 static mb_plan mb_make_plan(int type, int nch, int64_t tiles, int K, const int *fit) {
     mb_plan pl = {};
-    const int raw_bytes = MB_ROWS * mb_row_bytes(type) + nch * MB_CHUNK * MB_META, b_bytes = nch * MB_COLS * MB_BK * 2, nsb = K / 256;
+    const int raw_bytes = MB_ROWS * mb_row_bytes(type) + nch * MB_CHUNK * MB_META, b_bytes = nch * MB_COLS * (type == SKN_TYPE_Q6_K ? 128 : 256), nsb = K / 256;
     int64_t best = 0;
     for (int c = 1; c <= MB_MAX_SPLIT && c <= nsb; ++c) {
         if (fit[c] < 1 && c > 1) continue;
         const int64_t f = fit[c] > 0 ? fit[c] : 1, waves = (tiles * c + f - 1) / f;
-        const int64_t cost = waves * (9000 + (c > 1 ? 2000 : 0) + (int64_t)((nsb + c - 1) / c) * 4 * MB_STAGE_CLOCKS);
+        const int64_t cost = waves * (9000 + (c > 1 ? 2000 : 0) + (int64_t)((nsb + c - 1) / c) * 4 * MB_STAGE_CLOCKS * (type == SKN_TYPE_Q6_K ? 2 : 1));
         if (best == 0 || cost < best) { best = cost; pl.split = c; }
     }
     pl.d = 512 / (nch * MB_COLS * (type == SKN_TYPE_Q4_K ? 1 : 2));
@@ -644,7 +709,7 @@ int skn_batch_rows(int32_t type) { return type == SKN_TYPE_Q8_0 ? 24 : 32; }
 // whether skn_batch_try_group takes these tensors
 bool skn_batch_covers(int n, const skn_tensor *const *w) {
     const skn_tensor *w0 = w[0];
-    if (w0->type != SKN_TYPE_Q4_K && w0->type != SKN_TYPE_Q4_0 && w0->type != SKN_TYPE_Q8_0) return false;
+    if (w0->type != SKN_TYPE_Q4_K && w0->type != SKN_TYPE_Q4_0 && w0->type != SKN_TYPE_Q8_0 && w0->type != SKN_TYPE_Q6_K) return false;
     if (n < 1 || n > 3 || w0->n_cols % 256 || w0->n_cols < 256 || w0->n_cols > (1 << 18) || w0->pitch % 16) return false;
     for (int t = 0; t < n; ++t)
         if (w[t]->type != w0->type || w[t]->n_cols != w0->n_cols || w[t]->pitch != w0->pitch || w[t]->n_rows < 1 || w[t]->n_rows > (1 << 28)) return false;
@@ -665,6 +730,7 @@ static cudaError_t mb_by_type(int type, int M, A &&...a) {
     switch (type) {
     case SKN_TYPE_Q4_K: return mb_by_rows<SKN_TYPE_Q4_K, DUAL>(M, a...);
     case SKN_TYPE_Q4_0: return mb_by_rows<SKN_TYPE_Q4_0, DUAL>(M, a...);
+    case SKN_TYPE_Q6_K: return mb_by_rows<SKN_TYPE_Q6_K, DUAL>(M, a...);
     default: return mb_by_rows<SKN_TYPE_Q8_0, DUAL>(M, a...);
     }
 }

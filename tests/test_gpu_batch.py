@@ -10,7 +10,7 @@ from skainet_b200 import synth
 from skainet_b200.llama import LlamaConfig, LlamaDecoder
 
 pytestmark = pytest.mark.gpu
-TYPES = [synth.Q4_0, synth.Q8_0, synth.Q4_K]
+TYPES = [synth.Q4_0, synth.Q8_0, synth.Q4_K, synth.Q6_K]
 
 
 def check(ctx, qt, w, x, N, K, bias=None):
