@@ -1,5 +1,6 @@
 // Small element-wise kernels around the matmuls (no counterpart in the reference).
 #include "skn_internal.cuh"
+#include "skn_mma.cuh"
 #include "skn_ptx.cuh"
 
 // h = silu(g) * u, fp32 (the decode-size SwiGLU; the prefill path fuses this into the
@@ -22,11 +23,14 @@ cudaError_t skn_launch_silu_mul(const float *g, const float *u, float *h, int64_
 
 // ---- decoder glue (K8) ---------------------------------------------------------------------
 // y[m][:] = x[m][:] / sqrt(mean(x[m]^2) + eps) * gain[:]; one CTA per row
+// (T = bf16: what the tensor-core products read, without a pass of its own for the conversion)
+template <class T>
 __global__ void __launch_bounds__(256)
-skn_rmsnorm_kernel(const float *__restrict__ x, const float *__restrict__ gain, float *__restrict__ y, int D, float eps) {
+skn_rmsnorm_kernel(const float *__restrict__ x, const float *__restrict__ gain, T *__restrict__ y, int D, float eps) {
     __shared__ float red[8];
     const float *xr = x + (size_t)blockIdx.x * D;
-    float *yr = y + (size_t)blockIdx.x * D;
+    T *yr = y + (size_t)blockIdx.x * D;
+    if (sizeof(T) == 2) skn_pdl_launch_dependents();       // the product's CTAs may come in and unpack their first weights
     float ss = 0.f;
     for (int i = threadIdx.x * 4; i < D; i += blockDim.x * 4) {
         const float4 v = *reinterpret_cast<const float4 *>(xr + i);
@@ -42,7 +46,11 @@ skn_rmsnorm_kernel(const float *__restrict__ x, const float *__restrict__ gain, 
     for (int i = threadIdx.x * 4; i < D; i += blockDim.x * 4) {
         const float4 v = *reinterpret_cast<const float4 *>(xr + i);
         const float4 g = *reinterpret_cast<const float4 *>(gain + i);
-        *reinterpret_cast<float4 *>(yr + i) = make_float4(v.x * r * g.x, v.y * r * g.y, v.z * r * g.z, v.w * r * g.w);
+        const float4 o = make_float4(v.x * r * g.x, v.y * r * g.y, v.z * r * g.z, v.w * r * g.w);
+        if constexpr (sizeof(T) == 2)
+            *reinterpret_cast<uint2 *>(yr + i) = make_uint2(pack_bf16(o.x, o.y), pack_bf16(o.z, o.w));
+        else
+            *reinterpret_cast<float4 *>(yr + i) = o;
     }
 }
 
@@ -150,6 +158,11 @@ static int glue_blocks(int64_t n, int sm_count) {
 cudaError_t skn_launch_rmsnorm(const float *x, const float *gain, float *y, int M, int D, float eps, cudaStream_t st) {
     if (M == 0) return cudaSuccess;
     skn_rmsnorm_kernel<<<M, 256, 0, st>>>(x, gain, y, D, eps);
+    return cudaGetLastError();
+}
+cudaError_t skn_launch_rmsnorm_bf16(const float *x, const float *gain, void *y_bf16, int M, int D, float eps, cudaStream_t st) {
+    if (M == 0) return cudaSuccess;
+    skn_rmsnorm_kernel<<<M, 256, 0, st>>>(x, gain, (__nv_bfloat16 *)y_bf16, D, eps);
     return cudaGetLastError();
 }
 cudaError_t skn_launch_rope(float *x, const int32_t *len, int M, int T, int H, int D, float theta, int sm_count, cudaStream_t st) {

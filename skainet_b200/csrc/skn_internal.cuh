@@ -230,13 +230,15 @@ cudaError_t skn_launch_matvec_group(skn_ctx *ctx, int n, const skn_tensor *const
 bool skn_tc_supported(const skn_tensor *w, int32_t M);
 cudaError_t skn_launch_f32_to_bf16(const float *in, void *out_bf16, int64_t n, int sm_count, cudaStream_t stream);
 cudaError_t skn_launch_matmul_tc(skn_ctx *ctx, const skn_tensor *w, const void *a_bf16, int32_t M, const float *bias,
-                                 float *y, cudaStream_t stream);
+                                 float *y, cudaStream_t stream, const float *resid = nullptr);
 cudaError_t skn_launch_gate_up_tc(skn_ctx *ctx, const skn_tensor *wg, const skn_tensor *wu, const void *a_bf16,
                                   int32_t M, void *h_bf16, cudaStream_t stream);
 cudaError_t skn_launch_silu_mul(const float *g, const float *u, float *h, int64_t n, int sm_count, cudaStream_t stream);
 
 // decoder glue (skn_glue.cu)
 cudaError_t skn_launch_rmsnorm(const float *x, const float *gain, float *y, int M, int D, float eps, cudaStream_t st);
+// the same rows rounded to bf16
+cudaError_t skn_launch_rmsnorm_bf16(const float *x, const float *gain, void *y_bf16, int M, int D, float eps, cudaStream_t st);
 cudaError_t skn_launch_rope(float *x, const int32_t *len, int M, int T, int H, int D, float theta, int sm_count, cudaStream_t st);
 cudaError_t skn_launch_add(const float *a, const float *b, float *out, int64_t n, int sm_count, cudaStream_t st);
 cudaError_t skn_launch_fetch(const float *src, float *dst, int64_t n, cudaStream_t st);

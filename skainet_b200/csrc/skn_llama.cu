@@ -401,7 +401,24 @@ int32_t skn_llama_forward_dev(skn_llama *m, const int32_t *tokens_dev, int32_t T
             }
             continue;
         }
-        if (small) {
+        // prompts whose projections all run on the tensor cores: norms write the bf16 rows that the products read, once for Q/K/V,
+        // and the residual is added where the output and down projections store (18 launches a layer become 12; the same bits)
+        const bool tc = !small && ctx->prefill_min_m > 0 && M >= ctx->prefill_min_m && skn_tc_supported(l.wq, M) && skn_tc_supported(l.wk, M) &&
+                        skn_tc_supported(l.wv, M) && skn_tc_supported(l.wo, M) && skn_tc_supported(l.wg, M) && skn_tc_supported(l.wd, M) &&
+                        l.wu->type == l.wg->type && l.wu->pitch == l.wg->pitch;
+        void *a16 = nullptr, *h16 = nullptr;
+        if (tc) {
+            const size_t ab = ((size_t)M * (d > qd ? d : qd) * 2 + 255) / 256 * 256;
+            if ((rc = skn_stage_reserve(ctx, &ctx->d_scratch, &ctx->d_scratch_bytes, ab + (size_t)M * F * 2))) return rc;
+            a16 = ctx->d_scratch;
+            h16 = (uint8_t *)ctx->d_scratch + ab;
+        }
+        if (tc) {
+            SKN_CUDA(ctx, skn_launch_rmsnorm_bf16(m->x, l.attn_norm, a16, M, d, m->rms_eps, st));
+            SKN_CUDA(ctx, skn_launch_matmul_tc(ctx, l.wq, a16, M, nullptr, m->q, st));
+            SKN_CUDA(ctx, skn_launch_matmul_tc(ctx, l.wk, a16, M, nullptr, m->k, st));
+            SKN_CUDA(ctx, skn_launch_matmul_tc(ctx, l.wv, a16, M, nullptr, m->v, st));
+        } else if (small) {
             // decode-size batches, per activation row: RMSNorm folded into the preparation of x
             // for Q/K/V (one launch) ...
             bool fb = false;
@@ -485,6 +502,14 @@ int32_t skn_llama_forward_dev(skn_llama *m, const int32_t *tokens_dev, int32_t T
                     }
                 }
             }
+            if (tp && (rc = skn_allreduce_dev(m->comm, m->proj, m->x, m->x, (int64_t)M * d))) return rc;
+        } else if (tc) {
+            SKN_CUDA(ctx, skn_launch_f32_to_bf16(m->att, a16, (int64_t)M * qd, ctx->sm_count, st));
+            SKN_CUDA(ctx, skn_launch_matmul_tc(ctx, l.wo, a16, M, nullptr, tp ? m->proj : m->x, st, tp ? nullptr : m->x));
+            if (tp && (rc = skn_allreduce_dev(m->comm, m->proj, m->x, m->x, (int64_t)M * d))) return rc;
+            SKN_CUDA(ctx, skn_launch_rmsnorm_bf16(m->x, l.ffn_norm, a16, M, d, m->rms_eps, st));
+            SKN_CUDA(ctx, skn_launch_gate_up_tc(ctx, l.wg, l.wu, a16, M, h16, st));
+            SKN_CUDA(ctx, skn_launch_matmul_tc(ctx, l.wd, h16, M, nullptr, tp ? m->proj : m->x, st, tp ? nullptr : m->x));
             if (tp && (rc = skn_allreduce_dev(m->comm, m->proj, m->x, m->x, (int64_t)M * d))) return rc;
         } else {
             if ((rc = skn_matmul_dev(ctx, l.wo, m->att, M, qd, nullptr, m->proj))) return rc;

@@ -215,9 +215,10 @@ struct tc_plan {
     size_t smem;
 };
 
-// what the kernel computes: out_f32[m][n] = acc (+ bias[n]), or (DUAL) out_bf16[m][n] = silu(gate) * up
+// what the kernel computes: out_f32[m][n] = acc (+ resid[m][n]) (+ bias[n]), or (DUAL) out_bf16[m][n] = silu(gate) * up
 struct tc_out {
     const float *bias;
+    const float *resid;     // added to the product, laid out like f32 and possibly the same memory
     float *f32;
     __nv_bfloat16 *bf16;
     int64_t ld;
@@ -481,6 +482,12 @@ skn_matmul_tc_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_cons
                 if (f < N) {
                     const float bias = out.bias ? __ldg(out.bias + f) : 0.f;
                     float *dst = out.f32 + (int64_t)m * out.ld + f;
+                    if (out.resid) {                           // (all loads before the first store)
+                        const float *res = out.resid + (int64_t)m * out.ld + f;
+#pragma unroll
+                        for (int i = 0; i < TC_BLOCK; ++i)
+                            if (m + i < M) acc[i] = __float_as_uint(__uint_as_float(acc[i]) + res[(int64_t)i * out.ld]);
+                    }
 #pragma unroll
                     for (int i = 0; i < TC_BLOCK; ++i)
                         if (m + i < M) dst[(int64_t)i * out.ld] = __uint_as_float(acc[i]) + bias;
@@ -632,16 +639,16 @@ cudaError_t skn_launch_f32_to_bf16(const float *in, void *out_bf16, int64_t n, i
     return cudaGetLastError();
 }
 
-// Y = A_bf16 . W^T (+bias), fp32 out
+// Y = A_bf16 . W^T (+bias) (+resid), fp32 out
 cudaError_t skn_launch_matmul_tc(skn_ctx *ctx, const skn_tensor *w, const void *a_bf16, int32_t M, const float *bias,
-                                 float *y, cudaStream_t stream) {
+                                 float *y, cudaStream_t stream, const float *resid) {
     return dispatch_tc<false>((const __nv_bfloat16 *)a_bf16, M, (int)w->n_cols, w, nullptr,
-                              tc_out{bias, y, nullptr, w->n_rows}, ctx->d_status, stream);
+                              tc_out{bias, resid, y, nullptr, w->n_rows}, ctx->d_status, stream);
 }
 
 // H_bf16 = silu(A . Wg^T) * (A . Wu^T)
 cudaError_t skn_launch_gate_up_tc(skn_ctx *ctx, const skn_tensor *wg, const skn_tensor *wu, const void *a_bf16,
                                   int32_t M, void *h_bf16, cudaStream_t stream) {
     return dispatch_tc<true>((const __nv_bfloat16 *)a_bf16, M, (int)wg->n_cols, wg, wu,
-                             tc_out{nullptr, nullptr, (__nv_bfloat16 *)h_bf16, wg->n_rows}, ctx->d_status, stream);
+                             tc_out{nullptr, nullptr, nullptr, (__nv_bfloat16 *)h_bf16, wg->n_rows}, ctx->d_status, stream);
 }
