@@ -1,4 +1,4 @@
-// K2 for small batches (3 to 16 activation rows in ONE launch): Y[M, N] = X[M, K] . W_q[N, K]^T with the weights
+// K2 for small batches (3 to 8 rows, and 9 to 16 where skn_matvec_batch.cu does not take the tensors, in ONE launch): Y[M, N] = X[M, K] . W_q[N, K]^T with the weights
 // streamed from HBM exactly once.  Same arithmetic as skn_matvec_mma.cu -- exact integer dot products of 32-weight
 // sub-blocks with the digit planes of the activations on the tensor cores (mma.sync m16n8k32, one MMA serves two
 // activation rows), integer sub-block scales, fp32 across super-blocks -- but organised for many rows:
