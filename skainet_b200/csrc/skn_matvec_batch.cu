@@ -197,6 +197,16 @@ __device__ __forceinline__ float mb_byte(uint32_t w, int i) {       // byte i as
     return __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7440 + i)) - 8388608.f;
 }
 
+// The outliers of the record at m times their dequantised weights of the block at `blk`.  Rare and out of line: inlined for every
+// row of x it made the kernels' code a tenth larger; times are the same.
+template <int MM>
+static __device__ __noinline__ float mb_outliers(uint32_t blk, uint32_t m, int n) {
+    float sum = 0.f;
+#pragma unroll 1
+    for (int i = 0; i < n; ++i) sum = fmaf(mm_weight_at<MM>(blk, (int)mm_lds8(m + 8 + (uint32_t)i)), mm_lds32f(m + 16 + 4 * (uint32_t)i), sum);
+    return sum;
+}
+
 struct mb_args {
     int count, n_act;
     int tcum[4];                                  // tiles before tensor t
@@ -531,11 +541,7 @@ skn_matvec_batch_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_c
                     const int act = MB_CHUNK * (2 * (a / MB_CHUNK) + odd) + a % MB_CHUNK;
                     const uint32_t m = mt + (uint32_t)(act * MB_META);
                     const int n = act < ar.n_act ? (int)(mm_lds32(m + 4) & 0xFFu) : 0;
-                    float add = 0.f;
-#pragma unroll 1
-                    for (int i = 0; i < n; ++i)
-                        add = fmaf(mm_weight_at<MbFmt<TYPE>::MM>(blk, (int)mm_lds8(m + 8 + (uint32_t)i)), mm_lds32f(m + 16 + 4 * (uint32_t)i), add);
-                    y[a] += add;
+                    if (n > 0) y[a] += mb_outliers<MbFmt<TYPE>::MM>(blk, m, n);
                 }
             }
             __syncwarp();
