@@ -980,7 +980,8 @@ skn_dense_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
                 }
         }
     } else if (warp == DTC_MMA) {
-        // the whole warp follows the barriers, one elected lane issues
+        // The whole warp follows the barriers, one elected lane issues.  One lane polls for all of them: were each to give up by its own
+        // clock, some could leave the loop while the others stand in elect.sync for good.
         uint32_t idesc = tc_idesc(DTC_BM, NT);
         bool ok = true;
         int s = 0, tile = 0;
@@ -990,14 +991,14 @@ skn_dense_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
             const int kb = (int)((int64_t)ksteps * sp / splits), ke = (int)((int64_t)ksteps * (sp + 1) / splits);
             const int b = tile & 1;
             if (GROUPS) idesc = tc_idesc(DTC_BM, max(16, (tile_of(u).cols + 15) / 16 * 16));
-            if (!skn_mbar_wait(&acc_empty[b], ((uint32_t)(tile >> 1) & 1u) ^ 1u)) {
+            if (!tc_wait_warp(&acc_empty[b], ((uint32_t)(tile >> 1) & 1u) ^ 1u, lane)) {
                 if (lane == 0) atomicExch(status, SKN_ERR_TIMEOUT);
                 break;
             }
             tc_fence_after();
             const uint32_t d = tmem + (uint32_t)(b * acc_cols);
             for (int k = kb; k < ke; ++k) {
-                if (!skn_mbar_wait(&full_bar[s], ph)) {
+                if (!tc_wait_warp(&full_bar[s], ph, lane)) {
                     if (lane == 0) atomicExch(status, SKN_ERR_TIMEOUT);
                     ok = false;
                     break;
