@@ -980,8 +980,8 @@ skn_dense_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
                 }
         }
     } else if (warp == DTC_MMA) {
-        // The whole warp follows the barriers, one elected lane issues.  One lane polls for all of them: were each to give up by its own
-        // clock, some could leave the loop while the others stand in elect.sync for good.
+        // The whole warp follows the barriers, one elected lane issues.  The lanes get one answer from every wait: were each to give up
+        // by its own clock, some could leave the loop while the others stand in elect.sync for good.
         uint32_t idesc = tc_idesc(DTC_BM, NT);
         bool ok = true;
         int s = 0, tile = 0;
@@ -1023,7 +1023,7 @@ skn_dense_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
             const dtc_tile tl = tile_of(u);
             const int m0 = tl.m0, sp = tl.sp, nti = u / mt / splits, n0 = tl.n0;
             const int b = tile & 1;
-            if (ok && !skn_mbar_wait(&acc_full[b], (uint32_t)(tile >> 1) & 1u)) {
+            if (ok && !tc_wait_warp(&acc_full[b], (uint32_t)(tile >> 1) & 1u, lane)) {
                 if (lane == 0) atomicExch(status, SKN_ERR_TIMEOUT);
                 ok = false;
             }

@@ -369,17 +369,18 @@ skn_matvec_batch_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_c
         }
     } else if (warp == MB_MMA) {
         // ---------------- MMAs: 128 rows x NCOL columns, fp16 operands, one accumulator per scale block ----------------
+        // (a wait has one answer for the warp: its lanes elect, and fail, together)
         constexpr uint32_t idesc = (1u << 4) | ((uint32_t)(NCOL >> 3) << 17) | ((uint32_t)(MB_ROWS >> 4) << 24);
         const uint64_t a0 = tc_smem_desc(skn_smem_u32(smem)), b0 = tc_smem_desc(skn_smem_u32(b_ring));
         int s = 0, tb = 0, d = 0;
         uint32_t ph = 0, pb = 0, pd = 0;
         for (int it = 0; it < steps; ++it) {
-            if (!failed && !skn_mbar_wait(&b_full[tb], pb)) failed = true;
-            if (!failed && !skn_mbar_wait(&a_full[s], ph)) failed = true;
+            if (!failed && !tc_wait_warp(&b_full[tb], pb, lane)) failed = true;
+            if (!failed && !tc_wait_warp(&a_full[s], ph, lane)) failed = true;
             const uint64_t ad = a0 + (uint64_t)(s * (MB_A_BYTES >> 4)), bd = b0 + (uint64_t)(tb * (B_BYTES >> 4));
             // K step k (16 columns): 32 bytes inside a tile's swizzle atom = +2 in the address field
             if constexpr (TYPE == SKN_TYPE_Q6_K) {
-                if ((it & 3) == 0 && !failed && !skn_mbar_wait(&d_empty[d], pd ^ 1u)) failed = true;
+                if ((it & 3) == 0 && !failed && !tc_wait_warp(&d_empty[d], pd ^ 1u, lane)) failed = true;
                 tc_fence_after();
                 if (tc_elect()) {
 #pragma unroll
@@ -390,7 +391,7 @@ skn_matvec_batch_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_c
                 }
                 if ((it & 3) == 3 && ++d == nd) { d = 0; pd ^= 1u; }
             } else if constexpr (BLOCKS == 1) {
-                if ((it & 1) == 0 && !failed && !skn_mbar_wait(&d_empty[d], pd ^ 1u)) failed = true;
+                if ((it & 1) == 0 && !failed && !tc_wait_warp(&d_empty[d], pd ^ 1u, lane)) failed = true;
                 tc_fence_after();
                 if (tc_elect()) {
 #pragma unroll
@@ -404,7 +405,7 @@ skn_matvec_batch_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_c
                 // two blocks of 32 columns per tile, an accumulator each
 #pragma unroll
                 for (int v = 0; v < 2; ++v) {
-                    if (!failed && !skn_mbar_wait(&d_empty[d], pd ^ 1u)) failed = true;
+                    if (!failed && !tc_wait_warp(&d_empty[d], pd ^ 1u, lane)) failed = true;
                     tc_fence_after();
                     if (tc_elect()) {
 #pragma unroll

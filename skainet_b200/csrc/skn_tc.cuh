@@ -72,8 +72,11 @@ __device__ __forceinline__ void tc_cluster_sync() {
     asm volatile("barrier.cluster.arrive.release;" ::: "memory");
     asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
 }
-// one lane of a warp polls for all of it
+// A bounded wait of a whole warp with one answer for all its lanes.  All of them look once; where that does not settle it, one
+// lane polls by its clock and shares the result.  (One lane from the start: a broadcast on every wait, 333 -> 341 us for eight
+// 4096 x 14336 Q4_0 products of 16 rows and 4.49 -> 4.60 ms for a 2048-token Lugasun prompt; this form 288 us and 4.52 ms.)
 __device__ __forceinline__ bool tc_wait_warp(uint64_t *bar, uint32_t parity, int lane) {
+    if (__all_sync(0xffffffffu, skn_mbar_try_wait(bar, parity))) return true;
     bool ok = true;
     if (lane == 0) ok = skn_mbar_wait(bar, parity);
     return __shfl_sync(0xffffffffu, (int)ok, 0) != 0;

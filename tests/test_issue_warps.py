@@ -1,8 +1,8 @@
 """Waits of the warps that issue tcgen05 instructions, read from the kernels' source: nothing here can be tried on a GPU without hanging it.
 
 Such a warp elects a lane with elect.sync, which needs every lane of the warp.  A wait that each lane ends by its own clock lets the
-lanes disagree when a barrier completes around the limit: those that gave up leave, the others stand in elect.sync.  So one lane
-polls and shares the answer (tc_wait_warp), in every role that elects."""
+lanes disagree when a barrier completes around the limit: those that gave up leave, the others stand in elect.sync.  So a wait
+has one answer for the warp (tc_wait_warp), in every role that elects."""
 import os
 import re
 
@@ -35,8 +35,8 @@ def roles(text):
     return list(found.values())
 
 
-@pytest.mark.parametrize("name", ["skn_dense.cu"])
-def test_one_lane_polls_for_a_warp_that_elects(name):
+@pytest.mark.parametrize("name", ["skn_dense.cu", "skn_matmul_tc.cu", "skn_matvec_batch.cu"])
+def test_a_warp_that_elects_waits_as_one(name):
     with open(os.path.join(CSRC, name)) as f:
         blocks = roles(f.read())
     assert blocks, "no issuing role found"
