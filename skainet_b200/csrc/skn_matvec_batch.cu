@@ -2,12 +2,16 @@
 // single-row kernels, on the 5th-generation tensor cores.
 //
 // The arithmetic is the one of skn_matvec_mma.cu -- 30-bit fixed-point activations per super-block, integer products,
-// exact sums per scale block, outliers apart in fp32 -- in numbers that tcgen05 takes: a weight's integer (Q4_K: quant
-// times 6-bit sub-block scale, at most 945; Q4_0, Q8_0: the signed quant) is an exact fp16 number, an activation is
-// three exact fp16 digits (X = d0 2^22 + d1 2^11 + d2, |d0| <= 256, |d1|, |d2| <= 1024), and an fp32 accumulator holds
-// sums of such products exactly below 2^24, which those of the leading digit stay under but for contrived blocks (and
-// then lose one part in 2^23).  The scale d of a block multiplies the accumulator when it is drained: once per 256
-// columns for Q4_K, once per 32 for Q4_0 and Q8_0.
+// exact sums per scale block, outliers apart in fp32 -- in numbers that tcgen05 takes: a weight's integer is an exact fp16
+// number (Q4_0, Q8_0: the signed quant; Q4_K: quant times 6-bit sub-block scale less about half its range, s q - 8 (s & 60), at
+// most 480; Q6_K: quant times either part of its scale 16 h + l, at most 256), an activation is four signed byte digits
+// (X = d0 2^24 + d1 2^16 + d2 2^8 + d3, each at most 128) for the K-quants, three of eleven bits (d0 2^22 + d1 2^11 + d2, at most 1024)
+// for the others, and an fp32 accumulator holds the sum of such products exactly while it is at most 2^24: 256 columns of Q4_K stay
+// below 128 x 480 x 256 = 15.8 M whatever the input is, those of Q6_K below 2^23, the 32 of a Q8_0 or Q4_0 block below 2^22.
+// (Before, Q4_K took s q itself, Q6_K the scale as 2 h + b, both three digits: where activations of one sign met large scales the sums
+// passed 2^24 and every further step chopped, products 1.6e-7 and 4.3e-7 too small on the mean.)  What the weights of Q4_K lack,
+// 8 (s & 60) times the sum of x, joins the dmin term, which it nearly cancels: error against 64 bits 2.1e-7 -> 0.8e-7, time 28.2 ->
+// 28.9 us for 14336 x 4096 at 16 rows.  The scale d of a block multiplies what is drained.
 //
 // What bounded the mma.sync form of this (skn_matvec_rows.cu) was the chain load, MMA, integer multiply-add per 16 rows x
 // 32 columns of eight warps; here a thread that unpacks 64 weights needs about two instructions per weight, one thread
@@ -36,7 +40,7 @@ constexpr int MB_A_TILE = MB_ROWS * 128, MB_A_BYTES = 2 * MB_A_TILE;
 constexpr int MB_THREADS = 24 * 32;
 constexpr int MB_DQ_WARPS = 12, MB_DQ_GROUPS = 3, MB_DRAIN = 16, MB_DRAIN_WARPS = 8;
 constexpr int MB_MMA = 0, MB_TMA_X = 4, MB_TMA_W = 8;
-constexpr int MB_CHUNK = 8, MB_COLS = 32;         // activation rows of a chunk; its columns (three digits of eight rows, eight unused)
+constexpr int MB_CHUNK = 8, MB_COLS = 32;         // activation rows of a chunk; its columns (three or four digits of eight rows)
 constexpr int MB_MAX_A = 4, MB_MAX_B = 6, MB_MAX_RAW = 4, MB_MAX_D = 8, MB_MAX_SPLIT = 8;
 constexpr int MB_SMEM_MAX = 224 * 1024;
 
@@ -53,6 +57,8 @@ static_assert(MB_META == 64, "block record layout");
 // ---- activations -> digit planes and block records ------------------------------------------------------------------
 // One CTA per activation row; f(x) = x, x / rms(x) * gain, or silu(x) * u.  Row a's digit p goes to row
 // (a / 8) * 32 + p * 8 + a % 8 of `planes` ([32 * chunks][K] fp16); records to meta[super-block][8 * chunks].
+// DIGITS: 3 (eleven bits) or 4 (bytes), the leading one first
+template <int DIGITS>
 __global__ void __launch_bounds__(1024)
 skn_xsplit_kernel(const float *__restrict__ x, int K, const float *__restrict__ gain, float eps, const float *__restrict__ silu_u,
                   __half *__restrict__ planes, mb_meta *__restrict__ meta, int rows_pad) {
@@ -97,17 +103,23 @@ skn_xsplit_kernel(const float *__restrict__ x, int K, const float *__restrict__ 
         mb_meta *m = meta + (size_t)sb * rows_pad + a;
         int X[8];
         mm_fixed_point<false>(v0, v1, 0, lane, X, &m->scale, m->xsum, m->oval, &m->oidx, reinterpret_cast<uint8_t *>(&m->ocnt), nullptr);
-        __half dig[3][8];
+        __half dig[DIGITS][8];
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
-            const int d2 = ((X[i] + 1024) & 2047) - 1024, h = (X[i] - d2) >> 11;
-            const int d1 = ((h + 1024) & 2047) - 1024;
-            dig[0][i] = __int2half_rn((h - d1) >> 11);
-            dig[1][i] = __int2half_rn(d1);
-            dig[2][i] = __int2half_rn(d2);
+            if constexpr (DIGITS == 4) {
+                const uint32_t d = ((uint32_t)X[i] + 0x80808080u) ^ 0x80808080u;       // its bytes are the signed digits
+#pragma unroll
+                for (int p = 0; p < 4; ++p) dig[p][i] = __int2half_rn((int)(int8_t)(d >> (24 - 8 * p)));
+            } else {
+                const int d2 = ((X[i] + 1024) & 2047) - 1024, h = (X[i] - d2) >> 11;
+                const int d1 = ((h + 1024) & 2047) - 1024;
+                dig[0][i] = __int2half_rn((h - d1) >> 11);
+                dig[1][i] = __int2half_rn(d1);
+                dig[2][i] = __int2half_rn(d2);
+            }
         }
 #pragma unroll
-        for (int p = 0; p < 3; ++p) {
+        for (int p = 0; p < DIGITS; ++p) {
             uint2 *to = reinterpret_cast<uint2 *>(row + (size_t)p * MB_CHUNK * K + sb * 256) + lane;
             to[0] = *reinterpret_cast<const uint2 *>(&dig[p][0]);
             to[32] = *reinterpret_cast<const uint2 *>(&dig[p][4]);
@@ -117,12 +129,12 @@ skn_xsplit_kernel(const float *__restrict__ x, int K, const float *__restrict__ 
 
 // ---- raw blocks -> fp16 integers --------------------------------------------------------------------------------------
 template <int TYPE> struct MbFmt;
-template <> struct MbFmt<SKN_TYPE_Q4_K> { static constexpr int ROW = 144, MM = MM_FMT_Q4K, BLOCKS = 1, STAGES = 2; };
-template <> struct MbFmt<SKN_TYPE_Q4_0> { static constexpr int ROW = 144, MM = MM_FMT_Q40, BLOCKS = 8, STAGES = 2; };
-template <> struct MbFmt<SKN_TYPE_Q8_0> { static constexpr int ROW = 272, MM = MM_FMT_Q80, BLOCKS = 8, STAGES = 2; };
-// Q6_K: quant times 8-bit scale needs 12 bits.  The scale is taken as 2 h + b, b = 0 or 1: a stage is 64 columns in two weight
-// tiles, (q - 32) h and (q - 32) b, against one tile of digits, into two accumulators
-template <> struct MbFmt<SKN_TYPE_Q6_K> { static constexpr int ROW = 240, MM = MM_FMT_Q6K, BLOCKS = 1, STAGES = 4; };
+template <> struct MbFmt<SKN_TYPE_Q4_K> { static constexpr int ROW = 144, MM = MM_FMT_Q4K, BLOCKS = 1, STAGES = 2, DIGITS = 4; };
+template <> struct MbFmt<SKN_TYPE_Q4_0> { static constexpr int ROW = 144, MM = MM_FMT_Q40, BLOCKS = 8, STAGES = 2, DIGITS = 3; };
+template <> struct MbFmt<SKN_TYPE_Q8_0> { static constexpr int ROW = 272, MM = MM_FMT_Q80, BLOCKS = 8, STAGES = 2, DIGITS = 3; };
+// Q6_K: quant times 8-bit scale needs 12 bits.  The scale is taken as 16 h + l, -8 <= l < 8: a stage is 64 columns in two weight
+// tiles, (q - 32) h and (q - 32) l, against one tile of digits, into two accumulators
+template <> struct MbFmt<SKN_TYPE_Q6_K> { static constexpr int ROW = 240, MM = MM_FMT_Q6K, BLOCKS = 1, STAGES = 4, DIGITS = 4; };
 
 // four bytes b of w -> fp16 (b + 1024) * mul + add: 1024 + b is the byte under the high byte 0x64; all values here are exact
 __device__ __forceinline__ void mb_quad(uint32_t w, __half2 mul, __half2 add, uint32_t *out) {
@@ -133,14 +145,25 @@ __device__ __forceinline__ void mb_quad(uint32_t w, __half2 mul, __half2 add, ui
         out[i] = *reinterpret_cast<const uint32_t *>(&v);
     }
 }
+// bytes 0 and 1 of w as fp16
+__device__ __forceinline__ void mb_pair(uint32_t w, uint32_t &out) {
+    const uint32_t h = __byte_perm(w, 0x64646464u, 0x4140);
+    const __half2 v = __hsub2(*reinterpret_cast<const __half2 *>(&h), __float2half2_rn(1024.f));
+    out = *reinterpret_cast<const uint32_t *>(&v);
+}
 // half g of stage u of the row at `row` (see the formats' notes in skn_matmul_tc.cu: same cut, same chunks)
 template <int TYPE>
 __device__ __forceinline__ void mb_half(uint32_t row, int u, int g, uint32_t sc2, uint32_t (&out)[16], int lead = 0, int v = 0) {
     if constexpr (TYPE == SKN_TYPE_Q4_K) {
         const uint4 q = tc_lds128(row + 16 + 32 * u + 16 * g);
         const uint32_t qw[4] = {q.x, q.y, q.z, q.w};
-        const __half2 s0 = __half2half2(__uint2half_rn(sc2 & 0xFFu)), s1 = __half2half2(__uint2half_rn(sc2 >> 8));
-        const __half2 a0 = __hmul2(s0, __float2half2_rn(-1024.f)), a1 = __hmul2(s1, __float2half2_rn(-1024.f));
+        // (1024 + q) s + a = s q - 8 (s & 60): a is a multiple of 32 down to -64992, so an fp16 number
+        uint32_t sp, tp;
+        mb_pair(sc2, sp);
+        mb_pair(sc2 & 0x3C3Cu, tp);
+        const __half2 s = *reinterpret_cast<const __half2 *>(&sp);
+        const __half2 a = __hfma2(*reinterpret_cast<const __half2 *>(&tp), __float2half2_rn(-8.f), __hmul2(s, __float2half2_rn(-1024.f)));
+        const __half2 s0 = __low2half2(s), s1 = __high2half2(s), a0 = __low2half2(a), a1 = __high2half2(a);
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             mb_quad(qw[i] & 0x0F0F0F0Fu, s0, a0, out + 2 * i);
@@ -166,7 +189,8 @@ __device__ __forceinline__ void mb_half(uint32_t row, int u, int g, uint32_t sc2
         tc_shift(wh, lead >> 2, sh, qh);
         asm volatile("ld.shared.u16 %0, [%1];" : "=r"(s8) : "r"(row + (uint32_t)lead + 192 + 8 * (u >> 1) + 4 * (u & 1) + 2 * g));   // two int8 scales
         const int i0 = (int)(int8_t)(s8 & 0xFFu), i1 = (int)(int8_t)(s8 >> 8);
-        const __half2 s0 = __half2half2(__int2half_rn(v ? i0 & 1 : i0 >> 1)), s1 = __half2half2(__int2half_rn(v ? i1 & 1 : i1 >> 1));
+        const int l0 = ((i0 + 8) & 15) - 8, l1 = ((i1 + 8) & 15) - 8;
+        const __half2 s0 = __half2half2(__int2half_rn(v ? l0 : (i0 - l0) >> 4)), s1 = __half2half2(__int2half_rn(v ? l1 : (i1 - l1) >> 4));
         const int lsh = 4 * (u & 1), hsh = 4 * (u & 1) + 2 * g;
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
@@ -193,8 +217,15 @@ __device__ __forceinline__ void mb_q4k_scales(const uint4 &h, uint32_t (&sc)[2],
     mn[0] = h.z & 0x3F3F3F3Fu;
     mn[1] = ((h.w >> 4) & 0x0F0F0F0Fu) | ((h.z >> 2) & 0x30303030u);
 }
-__device__ __forceinline__ float mb_byte(uint32_t w, int i) {       // byte i as a float: 2^23 + byte, exactly, less 2^23
-    return __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7440 + i)) - 8388608.f;
+// bytes i and i + 1 as floats: 2^23 + byte, exactly, less 2^23
+__device__ __forceinline__ uint64_t mb_bytes2(uint32_t w, int i) {
+    return skn_add2(skn_pack2u(__byte_perm(w, 0x4B000000u, 0x7440 + i), __byte_perm(w, 0x4B000000u, 0x7441 + i)), skn_pack2(-8388608.f, -8388608.f));
+}
+
+// the sum that row a's digit sums stand for
+template <int DIGITS> __device__ __forceinline__ float mb_join(const uint32_t (&D)[32], int a) {
+    if constexpr (DIGITS == 3) return fmaf(__uint_as_float(D[a]), 4194304.f, fmaf(__uint_as_float(D[8 + a]), 2048.f, __uint_as_float(D[16 + a])));
+    return fmaf(fmaf(__uint_as_float(D[a]), 256.f, __uint_as_float(D[8 + a])), 65536.f, fmaf(__uint_as_float(D[16 + a]), 256.f, __uint_as_float(D[24 + a])));
 }
 
 // The outliers of the record at m times their dequantised weights of the block at `blk`.  Rare and out of line: inlined for every
@@ -449,16 +480,18 @@ skn_matvec_batch_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_c
                     const int ch = 2 * i + odd;
                     if (ch >= NCH) break;
                     const uint32_t at = tmem_base + (uint32_t)(d * SET_COLS + ch * MB_COLS) + ((uint32_t)(wq * 32) << 16);
-                    float hi[MB_CHUNK];
+                    float v[MB_CHUNK];
 #pragma unroll
-                    for (int v = 0; v < 2; ++v) {
-                        uint32_t D[32];
-                        tc_ld32(at + (uint32_t)(v * NCOL), D);
+                    for (int p = 0; p < 2; ++p) {                   // digits d3 and d2, then d1 and d0; the scale's parts join digit by digit
+                        uint32_t H[16], L[16];
+                        tc_ld16x2(at + (uint32_t)(16 * p), at + (uint32_t)(16 * p + NCOL), H, L);
 #pragma unroll
                         for (int a = 0; a < MB_CHUNK; ++a) {
-                            const float t = fmaf(__uint_as_float(D[a]), 4194304.f, fmaf(__uint_as_float(D[8 + a]), 2048.f, __uint_as_float(D[16 + a])));
-                            if (v == 0) hi[a] = t;
-                            else y[i * MB_CHUNK + a] = fmaf(fmaf(hi[a], 2.f, t), db * mm_lds32f(mt + (uint32_t)((ch * MB_CHUNK + a) * MB_META)), y[i * MB_CHUNK + a]);
+                            const float t1 = fmaf(__uint_as_float(H[a]), 16.f, __uint_as_float(L[a])),
+                                        t0 = fmaf(__uint_as_float(H[8 + a]), 16.f, __uint_as_float(L[8 + a]));
+                            const float t = fmaf(t1, 256.f, t0);
+                            if (p == 0) v[a] = t;
+                            else y[i * MB_CHUNK + a] = fmaf(fmaf(v[a], 65536.f, t), db * mm_lds32f(mt + (uint32_t)((ch * MB_CHUNK + a) * MB_META)), y[i * MB_CHUNK + a]);
                         }
                     }
                 }
@@ -471,9 +504,12 @@ skn_matvec_batch_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_c
                 const float2 dd = __half22float2(*reinterpret_cast<const __half2 *>(&hdr.x));
                 uint32_t sc[2], mn[2];
                 mb_q4k_scales(hdr, sc, mn);
-                float mf[8];
+                // what a sub-block's sum of x counts, 8 (s & 60) d - m dmin (products exact, one rounding): sub-blocks 2 j and 2 j + 1
+                uint64_t of[4];
+                const uint64_t d8 = skn_pack2(8.f * dd.x, 8.f * dd.x), dm = skn_pack2(-dd.y, -dd.y);
 #pragma unroll
-                for (int j = 0; j < 8; ++j) mf[j] = mb_byte(mn[j >> 2], j & 3);
+                for (int j = 0; j < 4; ++j)
+                    of[j] = skn_fma2(d8, mb_bytes2(sc[j >> 1] & 0x3C3C3C3Cu, 2 * (j & 1)), skn_fma2(dm, mb_bytes2(mn[j >> 1], 2 * (j & 1)), 0ull));
                 if (!failed && !tc_wait_warp(&d_full[d], pd, lane)) give_up();
                 tc_fence_after();
 #pragma unroll
@@ -487,13 +523,13 @@ skn_matvec_batch_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_c
                         const uint32_t m = mt + (uint32_t)((ch * MB_CHUNK + a) * MB_META);
                         const float sx = mm_lds32f(m);
                         const uint4 s0 = tc_lds128(m + 32), s1 = tc_lds128(m + 48);
-                        const float v = fmaf(__uint_as_float(D[a]), 4194304.f, fmaf(__uint_as_float(D[8 + a]), 2048.f, __uint_as_float(D[16 + a])));
-                        float off = mf[0] * __uint_as_float(s0.x);
-                        off = fmaf(mf[1], __uint_as_float(s0.y), off); off = fmaf(mf[2], __uint_as_float(s0.z), off);
-                        off = fmaf(mf[3], __uint_as_float(s0.w), off); off = fmaf(mf[4], __uint_as_float(s1.x), off);
-                        off = fmaf(mf[5], __uint_as_float(s1.y), off); off = fmaf(mf[6], __uint_as_float(s1.z), off);
-                        off = fmaf(mf[7], __uint_as_float(s1.w), off);
-                        y[i * MB_CHUNK + a] += fmaf(v, dd.x * sx, -dd.y * off);
+                        uint64_t off = skn_fma2(of[0], skn_pack2u(s0.x, s0.y), 0ull);
+                        off = skn_fma2(of[1], skn_pack2u(s0.z, s0.w), off);
+                        off = skn_fma2(of[2], skn_pack2u(s1.x, s1.y), off);
+                        off = skn_fma2(of[3], skn_pack2u(s1.z, s1.w), off);
+                        float even, uneven;
+                        skn_unpack2(off, even, uneven);
+                        y[i * MB_CHUNK + a] += fmaf(mb_join<4>(D, a), dd.x * sx, even + uneven);
                     }
                 }
                 tc_fence_before();
@@ -518,10 +554,7 @@ skn_matvec_batch_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_c
                             uint32_t D[32];
                             tc_ld32(tmem_base + (uint32_t)(d * SET_COLS + j * NCOL + ch * MB_COLS) + ((uint32_t)(wq * 32) << 16), D);
 #pragma unroll
-                            for (int a = 0; a < MB_CHUNK; ++a) {
-                                const float v = fmaf(__uint_as_float(D[a]), 4194304.f, fmaf(__uint_as_float(D[8 + a]), 2048.f, __uint_as_float(D[16 + a])));
-                                z[i * MB_CHUNK + a] = fmaf(v, dj, z[i * MB_CHUNK + a]);
-                            }
+                            for (int a = 0; a < MB_CHUNK; ++a) z[i * MB_CHUNK + a] = fmaf(mb_join<3>(D, a), dj, z[i * MB_CHUNK + a]);
                         }
                     }
                     tc_fence_before();
@@ -705,7 +738,7 @@ static cudaError_t mb_launch(skn_ctx *ctx, int n, const skn_tensor *const *w, co
     covered = true;
     const int warps = K / 256 < 32 ? K / 256 : 32;
     const cudaLaunchConfig_t prep = mb_config(dim3((unsigned)M), dim3((unsigned)warps * 32), 1, 0, stream, attr);
-    if ((e = cudaLaunchKernelEx(&prep, skn_xsplit_kernel, x, K, gain, eps, silu_u, xp, meta, rows_pad)) != cudaSuccess) return e;
+    if ((e = cudaLaunchKernelEx(&prep, skn_xsplit_kernel<MbFmt<TYPE>::DIGITS>, x, K, gain, eps, silu_u, xp, meta, rows_pad)) != cudaSuccess) return e;
     const cudaLaunchConfig_t cfg = mb_config(dim3((unsigned)(tiles * pl.split)), dim3(MB_THREADS), pl.split, pl.smem, stream, attr);
     return cudaLaunchKernelEx(&cfg, kern, tx, tw[0], tw[1], tw[2], ar, K, pl, (const mb_meta *)meta, ctx->d_status);
 }

@@ -57,6 +57,19 @@ __device__ __forceinline__ void tc_ld32(uint32_t taddr, uint32_t (&r)[32]) {
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
+// 16 columns at each of two addresses
+__device__ __forceinline__ void tc_ld16x2(uint32_t at0, uint32_t at1, uint32_t (&r)[16], uint32_t (&q)[16]) {
+#define TC_LD16(at, r)                                                                                                          \
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"        \
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),   \
+                   "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])                      \
+                 : "r"(at))
+    TC_LD16(at0, r);
+    TC_LD16(at1, q);
+#undef TC_LD16
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+
 // ---- clusters, warp-wide waits, shared-memory windows ------------------------------------------------------------
 __device__ __forceinline__ uint32_t tc_cluster_rank() {
     uint32_t r;

@@ -63,6 +63,50 @@ def test_batch_rows_that_are_not_finite_stay_apart(ctx, qt):
     assert np.array_equal(y[keep], clean[keep])
 
 
+def _near_the_largest(g, qt, n, k):
+    """Blocks of positive weights whose quants and integer scales are at or near their largest, d a power of two."""
+    half = np.frombuffer(np.float16(2.0 ** -6).tobytes(), dtype=np.uint8)
+    nibbles = lambda *shape: (0xEE | g.integers(0, 2, shape) | g.integers(0, 2, shape) << 4).astype(np.uint8)        # 14 and 15
+    if qt == synth.Q4_K:
+        b = np.zeros((n, k // 256, 144), dtype=np.uint8)
+        sc = g.integers(61, 64, (n, k // 256, 8)).astype(np.uint8)
+        b[..., 0:2], b[..., 16:] = half, nibbles(n, k // 256, 128)
+        b[..., 4:8], b[..., 12:16] = sc[..., :4] | sc[..., 4:] >> 4 << 6, sc[..., 4:] & 15
+    elif qt == synth.Q6_K:
+        b = np.full((n, k // 256, 210), 0xFF, dtype=np.uint8)
+        b[..., 208:], b[..., :128], b[..., 192:208] = half, nibbles(n, k // 256, 128), g.integers(118, 128, (n, k // 256, 16))
+    elif qt == synth.Q4_0:
+        b = np.zeros((n, k // 32, 18), dtype=np.uint8)
+        b[..., :2], b[..., 2:] = half, nibbles(n, k // 32, 16)
+    else:
+        b = np.zeros((n, k // 32, 34), dtype=np.uint8)
+        b[..., :2], b[..., 2:] = half, g.integers(118, 128, (n, k // 32, 32))
+    return b.reshape(-1)
+
+
+@pytest.mark.parametrize("qt", TYPES)
+@pytest.mark.parametrize("K", [256, 4096])
+@pytest.mark.parametrize("digit", [0, -128, 127])
+def test_batch_sums_of_one_sign_are_exact(ctx, qt, K, digit):
+    """Activations and weights of one sign near their largest, with the second byte digit of the activations near `digit`: the integer sums
+    are the largest there are.  They are exact, so what is left are roundings to nearest: joining the digits (3), sums of x and
+    offset, scale and accumulation of a super-block (4) and the parts of K (2), each at most 2^-24 of a sum of terms of one sign --
+    and without a preferred direction: the mean over some thousand outputs is far below one of them."""
+    g = synth.rng(K + digit + 200)
+    M, N = 12 if K == 256 else 30, 256
+    w = _near_the_largest(g, qt, N, K)
+    top, low = g.integers(56, 63, (M, K)), g.integers(-128, 128, (M, K))
+    second = np.clip(digit + g.integers(-3, 4, (M, K)), -128, 127)
+    x = ((top * 2.0 ** 24 + second * 2.0 ** 16 + low * 2.0 ** 8) * 2.0 ** -29).astype(np.float32)       # at most 23 bits: exact
+    t = skn.QuantTensor(ctx, (N, K), qt, w)
+    y = t.matmul_t(x)
+    t.close()
+    ref, _ = oracle.matmul(qt, w, N, K, x)
+    err = (y - ref) / ref
+    assert np.abs(err).max() <= (9 + K // 256 / 8) * 2.0 ** -24
+    assert abs(err.mean()) <= 2.0 ** -26
+
+
 @pytest.mark.parametrize("batch", [9, 20, 40])
 def test_decoder_batch_agrees_with_single_sequences(ctx, batch):
     """Q/K/V grouped, gate / up / SwiGLU interleaved, residuals and folded norms: a batch of sequences against the same
