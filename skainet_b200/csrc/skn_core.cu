@@ -50,6 +50,27 @@ int32_t skn_stage_reserve(skn_ctx *ctx, void **buf, size_t *cap, size_t need) {
     return SKN_OK;
 }
 
+// The prepared activations' buffer.  A captured graph holds its address, and a later call with more rows may need a larger one: the old
+// buffer stays until the context goes.  Sizes at least double, so all of them together take less than the last one again, and 24 of
+// them are more than an address space holds.  While `stream` captures nothing can be allocated: the caller is told (SKN_ERR_BUSY)
+// before anything has touched the capture, and may take a route without this buffer.
+int32_t skn_xq_reserve(skn_ctx *ctx, size_t need, cudaStream_t stream) {
+    if (need <= ctx->d_xq_bytes) return SKN_OK;
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    SKN_CUDA(ctx, cudaStreamIsCapturing(stream, &capture));
+    if (capture != cudaStreamCaptureStatusNone) return SKN_ERR_BUSY;
+    constexpr int most = (int)(sizeof(ctx->xq_outgrown) / sizeof(ctx->xq_outgrown[0]));
+    if (ctx->n_xq_outgrown >= most) return skn_fail(ctx, SKN_ERR_OOM, "prepared activations of %zu bytes", need);
+    size_t want = need < (1u << 20) ? (1u << 20) : need;
+    if (want < 2 * ctx->d_xq_bytes) want = 2 * ctx->d_xq_bytes;
+    void *grown = nullptr;
+    SKN_CUDA(ctx, cudaMalloc(&grown, want));
+    if (ctx->d_xq) ctx->xq_outgrown[ctx->n_xq_outgrown++] = ctx->d_xq;
+    ctx->d_xq = grown;
+    ctx->d_xq_bytes = want;
+    return SKN_OK;
+}
+
 extern "C" {
 
 int32_t skn_version(void) { return SKN_VERSION; }
@@ -119,6 +140,7 @@ int32_t skn_ctx_destroy(skn_ctx *ctx) {
     if (ctx->d_scratch) cudaFree(ctx->d_scratch);
     if (ctx->d_scratch2) cudaFree(ctx->d_scratch2);
     if (ctx->d_xq) cudaFree(ctx->d_xq);
+    for (int i = 0; i < ctx->n_xq_outgrown; ++i) cudaFree(ctx->xq_outgrown[i]);
     if (ctx->d_status_base) cudaFree(ctx->d_status_base);
     if (ctx->h_status_base) cudaFreeHost(ctx->h_status_base);
     if (ctx->own_stream) cudaStreamDestroy(ctx->own_stream);

@@ -53,7 +53,9 @@ struct skn_ctx {
     void *d_stage_out; size_t d_stage_out_bytes;
     void *d_scratch;   size_t d_scratch_bytes;   // kernel scratch (bf16 operands, FFN intermediates)
     void *d_scratch2;  size_t d_scratch2_bytes;  // attention split partials
-    void *d_xq;        size_t d_xq_bytes;        // prepared activations of the many-row matvec (digit planes, block records)
+    void *d_xq;        size_t d_xq_bytes;        // prepared activations of the matvec of several rows (digit planes, block records)
+    void *xq_outgrown[24];                       // ... and its smaller predecessors, which captured graphs may still use (skn_xq_reserve)
+    int n_xq_outgrown;
     uint32_t rows_cfg;                           // many-row matvec variants whose attributes are set on this device
     skn_group_plan group_plans[32];
     int n_group_plans;
@@ -158,6 +160,7 @@ bool skn_ctx_ok(const skn_ctx *ctx);
 bool skn_tensor_ok(const skn_tensor *t);
 bool skn_kv_ok(const skn_kvcache *kv);
 int32_t skn_stage_reserve(skn_ctx *ctx, void **buf, size_t *cap, size_t need);
+int32_t skn_xq_reserve(skn_ctx *ctx, size_t need, cudaStream_t stream);
 int32_t skn_status_check(skn_ctx *ctx);
 
 #define SKN_CUDA(ctx, call)                                            \

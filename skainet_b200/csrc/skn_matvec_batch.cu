@@ -728,7 +728,9 @@ static cudaError_t mb_launch(skn_ctx *ctx, int n, const skn_tensor *const *w, co
     const int K = (int)w[0]->n_cols, rows_pad = NCH * MB_CHUNK;
     const mb_plan pl = mb_make_plan(TYPE, NCH, tiles, K, f);
     const size_t planes = (size_t)NCH * MB_COLS * K * 2;           // a multiple of 1024
-    if (skn_stage_reserve(ctx, &ctx->d_xq, &ctx->d_xq_bytes, planes + (size_t)(K / 256) * rows_pad * MB_META) != SKN_OK) return cudaErrorMemoryAllocation;
+    // (while a graph is captured and the buffer is too small, the routes with smaller buffers or none take the call)
+    const int32_t rc = skn_xq_reserve(ctx, planes + (size_t)(K / 256) * rows_pad * MB_META, stream);
+    if (rc != SKN_OK) return rc == SKN_ERR_BUSY ? cudaErrorNotSupported : cudaErrorMemoryAllocation;
     __half *xp = (__half *)ctx->d_xq;
     mb_meta *meta = reinterpret_cast<mb_meta *>((uint8_t *)ctx->d_xq + planes);
     CUtensorMap tx, tw[3];

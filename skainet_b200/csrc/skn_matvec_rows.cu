@@ -704,7 +704,7 @@ bool skn_rows_try_group(skn_ctx *ctx, int n, const skn_tensor *const *w, const f
     }
     const int nb = (int)(K / 256);
     const int nks = (nb + pl.geo.KSB - 1) / pl.geo.KSB;
-    if (skn_stage_reserve(ctx, &ctx->d_xq, &ctx->d_xq_bytes, (size_t)nks * M * pl.geo.prow + 256) != SKN_OK) {
+    if (skn_xq_reserve(ctx, (size_t)nks * M * pl.geo.prow + 256, stream) != SKN_OK) {
         err = cudaErrorMemoryAllocation;
         return true;
     }

@@ -2,6 +2,7 @@
 launches and parts of K; the tolerance of the single-row kernels."""
 import numpy as np
 import pytest
+import torch
 
 import skainet_b200 as skn
 from conftest import FP32_TOL, assert_close_dot
@@ -105,6 +106,66 @@ def test_batch_sums_of_one_sign_are_exact(ctx, qt, K, digit):
     err = (y - ref) / ref
     assert np.abs(err).max() <= (9 + K // 256 / 8) * 2.0 ** -24
     assert abs(err.mean()) <= 2.0 ** -26
+
+
+def _captured(ctx, t, x, y):
+    """A graph of one product on a stream of its own."""
+    stream, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    ctx.set_stream(stream.cuda_stream)
+    with torch.cuda.stream(stream), torch.cuda.graph(graph, stream=stream):
+        t.matmul_t_dev(x, x.shape[0], y)
+    ctx.set_stream(None)
+    return graph
+
+
+@pytest.mark.parametrize("qt,M", [(synth.Q4_K, 30), (synth.Q6_K, 30)])
+def test_batch_captured_before_its_buffer_is_large_enough(qt, M):
+    """Nothing can be allocated while a graph is captured: a route takes the call that needs no larger buffer than there is.  Q6_K has one
+    without any; the others' takes up to 16 rows a launch and has what a call of five rows left."""
+    g = synth.rng(11)
+    N, K = 256, 8192
+    w, x = synth.make_weight(g, qt, N, K), torch.from_numpy(synth.make_activations(g, M, K)).cuda()
+    ctx = skn.Context(0)
+    t = skn.QuantTensor(ctx, (N, K), qt, w)
+    y = torch.zeros(M, N, device="cuda")
+    if qt != synth.Q6_K:
+        torch.cuda.synchronize()
+        t.matmul_t_dev(x, 5, y)
+        ctx.sync()
+    graph = _captured(ctx, t, x, y)
+    graph.replay()
+    torch.cuda.synchronize()
+    ref, absdot = oracle.matmul(qt, w, N, K, x.cpu().numpy())
+    assert_close_dot(y.cpu().numpy(), ref, absdot, FP32_TOL, f"type {qt}")
+    del graph
+    t.close()
+    ctx.close()
+
+
+@pytest.mark.parametrize("qt", TYPES)
+def test_batch_graph_outlives_a_larger_call(qt):
+    """A later call whose prepared activations need a larger buffer leaves the one a captured graph works in."""
+    g = synth.rng(12)
+    ctx = skn.Context(0)
+    small, large = (skn.QuantTensor(ctx, s, qt, synth.make_weight(g, qt, *s)) for s in ((256, 512), (16, 32768)))
+    x, big = (torch.from_numpy(synth.make_activations(g, *s)).cuda() for s in ((16, 512), (32, 32768)))
+    y, y_big = torch.zeros(16, 256, device="cuda"), torch.zeros(32, 16, device="cuda")
+    torch.cuda.synchronize()
+    small.matmul_t_dev(x, 16, y)
+    ctx.sync()
+    want = y.clone()
+    graph = _captured(ctx, small, x, y)
+    large.matmul_t_dev(big, 32, y_big)
+    ctx.sync()
+    y.zero_()
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(y, want)
+    del graph
+    small.close()
+    large.close()
+    ctx.close()
 
 
 @pytest.mark.parametrize("batch", [9, 20, 40])
