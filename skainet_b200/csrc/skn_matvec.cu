@@ -992,6 +992,7 @@ cudaError_t skn_launch_matvec_acts(skn_ctx *ctx, int n, const skn_tensor *const 
     }
     // three rows or more: the many-row kernel (x prepared once per launch by its own kernel, up to sixteen rows
     // per pass over the weights); it has no rotary epilogue and no exchange
+    int done = 0;
     if (M >= 3 && !xc && !rope) {
         const int maxr = skn_rows_max_acts(ctx, n, w);
         if (maxr >= 4) {
@@ -1009,20 +1010,19 @@ cudaError_t skn_launch_matvec_acts(skn_ctx *ctx, int n, const skn_tensor *const 
                 cudaError_t err = cudaSuccess;
                 if (!skn_rows_try_group(ctx, n, w, x + (int64_t)m0 * K, na, ys, add ? as : nullptr, add_per_act, norm_gain, norm_eps,
                                         silu_u ? silu_u + (int64_t)m0 * K : nullptr, swiglu, stream, err)) {
-                    if (i == 0) break;                                        // not covered after all: the route below
-                    return cudaErrorUnknown;
+                    break;          // this share is not covered (Q8_0 takes five rows a launch where four do not fit): the route below
                 }
                 if (err != cudaSuccess) return err;
-                m0 += na;
+                done = m0 += na;
                 if (m0 == M) return cudaSuccess;
             }
         }
     }
     const int maxa = skn_mma_max_acts(ctx, w[0]->type, tot, w[0]->n_cols);
-    if (maxa < 1) return cudaErrorNotSupported;
-    const int launches = (M + maxa - 1) / maxa;
+    if (maxa < 1) return done ? cudaErrorUnknown : cudaErrorNotSupported;      // (rows already added to must not run again)
+    const int launches = (M - done + maxa - 1) / maxa;
     if (xc && launches != 1) return cudaErrorNotSupported;      // an exchange covers all rows of one launch
-    for (int i = 0, m0 = 0; i < launches; ++i) {
+    for (int i = 0, m0 = done; i < launches; ++i) {
         const int na = (M - m0 + (launches - i) - 1) / (launches - i);       // even shares
         float *ys[3] = {nullptr, nullptr, nullptr};
         const float *as[3] = {nullptr, nullptr, nullptr};
@@ -1038,7 +1038,7 @@ cudaError_t skn_launch_matvec_acts(skn_ctx *ctx, int n, const skn_tensor *const 
         }
         if (!skn_mma_try_group(ctx, n, w, x + (int64_t)m0 * K, ys, add ? as : nullptr, norm_gain, norm_eps,
                                silu_u ? silu_u + (int64_t)m0 * K : nullptr, stream, err, swiglu, na, add_per_act, xc, rope ? &rp : nullptr))
-            return cudaErrorNotSupported;
+            return done ? cudaErrorUnknown : cudaErrorNotSupported;
         if (err != cudaSuccess) return err;
         m0 += na;
     }

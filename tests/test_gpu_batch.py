@@ -119,7 +119,7 @@ def _captured(ctx, t, x, y):
     return graph
 
 
-@pytest.mark.parametrize("qt,M", [(synth.Q4_K, 30), (synth.Q6_K, 30)])
+@pytest.mark.parametrize("qt,M", [(synth.Q4_K, 30), (synth.Q6_K, 30), (synth.Q8_0, 9)])
 def test_batch_captured_before_its_buffer_is_large_enough(qt, M):
     """Nothing can be allocated while a graph is captured: a route takes the call that needs no larger buffer than there is.  Q6_K has one
     without any; the others' takes up to 16 rows a launch and has what a call of five rows left."""
