@@ -408,8 +408,9 @@ int32_t skn_llama_forward_dev(skn_llama *m, const int32_t *tokens_dev, int32_t T
                         l.wu->type == l.wg->type && l.wu->pitch == l.wg->pitch;
         void *a16 = nullptr, *h16 = nullptr;
         if (tc) {
-            const size_t ab = ((size_t)M * (d > qd ? d : qd) * 2 + 255) / 256 * 256;
-            if ((rc = skn_stage_reserve(ctx, &ctx->d_scratch, &ctx->d_scratch_bytes, ab + (size_t)M * F * 2))) return rc;
+            // (the rows of the output projection, qd wide, are done with before the feed-forward's are written: no more memory than its own)
+            const size_t ab = ((size_t)M * d * 2 + 255) / 256 * 256, need = ab + (size_t)M * F * 2, rows = (size_t)M * qd * 2;
+            if ((rc = skn_stage_reserve(ctx, &ctx->d_scratch, &ctx->d_scratch_bytes, need > rows ? need : rows))) return rc;
             a16 = ctx->d_scratch;
             h16 = (uint8_t *)ctx->d_scratch + ab;
         }

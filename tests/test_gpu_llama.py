@@ -181,6 +181,48 @@ def test_decoder_argument_errors(ctx):
     dec.close()
 
 
+def test_captured_prompt_needs_no_more_scratch_than_its_widest_product(ctx):
+    """Heads together wider than the model: the scratch memory of a prompt is that of its feed-forward (or of the output projection
+    where that is larger), so a prompt that another decoder's forward made room for can be captured; it replays to the eager result."""
+    import torch
+    M = 128
+    base = dict(n_layers=1, ffn_dim=4608, vocab=512, head_dim=64)
+    first = LlamaConfig(d_model=768, n_heads=12, n_kv_heads=3, **base)
+    wide = LlamaConfig(d_model=512, n_heads=16, n_kv_heads=4, **base)
+    own = skn.Context(0)
+
+    def make(cfg, max_ctx):
+        layers, head = random_model_blocks(cfg, seed=8)
+        ones = np.ones(cfg.d_model, dtype=np.float32)
+        d = LlamaDecoder(own, cfg, batch=1, max_tokens=M, max_ctx=max_ctx)
+        d.set_layer(0, layers[0], ones, ones)
+        d.set_head(head[0], ones, head[1])
+        return d
+
+    prompt = synth.rng(80).integers(0, 512, size=(1, M)).astype(np.int32)
+    a, b = make(first, 1024), make(wide, 256)
+    a.forward(prompt)                                    # 128 x (768 + 4608) bf16; the other's 128 x (1024 + 4608) would be more
+    tokens = torch.from_numpy(prompt).cuda()
+    stream, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    own.set_stream(stream.cuda_stream)
+    with torch.cuda.stream(stream), torch.cuda.graph(graph, stream=stream):
+        b.forward_dev(tokens, M)
+    with torch.cuda.stream(stream):
+        graph.replay()
+    own.sync()
+    got = b.forward(prompt[:, :1], want_logits=True)[1]
+    b.reset()
+    b.forward(prompt)
+    want = b.forward(prompt[:, :1], want_logits=True)[1]
+    assert np.isfinite(want).all() and np.array_equal(got, want)
+    own.set_stream(None)
+    del graph
+    for d in (a, b):
+        d.close()
+    own.close()
+
+
 def test_replayed_steps_stop_at_the_cache_capacity(ctx):
     """A single-token step captured into a CUDA graph advances the caches on the device but not the host's
     position.  Replaying it up to the capacity (a multiple of the attention chunk) works and equals eager
