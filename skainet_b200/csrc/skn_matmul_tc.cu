@@ -578,30 +578,41 @@ static cudaLaunchConfig_t tc_config(dim3 grid, int split, size_t smem, cudaStrea
     return cfg;
 }
 
+// Pairs in flight when clusters hold 1 .. TC_MAX_SPLIT of them.  Asked of the driver once per device, of whichever kernel comes first: threads,
+// shared memory and one CTA per SM are the same for all of them (asked of each, the first call of each took 5 to 15 us longer on the host).
+static cudaError_t tc_pairs(int dev, const void *kern, cudaStream_t stream, int (&pairs)[TC_MAX_SPLIT + 1]) {
+    static std::atomic<int> fits[64][TC_MAX_SPLIT + 1];            // 0: not asked yet, -1: none
+    std::atomic<int> *fit = fits[dev & 63];
+    for (int s = TC_MAX_SPLIT; s >= 1; --s) {
+        pairs[s] = fit[s].load(std::memory_order_relaxed);
+        if (pairs[s]) continue;
+        cudaLaunchAttribute attr[2];
+        const cudaLaunchConfig_t cfg = tc_config(dim3(2 * s), s, TC_SMEM_MAX, stream, attr);
+        int n = 0;
+        const cudaError_t e = cudaOccupancyMaxActiveClusters(&n, kern, &cfg);
+        if (e != cudaSuccess) return e;
+        pairs[s] = n > 0 ? n * s : -1;
+        fit[s].store(pairs[s], std::memory_order_relaxed);
+    }
+    return cudaSuccess;
+}
+
 template <int TYPE, bool DUAL>
 static cudaError_t launch_tc(const __nv_bfloat16 *A, int M, int K, const skn_tensor *w, const skn_tensor *w2, const tc_out &out,
                              int32_t *status, cudaStream_t stream) {
     auto kern = skn_matmul_tc_kernel<TYPE, DUAL>;
-    // per device: pairs in flight when clusters hold 1 .. 4 of them (0: not asked yet; the attribute is set before)
-    static std::atomic<int> fits[64][TC_MAX_SPLIT + 1];
+    static std::atomic<bool> large[64];                            // per device: may use TC_SMEM_MAX
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
-    std::atomic<int> *fit = fits[dev & 63];
     cudaLaunchAttribute attr[2];
-    if (fit[TC_MAX_SPLIT].load(std::memory_order_acquire) == 0) {
+    if (!large[dev & 63].load(std::memory_order_acquire)) {
         e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM_MAX);
         if (e != cudaSuccess) return e;
-        for (int s = 1; s <= TC_MAX_SPLIT; ++s) {
-            const cudaLaunchConfig_t cfg = tc_config(dim3(2 * s), s, TC_SMEM_MAX, stream, attr);
-            int n = 0;
-            e = cudaOccupancyMaxActiveClusters(&n, kern, &cfg);
-            if (e != cudaSuccess) return e;
-            fit[s].store(n > 0 ? n * s : -1, std::memory_order_release);
-        }
+        large[dev & 63].store(true, std::memory_order_release);
     }
     int pairs[TC_MAX_SPLIT + 1] = {0};
-    for (int s = 1; s <= TC_MAX_SPLIT; ++s) pairs[s] = fit[s].load(std::memory_order_acquire);
+    if ((e = tc_pairs(dev, (const void *)kern, stream, pairs)) != cudaSuccess) return e;
     const int64_t tiles = DUAL ? (w->n_rows + TC_ROWS - 1) / TC_ROWS : (w->n_rows + 2 * TC_ROWS - 1) / (2 * TC_ROWS);
     const tc_plan pl = tc_make_plan(TYPE, M, tiles, K, pairs);
     CUtensorMap tx, tw, tw2;
@@ -624,10 +635,11 @@ static cudaError_t dispatch_tc(const __nv_bfloat16 *A, int M, int K, const skn_t
     }
 }
 
+// (the tensor map's base: 16 bytes)
 bool skn_tc_supported(const skn_tensor *w, int32_t M) {
     const bool type_ok = w->type == SKN_TYPE_Q4_0 || w->type == SKN_TYPE_Q8_0 || w->type == SKN_TYPE_Q4_K || w->type == SKN_TYPE_Q6_K;
     return type_ok && M >= 1 && (w->n_cols % TC_BK) == 0 && w->n_cols >= TC_BK && (w->n_rows % 8) == 0 && (w->pitch % 16) == 0 &&
-           (reinterpret_cast<uintptr_t>(w->d_blocks) & 1) == 0;
+           (reinterpret_cast<uintptr_t>(w->d_blocks) & 15) == 0;
 }
 
 cudaError_t skn_launch_f32_to_bf16(const float *in, void *out_bf16, int64_t n, int sm_count, cudaStream_t stream) {

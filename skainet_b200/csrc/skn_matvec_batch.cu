@@ -704,27 +704,40 @@ static cudaLaunchConfig_t mb_config(dim3 grid, dim3 block, int cluster, size_t s
     return cfg;
 }
 
+// CTAs in flight in clusters of 1 .. MB_MAX_SPLIT, asked of the driver once per device: the same for all kernels here (threads, shared memory,
+// one CTA per SM); asked of each of them, its first call took 15 to 30 us longer on the host.
+static cudaError_t mb_fits(const skn_ctx *ctx, const void *kern, cudaStream_t stream, int (&f)[MB_MAX_SPLIT + 1]) {
+    static std::atomic<int> fits[64][MB_MAX_SPLIT + 1];            // 0: not asked yet, -1: none
+    std::atomic<int> *fit = fits[ctx->device & 63];
+    f[1] = ctx->sm_count;
+    for (int s = MB_MAX_SPLIT; s > 1; --s) {
+        f[s] = fit[s].load(std::memory_order_relaxed);
+        if (f[s]) continue;
+        cudaLaunchAttribute attr[2];
+        const cudaLaunchConfig_t cfg = mb_config(dim3(s), dim3(MB_THREADS), s, MB_SMEM_MAX, stream, attr);
+        int k = 0;
+        const cudaError_t e = cudaOccupancyMaxActiveClusters(&k, kern, &cfg);
+        if (e != cudaSuccess) return e;
+        f[s] = k > 0 ? k * s : -1;
+        fit[s].store(f[s], std::memory_order_relaxed);
+    }
+    return cudaSuccess;
+}
+
 template <int TYPE, int NCH, bool DUAL>
 static cudaError_t mb_launch(skn_ctx *ctx, int n, const skn_tensor *const *w, const float *x, int M, const mb_args &ar, int64_t tiles, const float *gain,
                              float eps, const float *silu_u, cudaStream_t stream, bool &covered) {
     auto kern = skn_matvec_batch_kernel<TYPE, NCH, DUAL>;
-    // per device: CTAs in flight in clusters of 1 .. 8 (0: not asked yet)
-    static std::atomic<int> fits[64][MB_MAX_SPLIT + 1];
-    std::atomic<int> *fit = fits[ctx->device & 63];
+    static std::atomic<bool> large[64];                            // per device: may use MB_SMEM_MAX
     cudaLaunchAttribute attr[2];
     cudaError_t e;
-    if (fit[MB_MAX_SPLIT].load(std::memory_order_acquire) == 0) {
+    if (!large[ctx->device & 63].load(std::memory_order_acquire)) {
         e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, MB_SMEM_MAX);
         if (e != cudaSuccess) return e;
-        for (int s = 1; s <= MB_MAX_SPLIT; ++s) {
-            const cudaLaunchConfig_t cfg = mb_config(dim3(s), dim3(MB_THREADS), s, MB_SMEM_MAX, stream, attr);
-            int k = ctx->sm_count;
-            if (s > 1 && (e = cudaOccupancyMaxActiveClusters(&k, kern, &cfg)) != cudaSuccess) return e;
-            fit[s].store(k > 0 ? k * s : -1, std::memory_order_release);
-        }
+        large[ctx->device & 63].store(true, std::memory_order_release);
     }
     int f[MB_MAX_SPLIT + 1] = {0};
-    for (int s = 1; s <= MB_MAX_SPLIT; ++s) f[s] = fit[s].load(std::memory_order_acquire);
+    if ((e = mb_fits(ctx, (const void *)kern, stream, f)) != cudaSuccess) return e;
     const int K = (int)w[0]->n_cols, rows_pad = NCH * MB_CHUNK;
     const mb_plan pl = mb_make_plan(TYPE, NCH, tiles, K, f);
     const size_t planes = (size_t)NCH * MB_COLS * K * 2;           // a multiple of 1024
@@ -764,7 +777,9 @@ static cudaError_t mb_by_rows(int M, A &&...a) {
     case 1: return mb_launch<TYPE, 1, DUAL>(a...);
     case 2: return mb_launch<TYPE, 2, DUAL>(a...);
     case 3: return mb_launch<TYPE, 3, DUAL>(a...);
-    default: return mb_launch<TYPE, 4, DUAL>(a...);
+    default:
+        if constexpr (TYPE != SKN_TYPE_Q8_0) return mb_launch<TYPE, 4, DUAL>(a...);     // (skn_batch_rows)
+        return cudaErrorNotSupported;
     }
 }
 template <bool DUAL, class... A>
