@@ -383,8 +383,7 @@ skn_matmul_tc_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_cons
         int s = 0, t = 0;
         uint32_t ph = 0, pt = 0;
         for (int it = 0; it < steps; ++it) {
-            if (!failed && !tc_wait_warp(&b_full[t], pt, lane)) failed = true;      // (one answer for the warp: its lanes elect, and fail, together)
-            if (!failed && !tc_wait_warp(&a_full[s], ph, lane)) failed = true;
+            if (!failed && !tc_wait_warp(&b_full[t], pt, &a_full[s], ph, lane)) failed = true;      // (one answer for the warp: its lanes elect, and fail, together)
             tc_fence_after();
             const uint64_t ad = a0 + (uint64_t)(s * (TC_A_BYTES >> 4)), bd = b0 + (uint64_t)(t * b_step);
             if (tc_elect()) {

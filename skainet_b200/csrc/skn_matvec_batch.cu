@@ -406,8 +406,7 @@ skn_matvec_batch_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_c
         int s = 0, tb = 0, d = 0;
         uint32_t ph = 0, pb = 0, pd = 0;
         for (int it = 0; it < steps; ++it) {
-            if (!failed && !tc_wait_warp(&b_full[tb], pb, lane)) failed = true;
-            if (!failed && !tc_wait_warp(&a_full[s], ph, lane)) failed = true;
+            if (!failed && !tc_wait_warp(&b_full[tb], pb, &a_full[s], ph, lane)) failed = true;
             const uint64_t ad = a0 + (uint64_t)(s * (MB_A_BYTES >> 4)), bd = b0 + (uint64_t)(tb * (B_BYTES >> 4));
             // K step k (16 columns): 32 bytes inside a tile's swizzle atom = +2 in the address field
             if constexpr (TYPE == SKN_TYPE_Q6_K) {

@@ -94,6 +94,11 @@ __device__ __forceinline__ bool tc_wait_warp(uint64_t *bar, uint32_t parity, int
     if (lane == 0) ok = skn_mbar_wait(bar, parity);
     return __shfl_sync(0xffffffffu, (int)ok, 0) != 0;
 }
+// ... for two barriers: one vote where both are complete (two cost 14336 x 4096 Q4_K at 16 rows 29.8 us instead of 29.0)
+__device__ __forceinline__ bool tc_wait_warp(uint64_t *bar, uint32_t parity, uint64_t *bar2, uint32_t parity2, int lane) {
+    if (__all_sync(0xffffffffu, skn_mbar_try_wait(bar, parity) && skn_mbar_try_wait(bar2, parity2))) return true;
+    return tc_wait_warp(bar, parity, lane) && tc_wait_warp(bar2, parity2, lane);
+}
 __device__ __forceinline__ uint4 tc_lds128(uint32_t addr) {
     uint4 v;
     asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr));
