@@ -658,7 +658,9 @@ static int mb_row_bytes(int type) {
 }
 
 // K over as many CTAs of a cluster as make the launch shortest, in SM clocks: a start and end of 9000, MB_STAGE_CLOCKS per 64 columns
-// of 128 rows.  `fit[s]` = CTAs in flight in clusters of s.
+// of 128 rows (Q4_K and Q4_0 at 16 rows; the other types are off by one factor, which decides nothing), 500 for the exchange (at 2000
+// rows of two super-blocks stayed in one CTA: 512 x 512 at 16 rows 8.7 us, split 7.4, Q4_0 9.2 and 7.6, Q8_0 8192 x 768 13.3 and 11.0).
+// `fit[s]` = CTAs in flight in clusters of s.
 constexpr int MB_STAGE_CLOCKS = 500;
 static mb_plan mb_make_plan(int type, int nch, int64_t tiles, int K, const int *fit) {
     mb_plan pl = {};
@@ -667,7 +669,7 @@ static mb_plan mb_make_plan(int type, int nch, int64_t tiles, int K, const int *
     for (int c = 1; c <= MB_MAX_SPLIT && c <= nsb; ++c) {
         if (fit[c] < 1 && c > 1) continue;
         const int64_t f = fit[c] > 0 ? fit[c] : 1, waves = (tiles * c + f - 1) / f;
-        const int64_t cost = waves * (9000 + (c > 1 ? 2000 : 0) + (int64_t)((nsb + c - 1) / c) * 4 * MB_STAGE_CLOCKS * (type == SKN_TYPE_Q6_K ? 2 : 1));
+        const int64_t cost = waves * (9000 + (c > 1 ? 500 : 0) + (int64_t)((nsb + c - 1) / c) * 4 * MB_STAGE_CLOCKS * (type == SKN_TYPE_Q6_K ? 2 : 1));
         if (best == 0 || cost < best) { best = cost; pl.split = c; }
     }
     pl.d = 512 / (nch * MB_COLS * (type == SKN_TYPE_Q4_K ? 1 : 2));
