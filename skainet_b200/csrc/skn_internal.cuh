@@ -210,7 +210,7 @@ bool skn_rows_try_group(skn_ctx *ctx, int n, const skn_tensor *const *w, const f
                         bool swiglu, cudaStream_t stream, cudaError_t &err);
 // the same on tcgen05 (skn_matvec_batch.cu), 1 to skn_batch_rows(type) rows
 int skn_batch_rows(int32_t type);
-constexpr int SKN_BATCH_MIN = 9;               // rows from which it is the faster one (skn_launch_matvec_acts)
+constexpr int SKN_BATCH_MIN = 9;               // rows from which it is the faster one but for short rows (skn_launch_matvec_acts)
 bool skn_batch_covers(int n, const skn_tensor *const *w);
 bool skn_batch_try_group(skn_ctx *ctx, int n, const skn_tensor *const *w, const float *x, int M, float *const *y,
                          const float *const *add, bool add_per_act, const float *norm_gain, float norm_eps, const float *silu_u,

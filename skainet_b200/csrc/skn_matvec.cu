@@ -967,9 +967,18 @@ cudaError_t skn_launch_matvec_acts(skn_ctx *ctx, int n, const skn_tensor *const 
     if ((w[0]->pitch % 16) != 0) return cudaErrorNotSupported;
     const int64_t K = w[0]->n_cols;
     // nine rows or more: tcgen05, up to 32 rows per pass over the weights; it has no rotary epilogue and no exchange.  Its time
-    // hardly depends on the rows, that of the many-row kernel below grows with them: Q4_K 14336 x 4096 29 us at 3 to 16 rows
-    // against 18 / 34 / 69 at 4 / 8 / 16; 4096 x 4096 13.5 against 10.5 / 12.2 / 22; Q8_0 14336 x 4096 42 (M = 4), 50 (M = 16) against 20, 73.
-    if (M >= SKN_BATCH_MIN && !xc && !rope && skn_batch_covers(n, w)) {
+    // hardly depends on the rows, that of the many-row kernel below grows with them and doubles at nine.  Measured at 9 / 16 rows
+    // against that kernel (Q6_K: against four rows a launch), us:
+    //   Q4_K  14336 x 4096 28.8 / 29.0 (67.5 / 68.5), 4096 x 4096 13.0 / 13.1 (21.2 / 21.7), 8192 x 512 8.2 / 8.3 (8.3 / 8.8)
+    //   Q4_0  14336 x 4096 37.3 / 37.5 (80.2 / 81.0), 4096 x 4096 14.6 / 14.7 (24.0 / 24.6), 512 x 512 7.5 / 7.6 (7.9 / 8.2)
+    //   Q8_0  14336 x 4096 43.8 / 44.1 (71.4 / 73.1), 4096 x 4096 16.0 / 16.2 (10 rows 26.8), 8192 x 512 8.8 / 8.8 (8.5 / 8.8)
+    //   Q6_K  14336 x 4096 59 / 59 (92 / 134), 4096 x 4096 21.1 / 21.2 (38 / 57), 512 x 512 9.2 / 9.3 (12.7 / 18.8)
+    // Rows of two or three super-blocks of Q4_K with one group of 16 rows per SM stay with the many-row kernel to 16 rows:
+    // 2048 x 512 7.3 / 7.3 us there, 7.5 / 7.5 here; 512 x 768 7.2 / 7.3 and 7.4 / 7.5; from four super-blocks on they are level.
+    int64_t groups = 0;
+    for (int t = 0; t < n; ++t) groups += (w[t]->n_rows + 15) / 16;
+    const bool short_rows = w[0]->type == SKN_TYPE_Q4_K && M <= 16 && K <= 768 && groups <= ctx->sm_count && skn_rows_max_acts(ctx, n, w) >= M;
+    if (M >= SKN_BATCH_MIN && !short_rows && !xc && !rope && skn_batch_covers(n, w)) {
         const int rows = skn_batch_rows(w[0]->type), launches = (M + rows - 1) / rows;
         for (int i = 0, m0 = 0; i < launches; ++i) {
             const int na = (M - m0 + (launches - i) - 1) / (launches - i);       // even shares

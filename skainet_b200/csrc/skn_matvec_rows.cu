@@ -1,7 +1,8 @@
-// K2 for small batches (3 to 8 rows, and 9 to 16 where skn_matvec_batch.cu does not take the tensors, in ONE launch): Y[M, N] = X[M, K] . W_q[N, K]^T with the weights
-// streamed from HBM exactly once.  Same arithmetic as skn_matvec_mma.cu -- exact integer dot products of 32-weight
-// sub-blocks with the digit planes of the activations on the tensor cores (mma.sync m16n8k32, one MMA serves two
-// activation rows), integer sub-block scales, fp32 across super-blocks -- but organised for many rows:
+// K2 for small batches (3 to 8 rows, and 9 to 16 of short rows or in a graph captured without the larger buffer of
+// skn_matvec_batch.cu, in ONE launch): Y[M, N] = X[M, K] . W_q[N, K]^T with the weights streamed from HBM exactly once.
+// Same arithmetic as skn_matvec_mma.cu -- exact integer dot products of 32-weight sub-blocks with the digit planes of the
+// activations on the tensor cores (mma.sync m16n8k32, one MMA serves two activation rows), integer sub-block scales, fp32
+// across super-blocks -- but organised for many rows:
 //
 //   * x is prepared ONCE per launch by a kernel of its own (skn_xprep_kernel: one CTA per activation row applies
 //     the optional RMSNorm or silu(x) * u, then writes the four digit planes, the block scales, the group sums and

@@ -31,6 +31,14 @@ def test_batch_edges(ctx, qt, M, N, K):
     check(ctx, qt, synth.make_weight(g, qt, N, K), synth.make_activations(g, M, K), N, K, g.standard_normal(N).astype(np.float32) if M % 2 else None)
 
 
+@pytest.mark.parametrize("M", [9, 16, 17])
+@pytest.mark.parametrize("N,K", [(16 * 148, 512), (16 * 148 + 1, 512), (333, 768), (333, 1024)])
+def test_short_rows_on_both_sides_of_the_rule(ctx, N, K, M):
+    """Q4_K rows of two and three super-blocks, one group of 16 weight rows per SM and 16 activation rows at most: the many-row kernel."""
+    g = synth.rng(N + K + M)
+    check(ctx, synth.Q4_K, synth.make_weight(g, synth.Q4_K, N, K), synth.make_activations(g, M, K), N, K, g.standard_normal(N).astype(np.float32))
+
+
 @pytest.mark.parametrize("qt", TYPES)
 def test_batch_outliers_zeros_and_scales(ctx, qt):
     """Rows of zeros, of one element, of outliers up to 1e6 in the block, of very different sizes; the towering elements meet zero weights."""
