@@ -1,5 +1,7 @@
 """Batches of 9 to 63 activation rows (tcgen05 with exact fp16 integers) against the fp64 oracle, at the edges of chunks, tiles,
 launches and parts of K; the tolerance of the single-row kernels."""
+import threading
+
 import numpy as np
 import pytest
 import torch
@@ -9,6 +11,7 @@ from conftest import FP32_TOL, assert_close_dot
 from oracle import oracle
 from skainet_b200 import synth
 from skainet_b200.llama import LlamaConfig, LlamaDecoder
+from test_gpu_matvec import _zero_weight_at as zero_weight_at
 
 pytestmark = pytest.mark.gpu
 TYPES = [synth.Q4_0, synth.Q8_0, synth.Q4_K, synth.Q6_K]
@@ -40,11 +43,24 @@ def test_short_rows_on_both_sides_of_the_rule(ctx, N, K, M):
 
 
 @pytest.mark.parametrize("qt", TYPES)
-def test_batch_outliers_zeros_and_scales(ctx, qt):
-    """Rows of zeros, of one element, of outliers up to 1e6 in the block, of very different sizes; the towering elements meet zero weights."""
+@pytest.mark.parametrize("zero_weight", [False, True])
+def test_batch_outliers_zeros_and_scales(ctx, qt, zero_weight):
+    """Rows of zeros, of one element, of very different sizes, and of two outliers in every 256 elements, up to 1e6 times the others.  They meet
+    ordinary weights (an outlier's own product), or zero weights: then the bound is that of the others alone, which a fixed-point
+    form with the outliers left in would miss by far (2^-30 of 4e6)."""
     g = synth.rng(5)
     M, N, K = 12, 48, 1024
     w = synth.make_weight(g, qt, N, K)
+    cols = np.sort(np.concatenate([np.arange(5, K, 256), np.arange(130, K, 256)]))
+    if zero_weight:
+        e = synth.GEOMETRY[qt][0]
+        for first in (5, 130):
+            pos = np.full(K // e, -1)
+            pos[np.arange(first, K, 256) // e] = first % e
+            keep, w0 = pos < 0, w.reshape(N, K // e, -1).copy()
+            w = zero_weight_at(qt, w, N, K, np.where(keep, 0, pos))
+            w.reshape(N, K // e, -1)[:, keep] = w0[:, keep]
+        assert np.all(oracle.dequant(qt, w).reshape(N, K)[:, cols] == 0.0)
     x = synth.make_activations(g, M, K)
     x[0] = 0
     x[1] = 0
@@ -54,7 +70,12 @@ def test_batch_outliers_zeros_and_scales(ctx, qt):
         x[m, 130::256] *= -size
     x[5] *= 1e-20
     x[6] *= 1e20
-    check(ctx, qt, w, x, N, K)
+    t = skn.QuantTensor(ctx, (N, K), qt, w)
+    y = t.matmul_t(x)
+    t.close()
+    ref, absdot = oracle.matmul(qt, w, N, K, x)
+    for m in range(M):
+        assert_close_dot(y[m], ref[m], absdot[m], FP32_TOL, f"type {qt} row {m}")
 
 
 @pytest.mark.parametrize("qt", TYPES)
@@ -174,6 +195,114 @@ def test_batch_graph_outlives_a_larger_call(qt):
     small.close()
     large.close()
     ctx.close()
+
+
+@pytest.mark.parametrize("qt", TYPES)
+@pytest.mark.parametrize("M", [17, 24, 32])
+@pytest.mark.parametrize("N,K", [(14336, 2560), (1000, 14336)])
+def test_batch_rings_wrap(ctx, qt, N, K, M):
+    """Enough super-blocks per CTA (ten; seven of eight parts of K) that every ring is refilled several times, three and four chunks of rows; sampled outputs."""
+    g = synth.rng(N + M)
+    some = synth.make_weight(g, qt, 256, K).reshape(256, -1)
+    w = np.ascontiguousarray(some[np.arange(N) % 256])
+    x = synth.make_activations(g, M, K)
+    t = skn.QuantTensor(ctx, (N, K), qt, w.reshape(-1))
+    y = t.matmul_t(x)
+    t.close()
+    rows = np.unique(np.concatenate([g.choice(N, size=60, replace=False), [0, N - 1]]))
+    ref, absdot = oracle.matmul(qt, np.ascontiguousarray(w[rows]), rows.size, K, x)
+    assert_close_dot(y[:, rows], ref, absdot, FP32_TOL, f"type {qt} {N}x{K} M={M}")
+    assert np.array_equal(y[:, 256:512], y[:, :256])                 # the same weights in other tiles: the same bits
+
+
+def test_batch_at_the_longest_row(ctx):
+    g = synth.rng(13)
+    check(ctx, synth.Q4_K, synth.make_weight(g, synth.Q4_K, 3, 1 << 18), synth.make_activations(g, 32, 1 << 18), 3, 1 << 18)
+
+
+@pytest.mark.parametrize("qt", TYPES)
+def test_batch_in_relaxed_order_and_on_another_stream(qt):
+    """Products of different sizes share the buffer of prepared activations: declared independent, or on a stream of the caller's, they give the same bits."""
+    g = synth.rng(14)
+    ctx = skn.Context(0)
+    shapes = [(512, 2048, 16), (300, 512, 31), (4096, 4096, 9), (40, 8192, 24)]
+    ts = [skn.QuantTensor(ctx, (n, k), qt, synth.make_weight(g, qt, n, k)) for n, k, _ in shapes]
+    xs = [torch.from_numpy(synth.make_activations(g, m, k)).cuda() for _, k, m in shapes]
+    ys = [[torch.zeros(m, n, device="cuda") for n, _, m in shapes] for _ in range(3)]
+    torch.cuda.synchronize()
+    stream = torch.cuda.Stream()
+    for way in range(3):
+        ctx.set_relaxed_order(way == 1)
+        ctx.set_stream(stream.cuda_stream if way == 2 else None)
+        for _ in range(5):
+            for t, x, y in zip(ts, xs, ys[way]):
+                t.matmul_t_dev(x, x.shape[0], y)
+        ctx.sync()
+    for way in (1, 2):
+        assert all(torch.equal(a, b) for a, b in zip(ys[0], ys[way]))
+    for t in ts:
+        t.close()
+    ctx.close()
+
+
+def test_batch_from_two_threads():
+    """A context per thread: buffers and plans are the context's, what is kept for the device is the same for both."""
+    def work(seed, out):
+        g = synth.rng(seed)
+        ctx = skn.Context(0)
+        for i, qt in enumerate(TYPES * 3):
+            n, k, m = 128 + 40 * i, 512 + 256 * (i % 5), 9 + 2 * i
+            w, x = synth.make_weight(g, qt, n, k), synth.make_activations(g, m, k)
+            t = skn.QuantTensor(ctx, (n, k), qt, w)
+            out.append((qt, w, n, k, x, [t.matmul_t(x) for _ in range(5)]))
+            t.close()
+        ctx.close()
+
+    got = [[], []]
+    threads = [threading.Thread(target=work, args=(20 + i, got[i])) for i in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for out in got:
+        assert len(out) == 3 * len(TYPES)
+        for qt, w, n, k, x, ys in out:
+            ref, absdot = oracle.matmul(qt, w, n, k, x)
+            assert_close_dot(ys[0], ref, absdot, FP32_TOL, f"type {qt} {n}x{k}")
+            assert all(np.array_equal(y, ys[0]) for y in ys)
+
+
+@pytest.mark.parametrize("qt,batch", [(synth.Q4_0, 30), (synth.Q8_0, 24), (synth.Q4_K, 31), (synth.Q6_K, 25)])
+def test_decoder_gate_and_up_of_many_sequences(ctx, qt, batch):
+    """Gate and up interleaved, three and four chunks of rows, a tile for every SM and more super-blocks than a ring holds: a batch of sequences
+    against some of them one by one; fp32 sums, 1e-5 a product."""
+    d, f = 2560, 9472
+    g = synth.rng(batch)
+    cfg = LlamaConfig(n_layers=1, d_model=d, n_heads=4, n_kv_heads=2, head_dim=64, ffn_dim=f, vocab=320, proj_type=qt)
+
+    def weight(n, k):
+        some = synth.make_weight(g, qt, 128, k).reshape(128, -1)
+        return np.ascontiguousarray(some[np.arange(n) % 127]).reshape(-1)
+
+    shapes = dict(wq=(256, d), wk=(128, d), wv=(128, d), wo=(d, 256), w_gate=(f, d), w_up=(f, d), w_down=(d, f))
+    layer = {n: weight(*s) for n, s in shapes.items()}
+    embed, head = (synth.make_weight(g, synth.Q6_K, 320, d) for _ in range(2))
+    gain = np.ones(d, dtype=np.float32)
+    tokens = g.integers(0, 320, size=(batch, 2)).astype(np.int32)
+
+    def logits(rows):
+        m = LlamaDecoder(ctx, cfg, batch=len(rows), max_tokens=1, max_ctx=8)
+        m.set_layer(0, layer, gain, gain)
+        m.set_head(embed, gain, head)
+        out = np.stack([m.forward(np.ascontiguousarray(rows[:, i:i + 1]), want_logits=True)[1] for i in range(rows.shape[1])])
+        m.close()
+        return out.astype(np.float64)
+
+    many = logits(tokens)
+    assert np.isfinite(many).all()
+    for b in (0, 17, batch - 1):
+        one = logits(tokens[b:b + 1])[:, 0]
+        assert np.linalg.norm(many[:, b] - one) <= 1e-3 * np.linalg.norm(one)
 
 
 @pytest.mark.parametrize("batch", [9, 20, 40])

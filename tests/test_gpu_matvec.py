@@ -100,8 +100,8 @@ def test_cfg2_full_shapes_at_batch_16_and_64(ctx, qt, N, K, M):
 @pytest.mark.parametrize("N,K,M", [(28672, 4096, 16), (4096, 14336, 16), (6144, 4096, 8), (4096, 4096, 5), (32000, 4096, 16),
                                    (300, 2304, 7), (33, 256, 3), (1000, 5120, 12)])
 def test_many_rows_in_one_pass(ctx, qt, name, N, K, M):
-    """3 to 16 activation rows: every weight is read once (the many-row kernel for Q4_K / Q8_0 / Q4_0; Q6_K keeps four
-    rows per pass), decoder-size shapes and odd ones (short rows, a row count that does not fill a tile, a short
+    """3 to 16 activation rows: every weight is read once (the many-row kernel for Q4_K / Q8_0 / Q4_0 to eight rows, where Q6_K
+    keeps four rows per pass; the batch kernel from nine), decoder-size shapes and odd ones (short rows, a row count that does not fill a tile, a short
     last K chunk), with a bias."""
     _sampled_rows_case(ctx, qt, N, K, M, seed=6000 + N + K + M, tol=FP32_TOL, n_sample=64, bias=(M % 2 == 1))
 
