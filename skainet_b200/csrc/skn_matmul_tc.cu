@@ -22,8 +22,8 @@
 //
 // Measured (B200, stream of distinct weights with the conversion of x, before -> now; before: one CTA per 128 features x 128 or 256
 // tokens that read its weights with word loads from global memory), us:
-//   512 tokens: 28672 x 4096 Q4_K 187 -> 109; 4096 x 14336 Q4_K 138 -> 67, Q8_0 311 -> 75, Q6_K 213 -> 75; 4096 x 4096 46 -> 32
-//   96 tokens:  28672 x 4096 Q4_K 85 -> 69; 4096 x 14336 133 -> 44; 4096 x 4096 44 -> 24; 1024 x 4096 42 -> 19
+//   512 tokens: 28672 x 4096 Q4_K 187 -> 106; 4096 x 14336 Q4_K 138 -> 64, Q8_0 311 -> 71, Q6_K 213 -> 71; 4096 x 4096 46 -> 29
+//   96 tokens:  28672 x 4096 Q4_K 85 -> 66; 4096 x 14336 133 -> 42; 4096 x 4096 44 -> 22; 1024 x 4096 42 -> 18
 // At 512 tokens the tensor cores bound a stage (1020 clocks for 8 MMAs of 256 x 256 x 16); below 350 the dequantisation does.
 //
 // All waits are bounded.

@@ -23,19 +23,20 @@
 //   other warps < 16  unpack: raw super-block columns -> fp16 operand tiles, in three groups of four
 //   warps 16-23       drain: lane = weight row; scales, offsets (fp32 sums of x), outliers, sums over K in registers; output
 //
-// Measured (B200, graph of distinct weights, us per call with the preparation of x, before -> now):
-//   Q4_K 14336 x 4096: 8 rows 34 -> 31, 16 rows 69 -> 29, 32 rows 137 -> 37; 28672 x 4096: 16 rows 110 -> 57; 4096 x 4096: 22 -> 13.4
-//   Q4_0 4096 x 14336: 16 rows 75 -> 41, 60 rows 299 -> 116; Q8_0 14336 x 4096: 16 rows 73 -> 50
-//   Q6_K 32000 x 4096: 16 rows 236 -> 123; 4096 x 14336: 191 -> 57 (they ran four rows a launch)
-// Bound now: 600 clocks per 64 columns of 128 rows in the hand-overs between unpacking, issuing and draining warps (the products and the
-// arithmetic of each take less than half of that), and about 10 us a call of preparation, start and exchange.
+// Measured (B200, graph of distinct weights, us per call with the preparation of x, the kernels that took these rows before -> now):
+//   Q4_K 14336 x 4096: 16 rows 69 -> 29.0, 32 rows 137 -> 36.5; 28672 x 4096: 16 rows 110 -> 58; 4096 x 4096: 22 -> 13.1
+//   Q4_0 4096 x 14336: 16 rows 75 -> 35.6, 32 rows 149 -> 53; Q8_0 14336 x 4096: 16 rows 73 -> 44, 24 rows 143 -> 53
+//   Q6_K 28672 x 4096: 16 rows 221 -> 117; 4096 x 14336: 186 -> 54 (they ran four rows a launch)
+// Bound now by the hand-overs between unpacking, issuing and draining warps, 680 (Q4_K, 16 rows) to 1000 (Q4_0) clocks per 64 columns of
+// 128 rows (half of the issue slots, 9 to 12 % of the tensor pipe and 11 to 13 % of DRAM are used), and by about 7 us a call of preparation,
+// start and exchange.
 #include "skn_mma_common.cuh"
 #include "skn_tc.cuh"
 
 #include <atomic>
 
 constexpr int MB_ROWS = 128;                       // a stage: two 128-byte wide operand tiles of 64 columns (one tile per
-                                                  // stage left the issuing thread with 680 clocks of waits and commits per 64 columns)
+                                                  // stage cost the issuing thread its waits and commits every 64 columns)
 constexpr int MB_A_TILE = MB_ROWS * 128, MB_A_BYTES = 2 * MB_A_TILE;
 constexpr int MB_THREADS = 24 * 32;
 constexpr int MB_DQ_WARPS = 12, MB_DQ_GROUPS = 3, MB_DRAIN = 16, MB_DRAIN_WARPS = 8;
@@ -657,10 +658,10 @@ static int mb_row_bytes(int type) {
     return type == SKN_TYPE_Q8_0 ? MbFmt<SKN_TYPE_Q8_0>::ROW : (type == SKN_TYPE_Q6_K ? MbFmt<SKN_TYPE_Q6_K>::ROW : MbFmt<SKN_TYPE_Q4_K>::ROW);
 }
 
-// K over as many CTAs of a cluster as make the launch shortest, in SM clocks: a start and end of 9000, MB_STAGE_CLOCKS per 64 columns
-// of 128 rows (Q4_K and Q4_0 at 16 rows; the other types are off by one factor, which decides nothing), 500 for the exchange (at 2000
-// rows of two super-blocks stayed in one CTA: 512 x 512 at 16 rows 8.7 us, split 7.4, Q4_0 9.2 and 7.6, Q8_0 8192 x 768 13.3 and 11.0).
-// `fit[s]` = CTAs in flight in clusters of s.
+// K over as many CTAs of a cluster as make the launch shortest: a start and end of 9000, MB_STAGE_CLOCKS per 64 columns of 128 rows and 500 for
+// the exchange, in units of about 1.4 clocks (a launch of one super-block takes 7.3 us, 64 columns of Q4_K 680 clocks at 16 rows; Q4_0 and
+// Q8_0 weigh more than they are given).  At 2000 for the exchange rows of two super-blocks stayed in one CTA: 512 x 512 at 16 rows
+// 8.7 us, split 7.4, Q4_0 9.2 and 7.6, Q8_0 8192 x 768 13.3 and 11.0.  `fit[s]` = CTAs in flight in clusters of s.
 constexpr int MB_STAGE_CLOCKS = 500;
 static mb_plan mb_make_plan(int type, int nch, int64_t tiles, int K, const int *fit) {
     mb_plan pl = {};
