@@ -14,33 +14,32 @@
 // 28.9 us for 14336 x 4096 at 16 rows.  The scale d of a block multiplies what is drained.
 //
 // What bounded the mma.sync form of this (skn_matvec_rows.cu) was the chain load, MMA, integer multiply-add per 16 rows x
-// 32 columns of eight warps; here a thread that unpacks 64 weights needs about two instructions per weight, one thread
-// issues the MMAs for 128 rows, and a drained number stands for 256 (32) products.
+// 32 columns of eight warps; here a thread that unpacks 64 weights needs about two instructions per weight, two threads
+// issue the MMAs for 128 rows, and a drained number stands for 256 (32) products.
 //
 // A CTA owns 128 weight rows (DUAL: 16 gate rows, 16 up rows, ...) x a part of K; the c CTAs of a cluster share K and add their
 // sums through distributed shared memory in rank order.
-//   warps 4 i, i < 4  warp 0 issues MMAs, warp 4 the TMA of the digit planes, warp 8 that of the raw blocks and block records
-//   other warps < 16  unpack: raw super-block columns -> fp16 operand tiles, in three groups of four
-//   warps 16-23       drain: lane = weight row; scales, offsets (fp32 sums of x), outliers, sums over K in registers; output
+//   unpacking warps   raw super-block columns -> fp16 weight stages, in groups of four
+//   four warps        the TMA of the digit planes, that of the raw blocks and block records, and two that issue MMAs
+//   draining warps    lane = weight row; scales, offsets (fp32 sums of x), outliers, sums over K in registers; output
 //
-// Measured (B200, graph of distinct weights, us per call with the preparation of x, the kernels that took these rows before -> now):
-//   Q4_K 14336 x 4096: 16 rows 69 -> 29.0, 32 rows 137 -> 36.5; 28672 x 4096: 16 rows 110 -> 58; 4096 x 4096: 22 -> 13.1
-//   Q4_0 4096 x 14336: 16 rows 75 -> 35.6, 32 rows 149 -> 53; Q8_0 14336 x 4096: 16 rows 73 -> 44, 24 rows 143 -> 53
-//   Q6_K 28672 x 4096: 16 rows 221 -> 117; 4096 x 14336: 186 -> 54 (they ran four rows a launch)
-// Bound now by the hand-overs between unpacking, issuing and draining warps, 680 (Q4_K, 16 rows) to 1000 (Q4_0) clocks per 64 columns of
-// 128 rows (half of the issue slots, 9 to 12 % of the tensor pipe and 11 to 13 % of DRAM are used), and by about 7 us a call of preparation,
-// start and exchange.
+// Measured (B200, graph of distinct weights, us per call with the preparation of x; the kernels that took these rows before -> one issuing warp, weights
+// in shared memory, eight draining warps -> now):
+//   Q4_K 14336 x 4096: 16 rows 69 -> 28.1 -> 23.6, 32 rows 137 -> 35.6 -> 29.1; 28672 x 4096: 16 rows 110 -> 56 -> 46.6; 4096 x 4096: 22 -> 13.2 -> 11.5
+//   Q4_0 4096 x 14336: 16 rows 75 -> 35.5 -> 32.0, 32 rows 149 -> 52.5 -> 45.8; Q8_0 14336 x 4096: 16 rows 73 -> 43.6 -> 34.7, 24 rows 143 -> 52.2 -> 49.6
+//   Q6_K 32000 x 4096: 16 rows 116 -> 93; 4096 x 14336: 186 -> 53.6 -> 44
+// No one part bounds it: for 14336 x 4096 Q4_K with any of unpacking, products and draining left out it took 24 of 26 us, with all of them left out (rings,
+// barriers and loads of the blocks only) 15.4, of which 7.5 are preparation, start and end; two instead of one issuing warp gave 1.0, a second set of
+// draining warps 0.8, a fourth unpacking group 0.8.  A deeper ring of blocks, and blocks copied as contiguous pieces, gave nothing.
 #include "skn_mma_common.cuh"
 #include "skn_tc.cuh"
 
 #include <atomic>
 
-constexpr int MB_ROWS = 128;                       // a stage: two 128-byte wide operand tiles of 64 columns (one tile per
+constexpr int MB_ROWS = 128;                       // a stage: two weight tiles of 64 columns (one tile per
                                                   // stage cost the issuing thread its waits and commits every 64 columns)
-constexpr int MB_A_TILE = MB_ROWS * 128, MB_A_BYTES = 2 * MB_A_TILE;
-constexpr int MB_THREADS = 24 * 32;
-constexpr int MB_DQ_WARPS = 12, MB_DQ_GROUPS = 3, MB_DRAIN = 16, MB_DRAIN_WARPS = 8;
-constexpr int MB_MMA = 0, MB_TMA_X = 4, MB_TMA_W = 8;
+constexpr int MB_A_TILE = 32, MB_A_COLS = 2 * MB_A_TILE;           // ... in columns of tensor memory
+constexpr int MB_A_BYTES = 2 * MB_ROWS * 128;                      // ... in shared memory
 constexpr int MB_CHUNK = 8, MB_COLS = 32;         // activation rows of a chunk; its columns (three or four digits of eight rows)
 constexpr int MB_MAX_A = 4, MB_MAX_B = 6, MB_MAX_RAW = 4, MB_MAX_D = 8, MB_MAX_SPLIT = 8;
 constexpr int MB_SMEM_MAX = 224 * 1024;
@@ -223,10 +222,12 @@ __device__ __forceinline__ uint64_t mb_bytes2(uint32_t w, int i) {
     return skn_add2(skn_pack2u(__byte_perm(w, 0x4B000000u, 0x7440 + i), __byte_perm(w, 0x4B000000u, 0x7441 + i)), skn_pack2(-8388608.f, -8388608.f));
 }
 
-// the sum that row a's digit sums stand for
-template <int DIGITS> __device__ __forceinline__ float mb_join(const uint32_t (&D)[32], int a) {
-    if constexpr (DIGITS == 3) return fmaf(__uint_as_float(D[a]), 4194304.f, fmaf(__uint_as_float(D[8 + a]), 2048.f, __uint_as_float(D[16 + a])));
-    return fmaf(fmaf(__uint_as_float(D[a]), 256.f, __uint_as_float(D[8 + a])), 65536.f, fmaf(__uint_as_float(D[16 + a]), 256.f, __uint_as_float(D[24 + a])));
+// the sums that the digit sums of rows a and a + 1 stand for
+template <int DIGITS> __device__ __forceinline__ uint64_t mb_join(const uint32_t (&D)[32], int a) {
+    const uint64_t d0 = skn_pack2u(D[a], D[a + 1]), d1 = skn_pack2u(D[8 + a], D[9 + a]), d2 = skn_pack2u(D[16 + a], D[17 + a]);
+    if constexpr (DIGITS == 3) return skn_fma2(d0, skn_pack2(4194304.f, 4194304.f), skn_fma2(d1, skn_pack2(2048.f, 2048.f), d2));
+    const uint64_t b = skn_pack2(256.f, 256.f);
+    return skn_fma2(skn_fma2(d0, b, d1), skn_pack2(65536.f, 65536.f), skn_fma2(d2, b, skn_pack2u(D[24 + a], D[25 + a])));
 }
 
 // The outliers of the record at m times their dequantised weights of the block at `blk`.  Rare and out of line: inlined for every
@@ -247,20 +248,51 @@ struct mb_args {
     const float *add[3];
     int64_t addstride[3];
 };
+// Where the weight stages live.  In tensor memory a thread stores its row with two or four instructions and neither its stores nor the MMAs' reads of
+// them meet the digit tiles in shared memory (16 rows, one issuing warp: Q4_K 14336 x 4096 28.1 -> 26.2, Q8_0 43.6 -> 35.9, Q6_K 32000 x 4096 116 -> 100 us).  Q4_0 and Q8_0 from three chunks on keep shared memory: they drain two
+// blocks of 32 columns at a time, an accumulator each, and beside weights tensor memory would hold one such set (4096 x 14336 Q4_0 at 24 and 32
+// rows 49.8 and 52.5 us; with weights in tensor memory and a block at a time 58.7 and 61.7).
+__host__ __device__ constexpr bool mb_ts(int type, int nch) { return type == SKN_TYPE_Q4_K || type == SKN_TYPE_Q6_K || nch <= 2; }
+// columns of an accumulator set
+__host__ __device__ constexpr int mb_set_cols(int type, int nch) { return nch * MB_COLS * (type == SKN_TYPE_Q4_K ? 1 : 2); }
+// weight stages in tensor memory: one per unpacking group at least (a group tells its stage's turn by the parity of a phase), a fourth where that
+// leaves two accumulator sets; and the sets
+__host__ __device__ constexpr int mb_ts_stages(int type, int nch) { return (512 - 4 * MB_A_COLS) / mb_set_cols(type, nch) >= 2 ? 4 : 3; }
+__host__ __device__ constexpr int mb_sets(int type, int nch) {
+    const int n = (512 - (mb_ts(type, nch) ? mb_ts_stages(type, nch) * MB_A_COLS : 0)) / mb_set_cols(type, nch);
+    return n > 8 ? 8 : n;
+}
+// The warps of a kernel: unpacking groups of four, four special ones (MMA, digits, blocks, MMA), draining ones.
+//   GROUPS  a group per weight stage where there are four
+//   SETS    draining: the super-blocks of Q4_K, the 64-column tiles of Q4_0 and Q8_0 in turn
+//   PARTS   ... and the chunks of x
+// The threads share 64 K registers, and a draining thread holds its sums for all its rows of x, so what pays depends on those (us): Q4_0 4096 x 14336 and
+// Q8_0 14336 x 4096 at 16 rows, three groups and two sets 32.0 and 34.7, four groups and one set 35.2 and 37.9; Q4_K 14336 x 4096 at 16 rows, four groups
+// and two sets 23.6, three 24.5; at 24 and 32 rows three groups and one set 27.7 and 29.1, four groups 30.2 and 30.8.
+template <int TYPE, int NCH> struct MbWarps {
+    static constexpr bool FOUR = mb_ts(TYPE, NCH) && mb_ts_stages(TYPE, NCH) == 4, K4 = TYPE == SKN_TYPE_Q4_K, BLOCK = TYPE == SKN_TYPE_Q4_0 || TYPE == SKN_TYPE_Q8_0;
+    static constexpr int GROUPS = FOUR && !(BLOCK && NCH > 1) && !(K4 && NCH > 2) ? 4 : 3;
+    static constexpr int SETS = !(K4 || BLOCK) || NCH > 2 ? 1 : 2;
+    static constexpr int PARTS = NCH == 1 || (K4 && NCH == 2) ? 1 : 2;
+    static constexpr int MMA = 4 * GROUPS, TMA_X = MMA + 1, TMA_W = MMA + 2, MMA2 = MMA + 3, DRAIN = MMA + 4, DRAINS = 4 * SETS * PARTS, THREADS = 32 * (DRAIN + DRAINS);
+};
 struct mb_plan {
     int split, a, b, raw, d;                      // CTAs that share K; ring depths (weight tiles, digit tiles, raw columns, accumulators)
     size_t smem;
 };
 
 template <int TYPE, int NCH, bool DUAL>
-__global__ void __launch_bounds__(MB_THREADS, 1)
+__global__ void __launch_bounds__((MbWarps<TYPE, NCH>::THREADS), 1)
 skn_matvec_batch_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_w0, const __grid_constant__ CUtensorMap tm_w1,
                         const __grid_constant__ CUtensorMap tm_w2, const mb_args ar, int K, const mb_plan pl, const mb_meta *__restrict__ meta,
                         int32_t *__restrict__ status) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    constexpr bool TS = mb_ts(TYPE, NCH);
+    typedef MbWarps<TYPE, NCH> WP;
+    constexpr int SETS = WP::SETS, PARTS = WP::PARTS;
     constexpr int ROW = MbFmt<TYPE>::ROW, RAW_BYTES = MB_ROWS * ROW, BLOCKS = MbFmt<TYPE>::BLOCKS;
-    constexpr int NCOL = NCH * MB_COLS, SET_COLS = TYPE == SKN_TYPE_Q4_K ? NCOL : 2 * NCOL, B_TILE = NCOL * 128, STAGES = MbFmt<TYPE>::STAGES, B_TILES = 4 / STAGES, B_BYTES = B_TILES * B_TILE, META_BYTES = NCH * MB_CHUNK * MB_META;
+    constexpr int NCOL = NCH * MB_COLS, SET_COLS = mb_set_cols(TYPE, NCH), B_TILE = NCOL * 128, STAGES = MbFmt<TYPE>::STAGES, B_TILES = 4 / STAGES, B_BYTES = B_TILES * B_TILE, META_BYTES = NCH * MB_CHUNK * MB_META;
     __shared__ uint64_t a_full[MB_MAX_A], a_empty[MB_MAX_A], b_full[MB_MAX_B], b_empty[MB_MAX_B], raw_full[MB_MAX_RAW], meta_full[MB_MAX_RAW],
         raw_empty[MB_MAX_RAW], d_full[MB_MAX_D], d_empty[MB_MAX_D];
     __shared__ uint32_t tmem_slot;
@@ -268,7 +300,7 @@ skn_matvec_batch_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_c
     const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
     const int c = pl.split, kr = c > 1 ? (int)tc_cluster_rank() : 0, tile = (int)blockIdx.x / c;
     const int na = pl.a, nb = pl.b, nraw = pl.raw, nd = pl.d;
-    uint8_t *b_ring = smem + (size_t)na * MB_A_BYTES, *raw_ring = b_ring + (size_t)nb * B_BYTES, *meta_ring = raw_ring + (size_t)nraw * RAW_BYTES;
+    uint8_t *b_ring = smem + (TS ? 0 : (size_t)na * MB_A_BYTES), *raw_ring = b_ring + (size_t)nb * B_BYTES, *meta_ring = raw_ring + (size_t)nraw * RAW_BYTES;
     float *slots = reinterpret_cast<float *>(smem);                // over the rings, once all CTAs of the cluster are done with them
     const int nsb = K / 256, sb0 = kr * nsb / c, sb1 = (kr + 1) * nsb / c, steps = STAGES * (sb1 - sb0);
     // the tile's tensor and first row
@@ -280,15 +312,15 @@ skn_matvec_batch_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_c
     if (threadIdx.x == 0) {
         for (int s = 0; s < na; ++s) {
             skn_mbar_init(&a_full[s], 4);
-            skn_mbar_init(&a_empty[s], 1);
+            skn_mbar_init(&a_empty[s], TYPE == SKN_TYPE_Q4_K ? 1 : 2);       // a commit by every warp that reads the stage
         }
         for (int s = 0; s < nb; ++s) {
             skn_mbar_init(&b_full[s], 1);
-            skn_mbar_init(&b_empty[s], 1);
+            skn_mbar_init(&b_empty[s], TYPE == SKN_TYPE_Q4_K ? 1 : 2);
         }
         for (int s = 0; s < nd; ++s) {
-            skn_mbar_init(&d_full[s], 1);
-            skn_mbar_init(&d_empty[s], MB_DRAIN_WARPS);
+            skn_mbar_init(&d_full[s], TYPE == SKN_TYPE_Q6_K ? 2 : 1);
+            skn_mbar_init(&d_empty[s], 4 * PARTS);
         }
         skn_fence_mbar_init();
     }
@@ -310,30 +342,31 @@ skn_matvec_batch_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_c
         skn_bulk_g2s(meta_ring + (size_t)rs * META_BYTES, meta + (size_t)sb * (NCH * MB_CHUNK), META_BYTES, &meta_full[rs]);
     };
     const int early = min(nraw, sb1 - sb0);
-    if (warp == MB_TMA_W && lane == 0) {
+    if (warp == WP::TMA_W && lane == 0) {
         for (int s = 0; s < nraw; ++s) {
             skn_mbar_init(&raw_full[s], 1);
             skn_mbar_init(&meta_full[s], 1);
-            skn_mbar_init(&raw_empty[s], MB_DQ_WARPS + MB_DRAIN_WARPS);
+            skn_mbar_init(&raw_empty[s], 4 * WP::GROUPS + (BLOCKS == 1 ? 4 * PARTS : WP::DRAINS));
         }
         skn_fence_mbar_init();
         skn_fence_proxy_async();
         for (int i = 0; i < early; ++i) load_raw(sb0 + i, i);      // the weights depend on no launch before this one
     }
-    if (warp == MB_MMA) tc_alloc(&tmem_slot, TMEM_COLS);
+    if (warp == WP::MMA) tc_alloc(&tmem_slot, TMEM_COLS);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem_base = tmem_slot;
+    const uint32_t tmem_base = tmem_slot, tmem_a = tmem_base + TMEM_COLS - (uint32_t)(na * MB_A_COLS);      // accumulators, then weight stages
 
     bool failed = false;
     auto give_up = [&]() {
         failed = true;
         atomicExch(status, SKN_ERR_TIMEOUT);
     };
-    if (warp < MB_DRAIN && (warp & 3)) {
+    if (warp < WP::MMA) {
         // ---------------- unpack: group `turn` takes the stages 3 i + turn ----------------
-        const int dq = (warp >> 2) * 3 + (warp & 3) - 1, turn = dq >> 2, r = (dq & 3) * 32 + lane;
+        const int turn = warp >> 2, r = (warp & 3) * 32 + lane;
+        const uint32_t ta = tmem_a + ((uint32_t)(r & 96) << 16);
         const uint32_t raw0 = skn_smem_u32(raw_ring) + (uint32_t)(r * ROW);
         int s = turn % na, rs = 0, it = turn;
         uint32_t ph = (uint32_t)(turn / na), rph = 0;
@@ -343,35 +376,45 @@ skn_matvec_batch_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_c
             const uint32_t row = raw0 + (uint32_t)(rs * RAW_BYTES);
             const int lead = TYPE == SKN_TYPE_Q6_K ? ((sb0 + sb) * 210) & 15 : 0;
 #pragma unroll 1
-            for (; it / STAGES == sb; it += MB_DQ_GROUPS) {
+            for (; it / STAGES == sb; it += WP::GROUPS) {
                 uint32_t sc[2] = {0, 0}, mn[2];
                 if (TYPE == SKN_TYPE_Q4_K) mb_q4k_scales(tc_lds128(row), sc, mn);
                 const uint32_t sc4 = sc[it & 1];           // scales of the stage's four sub-blocks
 #pragma unroll 1
                 for (int v = 0; v < 2; ++v) {              // the stage's two tiles
-                    uint8_t *tile_a = smem + (size_t)s * MB_A_BYTES + v * MB_A_TILE;
+                    const uint32_t to = ta + (uint32_t)(s * MB_A_COLS + v * MB_A_TILE);
+                    uint8_t *tile_a = smem + (size_t)s * MB_A_BYTES + v * (MB_A_BYTES / 2);
 #pragma unroll
                     for (int g = 0; g < 2; ++g) {
                         uint32_t p[16];
                         mb_half<TYPE>(row, STAGES == 4 ? it & 3 : 2 * (it & 1) + v, g, (sc4 >> (16 * v)) & 0xFFFFu, p, lead, v);
                         if (v == 0 && g == 0 && !failed && !tc_wait_warp(&a_empty[s], ph ^ 1u, lane)) give_up();
+                        if constexpr (!TS) {
 #pragma unroll
-                        for (int i = 0; i < 4; ++i) {
-                            const int chunk = TYPE == SKN_TYPE_Q4_K ? 4 * (i >> 1) + 2 * g + (i & 1) : 4 * g + i;
-                            tc_store_chunk(tile_a, r, chunk, make_uint4(p[4 * i], p[4 * i + 1], p[4 * i + 2], p[4 * i + 3]));
+                            for (int i = 0; i < 4; ++i) tc_store_chunk(tile_a, r, 4 * g + i, make_uint4(p[4 * i], p[4 * i + 1], p[4 * i + 2], p[4 * i + 3]));
+                        } else if constexpr (TYPE == SKN_TYPE_Q4_K) {  // 16 columns of either sub-block
+                            tc_st8(to + (uint32_t)(8 * g), p);
+                            tc_st8(to + (uint32_t)(16 + 8 * g), p + 8);
+                        } else {
+                            tc_st16(to + (uint32_t)(16 * g), p);
                         }
                     }
                 }
-                skn_fence_proxy_async();
+                if constexpr (TS) {
+                    tc_wait_st();
+                    tc_fence_before();
+                } else {
+                    skn_fence_proxy_async();
+                }
                 __syncwarp();
                 if (lane == 0) skn_mbar_arrive(&a_full[s]);
-                for (s += MB_DQ_GROUPS; s >= na; s -= na) ph ^= 1u;
+                for (s += WP::GROUPS; s >= na; s -= na) ph ^= 1u;
             }
             __syncwarp();
             if (lane == 0) skn_mbar_arrive(&raw_empty[rs]);
             if (++rs == nraw) { rs = 0; rph ^= 1u; }
         }
-    } else if (warp == MB_TMA_W) {
+    } else if (warp == WP::TMA_W) {
         // ---------------- raw blocks, and the block records of the activations (previous launch's output) ----------------
         if (lane == 0) {
             skn_pdl_wait();
@@ -386,87 +429,100 @@ skn_matvec_batch_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_c
                 if (++rs == nraw) { rs = 0; rph ^= 1u; }
             }
         }
-    } else if (warp == MB_TMA_X) {
+    } else if (warp == WP::TMA_X) {
         if (lane == 0) {
             skn_pdl_wait();
             int s = 0;
             uint32_t ph = 0;
             for (int it = 0; it < steps; ++it) {
-                if (!failed && !skn_mbar_wait(&b_empty[s], ph ^ 1u)) give_up();
+                if (!failed && !skn_mbar_wait(TS ? &a_empty[s] : &b_empty[s], ph ^ 1u)) give_up();
                 skn_mbar_expect_tx(&b_full[s], B_BYTES);
                 for (int v = 0; v < B_TILES; ++v)
                     tc_tma_load_2d(b_ring + (size_t)s * B_BYTES + v * B_TILE, &tm_x, (sb0 * STAGES + it) * (64 * B_TILES) + 64 * v, 0, &b_full[s]);
                 if (++s == nb) { s = 0; ph ^= 1u; }
             }
         }
-    } else if (warp == MB_MMA) {
+    } else if (warp == WP::MMA || warp == WP::MMA2) {
         // ---------------- MMAs: 128 rows x NCOL columns, fp16 operands, one accumulator per scale block ----------------
+        // Two warps share them: Q4_K's super-blocks in turn, the two tiles of a stage of the others (of Q6_K the two parts of the scale).  A wait
+        // by parity tells a phase from the one before it only, so a warp has to see every phase of a barrier that it waits for: the tiles'
+        // warps see every stage, and Q4_K's super-blocks of two stages meet the same two of four stages, and the same half of the sets, each time.
+        // (The unpacking groups and the digits' warp see a stage of one warp free while one of the other two stages before is not: they are never two
+        // uses behind, because a raw column is loaded only when the super-block MB_MAX_RAW before it is drained.)
+        static_assert(TYPE != SKN_TYPE_Q4_K || (mb_ts_stages(TYPE, NCH) == 2 * STAGES && MB_MAX_RAW * STAGES <= 2 * mb_ts_stages(TYPE, NCH)), "a warp's stages");
+        static_assert(TYPE == SKN_TYPE_Q6_K || mb_sets(TYPE, NCH) % 2 == 0, "a warp's sets");
         // (a wait has one answer for the warp: its lanes elect, and fail, together)
         constexpr uint32_t idesc = (1u << 4) | ((uint32_t)(NCOL >> 3) << 17) | ((uint32_t)(MB_ROWS >> 4) << 24);
         const uint64_t a0 = tc_smem_desc(skn_smem_u32(smem)), b0 = tc_smem_desc(skn_smem_u32(b_ring));
+        const int p = warp == WP::MMA ? 0 : 1;
         int s = 0, tb = 0, d = 0;
         uint32_t ph = 0, pb = 0, pd = 0;
-        for (int it = 0; it < steps; ++it) {
-            if (!failed && !tc_wait_warp(&b_full[tb], pb, &a_full[s], ph, lane)) failed = true;
-            const uint64_t ad = a0 + (uint64_t)(s * (MB_A_BYTES >> 4)), bd = b0 + (uint64_t)(tb * (B_BYTES >> 4));
-            // K step k (16 columns): 32 bytes inside a tile's swizzle atom = +2 in the address field
-            if constexpr (TYPE == SKN_TYPE_Q6_K) {
-                if ((it & 3) == 0 && !failed && !tc_wait_warp(&d_empty[d], pd ^ 1u, lane)) failed = true;
-                tc_fence_after();
-                if (tc_elect()) {
-#pragma unroll
-                    for (int k = 0; k < 8; ++k)
-                        tc_mma_bf16(tmem_base + d * SET_COLS + (k >> 2) * NCOL, ad + (k >> 2) * (MB_A_TILE >> 4) + 2 * (k & 3), bd + 2 * (k & 3), idesc,
-                                    ((it & 3) || (k & 3)) ? 1u : 0u);
-                    if ((it & 3) == 3) tc_commit(&d_full[d]);
-                }
-                if ((it & 3) == 3 && ++d == nd) { d = 0; pd ^= 1u; }
-            } else if constexpr (BLOCKS == 1) {
-                if ((it & 1) == 0 && !failed && !tc_wait_warp(&d_empty[d], pd ^ 1u, lane)) failed = true;
-                tc_fence_after();
-                if (tc_elect()) {
-#pragma unroll
-                    for (int k = 0; k < 8; ++k)
-                        tc_mma_bf16(tmem_base + d * SET_COLS, ad + (k >> 2) * (MB_A_TILE >> 4) + 2 * (k & 3), bd + (k >> 2) * (B_TILE >> 4) + 2 * (k & 3), idesc,
-                                    ((it & 1) || k) ? 1u : 0u);
-                    if (it & 1) tc_commit(&d_full[d]);
-                }
-                if ((it & 1) && ++d == nd) { d = 0; pd ^= 1u; }
-            } else {
-                // two blocks of 32 columns per tile, an accumulator each
-#pragma unroll
-                for (int v = 0; v < 2; ++v) {
-                    if (!failed && !tc_wait_warp(&d_empty[d], pd ^ 1u, lane)) failed = true;
+        auto pass = [&](int stages, int sets) {            // on in the three rings
+            for (s += stages; s >= na; s -= na) ph ^= 1u;
+            for (tb += stages; tb >= nb; tb -= nb) pb ^= 1u;
+            for (d += sets; d >= nd; d -= nd) pd ^= 1u;
+        };
+        if constexpr (TYPE == SKN_TYPE_Q4_K) {
+            if (p) pass(STAGES, 1);
+            for (int sb = p; sb < steps / STAGES; sb += 2) {
+#pragma unroll 1
+                for (int j = 0; j < STAGES; ++j) {
+                    if (!failed && !tc_wait_warp(&b_full[tb], pb, &a_full[s], ph, lane)) failed = true;
+                    if (j == 0 && !failed && !tc_wait_warp(&d_empty[d], pd ^ 1u, lane)) failed = true;
                     tc_fence_after();
+                    const uint32_t ad = tmem_a + (uint32_t)(s * MB_A_COLS), to = tmem_base + (uint32_t)(d * SET_COLS);
+                    const uint64_t bd = b0 + (uint64_t)(tb * (B_BYTES >> 4));
                     if (tc_elect()) {
+                        // K step k (16 columns): 8 columns of weights; 32 bytes inside a digit tile's swizzle atom = +2 in the address field
 #pragma unroll
-                        for (int k = 0; k < 4; ++k)
-                            tc_mma_bf16(tmem_base + d * SET_COLS + (k >> 1) * NCOL, ad + v * (MB_A_TILE >> 4) + 2 * k, bd + v * (B_TILE >> 4) + 2 * k, idesc, (uint32_t)(k & 1));
-                        tc_commit(&d_full[d]);
+                        for (int k = 0; k < 8; ++k) tc_mma_ts(to, ad + 8 * k, bd + (k >> 2) * (B_TILE >> 4) + 2 * (k & 3), idesc, (j || k) ? 1u : 0u);
+                        tc_commit(&a_empty[s]);
+                        if (j == STAGES - 1) tc_commit(&d_full[d]);
                     }
-                    if (++d == nd) { d = 0; pd ^= 1u; }
+                    pass(1, 0);
                 }
+                pass(STAGES, 2);                           // the other warp's
             }
-            if (tc_elect()) {
-                tc_commit(&a_empty[s]);
-                tc_commit(&b_empty[tb]);
+        } else {
+            // Q6_K: a set of two accumulators, one per part, over four stages; Q4_0 and Q8_0: a set per tile, an accumulator for each of its two blocks
+            constexpr bool Q6 = TYPE == SKN_TYPE_Q6_K;
+            pass(0, Q6 ? 0 : p);
+            for (int it = 0; it < steps; ++it) {
+                const bool first = !Q6 || (it & 3) == 0, last = !Q6 || (it & 3) == 3;
+                if (!failed && !tc_wait_warp(&b_full[tb], pb, &a_full[s], ph, lane)) failed = true;
+                if (first && !failed && !tc_wait_warp(&d_empty[d], pd ^ 1u, lane)) failed = true;
+                tc_fence_after();
+                const uint32_t ad = tmem_a + (uint32_t)(s * MB_A_COLS + MB_A_TILE * p), to = tmem_base + (uint32_t)(d * SET_COLS + (Q6 ? p * NCOL : 0));
+                const uint64_t am = a0 + (uint64_t)(s * (MB_A_BYTES >> 4) + p * (MB_A_BYTES >> 5)), bd = b0 + (uint64_t)(tb * (B_BYTES >> 4) + (Q6 ? 0 : p * (B_TILE >> 4)));
+                if (tc_elect()) {
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {
+                        const uint32_t acc = Q6 ? ((it & 3) || k ? 1u : 0u) : (uint32_t)(k & 1), dst = to + (uint32_t)(Q6 ? 0 : (k >> 1) * NCOL);
+                        if constexpr (TS) tc_mma_ts(dst, ad + 8 * k, bd + 2 * k, idesc, acc);
+                        else tc_mma_bf16(dst, am + 2 * k, bd + 2 * k, idesc, acc);
+                    }
+                    if (last) tc_commit(&d_full[d]);
+                    tc_commit(&a_empty[s]);
+                    if constexpr (!TS) tc_commit(&b_empty[tb]);
+                }
+                pass(1, last ? (Q6 ? 1 : 2) : 0);
             }
-            if (++s == na) { s = 0; ph ^= 1u; }
-            if (++tb == nb) { tb = 0; pb ^= 1u; }
         }
         if (failed && lane == 0) atomicExch(status, SKN_ERR_TIMEOUT);
-    } else if (warp >= MB_DRAIN) {
+    } else if (warp >= WP::DRAIN) {
         // ---------------- drain: lane = weight row ----------------
-        const int wq = warp & 3, r = wq * 32 + lane, odd = (warp - MB_DRAIN) >> 2;     // the two warps of a row quarter take the chunks in turn
-        constexpr int MINE = (NCH + 1) / 2;
+        const int wq = warp & 3, r = wq * 32 + lane, part = ((warp - WP::DRAIN) >> 2) % PARTS, set = ((warp - WP::DRAIN) >> 2) / PARTS;
+        constexpr int MINE = (NCH + PARTS - 1) / PARTS;    // the chunks part, part + PARTS, ...
         const uint32_t raw0 = skn_smem_u32(raw_ring) + (uint32_t)(r * ROW), meta0 = skn_smem_u32(meta_ring);
         float y[MINE * MB_CHUNK];
 #pragma unroll
         for (int a = 0; a < MINE * MB_CHUNK; ++a) y[a] = 0.f;
-        int rs = 0, d = 0;
+        // (Q4_K: a set's super-blocks meet the same half of the raw columns and of the accumulators each time; see the issuing warps)
+        constexpr int TURN = BLOCKS == 1 ? SETS : 1;
+        int rs = TURN > 1 ? set : 0, d = set;
         uint32_t rph = 0, pd = 0;
 #pragma unroll 1
-        for (int sb = sb0; sb < sb1; ++sb) {
+        for (int sb = sb0 + (TURN > 1 ? set : 0); sb < sb1; sb += TURN) {
             if (!failed && !tc_wait_warp(&raw_full[rs], rph, lane)) give_up();
             if (!failed && !tc_wait_warp(&meta_full[rs], rph, lane)) give_up();
             const uint32_t row = raw0 + (uint32_t)(rs * RAW_BYTES), mt = meta0 + (uint32_t)(rs * META_BYTES);
@@ -477,7 +533,7 @@ skn_matvec_batch_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_c
                 tc_fence_after();
 #pragma unroll
                 for (int i = 0; i < MINE; ++i) {
-                    const int ch = 2 * i + odd;
+                    const int ch = PARTS * i + part;
                     if (ch >= NCH) break;
                     const uint32_t at = tmem_base + (uint32_t)(d * SET_COLS + ch * MB_COLS) + ((uint32_t)(wq * 32) << 16);
                     float v[MB_CHUNK];
@@ -499,7 +555,7 @@ skn_matvec_batch_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_c
                 __syncwarp();
                 if (lane == 0) skn_mbar_arrive(&d_empty[d]);
                 if (++d == nd) { d = 0; pd ^= 1u; }
-            } else if constexpr (BLOCKS == 1) {
+            } else if constexpr (TYPE == SKN_TYPE_Q4_K) {
                 const uint4 hdr = tc_lds128(row);
                 const float2 dd = __half22float2(*reinterpret_cast<const __half2 *>(&hdr.x));
                 uint32_t sc[2], mn[2];
@@ -514,34 +570,40 @@ skn_matvec_batch_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_c
                 tc_fence_after();
 #pragma unroll
                 for (int i = 0; i < MINE; ++i) {
-                    const int ch = 2 * i + odd;
+                    const int ch = PARTS * i + part;
                     if (ch >= NCH) break;
                     uint32_t D[32];
-                    tc_ld32(tmem_base + (uint32_t)(d * NCOL + ch * MB_COLS) + ((uint32_t)(wq * 32) << 16), D);
+                    tc_ld32(tmem_base + (uint32_t)(d * SET_COLS + ch * MB_COLS) + ((uint32_t)(wq * 32) << 16), D);
 #pragma unroll
-                    for (int a = 0; a < MB_CHUNK; ++a) {
-                        const uint32_t m = mt + (uint32_t)((ch * MB_CHUNK + a) * MB_META);
-                        const float sx = mm_lds32f(m);
-                        const uint4 s0 = tc_lds128(m + 32), s1 = tc_lds128(m + 48);
-                        uint64_t off = skn_fma2(of[0], skn_pack2u(s0.x, s0.y), 0ull);
-                        off = skn_fma2(of[1], skn_pack2u(s0.z, s0.w), off);
-                        off = skn_fma2(of[2], skn_pack2u(s1.x, s1.y), off);
-                        off = skn_fma2(of[3], skn_pack2u(s1.z, s1.w), off);
-                        float even, uneven;
-                        skn_unpack2(off, even, uneven);
-                        y[i * MB_CHUNK + a] += fmaf(mb_join<4>(D, a), dd.x * sx, even + uneven);
+                    for (int a = 0; a < MB_CHUNK; a += 2) {
+                        float off[2], sx[2];
+#pragma unroll
+                        for (int e = 0; e < 2; ++e) {
+                            const uint32_t m = mt + (uint32_t)((ch * MB_CHUNK + a + e) * MB_META);
+                            sx[e] = dd.x * mm_lds32f(m);
+                            const uint4 s0 = tc_lds128(m + 32), s1 = tc_lds128(m + 48);
+                            uint64_t o = skn_fma2(of[0], skn_pack2u(s0.x, s0.y), 0ull);
+                            o = skn_fma2(of[1], skn_pack2u(s0.z, s0.w), o);
+                            o = skn_fma2(of[2], skn_pack2u(s1.x, s1.y), o);
+                            o = skn_fma2(of[3], skn_pack2u(s1.z, s1.w), o);
+                            float even, uneven;
+                            skn_unpack2(o, even, uneven);
+                            off[e] = even + uneven;
+                        }
+                        float *to = y + i * MB_CHUNK + a;
+                        skn_unpack2(skn_add2(skn_pack2(to[0], to[1]), skn_fma2(mb_join<4>(D, a), skn_pack2(sx[0], sx[1]), skn_pack2(off[0], off[1]))), to[0], to[1]);
                     }
                 }
                 tc_fence_before();
                 __syncwarp();
                 if (lane == 0) skn_mbar_arrive(&d_empty[d]);
-                if (++d == nd) { d = 0; pd ^= 1u; }
+                for (d += SETS; d >= nd; d -= nd) pd ^= 1u;
             } else {
-                float z[MINE * MB_CHUNK];                           // sums over the super-block: short chains of roundings
+                uint64_t z[MINE * MB_CHUNK / 2];                    // sums over the super-block: short chains of roundings
 #pragma unroll
-                for (int a = 0; a < MINE * MB_CHUNK; ++a) z[a] = 0.f;
+                for (int a = 0; a < MINE * MB_CHUNK / 2; ++a) z[a] = 0ull;
 #pragma unroll 1
-                for (int u = 0; u < 4; ++u) {
+                for (int u = set; u < 4; u += SETS) {
                     if (!failed && !tc_wait_warp(&d_full[d], pd, lane)) give_up();
                     tc_fence_after();
 #pragma unroll
@@ -549,30 +611,35 @@ skn_matvec_batch_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_c
                         const float dj = mm_lds_half(row + (uint32_t)((2 * u + j) * (TYPE == SKN_TYPE_Q4_0 ? 18 : 34)));
 #pragma unroll
                         for (int i = 0; i < MINE; ++i) {
-                            const int ch = 2 * i + odd;
+                            const int ch = PARTS * i + part;
                             if (ch >= NCH) break;
                             uint32_t D[32];
                             tc_ld32(tmem_base + (uint32_t)(d * SET_COLS + j * NCOL + ch * MB_COLS) + ((uint32_t)(wq * 32) << 16), D);
 #pragma unroll
-                            for (int a = 0; a < MB_CHUNK; ++a) z[i * MB_CHUNK + a] = fmaf(mb_join<3>(D, a), dj, z[i * MB_CHUNK + a]);
+                            for (int a = 0; a < MB_CHUNK; a += 2)
+                                z[(i * MB_CHUNK + a) / 2] = skn_fma2(mb_join<3>(D, a), skn_pack2(dj, dj), z[(i * MB_CHUNK + a) / 2]);
                         }
                     }
                     tc_fence_before();
                     __syncwarp();
                     if (lane == 0) skn_mbar_arrive(&d_empty[d]);
-                    if (++d == nd) { d = 0; pd ^= 1u; }
+                    for (d += SETS; d >= nd; d -= nd) pd ^= 1u;
                 }
 #pragma unroll
                 for (int a = 0; a < MINE * MB_CHUNK; ++a)
-                    if (2 * (a / MB_CHUNK) + odd < NCH) y[a] = fmaf(z[a], mm_lds32f(mt + (uint32_t)((MB_CHUNK * (2 * (a / MB_CHUNK) + odd) + a % MB_CHUNK) * MB_META)), y[a]);
+                    if (PARTS * (a / MB_CHUNK) + part < NCH) {
+                        float z0, z1;
+                        skn_unpack2(z[a / 2], z0, z1);
+                        y[a] = fmaf(a & 1 ? z1 : z0, mm_lds32f(mt + (uint32_t)((MB_CHUNK * (PARTS * (a / MB_CHUNK) + part) + a % MB_CHUNK) * MB_META)), y[a]);
+                    }
             }
             // outliers (rare): their products with the whole dequantised weight
             uint32_t any = 0;
-            for (int a = lane; a < ar.n_act; a += 32) any |= mm_lds32(mt + (uint32_t)(a * MB_META) + 4) & 0xFFu;
+            for (int a = BLOCKS == 1 || set == 0 ? lane : ar.n_act; a < ar.n_act; a += 32) any |= mm_lds32(mt + (uint32_t)(a * MB_META) + 4) & 0xFFu;
             if (__any_sync(0xffffffffu, any != 0)) {
 #pragma unroll
                 for (int a = 0; a < MINE * MB_CHUNK; ++a) {
-                    const int act = MB_CHUNK * (2 * (a / MB_CHUNK) + odd) + a % MB_CHUNK;
+                    const int act = MB_CHUNK * (PARTS * (a / MB_CHUNK) + part) + a % MB_CHUNK;
                     const uint32_t m = mt + (uint32_t)(act * MB_META);
                     const int n = act < ar.n_act ? (int)(mm_lds32(m + 4) & 0xFFu) : 0;
                     if (n > 0) y[a] += mb_outliers<MbFmt<TYPE>::MM>(blk, m, n);
@@ -580,7 +647,19 @@ skn_matvec_batch_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_c
             }
             __syncwarp();
             if (lane == 0) skn_mbar_arrive(&raw_empty[rs]);
-            if (++rs == nraw) { rs = 0; rph ^= 1u; }
+            for (rs += TURN; rs >= nraw; rs -= nraw) rph ^= 1u;
+        }
+        if constexpr (SETS == 2) {
+            // the second set's sums join the first's, through the rings that both are done with
+            float *meet = slots + (part * MINE * MB_CHUNK) * MB_ROWS + r;
+            asm volatile("barrier.sync 1, %0;" ::"n"(32 * WP::DRAINS) : "memory");
+            if (set)
+#pragma unroll
+                for (int a = 0; a < MINE * MB_CHUNK; ++a) meet[a * MB_ROWS] = y[a];
+            asm volatile("barrier.sync 1, %0;" ::"n"(32 * WP::DRAINS) : "memory");
+            if (!set)
+#pragma unroll
+                for (int a = 0; a < MINE * MB_CHUNK; ++a) y[a] += meet[a * MB_ROWS];
         }
         skn_pdl_launch_dependents();
         skn_pdl_wait();                                            // y and add belong to earlier launches
@@ -589,8 +668,8 @@ skn_matvec_batch_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_c
             tc_cluster_sync();
 #pragma unroll
             for (int i = 0; i < MINE; ++i) {
-                const int ch = 2 * i + odd, owner = ch % c;
-                if (ch >= NCH || owner == kr) continue;
+                const int ch = PARTS * i + part, owner = ch % c;
+                if (set || ch >= NCH || owner == kr) continue;
                 const uint32_t to = tc_mapa(skn_smem_u32(slots) + (uint32_t)(((ch / c) * (c - 1) + (kr < owner ? kr : kr - 1)) * (MB_CHUNK * MB_ROWS) + r) * 4u,
                                             (uint32_t)owner);
 #pragma unroll
@@ -604,8 +683,8 @@ skn_matvec_batch_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_c
         const int64_t N = ar.n_rows[t];
 #pragma unroll
         for (int i = 0; i < MINE; ++i) {
-            const int ch = 2 * i + odd;
-            if (ch >= NCH || ch % c != kr) continue;
+            const int ch = PARTS * i + part;
+            if (set || ch >= NCH || ch % c != kr) continue;
             float v[MB_CHUNK];
 #pragma unroll
             for (int a = 0; a < MB_CHUNK; ++a) v[a] = y[i * MB_CHUNK + a];
@@ -641,13 +720,13 @@ skn_matvec_batch_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_c
         }
     }
     __syncwarp();
-    if (c > 1 && warp < MB_DRAIN) {                                // the other warps' part of the two cluster barriers
+    if (c > 1 && warp < WP::DRAIN) {                                // the other warps' part of the two cluster barriers
         tc_cluster_sync();
         tc_cluster_sync();
     }
     tc_fence_before();
     __syncthreads();
-    if (warp == MB_MMA) {
+    if (warp == WP::MMA) {
         tc_fence_after();
         tc_dealloc(tmem_base, TMEM_COLS);
     }
@@ -673,19 +752,20 @@ static mb_plan mb_make_plan(int type, int nch, int64_t tiles, int K, const int *
         const int64_t cost = waves * (9000 + (c > 1 ? 500 : 0) + (int64_t)((nsb + c - 1) / c) * 4 * MB_STAGE_CLOCKS * (type == SKN_TYPE_Q6_K ? 2 : 1));
         if (best == 0 || cost < best) { best = cost; pl.split = c; }
     }
-    pl.d = 512 / (nch * MB_COLS * (type == SKN_TYPE_Q4_K ? 1 : 2));
-    if (pl.d > MB_MAX_D) pl.d = MB_MAX_D;
-    // a weight tile per unpacking group at least (a group tells its tile's turn by the parity of a phase)
-    pl.a = MB_DQ_GROUPS;
-    pl.b = pl.raw = 2;
-    auto fits = [&](int a, int b, int raw) { return a * MB_A_BYTES + b * b_bytes + raw * raw_bytes <= MB_SMEM_MAX - 1024; };
+    const bool ts = mb_ts(type, nch);
+    pl.a = ts ? mb_ts_stages(type, nch) : 3;
+    pl.d = mb_sets(type, nch);
+    pl.b = ts ? pl.a : 2;                                          // (in tensor memory both tiles of a stage are freed by one commit)
+    pl.raw = 2;                                                    // (an even number: Q4_K's draining sets take them in turn)
+    auto bytes = [&](int a, int b, int raw) { return (ts ? 0 : a * MB_A_BYTES) + b * b_bytes + raw * raw_bytes; };
+    auto fits = [&](int a, int b, int raw) { return bytes(a, b, raw) <= MB_SMEM_MAX - 1024; };
     for (bool grown = true; grown;) {
         grown = false;
-        if (pl.raw < MB_MAX_RAW && fits(pl.a, pl.b, pl.raw + 1)) { ++pl.raw; grown = true; }
-        if (pl.b < MB_MAX_B && fits(pl.a, pl.b + 1, pl.raw)) { ++pl.b; grown = true; }
-        if (pl.a < MB_MAX_A && fits(pl.a + 1, pl.b, pl.raw)) { ++pl.a; grown = true; }
+        if (pl.raw < MB_MAX_RAW && fits(pl.a, pl.b, pl.raw + 2)) { pl.raw += 2; grown = true; }
+        if (!ts && pl.b < MB_MAX_B && fits(pl.a, pl.b + 1, pl.raw)) { ++pl.b; grown = true; }
+        if (!ts && pl.a < MB_MAX_A && fits(pl.a + 1, pl.b, pl.raw)) { ++pl.a; grown = true; }
     }
-    pl.smem = (size_t)pl.a * MB_A_BYTES + (size_t)pl.b * b_bytes + (size_t)pl.raw * raw_bytes + 1024;      // (the partial sums, 28 KB at most, meet in it)
+    pl.smem = (size_t)bytes(pl.a, pl.b, pl.raw) + 1024;      // (the partial sums, 28 KB at most, meet in it)
     return pl;
 }
 
@@ -708,7 +788,7 @@ static cudaLaunchConfig_t mb_config(dim3 grid, dim3 block, int cluster, size_t s
 
 // CTAs in flight in clusters of 1 .. MB_MAX_SPLIT, asked of the driver once per device: the same for all kernels here (threads, shared memory,
 // one CTA per SM); asked of each of them, its first call took 15 to 30 us longer on the host.
-static cudaError_t mb_fits(const skn_ctx *ctx, const void *kern, cudaStream_t stream, int (&f)[MB_MAX_SPLIT + 1]) {
+static cudaError_t mb_fits(const skn_ctx *ctx, const void *kern, int threads, cudaStream_t stream, int (&f)[MB_MAX_SPLIT + 1]) {
     static std::atomic<int> fits[64][MB_MAX_SPLIT + 1];            // 0: not asked yet, -1: none
     std::atomic<int> *fit = fits[ctx->device & 63];
     f[1] = ctx->sm_count;
@@ -716,7 +796,7 @@ static cudaError_t mb_fits(const skn_ctx *ctx, const void *kern, cudaStream_t st
         f[s] = fit[s].load(std::memory_order_relaxed);
         if (f[s]) continue;
         cudaLaunchAttribute attr[2];
-        const cudaLaunchConfig_t cfg = mb_config(dim3(s), dim3(MB_THREADS), s, MB_SMEM_MAX, stream, attr);
+        const cudaLaunchConfig_t cfg = mb_config(dim3(s), dim3(threads), s, MB_SMEM_MAX, stream, attr);
         int k = 0;
         const cudaError_t e = cudaOccupancyMaxActiveClusters(&k, kern, &cfg);
         if (e != cudaSuccess) return e;
@@ -739,7 +819,7 @@ static cudaError_t mb_launch(skn_ctx *ctx, int n, const skn_tensor *const *w, co
         large[ctx->device & 63].store(true, std::memory_order_release);
     }
     int f[MB_MAX_SPLIT + 1] = {0};
-    if ((e = mb_fits(ctx, (const void *)kern, stream, f)) != cudaSuccess) return e;
+    if ((e = mb_fits(ctx, (const void *)kern, MbWarps<TYPE, NCH>::THREADS, stream, f)) != cudaSuccess) return e;
     const int K = (int)w[0]->n_cols, rows_pad = NCH * MB_CHUNK;
     const mb_plan pl = mb_make_plan(TYPE, NCH, tiles, K, f);
     const size_t planes = (size_t)NCH * MB_COLS * K * 2;           // a multiple of 1024
@@ -756,7 +836,7 @@ static cudaError_t mb_launch(skn_ctx *ctx, int n, const skn_tensor *const *w, co
     const int warps = K / 256 < 32 ? K / 256 : 32;
     const cudaLaunchConfig_t prep = mb_config(dim3((unsigned)M), dim3((unsigned)warps * 32), 1, 0, stream, attr);
     if ((e = cudaLaunchKernelEx(&prep, skn_xsplit_kernel<MbFmt<TYPE>::DIGITS>, x, K, gain, eps, silu_u, xp, meta, rows_pad)) != cudaSuccess) return e;
-    const cudaLaunchConfig_t cfg = mb_config(dim3((unsigned)(tiles * pl.split)), dim3(MB_THREADS), pl.split, pl.smem, stream, attr);
+    const cudaLaunchConfig_t cfg = mb_config(dim3((unsigned)(tiles * pl.split)), dim3(MbWarps<TYPE, NCH>::THREADS), pl.split, pl.smem, stream, attr);
     return cudaLaunchKernelEx(&cfg, kern, tx, tw[0], tw[1], tw[2], ar, K, pl, (const mb_meta *)meta, ctx->d_status);
 }
 
