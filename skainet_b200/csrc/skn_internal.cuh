@@ -258,8 +258,13 @@ cudaError_t skn_launch_embed(const skn_tensor *emb, const int32_t *ids, int M, f
 // for all layers at the end of a step
 int32_t skn_kv_rope_append_pending(skn_kvcache *kv, float *q_dev, const float *k_new_dev, const float *v_new_dev,
                                    int32_t n_q_heads, int32_t T, float theta, int32_t host_len_upper);
+// host_len: no sequence had more tokens before the T pending ones.  out_bf16 (optional): where the tensor-core form puts its rows instead, rounded; *wrote_bf16 says whether it did
 int32_t skn_attn_causal_pending(skn_kvcache *kv, const float *q_dev, int32_t n_q_heads, int32_t T, float scale,
-                                float *out_dev);
+                                int32_t host_len, float *out_dev, void *out_bf16 = nullptr, bool *wrote_bf16 = nullptr);
+// the tensor-core form of the many-query kernels (skn_attn_prompt.cu), from this many (query, head) rows on; keys: no sequence holds more
+constexpr int64_t SKN_ATTN_PROMPT_ROWS = 2048;
+bool skn_attn_prompt_takes(const skn_kvcache *kv, int G, int T);
+cudaError_t skn_launch_attn_prompt(const skn_kvcache *kv, const float *q, int G, int T, float scale, int len_extra, int keys, float *out, void *out_bf16, cudaStream_t st);
 int32_t *skn_kv_len_dev(const skn_kvcache *kv);
 cudaError_t skn_kv_advance_all(int32_t *const *lens_dev, int n_layers, int B, int T, int cap, int32_t *status_dev,
                                cudaStream_t st);

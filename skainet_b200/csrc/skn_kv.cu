@@ -1279,7 +1279,7 @@ int32_t skn_kv_append_many_dev(skn_kvcache *kv, const float *k_new_dev, const fl
 // appended): q, out are [batch][T][n_q_heads][head_dim]; query t attends to the cache up to its
 // own token.  T = 1 is skn_attn_decode_dev.  Scratch: T times skn_attn_scratch_bytes().
 static int32_t attn_causal_impl(skn_kvcache *kv, const float *q_dev, int32_t n_q_heads, int32_t T, float scale,
-                                float *out_dev, void *scratch_dev, int len_extra) {
+                                float *out_dev, void *scratch_dev, int len_extra, int keys, void *out_bf16 = nullptr, bool *wrote_bf16 = nullptr) {
     int G = 0;
     int32_t rc = attn_check(kv, n_q_heads, q_dev, out_dev, &G);
     if (rc) return rc;
@@ -1290,6 +1290,11 @@ static int32_t attn_causal_impl(skn_kvcache *kv, const float *q_dev, int32_t n_q
     if ((((uintptr_t)q_dev) | ((uintptr_t)out_dev) | ((uintptr_t)scratch_dev)) & 15)
         return skn_fail(ctx, SKN_ERR_ALIGN, "q, out and scratch must be 16-byte aligned");
     SKN_CUDA(ctx, cudaSetDevice(ctx->device));
+    if (skn_attn_prompt_takes(kv, G, T)) {
+        SKN_CUDA(ctx, skn_launch_attn_prompt(kv, q_dev, G, T, scale, len_extra, keys, out_dev, out_bf16, ctx->stream));
+        if (wrote_bf16) *wrote_bf16 = out_bf16 != nullptr;
+        return SKN_OK;
+    }
     int chunk = ATT_CHUNK;
     float *part = (float *)scratch_dev;
     if (!part) {
@@ -1306,7 +1311,7 @@ static int32_t attn_causal_impl(skn_kvcache *kv, const float *q_dev, int32_t n_q
 
 int32_t skn_attn_causal_dev(skn_kvcache *kv, const float *q_dev, int32_t n_q_heads, int32_t T, float scale,
                             float *out_dev, void *scratch_dev) {
-    return attn_causal_impl(kv, q_dev, n_q_heads, T, scale, out_dev, scratch_dev, 0);
+    return attn_causal_impl(kv, q_dev, n_q_heads, T, scale, out_dev, scratch_dev, 0, skn_kv_ok(kv) ? kv->capacity : 0);
 }
 
 }  // extern "C"
@@ -1340,8 +1345,9 @@ int32_t skn_kv_rope_append_pending(skn_kvcache *kv, float *q_dev, const float *k
 }
 
 int32_t skn_attn_causal_pending(skn_kvcache *kv, const float *q_dev, int32_t n_q_heads, int32_t T, float scale,
-                                float *out_dev) {
-    return attn_causal_impl(kv, q_dev, n_q_heads, T, scale, out_dev, nullptr, T);
+                                int32_t host_len, float *out_dev, void *out_bf16, bool *wrote_bf16) {
+    if (wrote_bf16) *wrote_bf16 = false;
+    return attn_causal_impl(kv, q_dev, n_q_heads, T, scale, out_dev, nullptr, T, host_len + T, out_bf16, wrote_bf16);
 }
 
 int32_t *skn_kv_len_dev(const skn_kvcache *kv) { return kv_ok(kv) ? kv->d_len : nullptr; }

@@ -364,7 +364,7 @@ int32_t skn_llama_forward_dev(skn_llama *m, const int32_t *tokens_dev, int32_t T
                 if (pending) { float *tmp = xcur; xcur = xalt; xalt = tmp; pending = false; }
             }
             if (!rope_fused && (rc = skn_kv_rope_append_pending(l.kv, m->q, m->k, m->v, Hq, T, m->rope_theta, m->host_len))) return rc;
-            if ((rc = skn_attn_causal_pending(l.kv, m->q, Hq, T, scale, m->att))) return rc;
+            if ((rc = skn_attn_causal_pending(l.kv, m->q, Hq, T, scale, m->host_len, m->att))) return rc;
             {
                 const skn_tensor *ws[1] = {l.wo};
                 float *ys[1] = {tp ? m->proj : xcur};
@@ -445,7 +445,8 @@ int32_t skn_llama_forward_dev(skn_llama *m, const int32_t *tokens_dev, int32_t T
         // rotary embedding of q in place and of k on its way into the cache, v alongside; the
         // lengths advance once for all layers at the end of the step
         if ((rc = skn_kv_rope_append_pending(l.kv, m->q, m->k, m->v, Hq, T, m->rope_theta, m->host_len))) return rc;
-        if ((rc = skn_attn_causal_pending(l.kv, m->q, Hq, T, scale, m->att))) return rc;
+        bool att16 = false;
+        if ((rc = skn_attn_causal_pending(l.kv, m->q, Hq, T, scale, m->host_len, m->att, tc ? a16 : nullptr, &att16))) return rc;
         if (small) {
             // ... output projection with the residual added in its epilogue (x += att . Wo^T); with
             // K-sharded weights the partial products meet in the exchange, which adds the residual ...
@@ -505,7 +506,7 @@ int32_t skn_llama_forward_dev(skn_llama *m, const int32_t *tokens_dev, int32_t T
             }
             if (tp && (rc = skn_allreduce_dev(m->comm, m->proj, m->x, m->x, (int64_t)M * d))) return rc;
         } else if (tc) {
-            SKN_CUDA(ctx, skn_launch_f32_to_bf16(m->att, a16, (int64_t)M * qd, ctx->sm_count, st));
+            if (!att16) SKN_CUDA(ctx, skn_launch_f32_to_bf16(m->att, a16, (int64_t)M * qd, ctx->sm_count, st));
             SKN_CUDA(ctx, skn_launch_matmul_tc(ctx, l.wo, a16, M, nullptr, tp ? m->proj : m->x, st, tp ? nullptr : m->x));
             if (tp && (rc = skn_allreduce_dev(m->comm, m->proj, m->x, m->x, (int64_t)M * d))) return rc;
             SKN_CUDA(ctx, skn_launch_rmsnorm_bf16(m->x, l.ffn_norm, a16, M, d, m->rms_eps, st));
