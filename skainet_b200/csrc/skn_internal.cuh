@@ -232,6 +232,7 @@ cudaError_t skn_launch_matvec_group(skn_ctx *ctx, int n, const skn_tensor *const
 // tensor-core prefill path (skn_matmul_tc.cu)
 bool skn_tc_supported(const skn_tensor *w, int32_t M);
 cudaError_t skn_launch_f32_to_bf16(const float *in, void *out_bf16, int64_t n, int sm_count, cudaStream_t stream);
+cudaError_t skn_launch_matmul_tc_group(skn_ctx *ctx, int n, const skn_tensor *const *w, const void *a_bf16, int32_t M, float *const *y, cudaStream_t stream);
 cudaError_t skn_launch_matmul_tc(skn_ctx *ctx, const skn_tensor *w, const void *a_bf16, int32_t M, const float *bias,
                                  float *y, cudaStream_t stream, const float *resid = nullptr);
 cudaError_t skn_launch_gate_up_tc(skn_ctx *ctx, const skn_tensor *wg, const skn_tensor *wu, const void *a_bf16,

@@ -416,9 +416,13 @@ int32_t skn_llama_forward_dev(skn_llama *m, const int32_t *tokens_dev, int32_t T
         }
         if (tc) {
             SKN_CUDA(ctx, skn_launch_rmsnorm_bf16(m->x, l.attn_norm, a16, M, d, m->rms_eps, st));
-            SKN_CUDA(ctx, skn_launch_matmul_tc(ctx, l.wq, a16, M, nullptr, m->q, st));
-            SKN_CUDA(ctx, skn_launch_matmul_tc(ctx, l.wk, a16, M, nullptr, m->k, st));
-            SKN_CUDA(ctx, skn_launch_matmul_tc(ctx, l.wv, a16, M, nullptr, m->v, st));
+            const skn_tensor *ws[3] = {l.wq, l.wk, l.wv};
+            float *ys[3] = {m->q, m->k, m->v};
+            if (l.wk->type == l.wq->type && l.wv->type == l.wq->type) {
+                SKN_CUDA(ctx, skn_launch_matmul_tc_group(ctx, 3, ws, a16, M, ys, st));
+            } else {
+                for (int t = 0; t < 3; ++t) SKN_CUDA(ctx, skn_launch_matmul_tc(ctx, ws[t], a16, M, nullptr, ys[t], st));
+            }
         } else if (small) {
             // decode-size batches, per activation row: RMSNorm folded into the preparation of x
             // for Q/K/V (one launch) ...
