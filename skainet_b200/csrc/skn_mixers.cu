@@ -479,16 +479,137 @@ skn_head_prep_kernel(skn_attn_args a, skn_ret_args r, skn_step st, prep_args p, 
     }
 }
 
+// four numbers into a cache row or prepared queries
+__device__ __forceinline__ void put4(float *to, float4 v) { *reinterpret_cast<float4 *>(to) = v; }
+__device__ __forceinline__ void put4(__nv_bfloat16 *to, float4 v) { *reinterpret_cast<uint2 *>(to) = make_uint2(pack_bf16(v.x, v.y), pack_bf16(v.z, v.w)); }
+
+// The same with a head in registers, four elements per lane and register of NV: for widths, halves of rotations and row strides that are multiples of four
+// and rows on 16 bytes (head_prep_aligned).  The element-wise form above goes through shared memory three times and asks for 32 numbers at a time: 44 us
+// for 2048 rows of 5120 head elements (70 MB), 26 us here; a warp's next head is on its way while it prepares one.
+template <class CT, int NV>
+__global__ void __launch_bounds__(256)
+skn_head_prep_vec_kernel(skn_attn_args a, skn_ret_args r, skn_step st, prep_args p, CT *kc, CT *vc) {
+    skn_pdl_launch_dependents();
+    skn_pdl_wait();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, m = blockIdx.x;
+    const int slot = st.slot0 + m / st.T, pos = min(st.pos[slot] + m % st.T, st.max_pos - 1), at = p.cap ? pos % p.cap : 0;
+    const int nq = a.q16 ? p.H : 0, units = nq + 2 * p.G + 2 * p.RH;
+    // where the raw head of unit u is, and its width
+    auto source = [&](int u, int &w) -> float * {
+        if (u < nq) { w = p.dim; return const_cast<float *>(a.q) + (int64_t)m * a.ld + (int64_t)u * p.dim; }
+        if (u < nq + p.G) { w = p.dim; return const_cast<float *>(a.k) + (int64_t)m * a.ld + (int64_t)(u - nq) * p.dim; }
+        if (u < nq + 2 * p.G) { w = p.vdim; return const_cast<float *>(a.v) + (int64_t)m * a.ld + (int64_t)(u - nq - p.G) * p.vdim; }
+        const int i = u - nq - 2 * p.G;
+        w = p.rdk;
+        return ((i & 1) ? r.k : r.q) + (int64_t)m * r.ld + (int64_t)(i >> 1) * p.rdk;
+    };
+    auto fetch = [&](int u, float4 (&x)[NV]) {
+        int w = 0;
+        const float *src = u < units ? source(u, w) : nullptr;
+#pragma unroll
+        for (int c = 0; c < NV; ++c) {
+            const int d = (c * 32 + lane) * 4;
+            x[c] = d < w ? __ldcg(reinterpret_cast<const float4 *>(src + d)) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+    };
+    float4 x[NV], next[NV];
+    fetch(warp, x);
+    for (int u = warp; u < units; u += 8) {
+        fetch(u + 8, next);
+        int w;
+        float *src = source(u, w);
+        const bool value = u >= nq + p.G && u < nq + 2 * p.G, ret = u >= nq + 2 * p.G;
+        const float *gain = ret || value ? nullptr : u < nq ? a.q_gain : a.k_gain;
+        if (gain) {
+            float ss = 0.f;
+#pragma unroll
+            for (int c = 0; c < NV; ++c) ss += (x[c].x * x[c].x + x[c].y * x[c].y) + (x[c].z * x[c].z + x[c].w * x[c].w);
+            const float f = 1.f / sqrtf(warp_sum(ss) / (float)w + a.eps);
+#pragma unroll
+            for (int c = 0; c < NV; ++c) {
+                const int d = (c * 32 + lane) * 4;
+                if (d >= w) continue;
+                const float4 g = __ldg(reinterpret_cast<const float4 *>(gain + d));
+                x[c] = make_float4(x[c].x * f * g.x, x[c].y * f * g.y, x[c].z * f * g.z, x[c].w * f * g.w);
+            }
+        }
+        const skn_rot &rot = ret ? r.rot : a.rot;
+        if (!value && rot.half > 0) {
+            float4 y[NV];
+#pragma unroll
+            for (int c = 0; c < NV; ++c) {
+                // the other element of a pair is half a rotation away
+                const int d = (c * 32 + lane) * 4, o = (d < rot.half ? d + rot.half : d - rot.half) >> 2, from = o & 31;
+                y[c] = make_float4(__shfl_sync(0xffffffffu, x[0].x, from), __shfl_sync(0xffffffffu, x[0].y, from), __shfl_sync(0xffffffffu, x[0].z, from),
+                                   __shfl_sync(0xffffffffu, x[0].w, from));
+                if (NV > 1) {
+                    const float4 z = make_float4(__shfl_sync(0xffffffffu, x[NV - 1].x, from), __shfl_sync(0xffffffffu, x[NV - 1].y, from),
+                                                 __shfl_sync(0xffffffffu, x[NV - 1].z, from), __shfl_sync(0xffffffffu, x[NV - 1].w, from));
+                    if (o >= 32) y[c] = z;
+                }
+            }
+#pragma unroll
+            for (int c = 0; c < NV; ++c) {
+                const int d = (c * 32 + lane) * 4;
+                if (d >= 2 * rot.half) continue;
+                const bool low = d < rot.half;
+                const float4 *t = reinterpret_cast<const float4 *>(rot.table + (int64_t)m * rot.ld + (low ? d : d - rot.half));
+                const float4 t0 = __ldcg(t), t1 = __ldcg(t + 1);
+                const float sg = low ? -1.f : 1.f;                     // u c - v s, v c + u s
+                x[c] = make_float4(x[c].x * t0.x + sg * (y[c].x * t0.y), x[c].y * t0.z + sg * (y[c].y * t0.w), x[c].z * t1.x + sg * (y[c].z * t1.y),
+                                   x[c].w * t1.z + sg * (y[c].w * t1.w));
+            }
+        }
+        if (ret && ((u - nq - 2 * p.G) & 1) && r.k_scale != 1.f)
+#pragma unroll
+            for (int c = 0; c < NV; ++c) x[c] = make_float4(x[c].x * r.k_scale, x[c].y * r.k_scale, x[c].z * r.k_scale, x[c].w * r.k_scale);
+#pragma unroll
+        for (int c = 0; c < NV; ++c) {
+            const int d = (c * 32 + lane) * 4;
+            if (u < nq) {
+                if (d < p.kp) put4(a.q16 + ((int64_t)m * p.H + u) * p.kp + d, x[c]);
+            } else if (d < w) {
+                if (ret) put4(src + d, x[c]);
+                else if (value) put4(vc + (((size_t)slot * p.G + u - nq - p.G) * p.cap + at) * p.vp + d, x[c]);
+                else put4(kc + (((size_t)slot * p.G + u - nq) * p.cap + at) * p.kp + d, x[c]);
+            }
+            x[c] = next[c];
+        }
+    }
+}
+static bool head_prep_aligned(const skn_attn_args *a, const skn_ret_args *r, const prep_args &p) {
+    uintptr_t at = 0;
+    int64_t n = 0;
+    if (a) {
+        at |= (uintptr_t)a->q | (uintptr_t)a->k | (uintptr_t)a->v | (uintptr_t)a->q_gain | (uintptr_t)a->k_gain | (uintptr_t)a->rot.table | (uintptr_t)a->q16;
+        n |= a->ld | p.dim | p.vdim | p.kp | p.vp | a->rot.half | (a->rot.half ? a->rot.ld : 0);
+    }
+    if (r) {
+        at |= (uintptr_t)r->q | (uintptr_t)r->k | (uintptr_t)r->rot.table;
+        n |= r->ld | p.rdk | r->rot.half | (r->rot.half ? r->rot.ld : 0);
+    }
+    return !(at & 15) && !(n & 3);
+}
+
 // ---- attention on the tensor cores ---------------------------------------------------------------------------------
 constexpr int ATQ = 64, ATK = 32;      // queries and keys of a tile
 constexpr int AT_THREADS = ATQ * 2;    // a warp owns 16 queries
 
-// tanh through one exponential; absolute error a few 1e-7
-__device__ __forceinline__ float tanh_exp(float y) {
-    const float t = __expf(2.f * fminf(fmaxf(y, -20.f), 20.f));
-    return 1.f - __fdividef(2.f, t + 1.f);
+__device__ __forceinline__ float ex2(float x) {
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+__device__ __forceinline__ float rcp(float x) {
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
 }
 
+// What bounds it: the instructions beside the products.  It issued 66 per score and was busy with 8 x 8 products for a quarter of
+// its time (2048 tokens, 16 heads of 128, chunk 1024, soft cap: 135 us).  Now the soft cap is five instructions a score (c - 2 c / (e^(2 s / cap) + 1)
+// needs no clamp: the exponential may overflow), masks are looked at in tiles that have one, outputs are rescaled in tiles that raise a
+// maximum of the warp, fragments are fetched a step ahead of the products that take them, and CTAs with the most keys start first (86 us; 23 would be the products').
 template <int DV>
 __global__ void __launch_bounds__(AT_THREADS, DV <= 128 ? 3 : 1)
 skn_attn_tc_kernel(skn_attn_args a, skn_step st, skn_attn_keys src) {
@@ -499,7 +620,11 @@ skn_attn_tc_kernel(skn_attn_args a, skn_step st, skn_attn_keys src) {
     __nv_bfloat16 *Q = reinterpret_cast<__nv_bfloat16 *>(smb), *K = Q + ATQ * ks, *V = K + 2 * ATK * ks;
     skn_pdl_launch_dependents();
     skn_pdl_wait();
-    const int t0 = (gridDim.x - 1 - blockIdx.x) * ATQ, h = blockIdx.y, seq = blockIdx.z, slot = st.slot0 + seq, g = h / src.group;
+    // query tiles by the keys they see, most first: in chunks, by their place in the chunk
+    const int nt = (st.T + ATQ - 1) / ATQ, pc = a.chunk > 0 ? min(nt, (a.chunk + ATQ - 1) / ATQ) : nt, nc = (nt + pc - 1) / pc;
+    const int qt = ((int)blockIdx.y % nc) * pc + pc - 1 - (int)blockIdx.y / nc;
+    if (qt >= nt) return;
+    const int t0 = qt * ATQ, h = blockIdx.x, seq = blockIdx.z, slot = st.slot0 + seq, g = h / src.group;
     const int p0 = st.pos[slot], nq = min(ATQ, st.T - t0);
     const int pf = p0 + t0, pl = pf + nq - 1;                            // first and last query position
     const int lo = first_visible(a, pf);
@@ -542,7 +667,8 @@ skn_attn_tc_kernel(skn_attn_args a, skn_step st, skn_attn_keys src) {
 #pragma unroll
     for (int i = 0; i < 2; ++i) qlo[i] = first_visible(a, qi[i]);
     const int w0 = pf + warp * 16, wlo = first_visible(a, w0), whi = first_visible(a, w0 + 15);
-    const float inv_cap = a.softcap > 0.f ? a.scale / a.softcap : 0.f;
+    const bool capped = a.softcap > 0.f;
+    const float mul = capped ? 2.f * (a.scale / a.softcap) * L2E : a.scale * L2E, top = a.softcap * L2E;
 
     for (int t = 0; t < tiles; ++t) {
         const int buf = t & 1;
@@ -560,49 +686,83 @@ skn_attn_tc_kernel(skn_attn_args a, skn_step st, skn_attn_keys src) {
 #pragma unroll
         for (int i = 0; i < ATK / 8; ++i) s[i][0] = s[i][1] = s[i][2] = s[i][3] = 0.f;
         const __nv_bfloat16 *Kb = K + (size_t)buf * ATK * ks, *Vb = V + (size_t)buf * ATK * vs;
-        for (int kk = 0; kk < kp; kk += 16) {
-            uint32_t af[4];
-            ldsm4(af, skn_smem_u32(Q + (size_t)(warp * 16 + (lane & 15)) * ks + kk + (lane >> 4) * 8));
+        {
+            const uint32_t qa = skn_smem_u32(Q + (size_t)(warp * 16 + (lane & 15)) * ks + (lane >> 4) * 8),
+                           ka = skn_smem_u32(Kb + (size_t)((lane & 7) + ((lane >> 4) << 3)) * ks + ((lane >> 3) & 1) * 8);
+            uint32_t af[2][4], bf[2][ATK / 16][4];
+            auto load = [&](int kk, int x) {
+                ldsm4(af[x], qa + (uint32_t)kk * 2);
 #pragma unroll
-            for (int n = 0; n < ATK / 16; ++n) {
-                uint32_t bf[4];
-                ldsm4(bf, skn_smem_u32(Kb + (size_t)(n * 16 + (lane & 7) + ((lane >> 4) << 3)) * ks + kk + ((lane >> 3) & 1) * 8));
-                mma_bf16(s[2 * n], af, bf[0], bf[1]);
-                mma_bf16(s[2 * n + 1], af, bf[2], bf[3]);
-            }
+                for (int n = 0; n < ATK / 16; ++n) ldsm4(bf[x][n], ka + (uint32_t)(n * 16 * ks + kk) * 2);
+            };
+            load(0, 0);
+            for (int kk = 0; kk < kp; kk += 32)
+#pragma unroll
+                for (int x = 0; x < 2; ++x) {
+                    if (kk + 16 * x >= kp) break;
+                    if (kk + 16 * x + 16 < kp) load(kk + 16 * x + 16, x ^ 1);
+#pragma unroll
+                    for (int n = 0; n < ATK / 16; ++n) {
+                        mma_bf16(s[2 * n], af[x], bf[x][n][0], bf[x][n][1]);
+                        mma_bf16(s[2 * n + 1], af[x], bf[x][n][2], bf[x][n][3]);
+                    }
+                }
         }
-        float mx[2] = {mrow[0], mrow[1]};
+        if (capped) {
 #pragma unroll
-        for (int n = 0; n < ATK / 8; ++n)
+            for (int n = 0; n < ATK / 8; ++n)
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const int i = e >> 1, j = j0 + n * 8 + (lane & 3) * 2 + (e & 1);
-                float v = a.softcap > 0.f ? a.softcap * tanh_exp(s[n][e] * inv_cap) : s[n][e] * a.scale;
-                v = !masked || (j <= qi[i] && j >= qlo[i]) ? v * L2E : -INFINITY;
-                s[n][e] = v;
-                mx[i] = fmaxf(mx[i], v);
-            }
-        float corr[2], base[2];
+                for (int e = 0; e < 4; ++e) s[n][e] = fmaf(-2.f * top, rcp(ex2(s[n][e] * mul) + 1.f), top);
+        } else {
+#pragma unroll
+            for (int n = 0; n < ATK / 8; ++n)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) s[n][e] *= mul;
+        }
+        if (masked) {
+#pragma unroll
+            for (int n = 0; n < ATK / 8; ++n)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const int i = e >> 1, j = j0 + n * 8 + (lane & 3) * 2 + (e & 1);
+                    if (j > qi[i] || j < qlo[i]) s[n][e] = -INFINITY;
+                }
+        }
+        float base[2];
+        bool grown = false;
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
-            mx[i] = fmaxf(mx[i], __shfl_xor_sync(0xffffffffu, mx[i], 1));
-            mx[i] = fmaxf(mx[i], __shfl_xor_sync(0xffffffffu, mx[i], 2));
-            base[i] = mx[i] == -INFINITY ? 0.f : mx[i];
-            corr[i] = exp2f(mrow[i] - base[i]);
-            mrow[i] = mx[i];
-            lrow[i] *= corr[i];
+            float mx = mrow[i];
+#pragma unroll
+            for (int n = 0; n < ATK / 8; ++n) mx = fmaxf(mx, fmaxf(s[n][2 * i], s[n][2 * i + 1]));
+            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+            base[i] = mx;
+            grown = grown || mx > mrow[i];
         }
+        if (__any_sync(0xffffffffu, grown)) {
+            float corr[2];
 #pragma unroll
-        for (int n = 0; n < ATK / 8; ++n)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                s[n][e] = exp2f(s[n][e] - base[e >> 1]);
-                lrow[e >> 1] += s[n][e];
+            for (int i = 0; i < 2; ++i) {
+                corr[i] = ex2(mrow[i] - (base[i] == -INFINITY ? 0.f : base[i]));
+                mrow[i] = base[i];
+                lrow[i] *= corr[i];
             }
 #pragma unroll
-        for (int i = 0; i < DV / 8; ++i) {
-            o[i][0] *= corr[0]; o[i][1] *= corr[0];
-            o[i][2] *= corr[1]; o[i][3] *= corr[1];
+            for (int i = 0; i < DV / 8; ++i) {
+                o[i][0] *= corr[0]; o[i][1] *= corr[0];
+                o[i][2] *= corr[1]; o[i][3] *= corr[1];
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const float b = base[i] == -INFINITY ? 0.f : base[i];
+#pragma unroll
+            for (int n = 0; n < ATK / 8; ++n) {
+                s[n][2 * i] = ex2(s[n][2 * i] - b);
+                s[n][2 * i + 1] = ex2(s[n][2 * i + 1] - b);
+                lrow[i] += s[n][2 * i] + s[n][2 * i + 1];
+            }
         }
 #pragma unroll
         for (int kk = 0; kk < ATK / 16; ++kk) {
@@ -614,14 +774,17 @@ skn_attn_tc_kernel(skn_attn_args a, skn_step st, skn_attn_keys src) {
                 hi[x] = pack_bf16(w0, w1);
                 lw[x] = pack_bf16(w0 - __uint_as_float(hi[x] << 16), w1 - __uint_as_float(hi[x] & 0xFFFF0000u));
             }
+            const uint32_t va = skn_smem_u32(Vb + (size_t)(kk * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * vs + (lane >> 4) * 8);
+            uint32_t bf[2][4];
+            ldsm4t(bf[0], va);
 #pragma unroll
             for (int n = 0; n < DV / 16; ++n) {
-                uint32_t bf[4];
-                ldsm4t(bf, skn_smem_u32(Vb + (size_t)(kk * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * vs + n * 16 + (lane >> 4) * 8));
-                mma_bf16(o[2 * n], hi, bf[0], bf[1]);
-                mma_bf16(o[2 * n + 1], hi, bf[2], bf[3]);
-                mma_bf16(o[2 * n], lw, bf[0], bf[1]);
-                mma_bf16(o[2 * n + 1], lw, bf[2], bf[3]);
+                if (n + 1 < DV / 16) ldsm4t(bf[(n + 1) & 1], va + (uint32_t)(n + 1) * 32);
+                const uint32_t(&b)[4] = bf[n & 1];
+                mma_bf16(o[2 * n], lw, b[0], b[1]);
+                mma_bf16(o[2 * n + 1], lw, b[2], b[3]);
+                mma_bf16(o[2 * n], hi, b[0], b[1]);
+                mma_bf16(o[2 * n + 1], hi, b[2], b[3]);
             }
         }
         __syncthreads();
@@ -657,7 +820,9 @@ static cudaError_t launch_attn_tc(const skn_step &s, const skn_attn_args &a, con
     const size_t smem = ((size_t)(ATQ + 2 * ATK) * (k.kp + 8) + (size_t)2 * ATK * (DV + 8)) * 2;
     const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     if (e != cudaSuccess) return e;
-    return skn_launch_pdl(kern, dim3((s.T + ATQ - 1) / ATQ, a.heads, s.n_seqs), dim3(AT_THREADS), smem, st, 1, a, s, k);
+    // (whole chunks of query tiles: the kernel orders them)
+    const int nt = (s.T + ATQ - 1) / ATQ, per = (a.chunk + ATQ - 1) / ATQ, pc = a.chunk > 0 && per < nt ? per : nt;
+    return skn_launch_pdl(kern, dim3(a.heads, (nt + pc - 1) / pc * pc, s.n_seqs), dim3(AT_THREADS), smem, st, 1, a, s, k);
 }
 
 cudaError_t skn_launch_attn_tiles(const skn_step &s, const skn_attn_args &a, const skn_attn_keys &k, cudaStream_t st) {
@@ -1035,6 +1200,11 @@ static cudaError_t launch_prep(const skn_step &s, const skn_attn_args *a, const 
     if (r) {
         rr = *r;
         p.RH = r->state->heads; p.rdk = r->state->k_dim;
+    }
+    const int keys = p.kp > p.vdim ? p.kp : p.vdim, widest = keys > p.rdk ? keys : p.rdk;
+    if (widest <= 256 && head_prep_aligned(a ? &aa : nullptr, r, p)) {
+        auto kern = widest <= 128 ? skn_head_prep_vec_kernel<CT, 1> : skn_head_prep_vec_kernel<CT, 2>;
+        return skn_launch_pdl(kern, dim3(s.n_seqs * s.T), dim3(256), 0, st, 1, aa, rr, s, p, kc, vc);
     }
     const size_t smem = (size_t)8 * (p.kp > p.rdk ? p.kp : p.rdk) * sizeof(float);
     return skn_launch_pdl(skn_head_prep_kernel<CT>, dim3(s.n_seqs * s.T), dim3(256), smem, st, 1, aa, rr, s, p, kc, vc);
