@@ -9,7 +9,7 @@
 //                          the weights enter the second product as two bf16 terms, so they keep 16 bits
 //  skn_attn_rows_kernel    the split kernel on prepared keys (fp32 cache, or head widths beyond the tensor-core form)
 //  skn_ret_*_kernel        retention in chunks of 64 tokens: what each chunk adds to the state, the states at the chunk
-//                          starts, and the outputs; on the CUDA cores (fp32 decoder) or the tensor cores (two-term tf32)
+//                          starts, and the outputs; on the CUDA cores (fp32 decoder) or the tensor cores (three bf16 terms)
 #include "skn_mixers.cuh"
 #include "skn_mma.cuh"
 
@@ -911,13 +911,35 @@ skn_ret_scan_kernel(skn_ret_args r, skn_step st, float *S, int H, int dk, int vp
 // rows of O (shared): divided by their root mean square, gated, scaled, stored
 __device__ __forceinline__ void ret_finish(const skn_ret_args &r, const float *O, int os, int64_t row0, int L, int h, int dv) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    for (int t = warp; t < L; t += 8) {
-        float ss = 0.f;
-        for (int d = lane; d < dv; d += 32) ss = fmaf(O[t * os + d], O[t * os + d], ss);
-        const float rs = r.out_scale / sqrtf(warp_sum(ss) / (float)dv + r.eps);
-        for (int d = lane; d < dv; d += 32) {
-            const float g = __ldcg(r.g + (row0 + t) * r.ld + (int64_t)h * dv + d);
-            put_out(r.out, row0 + t, (int64_t)h * dv + d, O[t * os + d] * rs * (g / (1.f + expf(-g))));
+    constexpr int R = 4, C = 4;                    // rows of a warp at a time, and columns per lane: their gates are asked for together
+    for (int t0 = warp * R; t0 < L; t0 += 8 * R) {
+        float ss[R] = {}, g[R][C];
+#pragma unroll
+        for (int i = 0; i < R; ++i)
+#pragma unroll
+            for (int c = 0; c < C; ++c) {
+                const int d = lane + 32 * c;
+                g[i][c] = t0 + i < L && d < dv ? __ldcg(r.g + (row0 + t0 + i) * r.ld + (int64_t)h * dv + d) : 0.f;
+            }
+#pragma unroll
+        for (int i = 0; i < R; ++i)
+            if (t0 + i < L)
+                for (int d = lane; d < dv; d += 32) ss[i] = fmaf(O[(t0 + i) * os + d], O[(t0 + i) * os + d], ss[i]);
+#pragma unroll
+        for (int i = 0; i < R; ++i) ss[i] = r.out_scale / sqrtf(warp_sum(ss[i]) / (float)dv + r.eps);
+#pragma unroll
+        for (int i = 0; i < R; ++i) {
+            const int t = t0 + i;
+            if (t >= L) break;
+#pragma unroll
+            for (int c = 0; c < C; ++c) {
+                const int d = lane + 32 * c;
+                if (d < dv) put_out(r.out, row0 + t, (int64_t)h * dv + d, O[t * os + d] * ss[i] * (g[i][c] / (1.f + expf(-g[i][c]))));
+            }
+            for (int d = lane + 32 * C; d < dv; d += 32) {
+                const float x = __ldcg(r.g + (row0 + t) * r.ld + (int64_t)h * dv + d);
+                put_out(r.out, row0 + t, (int64_t)h * dv + d, O[t * os + d] * ss[i] * (x / (1.f + expf(-x))));
+            }
         }
     }
 }
@@ -1017,163 +1039,256 @@ skn_ret_out_kernel(skn_ret_args r, int T, int H, int dk, int dv, int vp, int nch
 }
 
 // ---- retention chunks on the tensor cores -----------------------------------------------------------------------------
-// Every fp32 operand enters as the sum of two tf32 terms and three products are formed (the lowest is below fp32
-// rounding), summed in fp32: the results carry fp32 accuracy.  Fragments are read from fp32 rows in shared memory; row
-// strides are 4 (rows along M or N) or 8 (rows along K) banks off a multiple of 32, which keeps the reads conflict-free.
-__device__ __forceinline__ void mma_tf32(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-    asm volatile("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
-                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-struct TwoTerm { uint32_t hi, lo; };
-__device__ __forceinline__ TwoTerm two_term(float x) {
-    TwoTerm t;
-    t.hi = __float_as_uint(x) & 0xFFFFE000u;
-    t.lo = __float_as_uint(x - __uint_as_float(t.hi)) & 0xFFFFE000u;
-    return t;
-}
-// c[n] += A (16 x 8 at rows m, column step k) times B (8 x 8 NT): at(row, k) and bt(k, col) read shared memory
-template <int NT, class AT, class BT>
-__device__ __forceinline__ void mma_two_term(float (&c)[NT][4], int k, AT at, BT bt) {
-    const int g = (threadIdx.x & 31) >> 2, t = threadIdx.x & 3;
-    uint32_t ah[4], al[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const TwoTerm x = two_term(at(g + (i & 1) * 8, k + t + (i >> 1) * 4));
-        ah[i] = x.hi;
-        al[i] = x.lo;
-    }
-#pragma unroll
-    for (int n = 0; n < NT; ++n) {
-        const TwoTerm b0 = two_term(bt(k + t, n * 8 + g)), b1 = two_term(bt(k + t + 4, n * 8 + g));
-        mma_tf32(c[n], al, b0.hi, b1.hi);
-        mma_tf32(c[n], ah, b0.lo, b1.lo);
-        mma_tf32(c[n], ah, b0.hi, b1.hi);
-    }
-}
-
+// Every fp32 operand enters as three bf16 terms (skn_mma.cuh), split once where it is stored to shared memory, and sums over 32 elements are
+// added in fp32.  (Two tf32 terms split where fragments were read, a dozen instructions and six scalar loads per product, were bound by
+// those: 2048 tokens, 8 heads of 128 x 128: outputs 61 us, chunk sums 22; now 43 and 18.)  The 32 columns of a block of a
+// warp's tiles share the fragments of its 16 rows; row strides are 16 bytes off a multiple of 128.
 constexpr int RT2 = 128;              // columns of a tile
-constexpr int RKS = RT2 + 8;          // row stride of operands whose rows run along K
+constexpr int RTS = (RT2 + 8) * 2;    // bytes of a row of its planes
 
-// the chunk sums of skn_ret_chunk_kernel, in 128 x 128 tiles; a warp owns 16 rows
-__global__ void __launch_bounds__(256)
+// planes of [rows][32 cols' words...]: pair (x, y) at `at` of the first
+__device__ __forceinline__ void put_terms(uint8_t *at, int plane, float x, float y) {
+    uint32_t w[3];
+    split_terms(x, y, w);
+#pragma unroll
+    for (int p = 0; p < 3; ++p) *reinterpret_cast<uint32_t *>(at + p * plane) = w[p];
+}
+// elements c, c + 1 of a row of n; even: rows start on 8 bytes and n is even
+__device__ __forceinline__ float2 pair_at(const float *row, int c, int n, bool even) {
+    if (even) return c < n ? __ldcg(reinterpret_cast<const float2 *>(row + c)) : make_float2(0.f, 0.f);
+    return make_float2(c < n ? __ldcg(row + c) : 0.f, c + 1 < n ? __ldcg(row + c + 1) : 0.f);
+}
+__device__ __forceinline__ bool pairs_even(const float *p, int64_t ld, int n) { return !((reinterpret_cast<uintptr_t>(p) & 7) | (ld & 1) | (n & 1)); }
+
+// what chunk c adds to the state by its end (see skn_ret_chunk_kernel).  CTA: a 128 x 128 tile, a warp 16 of its rows.
+__global__ void __launch_bounds__(256, 2)
 skn_ret_chunk_tc_kernel(skn_ret_args r, int T, int H, int dk, int dv, int vp, int nchunks, int vtiles) {
-    extern __shared__ __align__(16) float sm[];
+    extern __shared__ __align__(16) uint8_t smb[];
     __shared__ float pw[RC + 1];
-    float *Ks = sm, *Vs = sm + RC * RKS;
+    constexpr int PL = RC * RTS;
+    uint8_t *Ks = smb, *Vs = smb + 3 * PL;
     skn_pdl_launch_dependents();
     skn_pdl_wait();
     const int c = blockIdx.x, h = blockIdx.y % H, seq = blockIdx.y / H, i0 = (blockIdx.z / vtiles) * RT2, j0 = (blockIdx.z % vtiles) * RT2;
     const int t0 = c * RC, L = min(RC, T - t0), tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int64_t row0 = (int64_t)seq * T + t0;
     const float *k = r.k + row0 * r.ld + (int64_t)h * dk + i0, *v = r.v + row0 * r.ld + (int64_t)h * dv + j0;
+    const bool ke = pairs_even(k, r.ld, dk), ve = pairs_even(v, r.ld, dv);
     if (tid <= RC) pw[tid] = r.powers[(size_t)h * (RC + 1) + tid];
     __syncthreads();
-#pragma unroll 8
-    for (int i = tid; i < RC * RT2; i += 256) {
-        const int t = i / RT2, d = i % RT2;
-        Ks[t * RKS + d] = t < L && i0 + d < dk ? __ldcg(k + (int64_t)t * r.ld + d) * pw[L - 1 - t] : 0.f;
-        Vs[t * RKS + d] = t < L && j0 + d < dv ? __ldcg(v + (int64_t)t * r.ld + d) : 0.f;
+    for (int t1 = tid >> 6; t1 < RC; t1 += 32) {
+        float2 a[8], b[8];
+        const int d = (tid & 63) * 2;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const int t = t1 + 4 * i;
+            a[i] = t < L ? pair_at(k + (int64_t)t * r.ld, d, dk - i0, ke) : make_float2(0.f, 0.f);
+            b[i] = t < L ? pair_at(v + (int64_t)t * r.ld, d, dv - j0, ve) : make_float2(0.f, 0.f);
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const int t = t1 + 4 * i;
+            const float f = t < L ? pw[L - 1 - t] : 0.f;
+            put_terms(Ks + t * RTS + d * 2, PL, a[i].x * f, a[i].y * f);
+            put_terms(Vs + t * RTS + d * 2, PL, b[i].x, b[i].y);
+        }
     }
     __syncthreads();
-    float acc[RT2 / 8][4] = {};
-    if (i0 + warp * 16 < dk)
-        for (int kk = 0; kk < RC; kk += 8)
-            mma_two_term(acc, kk, [&](int m, int x) { return Ks[x * RKS + warp * 16 + m]; }, [&](int x, int n) { return Vs[x * RKS + n]; });
+    if (i0 + warp * 16 >= dk) return;
     float *out = r.chunks + ((((size_t)seq * nchunks + c) * H + h) * dk) * vp;
+#pragma unroll 1
+    for (int nb = 0; nb < RT2 / 32 && j0 + nb * 32 < vp; ++nb) {
+        float acc[4][4] = {};
 #pragma unroll
-    for (int e = 0; e < 2; ++e) {
-        const int row = i0 + warp * 16 + (lane >> 2) + e * 8;
-        if (row >= dk) continue;
+        for (int kk = 0; kk < RC; kk += 32) {
+            float s[4][4], m[4][4];
 #pragma unroll
-        for (int n = 0; n < RT2 / 8; ++n) {
-            const int col = j0 + n * 8 + (lane & 3) * 2;
-            if (col < vp) *reinterpret_cast<float2 *>(out + (size_t)row * vp + col) = make_float2(acc[n][2 * e], acc[n][2 * e + 1]);
+            for (int x = 0; x < 2; ++x) {
+                uint32_t af[3][4], bf[2][3][4];
+                const int t = kk + 16 * x;
+#pragma unroll
+                for (int p = 0; p < 3; ++p) {
+                    ldsm4t(af[p], skn_smem_u32(Ks + p * PL + (t + (lane & 7) + ((lane >> 4) << 3)) * RTS + (warp * 16 + ((lane >> 3) & 1) * 8) * 2));
+                    const uint32_t vb = skn_smem_u32(Vs + p * PL + (t + (lane & 7) + ((lane >> 3) & 1) * 8) * RTS + (nb * 32 + (lane >> 4) * 8) * 2);
+                    ldsm4t(bf[0][p], vb);
+                    ldsm4t(bf[1][p], vb + 32);
+                }
+                if (x == 0) mma_terms<3, true>(s, m, af, bf);
+                else mma_terms<3, false>(s, m, af, bf);
+            }
+#pragma unroll
+            for (int n = 0; n < 4; ++n)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) acc[n][e] += m[n][e] + s[n][e];
+        }
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            const int row = i0 + warp * 16 + (lane >> 2) + e * 8;
+            if (row >= dk) continue;
+#pragma unroll
+            for (int n = 0; n < 4; ++n) {
+                const int col = j0 + nb * 32 + n * 8 + (lane & 3) * 2;
+                if (col < vp) *reinterpret_cast<float2 *>(out + (size_t)row * vp + col) = make_float2(acc[n][2 * e], acc[n][2 * e + 1]);
+            }
         }
     }
 }
 
-// the chunk outputs of skn_ret_out_kernel; warp w owns tokens 16 (w & 3) .. and one half of the columns
-// smem (floats): q [RC][dkp + 4] | A [RC][RC + 4] | max(k [RC][dkp + 4], b [32][RKS] and o [RC][vw + 4])
-static size_t ret_out_tc_smem(int dk, int dv) {
-    const size_t qk = (size_t)RC * ((dk + 31) / 32 * 32 + 4), bo = 32 * RKS + (size_t)RC * ((dv + RT2 - 1) / RT2 * RT2 + 4);
-    return (qk + RC * (RC + 4) + (qk > bo ? qk : bo)) * sizeof(float);
-}
+// Outputs of one chunk (see skn_ret_out_kernel).  Bytes of shared memory: planes of q [RC][dkp + 8] | of the scores [RC][RC + 8] | of a tile
+// [32][RT2 + 8] (keys, then rows of the state and values), the fp32 outputs [RC][vw + 4] over the first two when there is one block of
+// columns, else behind.  A warp owns 16 rows and half of a tile's columns.
+struct ret_out_layout {
+    int dkp, vw, lq, la, scores, tile, out, bytes;                      // row strides and offsets in bytes
+    __host__ __device__ ret_out_layout(int dk, int dv) {
+        dkp = (dk + 31) / 32 * 32;
+        vw = (dv + RT2 - 1) / RT2 * RT2;
+        lq = (dkp + 8) * 2;
+        la = (RC + 8) * 2;
+        scores = 3 * RC * lq;
+        tile = scores + 3 * RC * la;
+        const int end = tile + 3 * 32 * RTS, o = RC * (vw + 4) * 4;
+        out = vw == RT2 ? 0 : end;
+        bytes = out ? end + o : end > o ? end : o;
+    }
+};
+constexpr size_t RET_SMEM_MAX = 226 * 1024;
+static size_t ret_out_tc_smem(int dk, int dv) { return (size_t)ret_out_layout(dk, dv).bytes; }
 
 __global__ void __launch_bounds__(256, 2)
 skn_ret_out_tc_kernel(skn_ret_args r, int T, int H, int dk, int dv, int vp, int nchunks) {
-    extern __shared__ __align__(16) float sm[];
+    extern __shared__ __align__(16) uint8_t smb[];
     __shared__ float pw[RC + 1];
-    const int dkp = (dk + 31) / 32 * 32, qs = dkp + 4, vw = (dv + RT2 - 1) / RT2 * RT2, os = vw + 4;
-    constexpr int AS = RC + 4;
-    float *Q = sm, *A = Q + RC * qs, *Kb = A + RC * AS, *B = Kb, *O = Kb + 32 * RKS;
+    const ret_out_layout l(dk, dv);
+    uint8_t *Q = smb, *A = smb + l.scores, *B = smb + l.tile;
+    float *O = reinterpret_cast<float *>(smb + l.out);
+    const int QP = RC * l.lq, AP = RC * l.la, BP = 32 * RTS, os = l.vw + 4;
     skn_pdl_launch_dependents();
     skn_pdl_wait();
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, c = blockIdx.x, h = blockIdx.y, seq = blockIdx.z, t0 = c * RC, L = min(RC, T - t0);
     const int64_t row0 = (int64_t)seq * T + t0;
     const float *q = r.q + row0 * r.ld + (int64_t)h * dk, *k = r.k + row0 * r.ld + (int64_t)h * dk, *v = r.v + row0 * r.ld + (int64_t)h * dv;
+    const float *S = r.chunks + ((((size_t)seq * nchunks + c) * H + h) * dk) * vp;
+    const bool qe = pairs_even(q, r.ld, dk), ke = pairs_even(k, r.ld, dk), ve = pairs_even(v, r.ld, dv), se = pairs_even(S, vp, vp);
     if (tid <= RC) pw[tid] = r.powers[(size_t)h * (RC + 1) + tid];
-    for (int d0 = 0; d0 < dkp; d0 += 32)
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const int t = warp + i * 8, d = d0 + lane;
-            const bool in = t < L && d < dk;
-            Q[t * qs + d] = in ? __ldcg(q + (int64_t)t * r.ld + d) : 0.f;
-            Kb[t * qs + d] = in ? __ldcg(k + (int64_t)t * r.ld + d) : 0.f;
-        }
-    __syncthreads();
     const int m0 = (warp & 3) * 16, half = warp >> 2, g = lane >> 2, t = lane & 3;
-    {
-        float acc[RC / 16][4] = {};
-        const int n0 = half * (RC / 2);
-        if (n0 <= m0 + 15)                         // else every pair of this tile lies in the future
-            for (int kk = 0; kk < dkp; kk += 8)
-                mma_two_term(acc, kk, [&](int m, int x) { return Q[(m0 + m) * qs + x]; }, [&](int x, int n) { return Kb[(n0 + n) * qs + x]; });
+    // columns [from, end) of `rows` rows; a warp's 32 lanes take the words of 64 columns of a row
+    auto rows_in = [&](uint8_t *to, int stride, int plane, const float *src, bool even, int first, int rows, int from, int end) {
+        for (int d0 = from; d0 < end; d0 += 64) {
+            const int d = d0 + 2 * lane;
+            if (d >= end) continue;
+            for (int i = warp; i < rows; i += 64) {
+                float2 x[8];
 #pragma unroll
-        for (int n = 0; n < RC / 16; ++n)
+                for (int j = 0; j < 8; ++j) {
+                    const int y = first + i + 8 * j;
+                    x[j] = i + 8 * j < rows && y < L ? pair_at(src + (int64_t)y * r.ld, d, dk, even) : make_float2(0.f, 0.f);
+                }
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const int i = m0 + g + (e >> 1) * 8, j = n0 + n * 8 + t * 2 + (e & 1);
-                A[i * AS + j] = j <= i ? acc[n][e] * pw[i - j] : 0.f;
+                for (int j = 0; j < 8; ++j)
+                    if (i + 8 * j < rows) put_terms(to + (i + 8 * j) * stride + (d - from) * 2, plane, x[j].x, x[j].y);
+            }
+        }
+    };
+    rows_in(Q, l.lq, QP, q, qe, 0, RC, 0, l.dkp);
+#pragma unroll 1
+    for (int kt = 0; kt < RC; kt += 32) {
+        const int n0 = kt + half * 16;
+        float s[2][4] = {}, rest[2][4] = {};
+#pragma unroll 1
+        for (int d0 = 0; d0 < l.dkp; d0 += RT2) {
+            const int d1 = min(d0 + RT2, l.dkp);
+            if (kt | d0) __syncthreads();          // the keys before are done with
+            rows_in(B, RTS, BP, k, ke, kt, 32, d0, d1);
+            __syncthreads();
+            if (n0 > m0 + 15) continue;            // every pair of this tile lies in the future
+#pragma unroll 1
+            for (int kk = d0; kk < d1; kk += 32) {
+                float sm[2][4], mn[2][4];
+#pragma unroll
+                for (int x = 0; x < 2; ++x) {
+                    uint32_t af[3][4], bf[1][3][4];
+#pragma unroll
+                    for (int p = 0; p < 3; ++p) {
+                        ldsm4(af[p], skn_smem_u32(Q + p * QP + (m0 + (lane & 15)) * l.lq + (kk + 16 * x + (lane >> 4) * 8) * 2));
+                        ldsm4(bf[0][p], skn_smem_u32(B + p * BP + (half * 16 + (lane & 7) + ((lane >> 4) << 3)) * RTS + (kk - d0 + 16 * x + ((lane >> 3) & 1) * 8) * 2));
+                    }
+                    if (x == 0) mma_terms<3, true>(sm, mn, af, bf);
+                    else mma_terms<3, false>(sm, mn, af, bf);
+                }
+#pragma unroll
+                for (int n = 0; n < 2; ++n)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        s[n][e] += mn[n][e];
+                        rest[n][e] += sm[n][e];
+                    }
+            }
+        }
+#pragma unroll
+        for (int n = 0; n < 2; ++n)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const int i = m0 + g + e * 8, j = n0 + n * 8 + t * 2;
+                const float x = j <= i ? (s[n][2 * e] + rest[n][2 * e]) * pw[i - j] : 0.f, y = j + 1 <= i ? (s[n][2 * e + 1] + rest[n][2 * e + 1]) * pw[i - j - 1] : 0.f;
+                put_terms(A + i * l.la + j * 2, AP, x, y);
             }
     }
-    const float *S = r.chunks + ((((size_t)seq * nchunks + c) * H + h) * dk) * vp;
-    constexpr int NT = RT2 / 16;
-    for (int v0 = 0; v0 < vw; v0 += RT2) {
-        float o[NT][4] = {};
+    for (int v0 = 0; v0 < l.vw; v0 += RT2) {
+        float o[8][4] = {};
         const int c0 = half * (RT2 / 2);
         // tiles of 32 rows: the state's first, then the chunk's values
-        const int stiles = dkp / 32, tiles = stiles + (L + 31) / 32;
-        float pre[16];
+        const int stiles = l.dkp / 32, tiles = stiles + (L + 31) / 32;
+        float2 pre[8];
         auto fetch = [&](int x) {
 #pragma unroll
-            for (int i = 0; i < 16; ++i) {
-                const int row = (x < stiles ? x : x - stiles) * 32 + (tid >> 7) + i * 2, col = v0 + (tid & 127);
-                if (x < stiles) pre[i] = row < dk && col < vp ? __ldcg(S + (size_t)row * vp + col) : 0.f;
-                else pre[i] = row < L && col < dv ? __ldcg(v + (int64_t)row * r.ld + col) : 0.f;
+            for (int i = 0; i < 8; ++i) {
+                const int row = (x < stiles ? x : x - stiles) * 32 + (tid >> 6) + i * 4, col = v0 + (tid & 63) * 2;
+                if (x < stiles) pre[i] = row < dk ? pair_at(S + (size_t)row * vp, col, vp, se) : make_float2(0.f, 0.f);
+                else pre[i] = row < L ? pair_at(v + (int64_t)row * r.ld, col, dv, ve) : make_float2(0.f, 0.f);
             }
         };
         fetch(0);
+#pragma unroll 1
         for (int x = 0; x < tiles; ++x) {
-            __syncthreads();                       // the tile before (or k) is done with
+            __syncthreads();                       // the tile before (or the keys) is done with
 #pragma unroll
-            for (int i = 0; i < 16; ++i) B[((tid >> 7) + i * 2) * RKS + (tid & 127)] = pre[i];
+            for (int i = 0; i < 8; ++i) put_terms(B + ((tid >> 6) + i * 4) * RTS + (tid & 63) * 4, BP, pre[i].x, pre[i].y);
             __syncthreads();
             if (x + 1 < tiles) fetch(x + 1);
             if (x == stiles)
 #pragma unroll
-                for (int n = 0; n < NT; ++n)
+                for (int n = 0; n < 8; ++n)
 #pragma unroll
                     for (int e = 0; e < 4; ++e) o[n][e] *= pw[m0 + g + (e >> 1) * 8 + 1];
-            const float *a = x < stiles ? Q + x * 32 : A + (x - stiles) * 32;
-            const int lda = x < stiles ? qs : AS;
-            if (x < stiles || (x - stiles) * 32 <= m0 + 15)
+            const bool state = x < stiles;
+            if (!state && (x - stiles) * 32 > m0 + 15) continue;
+            const uint8_t *a = state ? Q + x * 64 : A + (x - stiles) * 64;
+            const int lda = state ? l.lq : l.la, pla = state ? QP : AP;
 #pragma unroll
-                for (int kk = 0; kk < 32; kk += 8)
-                    mma_two_term(o, kk, [&](int m, int y) { return a[(m0 + m) * lda + y]; }, [&](int y, int n) { return B[y * RKS + c0 + n]; });
+            for (int nb = 0; nb < 2; ++nb) {
+                float sm[4][4], mn[4][4];
+#pragma unroll
+                for (int y = 0; y < 2; ++y) {
+                    uint32_t af[3][4], bf[2][3][4];
+#pragma unroll
+                    for (int p = 0; p < 3; ++p) {
+                        ldsm4(af[p], skn_smem_u32(a + p * pla + (m0 + (lane & 15)) * lda + (y * 16 + (lane >> 4) * 8) * 2));
+                        const uint32_t bb = skn_smem_u32(B + p * BP + (y * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * RTS + (c0 + nb * 32 + (lane >> 4) * 8) * 2);
+                        ldsm4t(bf[0][p], bb);
+                        ldsm4t(bf[1][p], bb + 32);
+                    }
+                    if (y == 0) mma_terms<3, true>(sm, mn, af, bf);
+                    else mma_terms<3, false>(sm, mn, af, bf);
+                }
+#pragma unroll
+                for (int n = 0; n < 4; ++n)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) o[4 * nb + n][e] += mn[n][e] + sm[n][e];
+            }
         }
+        __syncthreads();                           // the outputs may lie over q and the scores
 #pragma unroll
-        for (int n = 0; n < NT; ++n)
+        for (int n = 0; n < 8; ++n)
 #pragma unroll
             for (int e = 0; e < 2; ++e)
                 *reinterpret_cast<float2 *>(O + (m0 + g + e * 8) * os + v0 + c0 + n * 8 + t * 2) = make_float2(o[n][2 * e], o[n][2 * e + 1]);
@@ -1224,13 +1339,13 @@ cudaError_t skn_launch_mix_prefill(skn_ctx *, const skn_step &s, const skn_attn_
     if (r) {
         const int H = r->state->heads, dk = r->state->k_dim, dv = r->state->v_dim, vp = r->state->v_pitch;
         const int nchunks = (s.T + RC - 1) / RC;
-        const bool tc = !r->exact && ret_out_tc_smem(dk, dv) <= 200 * 1024;
+        const bool tc = !r->exact && ret_out_tc_smem(dk, dv) <= RET_SMEM_MAX;
         const int tile = tc ? RT2 : 64, kt = (dk + tile - 1) / tile, vt = (dv + tile - 1) / tile;
         const dim3 cgrid(nchunks, H * s.n_seqs, kt * vt), ogrid(nchunks, H, s.n_seqs);
         if (tc) {
-            e = cudaFuncSetAttribute(skn_ret_chunk_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * RC * RKS * 4);
+            e = cudaFuncSetAttribute(skn_ret_chunk_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 6 * RC * RTS);
             if (e != cudaSuccess) return e;
-            e = skn_launch_pdl(skn_ret_chunk_tc_kernel, cgrid, dim3(256), (size_t)2 * RC * RKS * 4, st, 1, *r, s.T, H, dk, dv, vp, nchunks, vt);
+            e = skn_launch_pdl(skn_ret_chunk_tc_kernel, cgrid, dim3(256), (size_t)6 * RC * RTS, st, 1, *r, s.T, H, dk, dv, vp, nchunks, vt);
         } else {
             e = skn_launch_pdl(skn_ret_chunk_kernel, cgrid, dim3(256), 0, st, 1, *r, s.T, H, dk, dv, vp, nchunks, vt);
         }
@@ -1239,7 +1354,7 @@ cudaError_t skn_launch_mix_prefill(skn_ctx *, const skn_step &s, const skn_attn_
         e = skn_launch_pdl(skn_ret_scan_kernel, dim3((unsigned)((per + 127) / 128), s.n_seqs), dim3(128), 0, st, 1, *r, s, r->state->d, H, dk, vp, nchunks);
         if (e != cudaSuccess) return e;
         if (tc) {
-            e = cudaFuncSetAttribute(skn_ret_out_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+            e = cudaFuncSetAttribute(skn_ret_out_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, RET_SMEM_MAX);
             if (e != cudaSuccess) return e;
             e = skn_launch_pdl(skn_ret_out_tc_kernel, ogrid, dim3(256), ret_out_tc_smem(dk, dv), st, 1, *r, s.T, H, dk, dv, vp, nchunks);
         } else {

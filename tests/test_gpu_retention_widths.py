@@ -1,0 +1,24 @@
+"""Retention in chunks on the tensor cores at the edges of its shared memory: keys in several pieces of 128 columns, values in several blocks of
+128, and the widest that fits beside the first that does not (which runs in fp32 on the CUDA cores)."""
+import numpy as np
+import pytest
+
+from skainet_b200.mixers import RecurrentState
+from tests.test_gpu_lugasun import rel, retention_reference
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("H,D,V", [(2, 128, 129), (1, 129, 128), (1, 256, 256), (1, 257, 255), (1, 192, 384), (1, 256, 384), (1, 6, 2)])
+def test_retention_widths(ctx, H, D, V):
+    g = np.random.default_rng(D * 3 + V)
+    T, decay = 131, [0.998, 0.9][:H]
+    q, k, v, gate = (g.standard_normal((T, H, d)).astype(np.float32) for d in (D, D, V, V))
+    want, S = retention_reference(q, k, v, gate, decay, None, 1e-5)
+    st = RecurrentState(ctx, 1, H, D, V)
+    out = np.concatenate([st.retain(*(a[None, i:j] for a in (q, k, v, gate)), [i], decay)[0] for i, j in ((0, 67), (67, T))])
+    # sums of at most 64 + D products in fp32, the errors walking at random (2**-24 * sqrt(450) = 1.3e-6), and the norm of rows that can be ten
+    # times smaller than the largest
+    assert rel(out, want) < 2e-5
+    assert rel(st.read(0), S) < 2e-5
+    st.close()
