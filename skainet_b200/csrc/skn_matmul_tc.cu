@@ -215,18 +215,22 @@ struct tc_plan {
     size_t smem;
 };
 
-// what the kernel computes: f32[t][m][n] = acc (+ resid[m][n]) (+ bias[n]) for up to three weights of one type that share the tokens, or
-// (DUAL) bf16[m][n] = silu(gate) * up
+// what the kernel computes: (ONE) f32[0][m][n] = acc (+ resid[m][n]) (+ bias[n]), (GROUP) f32[t][m][n] = acc for two or three weights of one
+// type that share the tokens, or (DUAL) bf16[m][n] = silu(gate) * up.  A kernel of its own for the group: with the choice of a weight in every
+// launch the epilogue spills, and a kernel with local memory among others without starts later (48 products 936 x 256 Q4_K of 82 tokens,
+// each with its conversion: 543 us, without 422)
+enum { TC_ONE, TC_DUAL, TC_GROUP };
 struct tc_out {
     const float *bias;
     const float *resid;     // added to the product, laid out like f32 and possibly the same memory
     float *f32[3];
     __nv_bfloat16 *bf16;
     int n[3];               // features of each
+    int64_t ld;             // those of the first once more: 64 bits that ONE need not keep in registers
     int t1, t2;             // first tile of the second and of the third
 };
 
-template <int TYPE, bool DUAL>
+template <int TYPE, int KIND>
 __global__ void __launch_bounds__(TC_THREADS, 1)
 skn_matmul_tc_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_w2,
                      const __grid_constant__ CUtensorMap tm_w3, int M, int K, const tc_plan pl, const tc_out out, int32_t *__restrict__ status) {
@@ -234,6 +238,7 @@ skn_matmul_tc_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_cons
     // operand tiles need 1024-byte alignment for the 128-byte swizzle; the offset is the same in every CTA
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     constexpr int ROW = TcFmt<TYPE>::ROW, RAW_BYTES = TC_ROWS * ROW;
+    constexpr bool DUAL = KIND == TC_DUAL, GROUP = KIND == TC_GROUP;
     __shared__ uint64_t a_full[TC_MAX_A], a_empty[TC_MAX_A], b_full[TC_MAX_B], b_empty[TC_MAX_B], raw_full[TC_MAX_RAW], raw_empty[TC_MAX_RAW], accum_bar;
     __shared__ uint32_t tmem_slot;
 
@@ -248,8 +253,9 @@ skn_matmul_tc_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_cons
     const int nsb = (K + 255) / 256, sb0 = kr * nsb / c, sb1 = (kr + 1) * nsb / c;
     const int steps = min(K / TC_BK, sb1 * 4) - sb0 * 4;
     // features of this CTA: DUAL interleaves 16 gate and 16 up rows (lanes 0-15 and 16-31 of a warp)
-    const int wt = DUAL ? 0 : (tile >= out.t1 ? 1 : 0) + (tile >= out.t2 ? 1 : 0), N = out.n[wt];
-    const int n0 = DUAL ? tile * TC_ROWS + half * (TC_ROWS / 2) : (tile - (wt == 0 ? 0 : wt == 1 ? out.t1 : out.t2)) * 2 * TC_ROWS + half * TC_ROWS;
+    const bool w1 = GROUP && tile >= out.t1, w2 = GROUP && tile >= out.t2;
+    const int N = w2 ? out.n[2] : w1 ? out.n[1] : out.n[0];
+    const int n0 = DUAL ? tile * TC_ROWS + half * (TC_ROWS / 2) : (tile - (w2 ? out.t2 : w1 ? out.t1 : 0)) * 2 * TC_ROWS + half * TC_ROWS;
     const uint32_t tmem_cols = pl.nacc == 2 ? 512u : 256u;
     const uint16_t pair_mask = (uint16_t)(3u << (rank & ~1));
 
@@ -276,7 +282,7 @@ skn_matmul_tc_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_cons
                 tc_tma_load_2d(dst + (32 * i + 16) * ROW, &tm_w2, x, n0 + 16 * i, &raw_full[rs]);
             }
         } else {
-            tc_tma_load_2d(dst, wt == 0 ? &tm_w : (wt == 1 ? &tm_w2 : &tm_w3), x, n0, &raw_full[rs]);
+            tc_tma_load_2d(dst, w2 ? &tm_w3 : w1 ? &tm_w2 : &tm_w, x, n0, &raw_full[rs]);
         }
     };
     const int early = min(nraw, sb1 - sb0);
@@ -481,18 +487,19 @@ skn_matmul_tc_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_cons
                 }
             } else {
                 const int f = n0 + wq * 32 + lane;
+                const int64_t ld = GROUP ? N : out.ld;
                 if (f < N) {
-                    const float bias = out.bias ? __ldg(out.bias + f) : 0.f;
-                    float *dst = out.f32[wt] + (int64_t)m * N + f;
-                    if (out.resid) {                           // (all loads before the first store)
-                        const float *res = out.resid + (int64_t)m * N + f;
+                    const float bias = !GROUP && out.bias ? __ldg(out.bias + f) : 0.f;
+                    float *dst = (w2 ? out.f32[2] : w1 ? out.f32[1] : out.f32[0]) + m * ld + f;
+                    if (!GROUP && out.resid) {                           // (all loads before the first store)
+                        const float *res = out.resid + m * ld + f;
 #pragma unroll
                         for (int i = 0; i < TC_BLOCK; ++i)
-                            if (m + i < M) acc[i] = __float_as_uint(__uint_as_float(acc[i]) + res[(int64_t)i * N]);
+                            if (m + i < M) acc[i] = __float_as_uint(__uint_as_float(acc[i]) + res[i * ld]);
                     }
 #pragma unroll
                     for (int i = 0; i < TC_BLOCK; ++i)
-                        if (m + i < M) dst[(int64_t)i * N] = __uint_as_float(acc[i]) + bias;
+                        if (m + i < M) dst[i * ld] = __uint_as_float(acc[i]) + bias;
                 }
             }
         }
@@ -599,9 +606,10 @@ static cudaError_t tc_pairs(int dev, const void *kern, cudaStream_t stream, int 
     return cudaSuccess;
 }
 
-template <int TYPE, bool DUAL>
+template <int TYPE, int KIND>
 static cudaError_t launch_tc(const __nv_bfloat16 *A, int M, int K, int n, const skn_tensor *const *w, tc_out out, int32_t *status, cudaStream_t stream) {
-    auto kern = skn_matmul_tc_kernel<TYPE, DUAL>;
+    constexpr bool DUAL = KIND == TC_DUAL;
+    auto kern = skn_matmul_tc_kernel<TYPE, KIND>;
     static std::atomic<bool> large[64];                            // per device: may use TC_SMEM_MAX
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
@@ -616,6 +624,7 @@ static cudaError_t launch_tc(const __nv_bfloat16 *A, int M, int K, int n, const 
     if ((e = tc_pairs(dev, (const void *)kern, stream, pairs)) != cudaSuccess) return e;
     int64_t tiles = 0;
     out.t1 = out.t2 = 0x7fffffff;
+    out.ld = w[0]->n_rows;
     for (int t = 0; t < (DUAL ? 1 : n); ++t) {
         if (t == 1) out.t1 = (int)tiles;
         if (t == 2) out.t2 = (int)tiles;
@@ -632,14 +641,14 @@ static cudaError_t launch_tc(const __nv_bfloat16 *A, int M, int K, int n, const 
     return cudaLaunchKernelEx(&cfg, kern, tx, tw[0], tw[1], tw[2], M, K, pl, out, status);
 }
 
-template <bool DUAL>
+template <int KIND>
 static cudaError_t dispatch_tc(const __nv_bfloat16 *A, int M, int n, const skn_tensor *const *w, const tc_out &out, int32_t *status, cudaStream_t stream) {
     const int K = (int)w[0]->n_cols;
     switch (w[0]->type) {
-    case SKN_TYPE_Q4_0: return launch_tc<SKN_TYPE_Q4_0, DUAL>(A, M, K, n, w, out, status, stream);
-    case SKN_TYPE_Q8_0: return launch_tc<SKN_TYPE_Q8_0, DUAL>(A, M, K, n, w, out, status, stream);
-    case SKN_TYPE_Q4_K: return launch_tc<SKN_TYPE_Q4_K, DUAL>(A, M, K, n, w, out, status, stream);
-    case SKN_TYPE_Q6_K: return launch_tc<SKN_TYPE_Q6_K, DUAL>(A, M, K, n, w, out, status, stream);
+    case SKN_TYPE_Q4_0: return launch_tc<SKN_TYPE_Q4_0, KIND>(A, M, K, n, w, out, status, stream);
+    case SKN_TYPE_Q8_0: return launch_tc<SKN_TYPE_Q8_0, KIND>(A, M, K, n, w, out, status, stream);
+    case SKN_TYPE_Q4_K: return launch_tc<SKN_TYPE_Q4_K, KIND>(A, M, K, n, w, out, status, stream);
+    case SKN_TYPE_Q6_K: return launch_tc<SKN_TYPE_Q6_K, KIND>(A, M, K, n, w, out, status, stream);
     default: return cudaErrorInvalidValue;
     }
 }
@@ -665,19 +674,19 @@ cudaError_t skn_launch_matmul_tc(skn_ctx *ctx, const skn_tensor *w, const void *
                                  float *y, cudaStream_t stream, const float *resid) {
     tc_out out = {};
     out.bias = bias; out.resid = resid; out.f32[0] = y;
-    return dispatch_tc<false>((const __nv_bfloat16 *)a_bf16, M, 1, &w, out, ctx->d_status, stream);
+    return dispatch_tc<TC_ONE>((const __nv_bfloat16 *)a_bf16, M, 1, &w, out, ctx->d_status, stream);
 }
 
 // Y[t] = A_bf16 . W[t]^T for two or three weights of one type and width in one launch: the key and value projections of a model with grouped
 // heads have too few tiles for a launch of their own (512 tokens, 4096 x 4096 and twice 1024 x 4096 Q4_K: 74 us in three launches, 44 in one)
 cudaError_t skn_launch_matmul_tc_group(skn_ctx *ctx, int n, const skn_tensor *const *w, const void *a_bf16, int32_t M, float *const *y, cudaStream_t stream) {
-    if (n < 1 || n > 3) return cudaErrorInvalidValue;
+    if (n < 2 || n > 3) return cudaErrorInvalidValue;
     tc_out out = {};
     for (int t = 0; t < n; ++t) {
         if (w[t]->type != w[0]->type || w[t]->n_cols != w[0]->n_cols) return cudaErrorInvalidValue;
         out.f32[t] = y[t];
     }
-    return dispatch_tc<false>((const __nv_bfloat16 *)a_bf16, M, n, w, out, ctx->d_status, stream);
+    return dispatch_tc<TC_GROUP>((const __nv_bfloat16 *)a_bf16, M, n, w, out, ctx->d_status, stream);
 }
 
 // H_bf16 = silu(A . Wg^T) * (A . Wu^T)
@@ -686,5 +695,5 @@ cudaError_t skn_launch_gate_up_tc(skn_ctx *ctx, const skn_tensor *wg, const skn_
     const skn_tensor *w[2] = {wg, wu};
     tc_out out = {};
     out.bf16 = (__nv_bfloat16 *)h_bf16;
-    return dispatch_tc<true>((const __nv_bfloat16 *)a_bf16, M, 2, w, out, ctx->d_status, stream);
+    return dispatch_tc<TC_DUAL>((const __nv_bfloat16 *)a_bf16, M, 2, w, out, ctx->d_status, stream);
 }
