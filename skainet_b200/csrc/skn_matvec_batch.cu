@@ -281,10 +281,12 @@ struct mb_plan {
     size_t smem;
 };
 
+// (`ar` stays in the parameter space: indexed by the tensor of the CTA it would be copied to local memory, and a kernel that has any starts later:
+// 16 rows, Q4_0 8192 x 256 7.8 -> 5.7 us a call, Q4_K 14336 x 4096 23.6 -> 22.2)
 template <int TYPE, int NCH, bool DUAL>
 __global__ void __launch_bounds__((MbWarps<TYPE, NCH>::THREADS), 1)
 skn_matvec_batch_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_w0, const __grid_constant__ CUtensorMap tm_w1,
-                        const __grid_constant__ CUtensorMap tm_w2, const mb_args ar, int K, const mb_plan pl, const mb_meta *__restrict__ meta,
+                        const __grid_constant__ CUtensorMap tm_w2, const __grid_constant__ mb_args ar, int K, const mb_plan pl, const mb_meta *__restrict__ meta,
                         int32_t *__restrict__ status) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
