@@ -66,7 +66,7 @@ __global__ void skn_rope_kernel(float *__restrict__ x, const int32_t *__restrict
         // angle in double: at position 4096 an fp32 angle is already off by ~5e-4 rad
         const double ang = (double)pos * exp2(-(double)log2_theta * (2.0 * (double)p / (double)D));
         double sd, cd;
-        sincos(ang, &sd, &cd);
+        sincospi(ang * 0.31830988618379067, &sd, &cd);    // (sincos keeps local memory for the reduction of large angles)
         const float sn = (float)sd, cs = (float)cd;
         float2 *v = reinterpret_cast<float2 *>(x) + i;
         const float2 a = *v;

@@ -261,7 +261,7 @@ skn_rope_append_kernel(float *__restrict__ q, const float *__restrict__ k_new, c
     if ((int)threadIdx.x < half) {
         const double ang = (double)pos * exp2(-log2_theta * (2.0 * (double)threadIdx.x / (double)D));
         double sd, cd;
-        sincos(ang, &sd, &cd);
+        sincospi(ang * 0.31830988618379067, &sd, &cd);    // (sincos keeps local memory for the reduction of large angles)
         cs[threadIdx.x] = make_float2((float)cd, (float)sd);
     }
     auto source = [&](int i) -> const float2 * {

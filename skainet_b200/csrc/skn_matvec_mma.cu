@@ -156,14 +156,11 @@ skn_matvec_mma(const skn_mv_group grp, int64_t pitch, int K, int nst, const floa
     if (!relaxed) skn_pdl_wait();
     MV_STAMP(2);
     // rotary epilogue: positions and ring starts are requested now and used at the very end
-    int rp_pos[NAMAX], rp_start[NAMAX];
-#pragma unroll
-    for (int a = 0; a < NAMAX; ++a) {
-        rp_pos[a] = rp_start[a] = 0;
-        if (f_rope_hd && a < NA) {
-            rp_pos[a] = grp.rope_len[grp.rope_a0 + a];
-            rp_start[a] = grp.rope_start[grp.rope_a0 + a];
-        }
+    // (lane a keeps those of row a: an array indexed by the row at hand would be local memory, and a kernel that has any starts later)
+    int rp_pos = 0, rp_start = 0;
+    if (f_rope_hd && lane < NA) {
+        rp_pos = grp.rope_len[grp.rope_a0 + lane];
+        rp_start = grp.rope_start[grp.rope_a0 + lane];
     }
     // Tensor-parallel consumer: the previous launch of every rank pushed its partial products into
     // this rank's inbox; wait for the peers' flags (bounded), then every load of x adds them up.
@@ -244,7 +241,7 @@ skn_matvec_mma(const skn_mv_group grp, int64_t pitch, int K, int nst, const floa
                                         (r1.z * r1.z + r1.w * r1.w);
 #pragma unroll
                         for (int k = 0; k < NAMAX; ++k)
-                            if (k == ua[h]) sq[k] += e;
+                            sq[k] += k == ua[h] ? e : 0.f;
                         const float4 g0 = gq[h][0], g1 = gq[h][1];
                         r0.x *= g0.x; r0.y *= g0.y; r0.z *= g0.z; r0.w *= g0.w;
                         r1.x *= g1.x; r1.y *= g1.y; r1.z *= g1.z; r1.w *= g1.w;
@@ -655,16 +652,14 @@ skn_matvec_mma(const skn_mv_group grp, int64_t pitch, int K, int nst, const floa
     // are linear in x, and the digits were taken of x * gain)
     mm_bar_sync(1, W * 32);
     MV_STAMP(6);
-    float nscale[NAMAX];
-#pragma unroll
-    for (int a = 0; a < NAMAX; ++a) {
-        nscale[a] = 1.f;
-        if (f_gain && a < NA) {
-            float tot = 0.f;
-            for (int w2 = 0; w2 < W; ++w2) tot += red[a][w2];
-            nscale[a] = rsqrtf(tot / (float)K + grp.norm_eps);
-        }
+    // (that of row a in lane a)
+    float nscale = 1.f;
+    if (f_gain && lane < NA) {
+        float tot = 0.f;
+        for (int w2 = 0; w2 < W; ++w2) tot += red[lane][w2];
+        nscale = rsqrtf(tot / (float)K + grp.norm_eps);
     }
+    __syncwarp();
     // L lanes per row (16, 4 or 1, the most that still covers the CTA's rows in about one pass):
     // each adds its share of the row's partials in index order, then a fixed butterfly, so the
     // summation tree depends on the shape only
@@ -676,6 +671,8 @@ skn_matvec_mma(const skn_mv_group grp, int64_t pitch, int K, int nst, const floa
     const size_t push_off = SKN_COMM_FLAG_BYTES / sizeof(float) + ((size_t)(xq % SKN_COMM_NBUF) * grp.xc_world + grp.xc_rank) * grp.xc_cap;
     for (int a = 0; a < NA; ++a) {
         const float *pa = part + (size_t)a * rows * pw;
+        const float scale = __shfl_sync(0xffffffffu, nscale, a);
+        const int pos = F_ROPE ? __shfl_sync(0xffffffffu, rp_pos, a) : 0, ring0 = F_ROPE ? __shfl_sync(0xffffffffu, rp_start, a) : 0;
         for (int lb = warp * (32 >> lsh); lb < rows; lb += W * (32 >> lsh)) {     // warp-uniform trip count
             const int lr = lb + (lane >> lsh);
             const int sub = lane & (L - 1);
@@ -683,9 +680,7 @@ skn_matvec_mma(const skn_mv_group grp, int64_t pitch, int K, int nst, const floa
             if (lr < rows)
                 for (int cc = sub; cc < pw; cc += L) s += pa[(size_t)lr * pw + cc];
             for (int o = L >> 1; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-#pragma unroll
-            for (int k = 0; k < NAMAX; ++k)
-                if (k == a) s *= nscale[k];
+            if (F_PREP) s *= scale;
             const float up = __shfl_xor_sync(0xffffffffu, s, L);      // the next row: the `up` product of a gate row
             if (sub == 0 && lr < rows) {
                 int64_t local;
@@ -696,10 +691,6 @@ skn_matvec_mma(const skn_mv_group grp, int64_t pitch, int K, int nst, const floa
                     // rotary embedding of the pair (2i, 2i+1) this row belongs to (`up` is the other
                     // row of the pair), k and v straight into the cache
                     const int hd = F_ROPE ? f_rope_hd : 2, seq = grp.rope_a0 + a;
-                    int pos = 0, ring0 = 0;
-#pragma unroll
-                    for (int k = 0; k < NAMAX; ++k)
-                        if (k == a) { pos = rp_pos[k]; ring0 = rp_start[k]; }
                     // a full cache (a replayed step the host did not count): nothing is overwritten
                     const bool room = pos < grp.rope_cap;
                     if (!room) atomicExch(status, SKN_ERR_SHAPE);
@@ -707,16 +698,15 @@ skn_matvec_mma(const skn_mv_group grp, int64_t pitch, int K, int nst, const floa
                     const int h = (int)(local / hd), dd = (int)(local % hd);
                     float o = s;
                     if (tt < 2) {
-                        // the angle in double (positions reach thousands of radians), reduced to [-pi, pi] with a
-                        // two-term 2 pi, then the fp32 functions: a handful of fp64 instructions instead of a
-                        // double-precision sincos
+                        // the angle in double (positions reach thousands of radians), in half turns and reduced to [-1, 1], then
+                        // the fp32 functions of half turns: a handful of fp64 instructions instead of a double-precision sincos, and
+                        // no local memory (sincosf keeps some for the reduction of large angles)
                         const double f = grp.rope_inv_freq ? grp.rope_inv_freq[dd >> 1]
                                                            : exp2(-grp.rope_log2theta * (2.0 * (double)(dd >> 1) / (double)hd));
                         const double ang = (double)pos * f;
-                        const double turns = rint(ang * 0.15915494309189535);
-                        const float red_ang = (float)fma(-turns, 2.4492935982947064e-16, fma(-turns, 6.283185307179586, ang));
+                        const double turns = ang * 0.31830988618379067;
                         float sn, cs;
-                        sincosf(red_ang, &sn, &cs);
+                        sincospif((float)(turns - 2.0 * rint(0.5 * turns)), &sn, &cs);
                         o = (dd & 1) ? (up * sn + s * cs) : (s * cs - up * sn);
                     }
                     if (tt == 0) grp.y[0][(size_t)a * grp.ystride[0] + local] = o;
