@@ -217,8 +217,8 @@ struct tc_plan {
 
 // what the kernel computes: (ONE) f32[0][m][n] = acc (+ resid[m][n]) (+ bias[n]), (GROUP) f32[t][m][n] = acc for two or three weights of one
 // type that share the tokens, or (DUAL) bf16[m][n] = silu(gate) * up.  A kernel of its own for the group: with the choice of a weight in every
-// launch the epilogue spills, and a kernel with local memory among others without starts later (48 products 936 x 256 Q4_K of 82 tokens,
-// each with its conversion: 543 us, without 422)
+// launch each thread first copies these arguments to local memory and the epilogue spills (48 products 936 x 256 Q4_K of 82 tokens, each with
+// its conversion: 543 us, without 422)
 enum { TC_ONE, TC_DUAL, TC_GROUP };
 struct tc_out {
     const float *bias;

@@ -281,8 +281,8 @@ struct mb_plan {
     size_t smem;
 };
 
-// (`ar` stays in the parameter space: indexed by the tensor of the CTA it would be copied to local memory, and a kernel that has any starts later:
-// 16 rows, Q4_0 8192 x 256 7.8 -> 5.7 us a call, Q4_K 14336 x 4096 23.6 -> 22.2)
+// (`ar` stays in the parameter space: it is indexed by the tensor of the CTA, and by value every thread would first copy its 120 bytes to local
+// memory.  16 rows, Q4_0 8192 x 256 7.8 -> 5.7 us a call, Q4_K 14336 x 4096 23.6 -> 22.2)
 template <int TYPE, int NCH, bool DUAL>
 __global__ void __launch_bounds__((MbWarps<TYPE, NCH>::THREADS), 1)
 skn_matvec_batch_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_w0, const __grid_constant__ CUtensorMap tm_w1,

@@ -156,7 +156,7 @@ skn_matvec_mma(const skn_mv_group grp, int64_t pitch, int K, int nst, const floa
     if (!relaxed) skn_pdl_wait();
     MV_STAMP(2);
     // rotary epilogue: positions and ring starts are requested now and used at the very end
-    // (lane a keeps those of row a: an array indexed by the row at hand would be local memory, and a kernel that has any starts later)
+    // (lane a keeps those of row a: an array indexed by the row at hand would be local memory)
     int rp_pos = 0, rp_start = 0;
     if (f_rope_hd && lane < NA) {
         rp_pos = grp.rope_len[grp.rope_a0 + lane];
