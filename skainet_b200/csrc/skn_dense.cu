@@ -888,9 +888,9 @@ skn_dense_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
     // (through a shuffle: the compiler then knows that a warp's threads take one role together)
     const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
     const int stage_bytes = DTC_A_BYTES + NT * DTC_BK * 2;
-    const int acc_cols = NT < 32 ? 32 : NT;
-    uint32_t tmem_cols = 32;
-    while ((int)tmem_cols < 2 * acc_cols) tmem_cols *= 2;
+    uint32_t tmem_cols = 64;                    // two accumulators
+    while ((int)tmem_cols < 2 * NT) tmem_cols *= 2;
+    const int acc_cols = (int)(tmem_cols / 2);
     const int ksteps = (K + DTC_BK - 1) / DTC_BK;
     const int nt = (N + DTC_BM - 1) / DTC_BM;
     int mt = (M + NT - 1) / NT, units = mt * nt * splits;      // token tiles fastest, then splits, then weight tiles
@@ -1098,7 +1098,9 @@ static cudaError_t launch_dtc(skn_ctx *ctx, const skn_linear &l, const skn_dense
     const int nt = (N + DTC_BM - 1) / DTC_BM;
     const int ksteps = (K + DTC_BK - 1) / DTC_BK;
     // token tile: the narrowest that covers M; beyond that, of the widths whose operands the shared memory feeds at full
-    // rate, the one with the least time in waves (a wave of narrower tiles costs less, but loads more per product)
+    // rate, the one with the least time in waves (a wave of narrower tiles costs less, but loads more per product).  Every multiple of 16, so
+    // that the last wave is nearly full whatever M and N are: 2048 tokens of 7168 x 2048 take four waves of 208 instead of five of 192,
+    // 2048 x 8192 one of 240 instead of 256 (a prompt of Lugasun at width 2048: 3.88 -> 3.70 ms).
     int NT = 16;
     if (GROUPS) {
         // tiles that an expert's share of the rows fills about once
@@ -1106,19 +1108,18 @@ static cudaError_t launch_dtc(skn_ctx *ctx, const skn_linear &l, const skn_dense
     } else if (M <= 128) {
         while (NT < M) NT *= 2;
     } else {
-        const int width[3] = {256, 192, 128};
-        const double rate[3] = {1.0, 1.03, 1.12};
         double best = 1e30;
-        for (int i = 0; i < 3; ++i) {
-            const int64_t tiles = (int64_t)nt * ((M + width[i] - 1) / width[i]);
-            const double cost = (double)((tiles + sms - 1) / sms) * (width[i] + 8) * rate[i];
+        for (int w = 256; w >= 128; w -= 16) {
+            const double rate = w >= 192 ? 1.0 + (256 - w) * (0.03 / 64) : 1.03 + (192 - w) * (0.09 / 64);
+            const int64_t tiles = (int64_t)nt * ((M + w - 1) / w);
+            const double cost = (double)((tiles + sms - 1) / sms) * (w + 8) * rate;
             if (cost < best) {
                 best = cost;
-                NT = width[i];
+                NT = w;
             }
         }
     }
-    while (!GROUPS && NT > 32 && nt * ((M + NT - 1) / NT) * 2 <= sms) NT = NT == 192 ? 128 : NT / 2;
+    while (!GROUPS && NT > 32 && nt * ((M + NT - 1) / NT) * 2 <= sms) NT = NT > 128 ? 128 : NT / 2;
     const int mt = GROUPS ? group_tiles_bound(M, l.pick.n, NT) : (M + NT - 1) / NT;
     // K splits that even out the load of the SMs (the tiles of a decode-size step are fewer than the SMs, or not many more)
     int splits = 1;
