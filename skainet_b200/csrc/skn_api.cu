@@ -230,17 +230,6 @@ int32_t skn_ffn_swiglu(skn_ctx *ctx, const skn_tensor *wg, const skn_tensor *wu,
     return skn_sync(ctx);
 }
 
-// device-side address of a page-locked host buffer (registered or allocated by the CUDA runtime), or NULL for
-// pageable memory
-static void *host_mapped(const void *p) {
-    cudaPointerAttributes a;
-    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
-        cudaGetLastError();
-        return nullptr;
-    }
-    return a.type == cudaMemoryTypeHost ? a.devicePointer : nullptr;
-}
-
 // sync: return when y_host holds the result (and report the device status); otherwise return once the
 // copies and the launch are enqueued on the context's stream
 static int32_t matmul_host(skn_ctx *ctx, const skn_tensor *w, const float *x_host, int32_t M, int64_t K, const float *bias_host,
@@ -267,18 +256,48 @@ static int32_t matmul_host(skn_ctx *ctx, const skn_tensor *w, const float *x_hos
         // the bus 148 times), and the matvec writes y straight into the caller's mapped buffer.  A copy-engine
         // operation between two kernels costs several microseconds of hand-over each way; kernels hand over
         // to one another in one or two, and the matvec prefetches its weights under the fetch.
-        void *xm = host_mapped(x_host), *ym = host_mapped(y_host), *bm = bias_host ? host_mapped(bias_host) : nullptr;
-        if (xm && ym && (!bias_host || bm) && !((((uintptr_t)xm) | ((uintptr_t)ym) | ((uintptr_t)bm)) & 15)) {
+        // A blocking call on pageable buffers does the same from and to page-locked staging of the context.
+        bool plain = true;                                 // all of it memory that the host can read and write
+        auto mapped = [&plain](const void *p) -> void * {
+            void *d = nullptr;
+            if (p && !skn_host_mapped(p, &d)) plain = false;
+            return ((uintptr_t)d & 15) ? nullptr : d;
+        };
+        void *xm = mapped(x_host), *ym = mapped(y_host), *bm = mapped(bias_host);
+        if (w->n_rows % 4) bm = nullptr;                   // (fetched in fours)
+        const void *y_staged = nullptr;
+        const size_t bb_al = (bb + 255) / 256 * 256;
+        const size_t staged = xb_al + bb_al + yb;
+        const bool few = staged <= SKN_SMALL_OUT_BYTES;    // (the result area beside the status word is page-locked too)
+        if (sync && plain && (!xm || !ym || (bias_host && !bm)) && (few || skn_pin_reserve(ctx, staged))) {
+            uint8_t *h = few ? ctx->h_status_base : ctx->h_pin, *d = few ? (uint8_t *)ctx->h_status_dev - SKN_SMALL_OUT_BYTES : ctx->h_pin_dev;
+            if (!xm) {
+                memcpy(h, x_host, xb);
+                xm = d;
+            }
+            if (bias_host && !bm) {
+                memcpy(h + xb_al, bias_host, bb);
+                bm = d + xb_al;
+            }
+            if (!ym) {
+                ym = d + xb_al + bb_al;
+                y_staged = h + xb_al + bb_al;
+            }
+        }
+        if (xm && ym && (!bias_host || bm)) {
             SKN_CUDA(ctx, skn_launch_fetch((const float *)xm, dx, (int64_t)M * K, ctx->stream));
-            if (db) SKN_CUDA(ctx, skn_launch_fetch((const float *)bm, db, w->n_rows, ctx->stream));
+            if (db) SKN_CUDA(ctx, skn_launch_fetch((const float *)bm, db, (w->n_rows + 3) / 4 * 4, ctx->stream));
             // (measured: 12.8 us per 4096 x 4096 call this way, 14.8 with a second kernel pushing y out of device
-            // memory, 20.2 with a copy-engine transfer of y)
+            // memory, 20.2 with a copy-engine transfer of y; pageable buffers, from Python: 33.7 through
+            // the driver's staging, 27.5 through ours)
             rc = skn_matmul_dev(ctx, w, dx, M, K, db, (float *)ym);
             if (rc || !sync) return rc;
             // the blocking call: the status word follows through a kernel as well (16 bytes into the pinned mirror)
             SKN_CUDA(ctx, skn_launch_fetch((const float *)ctx->d_status, (float *)ctx->h_status_dev, 4, ctx->stream));
             SKN_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-            return skn_status_check(ctx);
+            rc = skn_status_check(ctx);
+            if (rc == SKN_OK && y_staged) memcpy(y_host, y_staged, yb);
+            return rc;
         }
     }
     if (sync && yb <= SKN_SMALL_OUT_BYTES) {
@@ -304,8 +323,12 @@ static int32_t matmul_host(skn_ctx *ctx, const skn_tensor *w, const float *x_hos
     if (db) SKN_CUDA(ctx, cudaMemcpyAsync(db, bias_host, bb, cudaMemcpyHostToDevice, ctx->stream));
     rc = skn_matmul_dev(ctx, w, dx, M, K, db, (float *)ctx->d_stage_out);
     if (rc) return rc;
+    if (sync) {
+        const skn_result r = {y_host, ctx->d_stage_out, yb};
+        return skn_sync_results(ctx, &r, 1);
+    }
     SKN_CUDA(ctx, cudaMemcpyAsync(y_host, ctx->d_stage_out, yb, cudaMemcpyDeviceToHost, ctx->stream));
-    return sync ? skn_sync(ctx) : SKN_OK;
+    return SKN_OK;
 }
 
 int32_t skn_matmul(skn_ctx *ctx, const skn_tensor *w, const float *x_host, int32_t M, int64_t K, const float *bias_host,

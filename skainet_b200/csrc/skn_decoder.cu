@@ -229,8 +229,16 @@ int32_t skn_decoder_forward(skn_decoder *m, int32_t seq0, int32_t n_seqs, const 
     SKN_CUDA(ctx, cudaSetDevice(ctx->device));
     if (tokens_host) SKN_CUDA(ctx, cudaMemcpyAsync(m->ids_in, tokens_host, sizeof(int32_t) * n_seqs * T, cudaMemcpyHostToDevice, ctx->stream));
     rc = skn_decoder_forward_dev(m, seq0, n_seqs, tokens_host ? m->ids_in : nullptr, T, next_host != nullptr);
-    if (rc == SKN_OK && next_host)
-        SKN_CUDA(ctx, cudaMemcpyAsync(next_host, m->ids_out + seq0, sizeof(int32_t) * n_seqs, cudaMemcpyDeviceToHost, ctx->stream));
+    if (rc) return rc;
+    // the wanted rows are the ones that the ids came from (the last of every sequence): their logits are there already
+    bool last = next_host && n_want == n_seqs;
+    for (int i = 0; last && i < n_want; ++i) last = want_rows_host[i] == i * T + T - 1;
+    if (last || n_want == 0) {
+        const skn_result r[2] = {{next_host, m->ids_out + seq0, next_host ? sizeof(int32_t) * n_seqs : 0},
+                                 {logits_host, m->logits, sizeof(float) * (size_t)n_want * m->vocab}};
+        return skn_sync_results(ctx, r, 2);
+    }
+    if (next_host) SKN_CUDA(ctx, cudaMemcpyAsync(next_host, m->ids_out + seq0, sizeof(int32_t) * n_seqs, cudaMemcpyDeviceToHost, ctx->stream));
     for (int i = 0; i < n_want && rc == SKN_OK; i += SKN_HEAD_ROWS) {
         const int n = n_want - i < SKN_HEAD_ROWS ? n_want - i : SKN_HEAD_ROWS;
         SKN_CUDA(ctx, cudaMemcpyAsync(m->want, want_rows_host + i, sizeof(int32_t) * n, cudaMemcpyHostToDevice, ctx->stream));

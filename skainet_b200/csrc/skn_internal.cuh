@@ -30,6 +30,8 @@ struct skn_group_plan {
 };
 
 constexpr size_t SKN_SMALL_OUT_BYTES = 96 * 1024;
+constexpr size_t SKN_PIN_MAX = 16 << 20;      // most page-locked staging a context holds
+constexpr int SKN_PIN_PIECES = 8;
 
 struct skn_ctx {
     uint32_t magic;
@@ -48,6 +50,9 @@ struct skn_ctx {
     uint8_t *d_status_base;     // allocation: [SKN_SMALL_OUT_BYTES of result area][status / trace area]
     uint8_t *h_status_base;     // pinned:     [SKN_SMALL_OUT_BYTES of result area][status word]
     int32_t *h_status_dev;      // device-side address of h_status (page-locked memory is mapped)
+    // page-locked staging between pageable host buffers and the device (skn_pin_reserve), used by calls that end with a synchronisation only
+    uint8_t *h_pin, *h_pin_dev; size_t h_pin_bytes;
+    cudaEvent_t pin_events[SKN_PIN_PIECES];
     // staging for the host-pointer entry points (grown on demand)
     void *d_stage_in;  size_t d_stage_in_bytes;
     void *d_stage_out; size_t d_stage_out_bytes;
@@ -162,6 +167,16 @@ bool skn_kv_ok(const skn_kvcache *kv);
 int32_t skn_stage_reserve(skn_ctx *ctx, void **buf, size_t *cap, size_t need);
 int32_t skn_xq_reserve(skn_ctx *ctx, size_t need, cudaStream_t stream);
 int32_t skn_status_check(skn_ctx *ctx);
+bool skn_pin_reserve(skn_ctx *ctx, size_t need);
+bool skn_host_mapped(const void *p, void **dev);
+
+// results of a host-pointer call, device -> the caller's memory, and the status: returns when they are there
+struct skn_result {
+    void *host;
+    const void *dev;
+    size_t bytes;
+};
+int32_t skn_sync_results(skn_ctx *ctx, const skn_result *r, int n);
 
 #define SKN_CUDA(ctx, call)                                            \
     do {                                                               \

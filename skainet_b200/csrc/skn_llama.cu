@@ -569,11 +569,9 @@ int32_t skn_llama_forward(skn_llama *m, const int32_t *tokens_host, int32_t T, i
         SKN_CUDA(ctx, cudaMemcpyAsync(m->ids_in, tokens_host, sizeof(int32_t) * B * T, cudaMemcpyHostToDevice, ctx->stream));
     int32_t rc = skn_llama_forward_dev(m, tokens_host ? m->ids_in : nullptr, T);
     if (rc) return rc;
-    if (next_host)
-        SKN_CUDA(ctx, cudaMemcpyAsync(next_host, m->ids_out, sizeof(int32_t) * B, cudaMemcpyDeviceToHost, ctx->stream));
-    if (logits_host)
-        SKN_CUDA(ctx, cudaMemcpyAsync(logits_host, m->logits, sizeof(float) * B * m->vocab_l, cudaMemcpyDeviceToHost, ctx->stream));
-    return skn_sync(ctx);
+    const skn_result r[2] = {{next_host, m->ids_out, next_host ? sizeof(int32_t) * B : 0},
+                             {logits_host, m->logits, logits_host ? sizeof(float) * (size_t)B * m->vocab_l : 0}};
+    return skn_sync_results(ctx, r, 2);
 }
 
 // number of tokens cached per sequence

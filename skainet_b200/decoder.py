@@ -78,6 +78,8 @@ class DenseDecoder:
         if n < 1 or T < 1 or any(x < 0 or x >= n * T for x in want):
             raise ValueError("Shapes do not align.")
         per = self.max_tokens // n
+        if T <= per:
+            return self._step(t, seq, n, T, want, want_next)
         logits = np.empty((len(want), self.vocab), dtype=np.float32) if want else None
         nxt = None
         for a in range(0, T, per):
