@@ -35,6 +35,7 @@
 // are prefetched before the programmatic dependent-launch wait, x is read after it.  Partial
 // sums per (row, super-chunk, warp) meet in shared memory and are added in a fixed order.
 #include "skn_mma_common.cuh"
+#include "skn_tc.cuh"
 
 // Register caps: the register file is split over the SM's four schedulers (16K registers each), so
 // two resident CTAs of 9 warps need five warps per scheduler, i.e. at most 102 registers per
@@ -49,6 +50,8 @@
 // exchange.  Code size matters: the kernels of a decoder layer take turns, so every launch starts from a cold
 // instruction cache and fetches its preparation code (run once) from L2; the rare paths (outliers) are out of
 // line for the same reason.  Single-row Q4_K variants: 38 / 50 / 56 / 82 KB.
+constexpr int MM_FEAT_SPLIT = 4;    // as 0, K over a cluster of two CTAs
+
 template <int FMT, int SPW, int NP, bool ODD, int FEAT>   // format; super-blocks of a tile per compute warp (W = KS / SPW warps); row pairs;
                                                 // ODD: the last pair has one row only (its odd columns are skipped)
 __global__ void __launch_bounds__(MmFmt<FMT>::KS / SPW == 16 ? 544 : (MmFmt<FMT>::KS / SPW == 8 ? 320 : 256),
@@ -60,7 +63,8 @@ skn_matvec_mma(const skn_mv_group grp, int64_t pitch, int K, int nst, const floa
     constexpr int XS = MmFmt<FMT>::XS;
     constexpr int W = MM_KS / SPW;
     constexpr int NAMAX = 2 * NP;
-    constexpr bool F_PREP = FEAT >= 1, F_ROPE = FEAT >= 2, F_XC = FEAT == 3;
+    constexpr bool F_SPLIT = FEAT == MM_FEAT_SPLIT;
+    constexpr bool F_PREP = FEAT >= 1 && !F_SPLIT, F_ROPE = FEAT >= 2 && !F_SPLIT, F_XC = FEAT == 3;
     const float *const f_gain = F_PREP ? grp.norm_gain : nullptr;
     const float *const f_silu = F_XC ? grp.silu_u : nullptr;       // (the rare silu(x) * u preparation rides with the largest variant)
     const bool f_swiglu = (FEAT == 1 || FEAT == 3) && grp.swiglu;
@@ -71,14 +75,20 @@ skn_matvec_mma(const skn_mv_group grp, int64_t pitch, int K, int nst, const floa
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;          // 0..W-1 compute, W = producer
     const int g = lane >> 2, t = lane & 3;
-    const int nb = K / 256;
+    // F_SPLIT: the two CTAs of a cluster multiply the rows of both by half of the K super-chunks each (rank 0 by the lower ones); a CTA adds up the
+    // rows that it would have alone, from the same partial sums in the same order
+    const int kr = F_SPLIT ? (int)tc_cluster_rank() : 0, nks_all = (K / 256 + MM_KS - 1) / MM_KS;
+    const int k0 = F_SPLIT ? kr * nks_all / 2 : 0;
+    const int nb = F_SPLIT ? min(K / 256, (kr + 1) * nks_all / 2 * MM_KS) - k0 * MM_KS : K / 256;
+    const int nb_most = F_SPLIT ? (nks_all + 1) / 2 * MM_KS : nb;      // (what the layout is made for, the same in both)
+    x += k0 * MM_KS * 256;
     // launches of three or four rows keep the digit planes of ONE K super-chunk at a time (their
     // planes would not fit otherwise); one or two rows prepare all of x up front
     constexpr bool CHUNKED = NP > 1;
-    const int nbp = ((CHUNKED ? MM_KS : nb) + 3) / 4 * 4;        // scale slots per activation row
-    const int nxs = CHUNKED ? MM_KS : nb;       // super-blocks of group sums per activation row
+    const int nbp = ((CHUNKED ? MM_KS : nb_most) + 3) / 4 * 4;        // scale slots per activation row
+    const int nxs = CHUNKED ? MM_KS : nb_most;       // super-blocks of group sums per activation row
     const int nks = (nb + MM_KS - 1) / MM_KS;   // K super-chunks
-    const int ksb = CHUNKED ? (nb < MM_KS ? nb : MM_KS) : nb;    // super-blocks whose digit planes are resident
+    const int ksb = CHUNKED ? (nb < MM_KS ? nb : MM_KS) : nb_most;    // super-blocks whose digit planes are resident
     const int PL = ksb * 256 + 32;              // plane stride: 8 words mod 32, the four planes on disjoint banks
     const int RS = MM_ND * PL + 64;             // activation-row stride: 16 words mod 32, the two rows of a pair apart
 
@@ -97,12 +107,15 @@ skn_matvec_mma(const skn_mv_group grp, int64_t pitch, int K, int nst, const floa
 
     // with interleaved gate / up rows every CTA owns whole (gate, up) pairs: even boundaries
     const int64_t even = (f_swiglu || f_rope_hd) ? ~(int64_t)1 : ~(int64_t)0;
-    const int64_t row_begin = ((int64_t)blockIdx.x * N / gridDim.x) & even;
-    const int64_t row_end = (blockIdx.x + 1 == gridDim.x) ? N : (((int64_t)(blockIdx.x + 1) * N / gridDim.x) & even);
+    const int64_t cta = F_SPLIT ? blockIdx.x / 2 : blockIdx.x, ctas = F_SPLIT ? gridDim.x / 2 : gridDim.x;
+    const int64_t row_begin = (cta * N / ctas) & even;
+    const int64_t row_end = (cta + 1 == ctas) ? N : (((cta + 1) * N / ctas) & even);
     const int rows = (int)(row_end - row_begin);
+    const int64_t own_begin = F_SPLIT ? (int64_t)blockIdx.x * N / gridDim.x : row_begin, own_end = F_SPLIT ? ((int64_t)blockIdx.x + 1) * N / gridDim.x : row_end;
+    const int own = (int)(own_end - own_begin), first = kr == 0 ? own : rows - own;      // rows of this CTA, of rank 0
     const int nrt = (rows + 15) >> 4;           // row tiles
     const int ntiles = nrt * nks;               // tile i -> super-chunk i / nrt, row tile i % nrt
-    const int pw = nks * W;                     // partial slots per (activation row, weight row)
+    const int pw = (F_SPLIT ? nks_all : nks) * W;                     // partial slots per (activation row, weight row)
 
     __shared__ int s_anyout;                    // some prepared block of x has outliers (rare): the tile loop looks only then
     if (threadIdx.x == 0) s_anyout = 0;
@@ -114,6 +127,7 @@ skn_matvec_mma(const skn_mv_group grp, int64_t pitch, int K, int nst, const floa
     }
     if (warp == W) skn_fence_mbar_init();
     __syncthreads();                            // barriers are initialised for everyone
+    if (F_SPLIT) asm volatile("barrier.cluster.arrive.relaxed;" ::: "memory");      // this CTA is there
 
     if (warp == W) {
         // ---- producer: one copy per valid row of a tile, all on the stage's full barrier ----
@@ -138,11 +152,15 @@ skn_matvec_mma(const skn_mv_group grp, int64_t pitch, int K, int nst, const floa
                 const int tt = skn_group_row(grp, row_begin + rt * 16 + lane, local);
                 skn_fence_proxy_async();
                 skn_bulk_g2s(ring + (size_t)stg * MM_STAGE + lane * MM_ROW_STRIDE,
-                             grp.W[tt] + local * pitch + (size_t)ks * MM_KS * MM_BLOCK_BYTES, bytes, &full[stg]);
+                             grp.W[tt] + local * pitch + (size_t)(k0 + ks) * MM_KS * MM_BLOCK_BYTES, bytes, &full[stg]);
             }
             if (i == nst - 1 || i == ntiles - 1) skn_pdl_launch_dependents();   // the first ring-full is on its way
             if (++rt == nrt) { rt = 0; ++ks; }
             if (++stg == nst) { stg = 0; par ^= 1u; }
+        }
+        if (F_SPLIT) {
+            asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+            tc_cluster_sync();
         }
         return;
     }
@@ -281,6 +299,7 @@ skn_matvec_mma(const skn_mv_group grp, int64_t pitch, int K, int nst, const floa
         for (int kc = 0; kc < nks; ++kc) prep_chunk(kc);
         mm_bar_sync(1, W * 32);
     }
+    if (F_SPLIT) asm volatile("barrier.cluster.wait.acquire;" ::: "memory");      // both CTAs are there: their partial sums may be written
     MV_STAMP(3);
     for (int i = 0; i < ntiles; ++i) {
         const uint32_t st = ring_s + (uint32_t)stg * MM_STAGE;
@@ -639,9 +658,19 @@ skn_matvec_mma(const skn_mv_group grp, int64_t pitch, int K, int nst, const floa
                 const int r0 = rt * 16 + g;
                 const float v0 = (a & 1) ? accB[a >> 1][0] : accA[a >> 1][0];
                 const float v1 = (a & 1) ? accB[a >> 1][1] : accA[a >> 1][1];
-                float *pa = part + (size_t)a * rows * pw;
-                if (r0 < rows) pa[(size_t)r0 * pw + ks * W + warp] = v0 - ms[a];
-                if (r0 + 8 < rows) pa[(size_t)(r0 + 8) * pw + ks * W + warp] = v1 - mo;
+                if constexpr (F_SPLIT) {
+                    auto put = [&](int r, float v) {
+                        const int to = r < first ? 0 : 1, n = to == kr ? own : rows - own;
+                        const uint32_t at = skn_smem_u32(part + ((size_t)a * n + r - (to ? first : 0)) * pw + (k0 + ks) * W + warp);
+                        asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(tc_mapa(at, to)), "f"(v) : "memory");
+                    };
+                    if (r0 < rows) put(r0, v0 - ms[a]);
+                    if (r0 + 8 < rows) put(r0 + 8, v1 - mo);
+                } else {
+                    float *pa = part + (size_t)a * rows * pw;
+                    if (r0 < rows) pa[(size_t)r0 * pw + ks * W + warp] = v0 - ms[a];
+                    if (r0 + 8 < rows) pa[(size_t)(r0 + 8) * pw + ks * W + warp] = v1 - mo;
+                }
             }
         }
         if (++rt == nrt) { rt = 0; ++ks; }
@@ -650,7 +679,8 @@ skn_matvec_mma(const skn_mv_group grp, int64_t pitch, int K, int nst, const floa
     MV_STAMP(5);
     // RMSNorm: the scalar 1 / rms of every activation row multiplies its outputs (the products above
     // are linear in x, and the digits were taken of x * gain)
-    mm_bar_sync(1, W * 32);
+    if (F_SPLIT) tc_cluster_sync();
+    else mm_bar_sync(1, W * 32);
     MV_STAMP(6);
     // (that of row a in lane a)
     float nscale = 1.f;
@@ -663,28 +693,28 @@ skn_matvec_mma(const skn_mv_group grp, int64_t pitch, int K, int nst, const floa
     // L lanes per row (16, 4 or 1, the most that still covers the CTA's rows in about one pass):
     // each adds its share of the row's partials in index order, then a fixed butterfly, so the
     // summation tree depends on the shape only
-    const int lsh = (rows * 16 <= W * 32) ? 4 : ((rows * 4 <= W * 32) ? 2 : 0);
+    const int lsh = (own * 16 <= W * 32) ? 4 : ((own * 4 <= W * 32) ? 2 : 0);
     const int L = 1 << lsh;
     const bool push = F_XC && grp.xc_push && grp.xc_world > 1;
     uint32_t xq = 0;
     if (push) xq = *reinterpret_cast<volatile uint32_t *>(grp.xc_state);        // number of this exchange
     const size_t push_off = SKN_COMM_FLAG_BYTES / sizeof(float) + ((size_t)(xq % SKN_COMM_NBUF) * grp.xc_world + grp.xc_rank) * grp.xc_cap;
     for (int a = 0; a < NA; ++a) {
-        const float *pa = part + (size_t)a * rows * pw;
+        const float *pa = part + (size_t)a * own * pw;
         const float scale = __shfl_sync(0xffffffffu, nscale, a);
         const int pos = F_ROPE ? __shfl_sync(0xffffffffu, rp_pos, a) : 0, ring0 = F_ROPE ? __shfl_sync(0xffffffffu, rp_start, a) : 0;
-        for (int lb = warp * (32 >> lsh); lb < rows; lb += W * (32 >> lsh)) {     // warp-uniform trip count
+        for (int lb = warp * (32 >> lsh); lb < own; lb += W * (32 >> lsh)) {     // warp-uniform trip count
             const int lr = lb + (lane >> lsh);
             const int sub = lane & (L - 1);
             float s = 0.f;
-            if (lr < rows)
+            if (lr < own)
                 for (int cc = sub; cc < pw; cc += L) s += pa[(size_t)lr * pw + cc];
             for (int o = L >> 1; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
             if (F_PREP) s *= scale;
             const float up = __shfl_xor_sync(0xffffffffu, s, L);      // the next row: the `up` product of a gate row
-            if (sub == 0 && lr < rows) {
+            if (sub == 0 && lr < own) {
                 int64_t local;
-                const int tt = skn_group_row(grp, row_begin + lr, local);
+                const int tt = skn_group_row(grp, own_begin + lr, local);
                 if (f_swiglu) {
                     if (tt == 0) grp.y[0][(size_t)a * grp.ystride[0] + local] = s / (1.f + expf(-s)) * up;
                 } else if (f_rope_hd) {
@@ -775,6 +805,7 @@ static mm_kernel_t mm_kernel_feat(int n_act, int feat) {
     case 0: return mm_kernel_na<FMT, SPW, 0>(n_act);
     case 1: return mm_kernel_na<FMT, SPW, 1>(n_act);
     case 2: return mm_kernel_na<FMT, SPW, 2>(n_act);
+    case MM_FEAT_SPLIT: return n_act == 1 ? skn_matvec_mma<FMT, SPW, 1, true, MM_FEAT_SPLIT> : skn_matvec_mma<FMT, SPW, 1, false, MM_FEAT_SPLIT>;
     default: return mm_kernel_na<FMT, SPW, 3>(n_act);
     }
 }
@@ -811,6 +842,12 @@ static int mm_max_acts(const skn_ctx *ctx, int fmt, int64_t n_rows, int64_t n_co
     return 1;
 }
 
+static cudaError_t mm_prepare(mm_kernel_t kern) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
+    // all of the SM's L1 / shared memory as shared memory, so that two CTAs (consecutive launches) fit
+    return e != cudaSuccess ? e : cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+}
+
 static cudaError_t mm_plan(skn_ctx *ctx, int fmt, int64_t n_rows, int64_t n_cols, int n_act, int feat, skn_mv_plan &pl, bool relaxed) {
     pl = skn_mv_plan{-1, 0, 0, 0, 0, 0};
     if (n_cols % 256 || n_cols > (1 << 18) || n_rows < 1 || n_act < 1 || n_act > 4) return cudaSuccess;
@@ -832,6 +869,29 @@ static cudaError_t mm_plan(skn_ctx *ctx, int fmt, int64_t n_rows, int64_t n_cols
     // ring matters more than the neighbour
     const size_t budget = (size_t)(budget_env > 0 ? budget_env : (ntiles >= 6 ? 200 : 110)) * 1024;
     const size_t fixed = mm_fixed_smem(fmt, nb, n_act, rows_max, nks, warps);
+    // Rows of several K super-chunks and few rows a CTA: K over the two CTAs of a cluster, which multiply the rows of both.  Each prepares half of
+    // x, the tiles of 16 rows are fuller, and the halved planes leave room for more stages or for the next launch's CTA.  The partial sums go
+    // to the CTA that would have had the row alone and are added in the same order: the results are the same bits.  us before and now:
+    //   Q4_K 2048 x 8192 6.3 5.1, 1024 x 8192 5.95 3.9, 2960 x 8192 8.9 6.3, 4096 x 14336 13.6 13.0, two rows 20.7 17.5, 9400 x 14336 two rows 44.8 27.5
+    //   Q8_0 4096 x 4096 7.9 7.1, 1024 x 4096 4.6 3.35, 4096 x 14336 20.0 18.5   Q4_0 2048 x 8192 6.8 5.6   Q6_K 1024 x 4096 4.95 3.7, 2048 x 8192 9.8 8.2
+    // Not with four tiles of 16 rows a CTA at one activation row (Q8_0 9400 x 4096 10.1 10.25), not where one half has more than three quarters of K
+    // (Q4_K 4736 x 4608 6.9 7.3), and of Q6_K, which its instructions bound, only up to four tiles (4096 x 14336 22.9 23.6).
+    const int half = (nks + 1) / 2, nrt = (int)((n_rows + grid - 1) / grid + 15) / 16;
+    if (feat == 0 && n_act <= 2 && nks >= 2 && grid % 2 == 0 && nrt <= 2 + n_act && half * mm_ks(fmt) * 4 <= nb * 3 && (fmt != MM_FMT_Q6K || nrt * nks <= 4)) {
+        const int64_t most = (n_rows + grid / 2 - 1) / (grid / 2);
+        const int tiles = (int)((most + 15) / 16) * half;
+        const size_t planes = mm_fixed_smem(fmt, half * mm_ks(fmt), n_act, (most + 1) / 2 + 1, nks, warps);
+        if (planes + 2 * stage <= budget) {
+            mm_kernel_t kern = mm_kernel(fmt, warps, n_act, MM_FEAT_SPLIT);
+            cudaError_t e = mm_prepare(kern);
+            if (e != cudaSuccess) return e;
+            int nst = tiles < 4 ? tiles : 4;
+            while (nst > 2 && planes + (size_t)nst * stage > budget) --nst;
+            pl.nch = warps; pl.wg = nst; pl.grid = (int)grid; pl.threads = (warps + 1) * 32; pl.smem = planes + (size_t)nst * stage;
+            pl.state = 2;
+            return cudaSuccess;
+        }
+    }
     int nst = nst_env > 0 ? nst_env : (ntiles < 4 ? ntiles : 4);
     while (nst > 1 && fixed + (size_t)nst * stage > budget) --nst;
     if (nst < 2 && ntiles > 1 && budget_env <= 0) {
@@ -843,10 +903,7 @@ static cudaError_t mm_plan(skn_ctx *ctx, int fmt, int64_t n_rows, int64_t n_cols
     const size_t smem = fixed + (size_t)nst * stage;
     if (smem > 220 * 1024) return cudaSuccess;
     mm_kernel_t kern = mm_kernel(fmt, warps, n_act, feat);
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
-    if (e != cudaSuccess) return e;
-    // all of the SM's L1 / shared memory as shared memory, so that two CTAs (consecutive launches) fit
-    e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+    cudaError_t e = mm_prepare(kern);
     if (e != cudaSuccess) return e;
     // wg carries the ring depth, nch the compute warps; threads = compute warps + the producer warp
     pl.nch = warps; pl.wg = nst; pl.grid = (int)grid; pl.threads = (warps + 1) * 32; pl.smem = smem;
@@ -913,20 +970,29 @@ bool skn_mma_try_group(skn_ctx *ctx, int n, const skn_tensor *const *w, const fl
         if (ctx->n_group_plans < 32)
             ctx->group_plans[ctx->n_group_plans++] = skn_group_plan{key_type, ctx->relaxed_order, tot, w[0]->n_cols, pl};
     }
-    if (pl.state != 1) return false;
+    if (pl.state < 1) return false;
+    const bool split = pl.state == 2;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)pl.grid);
     cfg.blockDim = dim3((unsigned)pl.threads);
     cfg.dynamicSmemBytes = pl.smem;
     cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchAttribute attr[2];
     static const int pdl = env_int("SKN_PDL", 1);
     static const int pdl_max_mb = env_int("SKN_PDL_MAX_MB", 1 << 20);   // tuning knob: largest launch (weight bytes) that may start early
     cfg.attrs = attr;
-    cfg.numAttrs = (pdl && tot * w[0]->pitch <= (int64_t)pdl_max_mb * (1 << 20)) ? 1 : 0;
-    err = cudaLaunchKernelEx(&cfg, mm_kernel(fmt, pl.nch, n_act, feat), grp, w[0]->pitch, (int)w[0]->n_cols, pl.wg, x, ctx->d_status,
+    cfg.numAttrs = 0;
+    if (pdl && tot * w[0]->pitch <= (int64_t)pdl_max_mb * (1 << 20)) {
+        attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (split) {
+        attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+        attr[cfg.numAttrs].val.clusterDim.x = 2;
+        attr[cfg.numAttrs].val.clusterDim.y = 1;
+        attr[cfg.numAttrs++].val.clusterDim.z = 1;
+    }
+    err = cudaLaunchKernelEx(&cfg, mm_kernel(fmt, pl.nch, n_act, split ? MM_FEAT_SPLIT : feat), grp, w[0]->pitch, (int)w[0]->n_cols, pl.wg, x, ctx->d_status,
                              ctx->relaxed_order);
     return true;
 }
