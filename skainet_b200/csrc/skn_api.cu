@@ -256,26 +256,35 @@ static int32_t matmul_host(skn_ctx *ctx, const skn_tensor *w, const float *x_hos
         // the bus 148 times), and the matvec writes y straight into the caller's mapped buffer.  A copy-engine
         // operation between two kernels costs several microseconds of hand-over each way; kernels hand over
         // to one another in one or two, and the matvec prefetches its weights under the fetch.
-        // A blocking call on pageable buffers does the same from and to page-locked staging of the context.
-        bool plain = true;                                 // all of it memory that the host can read and write
-        auto mapped = [&plain](const void *p) -> void * {
-            void *d = nullptr;
-            if (p && !skn_host_mapped(p, &d)) plain = false;
-            return ((uintptr_t)d & 15) ? nullptr : d;
-        };
-        void *xm = mapped(x_host), *ym = mapped(y_host), *bm = mapped(bias_host);
-        if (w->n_rows % 4) bm = nullptr;                   // (fetched in fours)
+        // A blocking call does the same from and to page-locked staging of the context where a buffer is pageable, or a result off a 16-byte
+        // boundary.  Only pageable memory is read by the host, and only once the stream has come this far: page-locked and
+        // managed inputs may be the results of calls that are still enqueued, and are read in stream order, the former by the
+        // fetch kernel wherever they start, the latter by the copies below.
+        void *xm, *ym, *bm = nullptr;
+        const skn_memory xk = skn_memory_of(x_host, &xm), yk = skn_memory_of(y_host, &ym), bk = bias_host ? skn_memory_of(bias_host, &bm) : SKN_MEM_LOCKED;
+        if ((uintptr_t)xm & 3) xm = nullptr;
+        if ((uintptr_t)bm & 3) bm = nullptr;
+        if ((uintptr_t)ym & 15) ym = nullptr;              // (the matvec stores in fours)
         const void *y_staged = nullptr;
         const size_t bb_al = (bb + 255) / 256 * 256;
         const size_t staged = xb_al + bb_al + yb;
         const bool few = staged <= SKN_SMALL_OUT_BYTES;    // (the result area beside the status word is page-locked too)
-        if (sync && plain && (!xm || !ym || (bias_host && !bm)) && (few || skn_pin_reserve(ctx, staged))) {
+        const bool stage_x = !xm, stage_b = bias_host && !bm;
+        const bool may = (!stage_x || xk == SKN_MEM_PAGEABLE) && (!stage_b || bk == SKN_MEM_PAGEABLE) && yk != SKN_MEM_DEVICE;
+        if (sync && may && (stage_x || stage_b || !ym) && (few || skn_pin_reserve(ctx, staged))) {
             uint8_t *h = few ? ctx->h_status_base : ctx->h_pin, *d = few ? (uint8_t *)ctx->h_status_dev - SKN_SMALL_OUT_BYTES : ctx->h_pin_dev;
-            if (!xm) {
+            if (stage_x || stage_b) {
+                const cudaError_t idle = cudaStreamQuery(ctx->stream);
+                if (idle != cudaSuccess) {
+                    cudaGetLastError();                    // (not ready is kept as an error, too)
+                    SKN_CUDA(ctx, idle == cudaErrorNotReady ? cudaStreamSynchronize(ctx->stream) : idle);
+                }
+            }
+            if (stage_x) {
                 memcpy(h, x_host, xb);
                 xm = d;
             }
-            if (bias_host && !bm) {
+            if (stage_b) {
                 memcpy(h + xb_al, bias_host, bb);
                 bm = d + xb_al;
             }
@@ -286,7 +295,7 @@ static int32_t matmul_host(skn_ctx *ctx, const skn_tensor *w, const float *x_hos
         }
         if (xm && ym && (!bias_host || bm)) {
             SKN_CUDA(ctx, skn_launch_fetch((const float *)xm, dx, (int64_t)M * K, ctx->stream));
-            if (db) SKN_CUDA(ctx, skn_launch_fetch((const float *)bm, db, (w->n_rows + 3) / 4 * 4, ctx->stream));
+            if (db) SKN_CUDA(ctx, skn_launch_fetch((const float *)bm, db, w->n_rows, ctx->stream));
             // (measured: 12.8 us per 4096 x 4096 call this way, 14.8 with a second kernel pushing y out of device
             // memory, 20.2 with a copy-engine transfer of y; pageable buffers, from Python: 33.7 through
             // the driver's staging, 27.5 through ours)

@@ -71,7 +71,8 @@ int32_t skn_xq_reserve(skn_ctx *ctx, size_t need, cudaStream_t stream) {
     return SKN_OK;
 }
 
-// Page-locked staging of at least `need` bytes.  Whoever uses it has synchronised with the device before returning, so it may move here.
+// Page-locked staging of at least `need` bytes.  Whoever uses it has synchronised with the device before returning, unless a launch failed:
+// it moves behind a synchronisation of its own.
 // False: more than SKN_PIN_MAX, or none to be had; the caller copies from and to pageable memory as it is.
 bool skn_pin_reserve(skn_ctx *ctx, size_t need) {
     if (need <= ctx->h_pin_bytes) return true;
@@ -84,24 +85,29 @@ bool skn_pin_reserve(skn_ctx *ctx, size_t need) {
         if (h) cudaFreeHost(h);
         return false;
     }
-    if (ctx->h_pin) cudaFreeHost(ctx->h_pin);
+    if (ctx->h_pin) {
+        cudaStreamSynchronize(ctx->stream);
+        cudaFreeHost(ctx->h_pin);
+    }
     ctx->h_pin = (uint8_t *)h;
     ctx->h_pin_dev = (uint8_t *)d;
     ctx->h_pin_bytes = want;
     return true;
 }
 
-// *dev: device-side address of a page-locked host buffer (registered or allocated by the CUDA runtime), NULL for any other memory.
-// False: memory of a device, which a copy by the host must not touch.
-bool skn_host_mapped(const void *p, void **dev) {
+// *dev: device-side address of page-locked memory, NULL for any other
+skn_memory skn_memory_of(const void *p, void **dev) {
     cudaPointerAttributes a;
     *dev = nullptr;
     if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
         cudaGetLastError();
-        return true;
+        return SKN_MEM_PAGEABLE;
     }
-    if (a.type == cudaMemoryTypeHost) *dev = a.devicePointer;
-    return a.type != cudaMemoryTypeDevice;
+    if (a.type == cudaMemoryTypeHost) {
+        *dev = a.devicePointer;
+        return SKN_MEM_LOCKED;
+    }
+    return a.type == cudaMemoryTypeDevice ? SKN_MEM_DEVICE : a.type == cudaMemoryTypeManaged ? SKN_MEM_MANAGED : SKN_MEM_PAGEABLE;
 }
 
 // A copy to pageable memory waits for the stream, moves the bytes through the driver's own staging and meets the page faults of a
@@ -115,7 +121,7 @@ int32_t skn_sync_results(skn_ctx *ctx, const skn_result *r, int n) {
     for (int i = 0; i < n; ++i) {
         total += (r[i].bytes + 255) / 256 * 256;
         void *dev = nullptr;
-        if (r[i].bytes && (!skn_host_mapped(r[i].host, &dev) || (dev && r[i].bytes > (64 << 10)))) staged = false;     // (page-locked already)
+        if (r[i].bytes && (skn_memory_of(r[i].host, &dev) == SKN_MEM_DEVICE || (dev && r[i].bytes > (64 << 10)))) staged = false;     // (page-locked already)
     }
     if (total == 0 || n > 4 || !staged || !skn_pin_reserve(ctx, total)) {
         for (int i = 0; i < n; ++i)

@@ -182,10 +182,17 @@ __global__ void skn_fetch_kernel(const float4 *__restrict__ src, float4 *__restr
     skn_pdl_wait();
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n4; i += (int64_t)gridDim.x * blockDim.x) dst[i] = src[i];
 }
+// the same for a source off a 16-byte boundary, or a number of elements that is no multiple of four
+__global__ void skn_fetch_odd_kernel(const float *__restrict__ src, float *__restrict__ dst, int64_t n) {
+    skn_pdl_launch_dependents();
+    skn_pdl_wait();
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) dst[i] = src[i];
+}
 cudaError_t skn_launch_fetch(const float *src, float *dst, int64_t n, cudaStream_t st) {
     if (n == 0) return cudaSuccess;
     const int64_t n4 = n / 4;
-    int blocks = (int)((n4 + 255) / 256);
+    const bool odd = (n & 3) || (reinterpret_cast<uintptr_t>(src) & 15);
+    int blocks = (int)(((odd ? n : n4) + 255) / 256);
     if (blocks > 32) blocks = 32;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)blocks);
@@ -196,6 +203,7 @@ cudaError_t skn_launch_fetch(const float *src, float *dst, int64_t n, cudaStream
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
+    if (odd) return cudaLaunchKernelEx(&cfg, skn_fetch_odd_kernel, src, dst, n);
     return cudaLaunchKernelEx(&cfg, skn_fetch_kernel, reinterpret_cast<const float4 *>(src), reinterpret_cast<float4 *>(dst), n4);
 }
 cudaError_t skn_launch_add(const float *a, const float *b, float *out, int64_t n, int sm_count, cudaStream_t st) {

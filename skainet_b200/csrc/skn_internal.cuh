@@ -168,7 +168,10 @@ int32_t skn_stage_reserve(skn_ctx *ctx, void **buf, size_t *cap, size_t need);
 int32_t skn_xq_reserve(skn_ctx *ctx, size_t need, cudaStream_t stream);
 int32_t skn_status_check(skn_ctx *ctx);
 bool skn_pin_reserve(skn_ctx *ctx, size_t need);
-bool skn_host_mapped(const void *p, void **dev);
+// Memory that a host-pointer call is given.  LOCKED: registered or allocated by the CUDA runtime, kernels reach it at an address of their own.
+// MANAGED: kernels reach it where it is.  DEVICE: the host must not touch it.  PAGEABLE: any other.
+enum skn_memory { SKN_MEM_PAGEABLE, SKN_MEM_LOCKED, SKN_MEM_MANAGED, SKN_MEM_DEVICE };
+skn_memory skn_memory_of(const void *p, void **dev);
 
 // results of a host-pointer call, device -> the caller's memory, and the status: returns when they are there
 struct skn_result {

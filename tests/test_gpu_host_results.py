@@ -1,5 +1,7 @@
 """Blocking calls on host buffers of any kind: results in one piece and in several, from and to pageable and page-locked memory."""
 
+import ctypes
+
 import numpy as np
 import pytest
 import torch
@@ -40,6 +42,53 @@ def test_matmul_from_any_host_memory(ctx, qt, M, N, K, kind):
         else:                                              # bf16 activations: 2**-9 of every term at most
             assert (np.abs(y - r) <= 2.0 ** -8 * a).all()
     t.close()
+
+
+def managed(n):
+    """n floats of managed memory and what frees them."""
+    rt, p = ctypes.CDLL("libcudart.so.12"), ctypes.c_void_p()
+    assert rt.cudaMallocManaged(ctypes.byref(p), ctypes.c_size_t(4 * n), 1) == 0
+    return np.ctypeslib.as_array((ctypes.c_float * n).from_address(p.value)), lambda: rt.cudaFree(p)
+
+
+@pytest.mark.parametrize("role", ["x", "bias"])
+@pytest.mark.parametrize("kind", ["pinned", "pinned, read off 16 bytes", "pinned, written off 16 bytes", "managed", "pageable"])
+def test_blocking_call_on_a_result_that_is_still_to_come(ctx, role, kind):
+    """A result of skn_matmul_async is the next, blocking call's x or bias while the GPU is milliseconds behind: stream order, whatever memory
+    it lies in.  As a bias of 513 and four rows of x it does not come in fours either."""
+    g = synth.rng(5)
+    N1, K, N2, K2, M = 520, 512, 513, 512, 4
+    w1, w2, w = synth.make_weight(g, synth.Q4_K, N1, K), synth.make_weight(g, synth.Q4_K, N2, K2), synth.make_weight(g, synth.Q4_K, 4096, 4096)
+    t1, t2, t = (skn.QuantTensor(ctx, s, synth.Q4_K, b) for s, b in (((N1, K), w1), ((N2, K2), w2), ((4096, 4096), w)))
+    x, x2, bias = synth.make_activations(g, 1, K)[0], synth.make_activations(g, M, K2), g.standard_normal(N2).astype(np.float32)
+    busy = [torch.zeros(2048, 4096, device="cuda") for _ in range(2)]
+    free = None
+    if kind == "managed":
+        buf, free = managed(M * N1 + 8)
+    else:
+        buf = np.zeros(M * N1 + 8, dtype=np.float32) if kind == "pageable" else torch.zeros(M * N1 + 8).pin_memory().numpy()
+    out = buf[1:1 + M * N1] if kind.endswith("written off 16 bytes") else buf[:M * N1]
+    at = 1 if kind.endswith("read off 16 bytes") else 0
+    first = np.concatenate([t1.matmul_t(np.roll(x, i)) for i in range(M)])             # blocking, on memory of its own
+    part = lambda a: a[at:at + M * K2].reshape(M, K2) if role == "x" else a[at:at + N2]
+    call = lambda a: t2.matmul_t(part(a), bias) if role == "x" else t2.matmul_t(x2, part(a))
+    want = call(first.copy())
+    rows = [np.roll(x, i) if kind == "pageable" else pinned(np.roll(x, i)) for i in range(M)]
+    for _ in range(3):
+        buf[:] = 0
+        ctx.sync()
+        for _ in range(20):
+            t.matmul_t_dev(busy[0], 2048, busy[1])
+        for i in range(M):
+            t1.matmul_t_async(rows[i], out[i * N1:(i + 1) * N1])
+        got = call(out)
+        assert np.array_equal(got, want)
+        assert np.array_equal(out, first)
+    ctx.sync()
+    for q in (t1, t2, t):
+        q.close()
+    if free:
+        free()
 
 
 def test_rows_that_are_the_last_of_their_sequences(ctx):
