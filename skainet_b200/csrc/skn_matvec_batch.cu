@@ -390,7 +390,10 @@ skn_matvec_batch_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_c
                     for (int g = 0; g < 2; ++g) {
                         uint32_t p[16];
                         mb_half<TYPE>(row, STAGES == 4 ? it & 3 : 2 * (it & 1) + v, g, (sc4 >> (16 * v)) & 0xFFFFu, p, lead, v);
-                        if (v == 0 && g == 0 && !failed && !tc_wait_warp(&a_empty[s], ph ^ 1u, lane)) give_up();
+                        if (v == 0 && g == 0) {
+                            if (!failed && !tc_wait_warp(&a_empty[s], ph ^ 1u, lane)) give_up();
+                            if constexpr (TS) tc_fence_after();                     // the stores follow the MMAs that read the stage
+                        }
                         if constexpr (!TS) {
 #pragma unroll
                             for (int i = 0; i < 4; ++i) tc_store_chunk(tile_a, r, 4 * g + i, make_uint4(p[4 * i], p[4 * i + 1], p[4 * i + 2], p[4 * i + 3]));

@@ -43,3 +43,21 @@ def test_a_warp_that_elects_waits_as_one(name):
     for body in blocks:
         assert "tc_wait_warp(" in body
         assert "skn_mbar_wait(" not in body
+
+
+@pytest.mark.parametrize("name", ["skn_dense.cu", "skn_matmul_tc.cu", "skn_matvec_batch.cu"])
+def test_tensor_memory_is_touched_behind_a_fence(name):
+    """Stores to tensor memory, loads from it and MMAs follow the barrier that they wait for only through tcgen05.fence::after_thread_sync: it
+    stands between every access and the wait before it."""
+    with open(os.path.join(CSRC, name)) as f:
+        text = re.sub(r"//[^\n]*", "", f.read())
+    waited, accesses = None, 0
+    for m in re.finditer(r"(tc_wait_warp|skn_mbar_wait)\(|(tc_fence_after)\(|(?<!void )\b(tc_(?:ld|st)(?:8|16|32)\w*|tc2?_mma_\w+)\(", text):
+        if m[1]:
+            waited = m.start()
+        elif m[2]:
+            waited = None
+        else:
+            accesses += 1
+            assert waited is None, f"{m[3]} at line {text.count(chr(10), 0, m.start()) + 1}, no fence since the wait at line {text.count(chr(10), 0, waited) + 1}"
+    assert accesses >= 2
