@@ -273,7 +273,8 @@ static int32_t matmul_host(skn_ctx *ctx, const skn_tensor *w, const float *x_hos
         const bool may = (!stage_x || xk == SKN_MEM_PAGEABLE) && (!stage_b || bk == SKN_MEM_PAGEABLE) && yk != SKN_MEM_DEVICE;
         if (sync && may && (stage_x || stage_b || !ym) && (few || skn_pin_reserve(ctx, staged))) {
             uint8_t *h = few ? ctx->h_status_base : ctx->h_pin, *d = few ? (uint8_t *)ctx->h_status_dev - SKN_SMALL_OUT_BYTES : ctx->h_pin_dev;
-            if (stage_x || stage_b) {
+            // (asking the stream takes 1.8 us of a 29 us call: not where the context's own stream was left empty by the call before this one)
+            if ((stage_x || stage_b) && !(ctx->stream == ctx->own_stream && ctx->quiet_at + 1 == ctx->entries)) {
                 const cudaError_t idle = cudaStreamQuery(ctx->stream);
                 if (idle != cudaSuccess) {
                     cudaGetLastError();                    // (not ready is kept as an error, too)
@@ -305,8 +306,10 @@ static int32_t matmul_host(skn_ctx *ctx, const skn_tensor *w, const float *x_hos
             SKN_CUDA(ctx, skn_launch_fetch((const float *)ctx->d_status, (float *)ctx->h_status_dev, 4, ctx->stream));
             SKN_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
             rc = skn_status_check(ctx);
-            if (rc == SKN_OK && y_staged) memcpy(y_host, y_staged, yb);
-            return rc;
+            if (rc) return rc;
+            ctx->quiet_at = ctx->entries;
+            if (y_staged) memcpy(y_host, y_staged, yb);
+            return SKN_OK;
         }
     }
     if (sync && yb <= SKN_SMALL_OUT_BYTES) {

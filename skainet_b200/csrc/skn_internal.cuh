@@ -69,6 +69,7 @@ struct skn_ctx {
     // (entry points call one another); a second thread gets SKN_ERR_BUSY
     uint64_t owner;
     int owner_depth;
+    uint64_t entries, quiet_at;  // calls that claimed the context, and the last one after which nothing was left on its stream
     char err[512];
 };
 
@@ -83,6 +84,7 @@ struct skn_busy_guard {
         if (__atomic_compare_exchange_n(&c->owner, &expected, me, false, __ATOMIC_ACQUIRE, __ATOMIC_RELAXED)) {
             ok = true;
             c->owner_depth = 1;
+            ++c->entries;
         } else if (expected == me) {
             ok = true;
             ++c->owner_depth;
