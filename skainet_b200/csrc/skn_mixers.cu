@@ -908,8 +908,9 @@ skn_ret_scan_kernel(skn_ret_args r, skn_step st, float *S, int H, int dk, int vp
     *sp = s;
 }
 
-// rows of O (shared): divided by their root mean square, gated, scaled, stored
-__device__ __forceinline__ void ret_finish(const skn_ret_args &r, const float *O, int os, int64_t row0, int L, int h, int dv) {
+// rows of outputs (at(row, column), in shared memory): divided by their root mean square, gated, scaled, stored
+template <class AT>
+__device__ __forceinline__ void ret_finish(const skn_ret_args &r, AT at, int64_t row0, int L, int h, int dv) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     constexpr int R = 4, C = 4;                    // rows of a warp at a time, and columns per lane: their gates are asked for together
     for (int t0 = warp * R; t0 < L; t0 += 8 * R) {
@@ -924,7 +925,7 @@ __device__ __forceinline__ void ret_finish(const skn_ret_args &r, const float *O
 #pragma unroll
         for (int i = 0; i < R; ++i)
             if (t0 + i < L)
-                for (int d = lane; d < dv; d += 32) ss[i] = fmaf(O[(t0 + i) * os + d], O[(t0 + i) * os + d], ss[i]);
+                for (int d = lane; d < dv; d += 32) ss[i] = fmaf(at(t0 + i, d), at(t0 + i, d), ss[i]);
 #pragma unroll
         for (int i = 0; i < R; ++i) ss[i] = r.out_scale / sqrtf(warp_sum(ss[i]) / (float)dv + r.eps);
 #pragma unroll
@@ -934,11 +935,11 @@ __device__ __forceinline__ void ret_finish(const skn_ret_args &r, const float *O
 #pragma unroll
             for (int c = 0; c < C; ++c) {
                 const int d = lane + 32 * c;
-                if (d < dv) put_out(r.out, row0 + t, (int64_t)h * dv + d, O[t * os + d] * ss[i] * (g[i][c] / (1.f + expf(-g[i][c]))));
+                if (d < dv) put_out(r.out, row0 + t, (int64_t)h * dv + d, at(t, d) * ss[i] * (g[i][c] / (1.f + expf(-g[i][c]))));
             }
             for (int d = lane + 32 * C; d < dv; d += 32) {
                 const float x = __ldcg(r.g + (row0 + t) * r.ld + (int64_t)h * dv + d);
-                put_out(r.out, row0 + t, (int64_t)h * dv + d, O[t * os + d] * ss[i] * (x / (1.f + expf(-x))));
+                put_out(r.out, row0 + t, (int64_t)h * dv + d, at(t, d) * ss[i] * (x / (1.f + expf(-x))));
             }
         }
     }
@@ -1035,7 +1036,7 @@ skn_ret_out_kernel(skn_ret_args r, int T, int H, int dk, int dv, int vp, int nch
             for (int y = 0; y < 4; ++y) O[(ti + x) * os + v0 + tj + y] = fmaf(pw[ti + x + 1], p[x][y], o[x][y]);
     }
     __syncthreads();
-    ret_finish(r, O, os, row0, L, h, dv);
+    ret_finish(r, [&](int t, int d) { return O[t * os + d]; }, row0, L, h, dv);
 }
 
 // ---- retention chunks on the tensor cores -----------------------------------------------------------------------------
@@ -1135,8 +1136,9 @@ skn_ret_chunk_tc_kernel(skn_ret_args r, int T, int H, int dk, int dv, int vp, in
 }
 
 // Outputs of one chunk (see skn_ret_out_kernel).  Bytes of shared memory: planes of q [RC][dkp + 8] | of the scores [RC][RC + 8] | of a tile
-// [32][RT2 + 8] (keys, then rows of the state and values), the fp32 outputs [RC][vw + 4] over the first two when there is one block of
-// columns, else behind.  A warp owns 16 rows and half of a tile's columns.
+// [32][RT2 + 8] (keys, then rows of the state and values) | the fp32 outputs of all blocks of RT2 columns but the last [RC][vw - RT2 + 4].  Those of
+// the last block [RC][RT2 + 4] lie over the planes, which nothing reads any more: with all of them behind, 128 x 512, 256 x 384 and 352 x 256
+// (keys x values) would not fit.  A warp owns 16 rows and half of a tile's columns.
 struct ret_out_layout {
     int dkp, vw, lq, la, scores, tile, out, bytes;                      // row strides and offsets in bytes
     __host__ __device__ ret_out_layout(int dk, int dv) {
@@ -1146,9 +1148,9 @@ struct ret_out_layout {
         la = (RC + 8) * 2;
         scores = 3 * RC * lq;
         tile = scores + 3 * RC * la;
-        const int end = tile + 3 * 32 * RTS, o = RC * (vw + 4) * 4;
-        out = vw == RT2 ? 0 : end;
-        bytes = out ? end + o : end > o ? end : o;
+        const int end = tile + 3 * 32 * RTS, last = RC * (RT2 + 4) * 4;
+        out = end > last ? end : last;
+        bytes = out + (vw > RT2 ? RC * (vw - RT2 + 4) * 4 : 0);
     }
 };
 constexpr size_t RET_SMEM_MAX = 226 * 1024;
@@ -1160,8 +1162,9 @@ skn_ret_out_tc_kernel(skn_ret_args r, int T, int H, int dk, int dv, int vp, int 
     __shared__ float pw[RC + 1];
     const ret_out_layout l(dk, dv);
     uint8_t *Q = smb, *A = smb + l.scores, *B = smb + l.tile;
-    float *O = reinterpret_cast<float *>(smb + l.out);
-    const int QP = RC * l.lq, AP = RC * l.la, BP = 32 * RTS, os = l.vw + 4;
+    float *O = reinterpret_cast<float *>(smb + l.out), *P = reinterpret_cast<float *>(smb);     // outputs up to column `first`, those of the last block
+    const int QP = RC * l.lq, AP = RC * l.la, BP = 32 * RTS, first = l.vw - RT2, os = first + 4;
+    constexpr int ps = RT2 + 4;
     skn_pdl_launch_dependents();
     skn_pdl_wait();
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, c = blockIdx.x, h = blockIdx.y, seq = blockIdx.z, t0 = c * RC, L = min(RC, T - t0);
@@ -1286,15 +1289,17 @@ skn_ret_out_tc_kernel(skn_ret_args r, int T, int H, int dk, int dv, int vp, int 
                     for (int e = 0; e < 4; ++e) o[4 * nb + n][e] += mn[n][e] + sm[n][e];
             }
         }
-        __syncthreads();                           // the outputs may lie over q and the scores
+        __syncthreads();                           // the last block's outputs lie over q, the scores and the tile
+        float *to = v0 < first ? O + v0 : P;
+        const int ts = v0 < first ? os : ps;
 #pragma unroll
         for (int n = 0; n < 8; ++n)
 #pragma unroll
             for (int e = 0; e < 2; ++e)
-                *reinterpret_cast<float2 *>(O + (m0 + g + e * 8) * os + v0 + c0 + n * 8 + t * 2) = make_float2(o[n][2 * e], o[n][2 * e + 1]);
+                *reinterpret_cast<float2 *>(to + (m0 + g + e * 8) * ts + c0 + n * 8 + t * 2) = make_float2(o[n][2 * e], o[n][2 * e + 1]);
     }
     __syncthreads();
-    ret_finish(r, O, os, row0, L, h, dv);
+    ret_finish(r, [&](int t, int d) { return d < first ? O[t * os + d] : P[t * ps + d - first]; }, row0, L, h, dv);
 }
 
 template <class CT>
