@@ -1,8 +1,10 @@
 // Causal attention of a prompt's queries over the ring cache (fp32, fp16 or Q8_0 rows), on the warp-level tensor cores in the
 // accuracy of the fp32 kernels of skn_kv.cu.
 //
-// Every fp32 operand (queries, keys, probabilities, values) is the exact sum of three bf16 numbers a + b + c, and a product is the six of
-// nine partial products that reach its 24 bits: ac + ca + bb, ab + ba, aa.  A chain of the six runs from zero for each 16 elements of a
+// Every fp32 operand (queries, keys, probabilities, values) from 2^-110 up to the last 0.4 % of the range is the exact sum of three bf16 numbers
+// a + b + c, and a product is the six of nine partial products that reach its 24 bits: ac + ca + bb, ab + ba, aa.  (Below, c loses its bits
+// under 2^-133.  Above, and where an operand is not finite, a tile of keys is computed in plain fp32: one that holds such a key or value, and
+// all of a CTA that holds such a query.)  A chain of the six runs from zero for each 16 elements of a
 // reduction and its result is added in an fp32 register: the tensor cores chop what they add to an accumulator, a sum that stayed there
 // would drift.  Probabilities, maxima, sums and outputs are fp32 as before; the error against 64 bits is not larger
 // (tests/test_gpu_attn_prompt.py).
@@ -13,9 +15,10 @@
 // for most of the time, twice as long.  A group's next tile is on its way into registers while this one is multiplied.
 // CTAs with the most keys start first.
 //
-// 512 tokens, 32 heads of 128 over 8 kv heads: 173 us with the fp32 split kernels and their merge, 70 here; 16 sequences of 20 tokens 35 and 19, 128 tokens after
-// 272 of 4 sequences in Q8_0 236 and 109.  The products alone would take 24 (m16n8k16: 8 clocks of a scheduler, 96 of them for 16 rows x 8
-// keys); the tensor pipe is busy a third of the time, the rest is the latency of conversions, exponentials and fragment loads at two warps per scheduler.
+// 512 tokens, 32 heads of 128 over 8 kv heads, launches back to back: 194 us with the fp32 split kernels and their merge, 71 here; 16 sequences
+// of 20 tokens 36 and 20, 128 tokens of 4 sequences after 384 others 262 and 117.  The products alone would take 23 (m16n8k16: 8 clocks of a scheduler, 96 of
+// them for 16 rows x 8 keys); the tensor pipe is busy a third of the time, the rest is the latency of conversions, exponentials and
+// fragment loads at two warps per scheduler.
 #include "skn_internal.cuh"
 #include "skn_mma.cuh"
 
@@ -81,6 +84,8 @@ __device__ __forceinline__ void ap_split_store(uint8_t *at, int plane_bytes, flo
     }
 }
 
+__device__ __forceinline__ bool ap_finite(__nv_bfloat162 x) { return fabsf(__low2float(x)) < INFINITY && fabsf(__high2float(x)) < INFINITY; }
+
 // barriers of one group
 __device__ __forceinline__ void ap_sync(int group) { asm volatile("barrier.sync %0, %1;" ::"r"(group + 1), "n"(AP_GROUP) : "memory"); }
 __device__ __forceinline__ bool ap_sync_or(int group, bool x) {
@@ -126,10 +131,28 @@ skn_attn_prompt_kernel(const ap_args a) {
         x.x *= a.scale; x.y *= a.scale; x.z *= a.scale; x.w *= a.scale;
         return x;
     };
-    for (int i = threadIdx.x; i < AP_ROWS * (D / 4); i += GROUPS * AP_GROUP) {
-        const int r = i / (D / 4), d = i % (D / 4) * 4;
-        __nv_bfloat162 any = __floats2bfloat162_rn(0.f, 0.f);
-        ap_split_store<3>(Q + r * LD + d * 2, QP, r < nrows ? query(r, d) : make_float4(0.f, 0.f, 0.f, 0.f), any);
+    __nv_bfloat162 qlast = __floats2bfloat162_rn(0.f, 0.f);
+    // (asked for in fours; not beside fp16 rows of 64, whose tile loop then comes out slower: 256 tokens over 2048, 124 us this way, 129 in fours)
+    if constexpr (D == 64 && DT == SKN_KV_F16) {
+        for (int i = threadIdx.x; i < AP_ROWS * (D / 4); i += GROUPS * AP_GROUP) {
+            const int r = i / (D / 4), d = i % (D / 4) * 4;
+            ap_split_store<3>(Q + r * LD + d * 2, QP, r < nrows ? query(r, d) : make_float4(0.f, 0.f, 0.f, 0.f), qlast);
+        }
+    } else {
+#pragma unroll
+        for (int i0 = 0; i0 < AP_ROWS * (D / 4) / (GROUPS * AP_GROUP); i0 += 4) {
+            float4 x[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int at = (i0 + i) * GROUPS * AP_GROUP + threadIdx.x, r = at / (D / 4);
+                x[i] = r < nrows ? query(r, at % (D / 4) * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int at = (i0 + i) * GROUPS * AP_GROUP + threadIdx.x;
+                ap_split_store<3>(Q + at / (D / 4) * LD + at % (D / 4) * 8, QP, x[i], qlast);
+            }
+        }
     }
     float4 rk[NLD], rv[NLD];
     auto fetch = [&](int t) {
@@ -144,7 +167,8 @@ skn_attn_prompt_kernel(const ap_args a) {
         }
     };
     if (group < tiles) fetch(group);
-    __syncthreads();                                                    // the queries are in place
+    // the queries are in place; where one of them has no three finite terms, all tiles are computed in plain fp32
+    const bool qplain = __syncthreads_or(!ap_finite(qlast)) != 0;
 
     float o[D / 8][4];
 #pragma unroll
@@ -210,7 +234,7 @@ skn_attn_prompt_kernel(const ap_args a) {
         }
         // a key or value without three finite bf16 terms must neither lose its meaning nor, times a masked weight of zero, reach
         // queries before it: such a tile is computed in plain fp32
-        const bool plain = ap_sync_or(group, !(fabsf(__low2float(last)) < INFINITY && fabsf(__high2float(last)) < INFINITY));
+        const bool plain = ap_sync_or(group, qplain || !ap_finite(last));
         const bool none = j0 >= wmax;                                   // no row of this warp sees the tile
         if (none && !plain) {
             if (t + GROUPS < tiles) fetch(t + GROUPS);

@@ -130,3 +130,26 @@ def test_what_is_not_finite_reaches_no_earlier_query(ctx, where, value):
         else:                                                                      # its own column alone, of the value's kind
             assert np.all((np.abs(out - ref) <= 2.0 ** -17 * size)[hit & ~col])
             assert np.isnan(out[col]).all() if np.isnan(value) else np.all((out[col] == value) | np.isnan(out[col]))
+
+
+@pytest.mark.parametrize("value", [np.nan, np.inf, -np.inf, 3.4e38, -3.4e38])
+@pytest.mark.parametrize("B,Hkv,G,D,T,keys,dtype", [(1, 8, 4, 128, 100, 100, "f32"), (1, 8, 4, 64, 128, 700, "f16"), (1, 8, 4, 128, 200, 700, "q8_0"), (9, 8, 4, 128, 20, 32, "f32")])
+def test_what_is_not_finite_in_a_query_reaches_no_other(ctx, B, Hkv, G, D, T, keys, dtype, value):
+    """A query off the range that three bf16 terms have: the scores of one that is finite are those of fp32, against keys so small there that they are ordinary."""
+    g, at = synth.rng(12), T // 2
+    k, v = (g.standard_normal((B, Hkv, keys, D), dtype=np.float32) for _ in range(2))
+    q = g.standard_normal((B, T, Hkv * G, D), dtype=np.float32) * np.float32(0.1)
+    k[..., 5] *= 1e-38
+    q[0, at, 9, 5] = value
+    kv = skn.KVCache(ctx, B, Hkv, D, keys, dtype=dtype)
+    kv.load(k, v, np.full(B, keys, dtype=np.int32))
+    out, pairs = causal(ctx, kv, q, T, 1.0), held(kv)
+    kv.close()
+    rows = np.ones(out.shape, dtype=bool)
+    if not np.isfinite(value):
+        rows[0, at, 9] = False
+        assert np.isnan(out[~rows]).all()
+        q[0, at, 9, 5] = 0.0
+    ref, size = expected(pairs, q, 1.0)
+    assert np.isfinite(out[rows]).all()
+    assert np.all(np.abs(out - ref)[rows] <= 2.0 ** -17 * size[rows])
