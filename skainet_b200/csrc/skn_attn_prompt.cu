@@ -22,6 +22,8 @@
 #include "skn_internal.cuh"
 #include "skn_mma.cuh"
 
+#include <math.h>
+
 constexpr int AP_ROWS = 64, AP_KEYS = 32, AP_RUN = 256, AP_GROUP = 128;
 
 // four consecutive elements of a cached row
@@ -443,10 +445,36 @@ static cudaError_t ap_by_type(int dtype, const ap_args &a, cudaStream_t st) {
     return dtype == SKN_KV_F32 ? ap_launch<D, SKN_KV_F32, GROUPS>(a, st) : dtype == SKN_KV_F16 ? ap_launch<D, SKN_KV_F16, GROUPS>(a, st) : ap_launch<D, SKN_KV_Q8_0, GROUPS>(a, st);
 }
 
-bool skn_attn_prompt_takes(const skn_kvcache *kv, int G, int T) {
+bool skn_attn_prompt_covers(const skn_kvcache *kv, int G, int T) {
     if (T < 2 || (kv->head_dim != 64 && kv->head_dim != 128)) return false;
     const int64_t heads = (int64_t)kv->n_kv_heads * kv->batch, rows = (int64_t)T * G, tiles = (rows + AP_ROWS - 1) / AP_ROWS;
     return tiles * heads < (1 << 30) && rows * heads >= SKN_ATTN_PROMPT_ROWS;
+}
+
+// Whether this kernel is expected to end before the split kernels.  Those share the keys out as well, so their time goes with rows x keys; here
+// a CTA walks all keys of its 64 rows, and the time goes with the keys and the waves of CTAs, however few rows there are.  Microseconds
+// on B200, fitted to 548 shapes (1 to 16 sequences, 1 to 8 heads a group, 2 to 1024 tokens, contexts to 16384): all but 9 of them take
+// the faster kernel to within 3 %, the others lose 4 us at most.  Tokens over cached ones, 32 heads of 128 over 8 kv heads, fp32, split
+// kernels / this one:
+//          context 512     2048          8192
+//   64     51 / 65         141 / 229     518 / 888
+//   96     67 / 65         203 / 228     771 / 887
+//   128    90 / 65         266 / 227     1018 / 887
+//   256    142 / 66        499 / 227     1997 / 887
+bool skn_attn_prompt_faster(const skn_kvcache *kv, int G, int T, int keys) {
+    const bool q8 = kv->dtype == SKN_KV_Q8_0, wide = kv->head_dim == 128;
+    const double heads = (double)kv->n_kv_heads * kv->batch, krows = heads * G * T / 1000.0, seen = keys - T / 2.0;
+    // split kernels: a key for a thousand rows, by heads of a group
+    static const double split[2][2][4] = {{{.061, .037, .025, .024}, {.075, .047, .031, .031}}, {{.081, .045, .028, .021}, {.093, .053, .034, .032}}};
+    const double per = split[q8][wide][G == 1 ? 0 : G == 2 ? 1 : G == 4 ? 2 : 3];
+    const double before = 14.0 + krows * (seen * per + 4.0 * (keys < 256 ? keys / 256.0 : 1.0));
+    // here: a key for a wave; fp16 rows are converted as they arrive, which waits for them where the cache is not in L2
+    static const double tile[3][2] = {{.057, .108}, {.055, .115}, {.071, .131}};
+    double key = tile[q8 ? 2 : kv->dtype == SKN_KV_F16 ? 1 : 0][wide];
+    if (kv->dtype == SKN_KV_F16 && heads * keys * kv->head_dim * 4.0 > 48e6) key *= 1.4;
+    const double ctas = heads * ((T * G + AP_ROWS - 1) / AP_ROWS), waves = ceil(ctas / kv->ctx->sm_count);
+    const double most = fmax(fmax((double)keys, (double)AP_KEYS), waves * seen);
+    return 12.0 + key * most + 1.0 <= before;
 }
 
 cudaError_t skn_launch_attn_prompt(const skn_kvcache *kv, const float *q, int G, int T, float scale, int len_extra, int keys, float *out, void *out_bf16, cudaStream_t st) {

@@ -282,9 +282,11 @@ int32_t skn_kv_rope_append_pending(skn_kvcache *kv, float *q_dev, const float *k
 // host_len: no sequence had more tokens before the T pending ones.  out_bf16 (optional): where the tensor-core form puts its rows instead, rounded; *wrote_bf16 says whether it did
 int32_t skn_attn_causal_pending(skn_kvcache *kv, const float *q_dev, int32_t n_q_heads, int32_t T, float scale,
                                 int32_t host_len, float *out_dev, void *out_bf16 = nullptr, bool *wrote_bf16 = nullptr);
-// the tensor-core form of the many-query kernels (skn_attn_prompt.cu), from this many (query, head) rows on; keys: no sequence holds more
+// the tensor-core form of the many-query kernels (skn_attn_prompt.cu), from this many (query, head) rows of all sequences on, where it is the
+// faster one; keys: no sequence holds more
 constexpr int64_t SKN_ATTN_PROMPT_ROWS = 2048;
-bool skn_attn_prompt_takes(const skn_kvcache *kv, int G, int T);
+bool skn_attn_prompt_covers(const skn_kvcache *kv, int G, int T);
+bool skn_attn_prompt_faster(const skn_kvcache *kv, int G, int T, int keys);
 cudaError_t skn_launch_attn_prompt(const skn_kvcache *kv, const float *q, int G, int T, float scale, int len_extra, int keys, float *out, void *out_bf16, cudaStream_t st);
 int32_t *skn_kv_len_dev(const skn_kvcache *kv);
 cudaError_t skn_kv_advance_all(int32_t *const *lens_dev, int n_layers, int B, int T, int cap, int32_t *status_dev,

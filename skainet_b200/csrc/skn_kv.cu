@@ -1299,20 +1299,33 @@ static int32_t attn_causal_impl(skn_kvcache *kv, const float *q_dev, int32_t n_q
     if ((((uintptr_t)q_dev) | ((uintptr_t)out_dev) | ((uintptr_t)scratch_dev)) & 15)
         return skn_fail(ctx, SKN_ERR_ALIGN, "q, out and scratch must be 16-byte aligned");
     SKN_CUDA(ctx, cudaSetDevice(ctx->device));
-    if (skn_attn_prompt_takes(kv, G, T)) {
+    const bool covered = skn_attn_prompt_covers(kv, G, T);
+    bool prompt = covered && skn_attn_prompt_faster(kv, G, T, keys);
+    int chunk = ATT_CHUNK;
+    float *part = (float *)scratch_dev;
+    if (!prompt && !part) {
+        chunk = attn_pick_chunk(kv, n_q_heads, T, (size_t)64 << 20);
+        const size_t S = (size_t)(kv->capacity + chunk - 1) / chunk, need = (size_t)kv->batch * T * n_q_heads * S * (kv->head_dim + 2) * sizeof(float);
+        // (the prompt kernel needs no room for partial results: it takes what it covers where there is none, and while a graph is captured none is made)
+        if (covered && need > ctx->d_scratch2_bytes) {
+            cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+            SKN_CUDA(ctx, cudaStreamIsCapturing(ctx->stream, &capture));
+            prompt = capture != cudaStreamCaptureStatusNone;
+        }
+        if (!prompt) {
+            rc = skn_stage_reserve(ctx, &ctx->d_scratch2, &ctx->d_scratch2_bytes, need);
+            if (rc && !covered) return rc;
+            if (rc) {
+                cudaGetLastError();
+                prompt = true;
+            }
+            part = (float *)ctx->d_scratch2;
+        }
+    }
+    if (prompt) {
         SKN_CUDA(ctx, skn_launch_attn_prompt(kv, q_dev, G, T, scale, len_extra, keys, out_dev, out_bf16, ctx->stream));
         if (wrote_bf16) *wrote_bf16 = out_bf16 != nullptr;
         return SKN_OK;
-    }
-    int chunk = ATT_CHUNK;
-    float *part = (float *)scratch_dev;
-    if (!part) {
-        chunk = attn_pick_chunk(kv, n_q_heads, T, (size_t)64 << 20);
-        const int S = (kv->capacity + chunk - 1) / chunk;
-        rc = skn_stage_reserve(ctx, &ctx->d_scratch2, &ctx->d_scratch2_bytes,
-                               (size_t)kv->batch * T * n_q_heads * S * (kv->head_dim + 2) * sizeof(float));
-        if (rc) return rc;
-        part = (float *)ctx->d_scratch2;
     }
     SKN_CUDA(ctx, dispatch_attn(kv, G, q_dev, scale, part, chunk, out_dev, ctx->stream, T, len_extra));
     return SKN_OK;

@@ -1,6 +1,8 @@
-"""Causal attention of many queries on the tensor cores (three bf16 terms per fp32 operand) against fp64 on what the cache holds: edges of
-tiles of 64 (query, head) rows and 32 keys, rings that wrap, queries before the first key, values without finite bf16 terms."""
+"""Causal attention of many queries against fp64 on what the cache holds, on the tensor cores (three bf16 terms per fp32 operand) and where the rule
+leaves it to the split kernels: edges of tiles of 64 (query, head) rows and 32 keys, rings that wrap, queries before the first key, operands
+without finite bf16 terms, few queries over many keys."""
 import ctypes
+import math
 
 import numpy as np
 import pytest
@@ -20,6 +22,28 @@ def causal(ctx, kv, q, T, scale):
     assert rc == 0
     ctx.sync()
     return out.cpu().numpy()
+
+
+def routed(ctx, kv, q, T, scale):
+    """The same with the caller's scratch memory, and whether the tensor-core kernel took the call: it leaves that alone."""
+    qd = torch.from_numpy(q).cuda()
+    out, scratch = torch.full_like(qd, np.nan), torch.full((T * kv.scratch_bytes(q.shape[2]) // 4,), 7.0, device="cuda")
+    torch.cuda.synchronize()
+    rc = _ffi.lib().skn_attn_causal_dev(kv.handle, qd.data_ptr(), q.shape[2], T, ctypes.c_float(scale), out.data_ptr(), scratch.data_ptr())
+    assert rc == 0
+    ctx.sync()
+    return out.cpu().numpy(), bool((scratch == 7.0).all())
+
+
+def faster(B, Hkv, G, D, dtype, T, keys):
+    """The rule of skn_attn_prompt_faster: estimated microseconds of the split kernels and of the tensor-core kernel."""
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    heads, seen, q8, f16 = B * Hkv, keys - T / 2, dtype == "q8_0", dtype == "f16"
+    per = {(64, 0): (.061, .037, .025, .024), (128, 0): (.075, .047, .031, .031), (64, 1): (.081, .045, .028, .021), (128, 1): (.093, .053, .034, .032)}[D, q8]
+    split = 14 + heads * G * T / 1000 * (seen * per[int(math.log2(G))] + 4 * min(1, keys / 256))
+    key = {"f32": (.057, .108), "f16": (.055, .115), "q8_0": (.071, .131)}[dtype][D == 128] * (1.4 if f16 and heads * keys * D * 4 > 48e6 else 1)
+    ctas = heads * -(-T * G // 64)
+    return heads * G * T >= 2048 and 12 + key * max(keys, 32, -(-ctas // sms) * seen) + 1 <= split
 
 
 def held(kv):
@@ -70,6 +94,71 @@ def test_prompt_attention(ctx, B, Hkv, G, D, T, cap, lens, dtype):
     kv.close()
 
 
+@pytest.mark.parametrize("dtype", ["f32", "f16", "q8_0"])
+@pytest.mark.parametrize("B,Hkv,G,D,T,cap,lens", [
+    (2, 8, 4, 128, 64, 64, [64, 64]), (2, 8, 4, 128, 65, 400, [97, 400]), (4, 4, 8, 64, 33, 300, [33, 260, 299, 64]), (3, 8, 1, 128, 129, 161, [161, 130, 129]),
+    (4, 8, 2, 128, 47, 96, [96, 48, 47, 50]), (1, 32, 1, 128, 64, 1000, [1000]), (16, 8, 8, 128, 5, 70, [5 + 4 * i for i in range(16)]),
+    (9, 8, 4, 128, 20, 32, [20, 32, 31, 21, 32, 25, 24, 30, 32]), (9, 8, 4, 128, 20, 33, [20, 33, 31, 21, 32, 25, 24, 30, 32]),
+    (9, 4, 8, 64, 17, 31, [17, 31, 18, 30, 24, 31, 31, 17, 20]), (1, 8, 4, 128, 200, 1300, [1300])])
+def test_prompt_attention_on_the_tensor_cores(ctx, B, Hkv, G, D, T, cap, lens, dtype):
+    g = synth.rng(T + cap + D)
+    kv = skn.KVCache(ctx, B, Hkv, D, cap, dtype=dtype)
+    k, v = (g.standard_normal((B, Hkv, cap, D), dtype=np.float32) for _ in range(2))
+    kv.load(k, v, np.array(lens, dtype=np.int32))
+    q = g.standard_normal((B, T, Hkv * G, D), dtype=np.float32)
+    out, taken = routed(ctx, kv, q, T, D ** -0.5)
+    assert taken
+    check(out, held(kv), q, D ** -0.5)
+    assert np.array_equal(out, causal(ctx, kv, q, T, D ** -0.5))
+    for _ in range(5):                                     # rings that were full go on: their first token is not in slot 0 any more
+        kv.append(*(g.standard_normal((B, Hkv, D), dtype=np.float32) for _ in range(2)))
+    check(causal(ctx, kv, q, T, D ** -0.5), held(kv), q, D ** -0.5)
+    kv.close()
+
+
+@pytest.mark.parametrize("dtype", ["f32", "f16", "q8_0"])
+@pytest.mark.parametrize("B,Hkv,G,D,T,keys,taken", [
+    (1, 8, 4, 128, 64, 4000, False), (1, 8, 4, 128, 100, 2000, False), (1, 8, 4, 128, 256, 2000, True), (1, 4, 8, 128, 64, 1500, False), (4, 8, 4, 128, 16, 2000, False),
+    (4, 8, 4, 128, 64, 1000, True), (16, 8, 8, 128, 2, 500, False), (1, 8, 2, 128, 128, 1000, False), (1, 8, 2, 128, 256, 1000, True), (1, 8, 1, 64, 256, 1500, True),
+    (1, 2, 1, 128, 1024, 1024, False), (1, 2, 4, 128, 256, 1000, False), (1, 8, 4, 128, 63, 100, False)])
+def test_few_queries_over_many_keys_are_left_to_the_split_kernels(ctx, B, Hkv, G, D, T, keys, dtype, taken):
+    """A CTA of the tensor-core kernel walks all keys whatever the number of CTAs: which kernel runs, and that both are right."""
+    assert faster(B, Hkv, G, D, dtype, T, keys) == taken
+    g = synth.rng(T + keys + D)
+    kv = skn.KVCache(ctx, B, Hkv, D, keys, dtype=dtype)
+    k, v = (g.standard_normal((B, Hkv, keys, D), dtype=np.float32) for _ in range(2))
+    kv.load(k, v, np.full(B, keys, dtype=np.int32))
+    q = g.standard_normal((B, T, Hkv * G, D), dtype=np.float32)
+    out, tensor_cores = routed(ctx, kv, q, T, D ** -0.5)
+    assert tensor_cores == taken
+    check(out, held(kv), q, D ** -0.5)
+    check(causal(ctx, kv, q, T, D ** -0.5), held(kv), q, D ** -0.5)
+    kv.close()
+
+
+def test_a_captured_call_without_scratch_memory():
+    """While a graph is captured nothing can be allocated: the tensor-core kernel takes what the rule would leave to the split kernels."""
+    with skn.Context(0) as own:
+        g = synth.rng(21)
+        Hkv, G, D, T, keys = 8, 4, 128, 64, 2000
+        kv = skn.KVCache(own, 1, Hkv, D, keys)
+        kv.load(*(g.standard_normal((1, Hkv, keys, D), dtype=np.float32) for _ in range(2)), np.array([keys], dtype=np.int32))
+        q = g.standard_normal((1, T, Hkv * G, D), dtype=np.float32)
+        qd = torch.from_numpy(q).cuda()
+        out = torch.full_like(qd, np.nan)
+        torch.cuda.synchronize()
+        stream, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+        own.set_stream(stream.cuda_stream)
+        with torch.cuda.stream(stream), torch.cuda.graph(graph, stream=stream):
+            rc = _ffi.lib().skn_attn_causal_dev(kv.handle, qd.data_ptr(), Hkv * G, T, ctypes.c_float(D ** -0.5), out.data_ptr(), None)
+        assert rc == 0
+        for _ in range(2):
+            graph.replay()
+        torch.cuda.synchronize()
+        check(out.cpu().numpy(), held(kv), q, D ** -0.5)
+        kv.close()
+
+
 def test_queries_before_the_first_key_are_zero(ctx):
     g = synth.rng(3)
     B, Hkv, G, D, T, cap = 3, 8, 4, 128, 70, 100
@@ -83,11 +172,12 @@ def test_queries_before_the_first_key_are_zero(ctx):
     kv.close()
 
 
+@pytest.mark.parametrize("T", [80, 128])
 @pytest.mark.parametrize("size_q,size_k,size_v", [(1.0, 1.0, 1e30), (1e-12, 1e12, 1e-30), (30.0, 1.0, 1.0)])
-def test_sizes_of_values(ctx, size_q, size_k, size_v):
+def test_sizes_of_values(ctx, size_q, size_k, size_v, T):
     """One element in eight is a thousand times the others: every term keeps its own 24 bits."""
     g = synth.rng(7)
-    B, Hkv, G, D, T = 1, 8, 4, 128, 80
+    B, Hkv, G, D = 1, 8, 4, 128
     kv = skn.KVCache(ctx, B, Hkv, D, T)
     k, v = (g.standard_normal((B, Hkv, T, D), dtype=np.float32) * size for size in (size_k, size_v))
     q = g.standard_normal((B, T, Hkv * G, D), dtype=np.float32) * size_q
@@ -104,6 +194,7 @@ def test_sizes_of_values(ctx, size_q, size_k, size_v):
 def test_what_is_not_finite_reaches_no_earlier_query(ctx, where, value):
     g = synth.rng(11)
     B, Hkv, G, D, T, at = 1, 8, 4, 128, 100, 70
+    assert faster(B, Hkv, G, D, "f32", T, T)
     k, v = (g.standard_normal((B, Hkv, T, D), dtype=np.float32) for _ in range(2))
     q = g.standard_normal((B, T, Hkv * G, D), dtype=np.float32)
     (k if where == "k" else v)[0, 2, at, 5] = value
@@ -136,6 +227,7 @@ def test_what_is_not_finite_reaches_no_earlier_query(ctx, where, value):
 @pytest.mark.parametrize("B,Hkv,G,D,T,keys,dtype", [(1, 8, 4, 128, 100, 100, "f32"), (1, 8, 4, 64, 128, 700, "f16"), (1, 8, 4, 128, 200, 700, "q8_0"), (9, 8, 4, 128, 20, 32, "f32")])
 def test_what_is_not_finite_in_a_query_reaches_no_other(ctx, B, Hkv, G, D, T, keys, dtype, value):
     """A query off the range that three bf16 terms have: the scores of one that is finite are those of fp32, against keys so small there that they are ordinary."""
+    assert faster(B, Hkv, G, D, dtype, T, keys)
     g, at = synth.rng(12), T // 2
     k, v = (g.standard_normal((B, Hkv, keys, D), dtype=np.float32) for _ in range(2))
     q = g.standard_normal((B, T, Hkv * G, D), dtype=np.float32) * np.float32(0.1)
