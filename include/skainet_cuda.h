@@ -183,7 +183,8 @@ int32_t skn_dequantize_dev(skn_ctx *ctx, const skn_tensor *t, float *out_dev);
  * (core/src/commonMain/kotlin/sk/ai/net/impl/DoublesTensor.kt:255-279) without the
  * per-call transposed copy (DoublesTensor.kt:362-387).  K != n_cols fails with
  * SKN_ERR_SHAPE ("Shapes do not align.", DoublesTensor.kt:256).  `bias` ([n_rows]
- * fp32, may be NULL) is added as Linear does. */
+ * fp32, may be NULL) is added as Linear does.  x_host and bias_host may be results of calls that are still
+ * enqueued. */
 int32_t skn_matmul(skn_ctx *ctx, const skn_tensor *w, const float *x_host, int32_t M, int64_t K,
                    const float *bias_host, float *y_host);
 int32_t skn_matmul_dev(skn_ctx *ctx, const skn_tensor *w, const float *x_dev, int32_t M, int64_t K,

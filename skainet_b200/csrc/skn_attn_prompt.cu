@@ -15,8 +15,8 @@
 // for most of the time, twice as long.  A group's next tile is on its way into registers while this one is multiplied.
 // CTAs with the most keys start first.
 //
-// 512 tokens, 32 heads of 128 over 8 kv heads, launches back to back: 194 us with the fp32 split kernels and their merge, 71 here; 16 sequences
-// of 20 tokens 36 and 20, 128 tokens of 4 sequences after 384 others 262 and 117.  The products alone would take 23 (m16n8k16: 8 clocks of a scheduler, 96 of
+// 512 tokens, 32 heads of 128 over 8 kv heads, launches back to back: 194 to 219 us with the fp32 split kernels and their merge, 72 here;
+// 16 sequences of 20 tokens 36 and 20, 128 tokens of 4 sequences after 384 others 262 and 118.  The products alone would take 23 (m16n8k16: 8 clocks of a scheduler, 96 of
 // them for 16 rows x 8 keys); the tensor pipe is busy a third of the time, the rest is the latency of conversions, exponentials and
 // fragment loads at two warps per scheduler.
 #include "skn_internal.cuh"
@@ -457,10 +457,10 @@ bool skn_attn_prompt_covers(const skn_kvcache *kv, int G, int T) {
 // the faster kernel to within 3 %, the others lose 4 us at most.  Tokens over cached ones, 32 heads of 128 over 8 kv heads, fp32, split
 // kernels / this one:
 //          context 512     2048          8192
-//   64     51 / 65         141 / 229     518 / 888
-//   96     67 / 65         203 / 228     771 / 887
-//   128    90 / 65         266 / 227     1018 / 887
-//   256    142 / 66        499 / 227     1997 / 887
+//   64     51 / 65         144 / 229     519 / 887
+//   96     67 / 65         206 / 229     769 / 888
+//   128    82 / 65         265 / 229     1014 / 887
+//   256    155 / 66        500 / 229     1997 / 888
 bool skn_attn_prompt_faster(const skn_kvcache *kv, int G, int T, int keys) {
     const bool q8 = kv->dtype == SKN_KV_Q8_0, wide = kv->head_dim == 128;
     const double heads = (double)kv->n_kv_heads * kv->batch, krows = heads * G * T / 1000.0, seen = keys - T / 2.0;

@@ -25,9 +25,9 @@
 //
 // Measured (B200, graph of distinct weights, us per call with the preparation of x; the kernels that took these rows before -> one issuing warp, weights
 // in shared memory, eight draining warps -> now):
-//   Q4_K 14336 x 4096: 16 rows 69 -> 28.1 -> 23.6, 32 rows 137 -> 35.6 -> 29.1; 28672 x 4096: 16 rows 110 -> 56 -> 46.6; 4096 x 4096: 22 -> 13.2 -> 11.5
-//   Q4_0 4096 x 14336: 16 rows 75 -> 35.5 -> 32.0, 32 rows 149 -> 52.5 -> 45.8; Q8_0 14336 x 4096: 16 rows 73 -> 43.6 -> 34.7, 24 rows 143 -> 52.2 -> 49.6
-//   Q6_K 32000 x 4096: 16 rows 116 -> 93; 4096 x 14336: 186 -> 53.6 -> 44
+//   Q4_K 14336 x 4096: 16 rows 69 -> 28.1 -> 22.4, 32 rows 137 -> 35.6 -> 28.3; 28672 x 4096: 16 rows 110 -> 56 -> 44.4; 4096 x 4096: 22 -> 13.2 -> 10.1
+//   Q4_0 4096 x 14336: 16 rows 75 -> 35.5 -> 31.9, 32 rows 149 -> 52.5 -> 46.0; Q8_0 14336 x 4096: 16 rows 73 -> 43.6 -> 34.1, 24 rows 143 -> 52.2 -> 48.8
+//   Q6_K 32000 x 4096: 16 rows 116 -> 92; 4096 x 14336: 186 -> 53.6 -> 43.6
 // No one part bounds it: for 14336 x 4096 Q4_K with any of unpacking, products and draining left out it took 24 of 26 us, with all of them left out (rings,
 // barriers and loads of the blocks only) 15.4, of which 7.5 are preparation, start and end; two instead of one issuing warp gave 1.0, a second set of
 // draining warps 0.8, a fourth unpacking group 0.8.  A deeper ring of blocks, and blocks copied as contiguous pieces, gave nothing.
@@ -268,7 +268,7 @@ __host__ __device__ constexpr int mb_sets(int type, int nch) {
 //   PARTS   ... and the chunks of x
 // The threads share 64 K registers, and a draining thread holds its sums for all its rows of x, so what pays depends on those (us): Q4_0 4096 x 14336 and
 // Q8_0 14336 x 4096 at 16 rows, three groups and two sets 32.0 and 34.7, four groups and one set 35.2 and 37.9; Q4_K 14336 x 4096 at 16 rows, four groups
-// and two sets 23.6, three 24.5; at 24 and 32 rows three groups and one set 27.7 and 29.1, four groups 30.2 and 30.8.
+// and two sets 23.6, three 24.5 (1.2 more than now: see the launch's arguments below); at 24 and 32 rows three groups and one set 27.7 and 29.1, four groups 30.2 and 30.8.
 template <int TYPE, int NCH> struct MbWarps {
     static constexpr bool FOUR = mb_ts(TYPE, NCH) && mb_ts_stages(TYPE, NCH) == 4, K4 = TYPE == SKN_TYPE_Q4_K, BLOCK = TYPE == SKN_TYPE_Q4_0 || TYPE == SKN_TYPE_Q8_0;
     static constexpr int GROUPS = FOUR && !(BLOCK && NCH > 1) && !(K4 && NCH > 2) ? 4 : 3;

@@ -595,6 +595,7 @@ static bool head_prep_aligned(const skn_attn_args *a, const skn_ret_args *r, con
 constexpr int ATQ = 64, ATK = 32;      // queries and keys of a tile
 constexpr int AT_THREADS = ATQ * 2;    // a warp owns 16 queries
 
+// (results below 2^-126 are zero: such a weight beside a largest one of 1)
 __device__ __forceinline__ float ex2(float x) {
     float y;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
